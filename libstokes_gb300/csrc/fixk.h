@@ -1,0 +1,87 @@
+// fixk.h -- data shared by the fixed-point tensor-core reciprocal sum
+// (kspace_fix.cu) and the host code that plans it (product_fix.cu).
+#pragma once
+
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <stddef.h>
+#include <stdint.h>
+
+#include <vector>
+
+namespace lsg {
+
+// Weights of one reciprocal vector: its direction and the six scalars of
+// recip_apply, times the weight of the vector in the sum over sign patterns.
+struct __align__ (16) FixCoef {
+  double ex, ey, ez, ya, yb, yc, yg, yh, ym, pad;
+};
+
+// Plan of one reciprocal sum.  The k vectors are (m1, m2, m3) with m1 along x;
+// an octant point is (|m1|, |m2|, |m3|).  Everything is expanded in products
+// of real functions: function index 0 of an axis is 1, 2 m - 1 is
+// cos(2 pi m u), 2 m is sin(2 pi m u), u the fractional coordinate.
+//   quarter  one (|m2|, |m3|) of the set, sorted by length
+//   row      4 quarter + 2 p2 + p3, p = 0 cosine, 1 sine: f_y f_z
+//   column   mi c + q, mi the x function index, q the vector component
+struct FixPlan {
+  int np = 0, c = 0;
+  double il[3] = {0, 0, 0};   // 1 / box
+  double l[3] = {0, 0, 0};
+  int M[3] = {0, 0, 0};       // largest |m| per axis
+  int nmi = 0;                // x functions, 2 M[0] + 1
+  int ncol = 0;               // nmi c
+  int nq = 0, nqp = 0;        // quarters; padded to 32 (a row tile)
+  int ldT = 0;                // particles padded to 128 (a backward row tile)
+  int oy = 0, oz = 0, zero = 0, nT = 0;   // table rows: x from 0, y, z, the zero row, total
+  int Rp = 0;                 // rows padded: 4 nqp
+  int nct = 0, mt = 0;        // column tiles, 128-particle tiles
+  int nsplit = 1, jper = 0;   // particle slices of the forward GEMM
+  int nfitem = 0, nbitem = 0; // work items
+  int fu = 0;                 // fractional bits of F
+  int stall = 0;              // tests: polls of a wait that nothing completes
+
+  const int4 *quart = nullptr;     // [nqp] table rows of (cos y, sin y, cos z, sin z)
+  const int *nqm = nullptr;        // [M0 + 1] quarters in use at |m1|
+  const FixCoef *coef = nullptr;   // octant points: [off[m1] + quarter][4 sign patterns]
+  const int *off = nullptr;        // [M0 + 2] first octant point of |m1|
+  void *T = nullptr;          // function table [nT][ldT]
+  void *F = nullptr;          // structure factors [nsplit][ncol][Rp], int64
+  void *G = nullptr;          // operator output [ncol][Rp]
+  void *ZF = nullptr;         // forward image [digits][ncol][ldT] f16
+  void *WB = nullptr;         // backward image [digits][ncol][Rp] f16
+  // high words of max |x_q| at [q] and of max |G| of the columns (m1, q) at
+  // [16 (|m1| + 1) + q]
+  unsigned *mx = nullptr;
+  const int4 *fitem = nullptr;     // forward: row tile, column tile, particle slice
+  const int4 *bitem = nullptr;     // backward: column tile, first K tile, K tiles
+  void *yp = nullptr;         // back-projection partials [nbitem][np][c]
+};
+
+struct FixMaps {
+  CUtensorMap zf, wb;
+};
+
+inline size_t fix_mx_words (const FixPlan &p) { return 16 * ((size_t) p.M[0] + 2); }
+
+// host entry points of kspace_fix.cu; ND: digits per number, 7 (FP64)
+size_t fix_bytes_T (int nd, const FixPlan &p);
+size_t fix_bytes_F (int nd, const FixPlan &p);
+size_t fix_bytes_G (int nd, const FixPlan &p);
+size_t fix_bytes_ZF (int nd, const FixPlan &p);
+size_t fix_bytes_WB (int nd, const FixPlan &p);
+size_t fix_bytes_yp (int nd, const FixPlan &p);
+void fix_plan_items (int nd, FixPlan &p, const std::vector<int> &nqm, std::vector<int4> &fwd,
+                     std::vector<int4> &bwd);
+int fix_maps (int nd, const FixPlan &p, FixMaps *m);
+struct Ctx;
+// y partials of the reciprocal sum from positions and x (device), in order
+// on st; *status is raised when a bounded wait ran out
+cudaError_t launch_fix_tables (int nd, const FixPlan &p, const double *pos, const double *x,
+                               cudaStream_t st, Ctx *prof);
+cudaError_t launch_fix_forward (int nd, int version, const FixPlan &p, const FixMaps &m, int *status,
+                                cudaStream_t st, Ctx *prof);
+cudaError_t launch_fix_backward (int nd, int version, const FixPlan &p, const FixMaps &m,
+                                 int *status, cudaStream_t st, Ctx *prof);
+
+}  // namespace lsg

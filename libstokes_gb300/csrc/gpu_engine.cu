@@ -9,6 +9,7 @@
 // own tests do (test/check-ewald.c:73-125).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdarg>
@@ -139,6 +140,7 @@ free_ctx (Ctx *c)
   if (c->hpos) cudaFreeHost (c->hpos);
   cudaStreamDestroy (c->stream);
   release_mixed (c);
+  release_fix (c);
   release_vjp_mixed (c);
   if (c->tuned) stokes_free (c->tuned);
   if (c->dense) stokes_free (c->dense);
@@ -331,10 +333,14 @@ upload_if_changed (DevBuf &buf, uint64_t &fp, const void *host, size_t bytes,
 // The reference's split xi = sqrt(pi) / L puts nearly all of the work in
 // real space (hundreds of lattice images at N = 1000).  The FP64 products
 // of equal and unequal spheres (not slip: libstokes' slip sum depends on xi
-// beyond the G term, 1e-2 between splits) run at xi = eta / V^(1/3) instead (eta 6 up to 1024
-// particles, 8 up to 4096, 10 above; LIBSTOKES_GB300_FP64_ETA sets it, 0
-// keeps the reference's split), set up by the reference's own rules on a
-// private copy of the system.  The sum is split-invariant to rounding
+// beyond the G term, 1e-2 between splits) run at xi = eta / V^(1/3) instead
+// (LIBSTOKES_GB300_FP64_ETA sets eta, 0 keeps the reference's split), set up
+// by the reference's own rules on a private copy of the system.  Equal spheres
+// take the fixed-point tensor-core reciprocal sum (product_fix.cu), so eta is
+// high: 12, at most xi = 0.7.  FTS N = 1000, phi 0.3, one GB300: 9.6 ms at eta
+// 6 with the SIMT sums, 1.6 ms now (real space 1.3 ms, GEMMs 110 + 121 us).
+// Unequal spheres keep the SIMT sums: eta 6 up to 1024 particles, 8 up to
+// 4096, 10 above.  The sum is split-invariant to rounding
 // (measured 5e-15 to 8e-15 against the reference's split) -- except under
 // the rmin clamp, which changes only the real-space part of the clamped
 // (overlapping) pairs: the real-space kernel adds that change at the
@@ -349,13 +355,21 @@ upload_if_changed (DevBuf &buf, uint64_t &fp, const void *host, size_t bytes,
 // G is linear in it, so the table's factors KT_GF (G) and KT_AF (the rest)
 // express the same correction.
 static double
-tuned_eta (int np)
+tuned_eta (const struct stokes *sys)
 {
   static const double env = [] {
     const char *s = getenv ("LIBSTOKES_GB300_FP64_ETA");
     return s ? atof (s) : -1.0;
   }();
   if (env >= 0.0) return env;
+  const int np = sys->np;
+  if (sys->a == nullptr)
+    {
+      // xi up to 0.7 (or eta 6 in a very small box): beyond, the self, real
+      // and reciprocal parts grow against their sum and cost digits
+      const double l = cbrt (sys->lx * sys->ly * sys->lz);
+      return std::min (12.0, std::max (6.0, 0.7 * l));
+    }
   return np <= 1024 ? 6.0 : (np <= 4096 ? 8.0 : 10.0);
 }
 
@@ -391,7 +405,7 @@ split_is_as_set (const struct stokes *sys)
 static bool
 tuned_applies (const Ctx *c, const struct stokes *sys, bool cube)
 {
-  const double eta = tuned_eta (sys->np);
+  const double eta = tuned_eta (sys);
   // the clamp (rmin > 0) of equal spheres, when only the minimum image of a
   // pair can be clamped
   bool clamp_ok = sys->rmin == 0.0;
@@ -411,7 +425,7 @@ static const struct stokes *
 tuned_system (Ctx *c, const struct stokes *sys)
 {
   const double eps = sys->ewald_eps > 0.0 ? sys->ewald_eps : 1e-12;
-  const double eta = tuned_eta (sys->np);
+  const double eta = tuned_eta (sys);
   const double key[7] = {sys->lx, sys->ly, sys->lz, (double) sys->np, (double) sys->version,
                          eta, eps};
   if (c->tuned && memcmp (c->tuned_key, key, sizeof key) == 0) return c->tuned;
@@ -485,6 +499,7 @@ prepare (Ctx *c, const struct stokes *sys, bool cube, int tables)
     return set_error (STOKES_GPU_EINVAL, "image table missing (stokes_set_xi not called?)");
   c->sys = sys;
   c->cube = cube;
+  c->use_fix = false;
   c->version = sys->version;
   c->np = sys->np;
   c->mode = sys->slip ? MODE_SLIP : (sys->a ? MODE_POLY : MODE_MONO);
@@ -534,6 +549,12 @@ prepare (Ctx *c, const struct stokes *sys, bool cube, int tables)
   rc = upload_if_changed (c->img, c->fp_img, c->h_img.data (), sizeof (Img4) * c->h_img.size (),
                           c->stream, "image table");
   if (rc) return rc;
+  // 2^22 particles: the range of the fixed-point sums
+  if (ts != sys && c->mode == MODE_MONO && sys->np <= (1 << 22))
+    {
+      c->use_fix = true;
+      return fix_setup (c, sys, ts);
+    }
   if (c->open)
     c->h_kt.clear ();
   else
@@ -572,6 +593,7 @@ int
 atimes_fp64_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
                  cudaStream_t st, bool timed)
 {
+  if (c->use_fix) return atimes_fix_dev (c, d_pos, d_x, d_y, st, timed);
   const int np = c->np, C = NCOMP (c->version);
   const int nchunk = choose_nchunk (np);
   cudaError_t e;
@@ -799,6 +821,7 @@ atimes_host (struct stokes *sys, const double *x, double *y, bool cube)
   // a bounded wait of this product's tensor-core kernels that ran out
   if (c->precision == STOKES_GPU_MIXED && !c->open && (rc = mixed_check_status (c)) != 0)
     return rc;
+  if (c->use_fix && (rc = fix_check_status (c)) != 0) return rc;
   collect_times (c);
   sys->cpu1 = c->times[0];
   sys->cpu2 = c->times[1];

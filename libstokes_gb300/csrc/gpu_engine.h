@@ -20,6 +20,7 @@ struct DevBuf {
 };
 
 struct MixedState;   // mixed-precision state (mixed.cu)
+struct FixState;     // FP64 product with the fixed-point reciprocal sum (product_fix.cu)
 
 struct Ctx {
   int device = 0;
@@ -67,6 +68,11 @@ struct Ctx {
   std::vector<const char *> kprof_name;
 
   MixedState *mixed = nullptr;
+
+  // the FP64 product with the fixed-point reciprocal sum (product_fix.cu);
+  // use_fix: the last prepare chose it
+  FixState *fix = nullptr;
+  bool use_fix = false;
 
   DevBuf openf;   // scratch of the mixed-precision free-space product
   DevBuf imgf;    // the images in FP32 (split-precision dense builder)
@@ -130,6 +136,14 @@ int atimes_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
                 cudaStream_t st, bool timed);
 int atimes_fp64_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
                      cudaStream_t st, bool timed);
+// the same for equal spheres at the tuned split (product_fix.cu)
+int atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cudaStream_t st,
+                    bool timed);
+// brings the tables of that product up to date: sys as the caller set it, ts
+// its private copy at the tuned split
+int fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts);
+int fix_check_status (Ctx *c);
+void release_fix (Ctx *c);
 void collect_times (Ctx *c);
 cudaEvent_t *phase_events (Ctx *c, bool timed);
 // record a kernel-profiling mark on st when the window is open

@@ -1,0 +1,1111 @@
+// kspace_fix.cu -- the reciprocal Ewald sum as exact integer GEMMs on the
+// tensor cores.
+//
+// A reciprocal vector is k = 2 pi (m1 / Lx, m2 / Ly, m3 / Lz) and every phase
+// factor is a product of one function of x, y and z each.  In the basis of
+// real functions f_0 = 1, f_(2m-1) = cos 2 pi m u, f_(2m) = sin 2 pi m u per
+// axis (u the fractional coordinate) the sum is, with row r = (y function, z
+// function) and column n = (x function mi, vector component q):
+//
+//   forward   F[n][r] = sum_j A[r][j] B[n][j],   A[r][j] = f_y(j) f_z(j),
+//                                                B[n][j] = f_x(j) x_q(j)
+//   operator  the four sign patterns of (|m1|, |m2|, |m3|): cosine and sine
+//             sums C, S by a 2-bit Walsh-Hadamard transform of the eight
+//             values, P, Q by the Ewald weights, G by the same transform back
+//   backward  y_q(i) = sum_mi f_x(i) sum_r A[r][i] G[n][r]
+//
+// which is half the multiplications of the complex form (k and -k share the
+// real products).
+//
+// Arithmetic.  FP64 runs at 1/64 of the FP32 rate here, the tensor cores
+// multiply f16.  Every operand is therefore a fixed-point number cut into ND
+// signed 8-bit digits, each an exact f16 integer (ND = 7: 55 fractional bits
+// below the largest magnitude of its kind, where FP64 has 53 significant
+// ones; |f| <= 1, x_q is scaled by a power of two per component and G by one
+// per column, since G falls off with |m1| and the rounding of a column is set
+// by its largest entry).
+// Digit products are at most 2^14 and at most 7 x 128 of them meet in one
+// accumulator, so the FP32 sums of the tensor core stay below 2^24 and are
+// exact integers.  The products of digits i and j with i + j = g < ND share
+// accumulator g; the dropped ones weigh less than the last digit.  Every 128
+// values of K the accumulators are drained: groups 0 to 3 into 64-bit
+// integers, the rest (below 2^-38 of full scale) into FP32.  The result
+// carries the rounding of its inputs, about 2^-56 of full scale each, and
+// none from the summation.
+//
+// Operands.  B comes from images [digit][column][K] of f16 by TMA.  A is
+// built in shared memory by the worker warps from the function table (int64,
+// 62 fractional bits): a 64-bit high product, one rounding shift, one add
+// that biases all digits at once, and per digit pair a byte permute, a mask
+// and an f16x2 subtraction.  Images of A would be 7 f16 planes of rows x
+// particles, re-read for every column tile.
+//
+// What bounds the GEMMs: shared-memory reads of the MMAs.  A 128 x 64 x 16
+// MMA reads 6 KB (48 clocks of shared memory against 32 of tensor pipe); a
+// 32-wide K tile has 56 of them (2700 clocks) next to about 900 clocks of
+// operand stores and 250 of drain per tile, spread over 16 worker warps.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <queue>
+#include <vector>
+
+#include "ewald_device.cuh"
+#include "fixk.h"
+#include "gpu_engine.h"
+#include "tc_umma.cuh"
+#include "tma_host.h"
+
+namespace lsg {
+namespace {
+
+constexpr int NT = 576;                 // 16 worker warps, a TMA and an MMA warp
+constexpr int NWORK = 512;
+constexpr int TMA_WARP = 16;
+constexpr int MMA_WARP = 17;
+constexpr int TM = 128;                 // MMA M
+constexpr int STAGES = 2;
+constexpr uint32_t TMEM_COLS = 512;
+constexpr uint32_t WAIT_LIMIT = 1u << 18;   // polls of up to ~20 us each
+
+// per precision: ND digits, operators in R
+template <int ND> struct Cfg;
+template <> struct Cfg<7> {
+  using R = double;
+  static constexpr int KT = 32;         // K values per tile
+  static constexpr int TN = 64;         // columns per tile (7 accumulators: 448 TMEM columns)
+  static constexpr int DK = 4;          // tiles per drain (K = 128)
+};
+
+template <int ND>
+struct Geo {
+  using C = Cfg<ND>;
+  static constexpr int ROWB = 2 * C::KT;                // bytes of a tile row
+  static constexpr uint32_t A_PLANE = TM * ROWB;
+  static constexpr uint32_t B_PLANE = C::TN * ROWB;
+  static constexpr uint32_t STAGE = ND * (A_PLANE + B_PLANE);
+  static constexpr uint32_t SMEM = STAGES * STAGE + 1024;
+  static constexpr int CPT = C::TN / 4;                 // accumulator columns per worker
+};
+
+struct Sync {
+  uint64_t full[STAGES], empty[STAGES], acc_full, acc_empty, done, never;
+  uint32_t tslot;
+  int err;
+};
+
+// ---- fixed point ----------------------------------------------------------
+// A table entry f (62 fractional bits) as hi 2^32 + lo with lo signed
+struct Limbs {
+  int hi, lo;
+};
+__device__ __forceinline__ Limbs
+limbs (long long f)
+{
+  const int lo = (int) f;
+  return Limbs {(int) (f >> 32) + (int) ((unsigned) lo >> 31), lo};
+}
+
+// f g as a biased string of 55 fractional bits: digit p is byte 6 - p minus
+// 128 (the top one a 16-bit field).  Three 32 x 32 bit products; the dropped
+// lo lo term is below 2^-61.
+__device__ __forceinline__ long long
+biased (Limbs f, Limbs g)
+{
+  const long long cross = (long long) f.hi * g.lo + (long long) f.lo * g.hi;
+  const long long v = (long long) f.hi * g.hi + (cross >> 32);      // 60 fractional bits
+  return (v + ((0x0080808080808080ll << 5) + 16)) >> 5;
+}
+
+// v 2^(frac - E) rounded to an integer, for |v| < 2^E: from the bits of v,
+// since FP64 arithmetic and conversions run at 1/64 of the integer rate
+__device__ __forceinline__ long long
+to_fixed (double v, int E, int frac)
+{
+  const long long bits = __double_as_longlong (v);
+  const int e = (int) (bits >> 52) & 0x7ff;
+  long long m = bits & 0x000fffffffffffffll;
+  if (e) m |= 0x0010000000000000ll;
+  const int sh = 1075 - max (e, 1) - frac + E;          // >= 53 - frac
+  if (sh > 54) m = 0;
+  else if (sh > 0) m = (m + (1ll << (sh - 1))) >> sh;
+  else m <<= -sh;
+  return bits < 0 ? -m : m;
+}
+
+// the f16 pairs (digit of a, digit of b) of two biased strings, plane by plane
+__device__ __forceinline__ uint32_t
+f16_digits (uint32_t bytes)
+{
+  // 0x6400 + n is the f16 number 1024 + n
+  const __half2 v = __hsub2 (*reinterpret_cast<__half2 *> (&bytes), __half2half2 (__ushort_as_half (0x6480)));
+  return *reinterpret_cast<const uint32_t *> (&v);
+}
+
+__device__ __forceinline__ void
+digits (long long a, long long b, uint32_t out[7])
+{
+  const uint32_t al = (uint32_t) a, ah = (uint32_t) ((unsigned long long) a >> 32);
+  const uint32_t bl = (uint32_t) b, bh = (uint32_t) ((unsigned long long) b >> 32);
+  auto pick = [] (uint32_t x, uint32_t y, uint32_t sel) {
+    return f16_digits ((__byte_perm (x, y, sel) & 0x00FF00FFu) | 0x64006400u);
+  };
+  out[0] = f16_digits (__byte_perm (ah, bh, 0x7632) + 0x64006400u);
+  out[1] = pick (ah, bh, 0x5511);
+  out[2] = pick (ah, bh, 0x4400);
+  out[3] = pick (al, bl, 0x7733);
+  out[4] = pick (al, bl, 0x6622);
+  out[5] = pick (al, bl, 0x5511);
+  out[6] = pick (al, bl, 0x4400);
+}
+
+// exponent E with |v| < 2^E for every v whose high word (sign cleared) is at
+// most hw; NaN and infinity: finite = false
+__device__ __forceinline__ int
+scale_exp (uint32_t hw, bool &finite)
+{
+  const int e = (int) (hw >> 20);
+  finite = e != 2047;
+  return e - 1022;
+}
+
+// 2^(E - log) as the factor that turns results in units of 2^-log into values;
+// NaN where an input was NaN or infinite, as a sum over it would be
+__device__ __forceinline__ double
+unit_of (uint32_t hw, int log)
+{
+  bool finite;
+  const int e = scale_exp (hw, finite) - log;
+  if (!finite) return __longlong_as_double (0x7ff8000000000000ll);
+  return e > -1022 ? __hiloint2double ((e + 1023) << 20, 0) : scalbn (1.0, e);
+}
+
+__device__ __forceinline__ uint32_t
+abs_hi (double v)
+{
+  return (uint32_t) __double2hiint (v) & 0x7fffffffu;
+}
+
+// ---- operand builders -----------------------------------------------------
+// byte offset of 16-byte chunk c of row r in a swizzled plane
+template <int ND>
+__device__ __forceinline__ uint32_t
+chunk_off (int r, int c)
+{
+  if (Geo<ND>::ROWB == 64) return (uint32_t) (r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
+  return (uint32_t) (r * 128 + ((c ^ (r & 7)) << 4));
+}
+
+// The A operand of a tile is built in two steps, so that the table loads of
+// the next tile are in flight while a worker waits for its stage: load()
+// reads the table entries of a thread's share into registers, store() forms
+// the products, cuts the digits and writes them to the stage.
+
+// Forward: rows r0 .. r0 + 127 (32 quarters, two per warp), particles j0 ..
+// j0 + 31.  Half a warp covers the 32 particles (two per lane) of one
+// quarter, whose four rows share its four table entries.  The upper half-warp
+// takes the rows in the order 1 0 3 2, so that the two halves write different
+// 64-byte halves of a 128-byte bank line.
+template <int ND>
+struct BuildF {
+  const long long *T;
+  int ldT, j0;
+  int4 f;                       // table rows of the thread's quarter
+  longlong2 y[2], z[2];         // cosine and sine entries of two particles
+  __device__ __forceinline__ BuildF (const FixPlan &p, int r0, int jb)
+    : T ((const long long *) p.T), ldT (p.ldT)
+  {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    f = p.quart[r0 / 4 + 2 * warp + (lane >> 4)];
+    j0 = jb + 2 * (lane & 15);
+  }
+  __device__ __forceinline__ void load (int t)
+  {
+    const size_t jo = (size_t) j0 + Cfg<ND>::KT * t;
+    y[0] = *reinterpret_cast<const longlong2 *> (T + (size_t) f.x * ldT + jo);
+    y[1] = *reinterpret_cast<const longlong2 *> (T + (size_t) f.y * ldT + jo);
+    z[0] = *reinterpret_cast<const longlong2 *> (T + (size_t) f.z * ldT + jo);
+    z[1] = *reinterpret_cast<const longlong2 *> (T + (size_t) f.w * ldT + jo);
+  }
+  __device__ __forceinline__ void store (unsigned char *stage) const
+  {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int jp = lane & 15, hs = lane >> 4, qd = 2 * warp + hs;
+    // z in the order of this half-warp's rows
+    const Limbs za[2] = {limbs (hs ? z[1].x : z[0].x), limbs (hs ? z[0].x : z[1].x)};
+    const Limbs zb[2] = {limbs (hs ? z[1].y : z[0].y), limbs (hs ? z[0].y : z[1].y)};
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      {
+        const int r = 4 * qd + (k ^ hs);                // row 2 p2 + p3 of the quarter
+        uint32_t d[7];
+        digits (biased (limbs (y[k >> 1].x), za[k & 1]), biased (limbs (y[k >> 1].y), zb[k & 1]), d);
+        unsigned char *o = stage + chunk_off<ND> (r, jp >> 2) + (jp & 3) * 4;
+#pragma unroll
+        for (int q = 0; q < ND; q++)
+          *reinterpret_cast<uint32_t *> (o + q * Geo<ND>::A_PLANE) = d[q];
+      }
+  }
+};
+
+// Backward: particles i0 .. i0 + 127, one per lane, rows 4 quart0 .. + 31, two
+// quarters (16 bytes per plane) per thread
+template <int ND>
+struct BuildB {
+  const long long *T;
+  const int4 *quart;
+  int ldT, i, c;
+  long long y[2][2], z[2][2];
+  __device__ __forceinline__ BuildB (const FixPlan &p, int i0, int quart0)
+    : T ((const long long *) p.T), quart (p.quart), ldT (p.ldT)
+  {
+    i = i0 + (threadIdx.x & 127);
+    c = threadIdx.x >> 7;
+    quart += quart0 + 2 * c;
+  }
+  __device__ __forceinline__ void load (int t)
+  {
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      {
+        const int4 f = __ldg (quart + t * (Cfg<ND>::KT / 4) + u);
+        y[u][0] = T[(size_t) f.x * ldT + i];
+        y[u][1] = T[(size_t) f.y * ldT + i];
+        z[u][0] = T[(size_t) f.z * ldT + i];
+        z[u][1] = T[(size_t) f.w * ldT + i];
+      }
+  }
+  __device__ __forceinline__ void store (unsigned char *stage) const
+  {
+    uint32_t w[ND][4];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      {
+        uint32_t d[7];
+        const Limbs fy = limbs (y[u >> 1][u & 1]);
+        digits (biased (fy, limbs (z[u >> 1][0])), biased (fy, limbs (z[u >> 1][1])), d);
+#pragma unroll
+        for (int q = 0; q < ND; q++) w[q][u] = d[q];
+      }
+    unsigned char *o = stage + chunk_off<ND> (threadIdx.x & 127, c);
+#pragma unroll
+    for (int q = 0; q < ND; q++)
+      *reinterpret_cast<uint4 *> (o + q * Geo<ND>::A_PLANE)
+        = make_uint4 (w[q][0], w[q][1], w[q][2], w[q][3]);
+  }
+};
+
+// ---- GEMM roles -----------------------------------------------------------
+__device__ __forceinline__ unsigned char *
+align1k (unsigned char *p)
+{
+  return p + ((1024u - (umma::smem_u32 (p) & 1023u)) & 1023u);
+}
+
+__device__ __forceinline__ void
+cta_setup (Sync &s)
+{
+  if (threadIdx.x < 32) umma::tmem_alloc (&s.tslot, TMEM_COLS);
+  if (threadIdx.x == 32)
+    {
+      for (int k = 0; k < STAGES; k++)
+        {
+          umma::mbar_init (&s.full[k], 1 + NWORK);
+          umma::mbar_init (&s.empty[k], 1);
+        }
+      umma::mbar_init (&s.acc_full, 1);
+      umma::mbar_init (&s.acc_empty, NWORK);
+      umma::mbar_init (&s.done, 1);
+      umma::mbar_init (&s.never, 1);
+      s.err = 0;
+      umma::fence_mbar_init ();
+    }
+  umma::fence_before_sync ();
+  __syncthreads ();
+  umma::fence_after_sync ();
+}
+
+// the TMA lane: all digit planes of the B tile at (K = k0 + KT t, column n0)
+template <int ND>
+__device__ __forceinline__ void
+tma_role (Sync &s, unsigned char *smem, const CUtensorMap *tb, int n0, int k0, int ntiles)
+{
+  using G = Geo<ND>;
+  volatile int *err = &s.err;
+  umma::tma_prefetch_desc (tb);
+  int issued = 0;
+  for (int t = 0; t < ntiles; t++)
+    {
+      const int st = t % STAGES;
+      if (t >= STAGES
+          && !umma::mbar_wait_or_abort (&s.empty[st], ((t / STAGES) - 1) & 1, WAIT_LIMIT, err))
+        break;
+      umma::mbar_expect_tx (&s.full[st], ND * G::B_PLANE);
+      umma::tma_load_3d (smem + (size_t) st * G::STAGE + ND * G::A_PLANE, tb,
+                         k0 + Cfg<ND>::KT * t, n0, 0, &s.full[st]);
+      issued = t + 1;
+    }
+  // the last load of each stage must land before the shared memory goes away
+  // (in an aborted CTA, whose workers may not arrive, the limit bounds the wait)
+  volatile int never = 0;
+  for (int t = issued > STAGES ? issued - STAGES : 0; t < issued; t++)
+    umma::mbar_wait_or_abort (&s.full[t % STAGES], (t / STAGES) & 1, WAIT_LIMIT, &never);
+}
+
+template <int ND>
+__device__ __forceinline__ uint64_t
+tile_desc (uint32_t a)
+{
+  return Geo<ND>::ROWB == 64 ? umma::smem_desc_sw64 (a) : umma::smem_desc_sw128 (a);
+}
+
+// the MMA lane: digit products by group (i + j), accumulator group g in TMEM
+// columns g TN; a new set of accumulators every DK tiles
+template <int ND>
+__device__ __forceinline__ void
+mma_role (Sync &s, const unsigned char *smem, uint32_t tmem, int ntiles, int stall)
+{
+  using G = Geo<ND>;
+  using C = Cfg<ND>;
+  volatile int *err = &s.err;
+  const uint32_t idesc = umma::idesc_f16 (TM, C::TN);
+  if (stall > 0 && !umma::mbar_wait_or_abort (&s.never, 0, (uint32_t) stall, err)) ntiles = 0;
+  for (int t = 0; t < ntiles; t++)
+    {
+      const int st = t % STAGES, set = t / C::DK;
+      if (!umma::mbar_wait_or_abort (&s.full[st], (t / STAGES) & 1, WAIT_LIMIT, err)) break;
+      if (t % C::DK == 0 && set > 0
+          && !umma::mbar_wait_or_abort (&s.acc_empty, (set - 1) & 1, WAIT_LIMIT, err))
+        break;
+      umma::fence_after_sync ();
+      const uint32_t a = umma::smem_u32 (smem) + (uint32_t) st * G::STAGE;
+      const uint32_t b = a + ND * G::A_PLANE;
+      const uint32_t first = t % C::DK == 0 ? 1u : 0u;
+#pragma unroll
+      for (int g = 0; g < ND; g++)
+#pragma unroll
+        for (int i = 0; i <= g; i++)
+#pragma unroll
+          for (int k = 0; k < C::KT / 16; k++)
+            umma::mma_f16 (tmem + (uint32_t) (g * C::TN), tile_desc<ND> (a + i * G::A_PLANE + 32 * k),
+                           tile_desc<ND> (b + (g - i) * G::B_PLANE + 32 * k), idesc,
+                           (first && i == 0 && k == 0) ? 0u : 1u);
+      umma::mma_commit (&s.empty[st]);
+      if (t % C::DK == C::DK - 1 || t == ntiles - 1) umma::mma_commit (&s.acc_full);
+    }
+  umma::mma_commit (&s.done);
+  volatile int never = 0;
+  umma::mbar_wait_or_abort (&s.done, 0, WAIT_LIMIT, &never);
+}
+
+// running sums of one worker: CPT columns of one row.  Value of a column:
+// (hi + lo) 2^-38; hi exact.
+template <int ND> struct Acc;
+template <> struct Acc<7> {
+  static constexpr int CPT = Geo<7>::CPT;
+  long long hi[CPT];
+  float lo[CPT];
+  __device__ __forceinline__ void zero ()
+  {
+#pragma unroll
+    for (int u = 0; u < CPT; u++) { hi[u] = 0; lo[u] = 0.f; }
+  }
+  __device__ __forceinline__ void drain (uint32_t d)
+  {
+    static_assert (CPT == 16, "one TMEM load per group");
+    float f[2][16];
+    umma::tmem_ld16_issue (d, f[0]);
+#pragma unroll
+    for (int g = 0; g < 7; g++)
+      {
+        umma::tmem_ld_wait (f[g & 1]);
+        if (g < 6) umma::tmem_ld16_issue (d + (g + 1) * Cfg<7>::TN, f[(g + 1) & 1]);
+#pragma unroll
+        for (int u = 0; u < 16; u++)
+          {
+            const float v = f[g & 1][u];
+            if (g < 4) hi[u] += (long long) __float2int_rn (v) * (1 << (8 * (3 - g)));
+            else lo[u] = fmaf (v, 1.0f / (float) (1u << (8 * (g - 3))), lo[u]);
+          }
+      }
+  }
+  // column u in units of 2^-fu, fu >= 38
+  __device__ __forceinline__ long long fixed (int u, int fu) const
+  {
+    const int whole = __float2int_rn (lo[u]);
+    const float rest = (lo[u] - (float) whole) * (float) (1u << (fu - 38));
+    return ((hi[u] + whole) << (fu - 38)) + __float2int_rn (rest);
+  }
+};
+
+// worker warps: build tile t + 2 once the MMAs of tile t are done; at the end
+// of a set drain first, so that the next set's MMAs start early
+template <int ND, class Build>
+__device__ __forceinline__ bool
+worker_role (Sync &s, unsigned char *smem, uint32_t tmem, int ntiles, Acc<ND> &acc, Build &build)
+{
+  using G = Geo<ND>;
+  using C = Cfg<ND>;
+  const int warp = threadIdx.x >> 5;
+  volatile int *err = &s.err;
+  auto put = [&] (int t) {
+    build.store (smem + (size_t) (t % STAGES) * G::STAGE);
+    umma::fence_async_smem ();
+    umma::mbar_arrive (&s.full[t % STAGES]);
+    if (t + 1 < ntiles) build.load (t + 1);
+  };
+  if (ntiles > 0) build.load (0);
+  for (int t = 0; t < STAGES && t < ntiles; t++) put (t);
+  const uint32_t dm = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + (uint32_t) ((warp >> 2) * G::CPT);
+  for (int t = 0; t < ntiles; t++)
+    {
+      if (t % C::DK == C::DK - 1 || t == ntiles - 1)
+        {
+          if (!umma::mbar_wait_or_abort (&s.acc_full, (t / C::DK) & 1, WAIT_LIMIT, err))
+            return false;
+          umma::fence_after_sync ();
+          acc.drain (dm);
+          umma::fence_before_sync ();
+          umma::mbar_arrive (&s.acc_empty);
+        }
+      if (t + STAGES < ntiles)
+        {
+          if (!umma::mbar_wait_or_abort (&s.empty[t % STAGES], (t / STAGES) & 1, WAIT_LIMIT, err))
+            return false;
+          put (t + STAGES);
+        }
+    }
+  return true;
+}
+
+__device__ __forceinline__ int
+col_m (const FixPlan &p, int n)
+{
+  return (n / p.c + 1) / 2;              // |m1| of column n
+}
+
+// first column of component q in the tile that starts at column n0
+__device__ __forceinline__ int
+first_col (const FixPlan &p, int n0, int q)
+{
+  return (q + p.c - n0 % p.c) % p.c;
+}
+
+constexpr int NOT_FINITE = 1 << 20;
+
+__device__ __forceinline__ void
+cta_finish (Sync &s, uint32_t tmem, int *status)
+{
+  if (threadIdx.x == 0 && s.err) atomicExch (status, 1);
+  umma::fence_before_sync ();
+  __syncthreads ();
+  if (threadIdx.x < 32) umma::tmem_dealloc (tmem, TMEM_COLS);
+}
+
+// forward: a CTA takes one item (row tile, column tile, particle slice) and
+// writes F[slice][column][row]; lanes are consecutive rows, so the stores
+// coalesce
+template <int ND>
+__global__ void __launch_bounds__ (NT, 1)
+k_fix_fwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
+{
+  using C = Cfg<ND>;
+  extern __shared__ unsigned char dsm[];
+  __shared__ Sync s;
+  const int4 it = p.fitem[blockIdx.x];
+  const int r0 = it.x * TM, n0 = it.y * C::TN;
+  unsigned char *smem = align1k (dsm);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int jb = it.z * p.jper, je = min (p.ldT, jb + p.jper);
+  const int ntiles = je > jb ? (je - jb + C::KT - 1) / C::KT : 0;
+  cta_setup (s);
+  const uint32_t tmem = s.tslot;
+  if (warp == TMA_WARP)
+    {
+      if (lane == 0) tma_role<ND> (s, smem, &tmB, n0, jb, ntiles);
+      __syncwarp ();
+    }
+  else if (warp == MMA_WARP)
+    {
+      if (lane == 0) mma_role<ND> (s, smem, tmem, ntiles, p.stall);
+      __syncwarp ();
+    }
+  else
+    {
+      Acc<ND> acc;
+      acc.zero ();
+      BuildF<ND> build (p, r0, jb);
+      if (worker_role<ND> (s, smem, tmem, ntiles, acc, build))
+        {
+          const int r = r0 + (warp & 3) * 32 + lane, c0 = n0 + (warp >> 2) * Geo<ND>::CPT;
+          long long *F = (long long *) p.F + (size_t) it.z * p.ncol * p.Rp + r;
+#pragma unroll
+          for (int u = 0; u < Geo<ND>::CPT; u++)
+            if (c0 + u < p.ncol) F[(size_t) (c0 + u) * p.Rp] = acc.fixed (u, p.fu);
+        }
+    }
+  cta_finish (s, tmem, status);
+}
+
+// backward: a CTA takes 128 particles and one item (column tile, first K
+// tile, K tiles), the item number is the slot of its partial y.  The sums H are
+// parked in the freed stages and reduced over the x functions of the tile in
+// 128-bit integers (an FP64 operation on the 128 x 64 tile takes the FP64 pipe
+// 4096 clocks, a 64 x 64 bit product of integers about a tenth): the columns'
+// different units 2^E come in as a right shift of the table entry.
+template <int ND>
+__global__ void __launch_bounds__ (NT, 1)
+k_fix_bwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
+{
+  using C = Cfg<ND>;
+  constexpr int HLD = C::TN + 1;
+  constexpr uint32_t H_LO = TM * HLD * sizeof (long long);
+  static_assert (H_LO + TM * HLD * sizeof (float) <= STAGES * Geo<ND>::STAGE, "parked tile");
+  extern __shared__ unsigned char dsm[];
+  __shared__ Sync s;
+  __shared__ int s_exp[C::TN], s_top[16];
+  unsigned char *smem = align1k (dsm);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int4 it = p.bitem[blockIdx.y];
+  const int i0 = blockIdx.x * TM, n0 = it.x * C::TN;
+  const int ne = min (C::TN, p.ncol - n0);
+  if ((int) threadIdx.x < ne)
+    {
+      const int n = n0 + threadIdx.x;
+      bool finite;
+      const int E = scale_exp (p.mx[16 * (col_m (p, n) + 1) + n % p.c], finite);
+      s_exp[threadIdx.x] = finite ? E : NOT_FINITE;
+    }
+  const int tb = it.y, ntiles = it.z;
+  cta_setup (s);
+  const uint32_t tmem = s.tslot;
+  // the largest unit of each component
+  if ((int) threadIdx.x < p.c)
+    {
+      int top = -2000;
+      for (int n = first_col (p, n0, threadIdx.x); n < ne; n += p.c) top = max (top, s_exp[n]);
+      s_top[threadIdx.x] = top;
+    }
+  if (warp == TMA_WARP)
+    {
+      if (lane == 0) tma_role<ND> (s, smem, &tmB, n0, tb * C::KT, ntiles);
+      __syncwarp ();
+    }
+  else if (warp == MMA_WARP)
+    {
+      if (lane == 0) mma_role<ND> (s, smem, tmem, ntiles, p.stall);
+      __syncwarp ();
+    }
+  else
+    {
+      Acc<ND> acc;
+      acc.zero ();
+      BuildB<ND> build (p, i0, tb * (C::KT / 4));
+      if (worker_role<ND> (s, smem, tmem, ntiles, acc, build))
+        {
+          // the last set is drained, so every build, load and MMA is done and
+          // the stages are free
+          const int o = ((warp & 3) * 32 + lane) * HLD + (warp >> 2) * Geo<ND>::CPT;
+          long long *Hi = reinterpret_cast<long long *> (smem) + o;
+          float *Lo = reinterpret_cast<float *> (smem + H_LO) + o;
+#pragma unroll
+          for (int u = 0; u < Geo<ND>::CPT; u++)
+            {
+              Hi[u] = acc.hi[u];
+              Lo[u] = acc.lo[u];
+            }
+        }
+    }
+  __syncthreads ();
+  if (!s.err)
+    {
+      const long long *Hi = reinterpret_cast<const long long *> (smem);
+      const float *Lo = reinterpret_cast<const float *> (smem + H_LO);
+      double *yp = (double *) p.yp + (size_t) blockIdx.y * p.np * p.c;
+      const long long *T = (const long long *) p.T;
+      for (int e = threadIdx.x; e < TM * p.c; e += NT)
+        {
+          const int q = e / TM, r = e - q * TM, i = i0 + r;
+          if (i >= p.np) continue;
+          const int top = s_top[q];
+          __int128 y = 0;
+          float yl = 0.f;
+          for (int n = first_col (p, n0, q); n < ne; n += p.c)
+            {
+              const int sh = top - s_exp[n];
+              if (sh > 62) continue;              // below the last bit
+              const long long f = T[(size_t) ((n0 + n) / p.c) * p.ldT + i] >> sh;
+              y += (__int128) f * Hi[r * HLD + n];
+              yl = fmaf ((float) (int) (f >> 32), Lo[r * HLD + n], yl);
+            }
+          // y: 62 + 38 fractional bits, yl: 30 + 38
+          const double v = (double) (long long) (y >> 64) * 0x1p-36
+                           + (double) (unsigned long long) y * 0x1p-100 + (double) yl * 0x1p-68;
+          yp[(size_t) i * p.c + q] = top == NOT_FINITE ? __longlong_as_double (0x7ff8000000000000ll)
+                                                       : scalbn (v, top);
+        }
+    }
+  cta_finish (s, tmem, status);
+}
+
+// ---- tables and images ----------------------------------------------------
+constexpr int TAB_P = 32, TAB_R = 4;
+
+// Function table, one (axis, m) pair of rows (cos, sin) per warp and 32
+// particles.  The fractional coordinate is a 64-bit fixed-point number (the
+// quotient's rounding error added back), so m u mod 1 is an exact integer
+// product.  The blocks of the first group also take the maxima of |x_q|; a
+// position that is not finite makes them NaN, which every result inherits.
+__global__ void __launch_bounds__ (TAB_P * TAB_R)
+k_fix_tables (FixPlan p, const double *pos, const double *x)
+{
+  __shared__ unsigned long long s_u[3][TAB_P];
+  __shared__ unsigned s_mx[16];
+  const int t = threadIdx.x, jb = blockIdx.x * TAB_P;
+  long long *T = (long long *) p.T;
+  if (t < 16) s_mx[t] = 0u;
+  __syncthreads ();
+  if (t < 3 * TAB_P)
+    {
+      const int d = t / TAB_P, jl = t % TAB_P, j = jb + jl;
+      unsigned long long u = 0;
+      if (j < p.np)
+        {
+          const double v = pos[3 * j + d], f = v * p.il[d];
+          const double rest = fma (-f, p.l[d], v) * p.il[d];
+          if (!(fabs (f) < 1e300) && blockIdx.y == 0) s_mx[0] = 0x7ff80000u;
+          u = __double2ull_rz ((f - floor (f)) * 18446744073709551616.0)
+              + (unsigned long long) __double2ll_rn (rest * 18446744073709551616.0);
+        }
+      s_u[d][jl] = u;
+    }
+  __syncthreads ();
+  const int item = blockIdx.y * TAB_R + t / TAB_P, j = jb + t % TAB_P;
+  const int n0 = p.M[0] + 1, n1 = n0 + p.M[1] + 1, n2 = n1 + p.M[2] + 1;
+  if (item < n2 && j < p.np)
+    {
+      const int d = item < n0 ? 0 : (item < n1 ? 1 : 2);
+      const int m = item - (d == 0 ? 0 : (d == 1 ? n0 : n1));
+      const long long ph = (long long) ((unsigned long long) m * s_u[d][t % TAB_P]);
+      double sn, cs;
+      sincospi ((double) ph * 1.0842021724855044e-19, &sn, &cs);     // 2^-63
+      long long *row = T + (size_t) ((d == 0 ? 0 : (d == 1 ? p.oy : p.oz)) + (m ? 2 * m - 1 : 0)) * p.ldT;
+      const double one = 4611686018427387904.0;                      // 2^62
+      row[j] = __double2ll_rn (cs * one);
+      if (m) row[p.ldT + j] = __double2ll_rn (sn * one);
+    }
+  if (blockIdx.y) return;
+  for (int e = t; e < TAB_P * p.c; e += TAB_P * TAB_R)
+    if ((size_t) jb * p.c + e < (size_t) p.np * p.c)
+      atomicMax (&s_mx[e % p.c], abs_hi (x[(size_t) jb * p.c + e]));
+  __syncthreads ();
+  if (t < p.c) atomicMax (p.mx + t, s_mx[t]);
+}
+
+// Forward image: digits of f_x(j) x_q(j), 64 particles and IMG_M x functions
+// per block, eight particles (16 bytes per plane) per thread
+constexpr int IMG_M = 4;
+
+__global__ void __launch_bounds__ (128)
+k_fix_image (FixPlan p, const double *x)
+{
+  __shared__ long long s_x[11][64];
+  const int t = threadIdx.x, jb = blockIdx.x * 64;
+  for (int e = t; e < 64 * p.c; e += 128)
+    {
+      const int jl = e / p.c, q = e - jl * p.c;
+      bool finite;
+      const int E = scale_exp (p.mx[q], finite);
+      s_x[q][jl] = jb + jl < p.np && finite ? to_fixed (x[(size_t) jb * p.c + e], E, 62) : 0ll;
+    }
+  __syncthreads ();
+  const long long *T = (const long long *) p.T;
+  for (int e = t; e < IMG_M * p.c * 8; e += 128)
+    {
+      const int j8 = e & 7, q = (e >> 3) % p.c, mi = blockIdx.y * IMG_M + (e >> 3) / p.c;
+      if (mi >= p.nmi) continue;
+      const long long *f = T + (size_t) mi * p.ldT + jb + 8 * j8;
+      uint32_t w[4][7];
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        {
+          const longlong2 v = *reinterpret_cast<const longlong2 *> (f + 2 * k);
+          digits (biased (limbs (v.x), limbs (s_x[q][8 * j8 + 2 * k])),
+                  biased (limbs (v.y), limbs (s_x[q][8 * j8 + 2 * k + 1])), w[k]);
+        }
+      uint4 *o = reinterpret_cast<uint4 *> ((__half *) p.ZF + (size_t) (mi * p.c + q) * p.ldT + jb)
+                 + j8;
+#pragma unroll
+      for (int d = 0; d < 7; d++)
+        o[(size_t) d * p.ncol * p.ldT / 8] = make_uint4 (w[0][d], w[1][d], w[2][d], w[3][d]);
+    }
+}
+
+// Operators: four lanes per octant point, lane b = 2 p2 + p3 holding row b of
+// the quarter; after the transform lane sigma holds the sign pattern
+// (s2, s3) = (1 - 2 (sigma >> 1), 1 - 2 (sigma & 1)).
+template <typename R>
+__device__ __forceinline__ R
+walsh4 (R v, int b)
+{
+  const R o = __shfl_xor_sync (0xffffffffu, v, 1);
+  v = (b & 1) ? o - v : v + o;
+  const R q = __shfl_xor_sync (0xffffffffu, v, 2);
+  return (b & 2) ? q - v : v + q;
+}
+
+// The transverse parts of a generalised force v at direction e: F, T x e and
+// S' e without their components along e.  Every reciprocal coupling acts
+// through these (a force and its derivatives drive an incompressible flow).
+template <int V, typename R> struct Trans { R f[3], t[3], s[3]; };
+
+template <int V, typename R>
+__device__ __forceinline__ void
+transverse (const R e[3], const R *x, Trans<V, R> &o)
+{
+  GenF<V, R> g;
+  load_genf<V, R> (x, g);
+  const R eF = e[0] * g.F[0] + e[1] * g.F[1] + e[2] * g.F[2];
+#pragma unroll
+  for (int d = 0; d < 3; d++) o.f[d] = fma (-eF, e[d], g.F[d]);
+  if (V == V_F) return;
+  o.t[0] = g.T[1] * e[2] - g.T[2] * e[1];
+  o.t[1] = g.T[2] * e[0] - g.T[0] * e[2];
+  o.t[2] = g.T[0] * e[1] - g.T[1] * e[0];
+  if (V == V_FT) return;
+  const R s0 = g.S[0] * e[0] + g.S[2] * e[1] + g.S[3] * e[2];
+  const R s1 = g.S[2] * e[0] + g.S[1] * e[1] + g.S[4] * e[2];
+  const R s2 = g.S[3] * e[0] + g.S[4] * e[1];
+  const R es = e[0] * s0 + e[1] * s1 + e[2] * s2;
+  o.s[0] = fma (-es, e[0], s0);
+  o.s[1] = fma (-es, e[1], s1);
+  o.s[2] = fma (-es, e[2], s2);
+}
+
+// the couplings of recip_apply on transverse parts: c of the vector that
+// meets the cosine-type weights (ya, yc, yh, ym), s of the one that meets the
+// sine-type weights (yb, yg); the sine part enters with the factor sg
+template <int V, typename R>
+__device__ __forceinline__ void
+couple (const R e[3], const FixCoef &K, R sg, const Trans<V, R> &c, const Trans<V, R> &s, R *y)
+{
+  const R ya = (R) K.ya, yb = sg * (R) K.yb, yc = (R) K.yc, yg = sg * (R) K.yg, yh = (R) K.yh,
+          ym = (R) K.ym;
+  R w[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++)
+    {
+      y[d] = ya * c.f[d];
+      if (V >= V_FT)
+        {
+          y[d] = fma (yb, s.t[d], y[d]);
+          w[d] = fma (yc, c.t[d], -yb * s.f[d]);
+        }
+      if (V == V_FTS)
+        {
+          y[d] = fma (R (-2) * yg, s.s[d], y[d]);
+          w[d] = fma (R (2) * yh, c.s[d], w[d]);
+        }
+    }
+  if (V == V_F) return;
+  y[3] = e[1] * w[2] - e[2] * w[1];
+  y[4] = e[2] * w[0] - e[0] * w[2];
+  y[5] = e[0] * w[1] - e[1] * w[0];
+  if (V == V_FT) return;
+  R v[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) v[d] = fma (yg, s.f[d], fma (yh, c.t[d], ym * c.s[d]));
+  y[6] = R (2) * e[0] * v[0];
+  y[7] = fma (e[0], v[1], e[1] * v[0]);
+  y[8] = fma (e[0], v[2], e[2] * v[0]);
+  y[9] = fma (e[1], v[2], e[2] * v[1]);
+  y[10] = R (2) * e[1] * v[1];
+}
+
+constexpr int KOP_T = 64;               // threads per CTA: 16 octant points
+
+template <int ND, int V>
+__global__ void __launch_bounds__ (KOP_T)
+k_fix_kop (FixPlan p)
+{
+  using R = typename Cfg<ND>::R;
+  constexpr int C = NComp<V>::value;
+  const int m1 = blockIdx.y, b = threadIdx.x & 3;
+  const int nqm = p.nqm[m1];
+  if ((int) (blockIdx.x * (KOP_T / 4)) >= nqm) return;
+  const int qr = blockIdx.x * (KOP_T / 4) + threadIdx.x / 4;
+  const bool live = qr < nqm;
+  const int row = 4 * (live ? qr : 0) + b;
+  const int colc = (m1 ? 2 * m1 - 1 : 0) * C, cols = 2 * m1 * C;
+  // a: this row's part of the cosine sums, s: of the sine sums
+  long long ia[C], is[C];
+#pragma unroll
+  for (int q = 0; q < C; q++) ia[q] = is[q] = 0;
+  for (int s = 0; s < p.nsplit; s++)
+    {
+      const long long *F = (const long long *) p.F + (size_t) s * p.ncol * p.Rp + row;
+#pragma unroll
+      for (int q = 0; q < C; q++) ia[q] += F[(size_t) (colc + q) * p.Rp];
+      if (m1)
+#pragma unroll
+        for (int q = 0; q < C; q++) is[q] += F[(size_t) (cols + q) * p.Rp];
+    }
+  R a[C], sn[C];
+#pragma unroll
+  for (int q = 0; q < C; q++)
+    {
+      const R u = (R) unit_of (p.mx[q], p.fu);
+      const long long fc = ia[q], fs = is[q];
+      a[q] = (R) walsh4 (b == 0 ? fc : (b == 3 ? -fc : -fs), b) * u;
+      sn[q] = (R) walsh4 (b == 0 ? fs : (b == 3 ? -fs : fc), b) * u;
+    }
+  const FixCoef K = p.coef[(size_t) 4 * (p.off[m1] + (live ? qr : 0)) + b];
+  const R e[3] = {(R) K.ex, (R) K.ey, (R) K.ez};
+  Trans<V, R> tc, ts;
+  transverse<V, R> (e, a, tc);
+  transverse<V, R> (e, sn, ts);
+  R P[C], Q[C];
+  couple<V, R> (e, K, R (-1), tc, ts, P);
+  couple<V, R> (e, K, R (1), ts, tc, Q);
+  R *G = (R *) p.G + row;
+#pragma unroll
+  for (int q = 0; q < C; q++)
+    {
+      const R wp = walsh4 (P[q], b), wq = walsh4 (Q[q], b);
+      // the cosine and the sine column of this row
+      const R gc = b == 0 ? wp : (b == 3 ? -wp : wq);
+      const R gs = b == 0 ? wq : (b == 3 ? -wq : -wp);
+      uint32_t mx = 0u;
+      if (live)
+        {
+          G[(size_t) (colc + q) * p.Rp] = gc;
+          mx = abs_hi ((double) gc);
+          if (m1)
+            {
+              G[(size_t) (cols + q) * p.Rp] = gs;
+              mx = max (mx, abs_hi ((double) gs));
+            }
+        }
+      mx = __reduce_max_sync (0xffffffffu, mx);
+      if ((threadIdx.x & 31) == 0 && mx) atomicMax (p.mx + 16 * (m1 + 1) + q, mx);
+    }
+}
+
+// Backward image: digits of G, eight rows per thread
+__global__ void __launch_bounds__ (128)
+k_fix_gimage (FixPlan p)
+{
+  const int n = blockIdx.y, r8 = blockIdx.x * 128 + threadIdx.x;
+  if (8 * r8 >= 4 * p.nqm[col_m (p, n)]) return;
+  bool finite;
+  const int E = scale_exp (p.mx[16 * (col_m (p, n) + 1) + n % p.c], finite);
+  const double *g = (const double *) p.G + (size_t) n * p.Rp + 8 * r8;
+  uint32_t w[4][7];
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    {
+      const double2 v = *reinterpret_cast<const double2 *> (g + 2 * k);
+      const long long bias = 0x0080808080808080ll;
+      digits ((finite ? to_fixed (v.x, E, 55) : 0ll) + bias,
+              (finite ? to_fixed (v.y, E, 55) : 0ll) + bias, w[k]);
+    }
+  uint4 *o = reinterpret_cast<uint4 *> ((__half *) p.WB + (size_t) n * p.Rp) + r8;
+#pragma unroll
+  for (int d = 0; d < 7; d++)
+    o[(size_t) d * p.ncol * p.Rp / 8] = make_uint4 (w[0][d], w[1][d], w[2][d], w[3][d]);
+}
+
+template <int ND, int V>
+cudaError_t
+kop_v (const FixPlan &p, cudaStream_t st)
+{
+  k_fix_kop<ND, V><<<dim3 (4 * p.nqp / KOP_T, p.M[0] + 1), KOP_T, 0, st>>> (p);
+  return cudaGetLastError ();
+}
+
+// the shared-memory opt-in is a per-device function attribute
+cudaError_t
+gemm_attrs ()
+{
+  static int attr_dev = -1;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice (&dev);
+  if (e != cudaSuccess || attr_dev == dev) return e;
+  if ((e = cudaFuncSetAttribute (k_fix_fwd<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int) Geo<7>::SMEM)) != cudaSuccess)
+    return e;
+  if ((e = cudaFuncSetAttribute (k_fix_bwd<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int) Geo<7>::SMEM)) != cudaSuccess)
+    return e;
+  attr_dev = dev;
+  return cudaSuccess;
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+size_t fix_bytes_T (int, const FixPlan &p) { return sizeof (long long) * (size_t) p.nT * p.ldT; }
+size_t
+fix_bytes_F (int, const FixPlan &p)
+{
+  return sizeof (long long) * (size_t) p.nsplit * p.ncol * p.Rp;
+}
+size_t fix_bytes_G (int, const FixPlan &p) { return sizeof (double) * (size_t) p.ncol * p.Rp; }
+size_t fix_bytes_ZF (int nd, const FixPlan &p) { return 2 * (size_t) nd * p.ncol * p.ldT; }
+size_t fix_bytes_WB (int nd, const FixPlan &p) { return 2 * (size_t) nd * p.ncol * p.Rp; }
+size_t
+fix_bytes_yp (int, const FixPlan &p)
+{
+  return sizeof (double) * (size_t) p.nbitem * p.np * p.c;
+}
+
+// The time of a set of CTAs (their K tiles, longest first) on one CTA per SM,
+// in K tiles; a CTA's start and end cost about START tiles (measured: a
+// 4-tile forward CTA takes as long as 7 tiles of a long one).
+constexpr int SMS = 152, START = 3;
+
+static long long
+makespan (std::vector<int> &len, int copies)
+{
+  std::sort (len.begin (), len.end (), [] (int a, int b) { return a > b; });
+  std::priority_queue<long long, std::vector<long long>, std::greater<long long>> free;
+  for (int k = 0; k < SMS; k++) free.push (0);
+  long long last = 0;
+  for (int l : len)
+    for (int k = 0; k < copies; k++)
+      {
+        const long long t = free.top () + l + START;
+        free.pop ();
+        free.push (t);
+        last = std::max (last, t);
+      }
+  return last;
+}
+
+// Work items of the two GEMMs.  A column tile needs the quarters that its
+// smallest |m1| uses (nqm): the forward has no item for row tiles past them,
+// the backward's K ends there.  K is sliced as evens out the SMs.
+void
+fix_plan_items (int, FixPlan &p, const std::vector<int> &nqm, std::vector<int4> &fwd,
+                std::vector<int4> &bwd)
+{
+  using C = Cfg<7>;
+  p.nct = (p.ncol + C::TN - 1) / C::TN;
+  p.mt = (p.np + TM - 1) / TM;
+  std::vector<int> rows (p.nct);
+  long long act = 0;
+  for (int ct = 0; ct < p.nct; ct++)
+    {
+      rows[ct] = 4 * nqm[(ct * C::TN / p.c + 1) / 2];
+      act += (rows[ct] + TM - 1) / TM;
+    }
+  // forward: the same number of particle slices for every tile (the operator
+  // kernel adds them), of at least 128 particles
+  long long best = -1;
+  const int kt = p.ldT / C::KT;
+  for (int ns = 1; ns <= std::min (16, p.ldT / 128); ns++)
+    {
+      const int per = (kt + ns - 1) / ns, used = (kt + per - 1) / per;
+      const long long t = (act * used + SMS - 1) / SMS * (per + START);
+      if (best < 0 || t < best)
+        {
+          best = t;
+          p.jper = per * C::KT;
+          p.nsplit = used;
+        }
+    }
+  fwd.clear ();
+  for (int z = 0; z < p.nsplit; z++)
+    for (int ct = 0; ct < p.nct; ct++)
+      for (int rt = 0; rt * TM < rows[ct]; rt++) fwd.push_back (make_int4 (rt, ct, z, 0));
+  p.nfitem = (int) fwd.size ();
+  // backward: row slices of about equal length
+  best = -1;
+  int slice = 1;
+  const int most = (rows[0] + C::KT - 1) / C::KT;
+  for (int s = 1; s <= 24; s++)
+    {
+      const int l = (most + s - 1) / s;
+      if (s > 1 && l < 4) break;
+      std::vector<int> len;
+      for (int ct = 0; ct < p.nct; ct++)
+        {
+          const int k = (rows[ct] + C::KT - 1) / C::KT, n = (k + l - 1) / l;
+          for (int z = 0; z < n; z++) len.push_back ((k + n - 1) / n);
+        }
+      if (s > 1 && len.size () > 96) break;
+      const long long t = makespan (len, p.mt);
+      if (best < 0 || t < best)
+        {
+          best = t;
+          slice = l;
+        }
+    }
+  bwd.clear ();
+  for (int ct = 0; ct < p.nct; ct++)
+    {
+      const int k = (rows[ct] + C::KT - 1) / C::KT, n = std::max (1, (k + slice - 1) / slice);
+      for (int z = 0; z < n; z++)
+        {
+          const int a = (int) ((long long) k * z / n), b = (int) ((long long) k * (z + 1) / n);
+          bwd.push_back (make_int4 (ct, a, b - a, 0));
+        }
+    }
+  std::stable_sort (bwd.begin (), bwd.end (), [] (const int4 &a, const int4 &b) { return a.z > b.z; });
+  p.nbitem = (int) bwd.size ();
+  // |F| <= np in units of its component, and the operators add four of them
+  int lg = 0;
+  while ((1ll << lg) < p.ldT) lg++;
+  p.fu = 60 - lg;
+}
+
+int
+fix_maps (int nd, const FixPlan &p, FixMaps *m)
+{
+  int e = encode_planes_f16 (&m->zf, p.ZF, nd, p.ncol, p.ldT, Cfg<7>::KT, Cfg<7>::TN);
+  if (!e) e = encode_planes_f16 (&m->wb, p.WB, nd, p.ncol, p.Rp, Cfg<7>::KT, Cfg<7>::TN);
+  return e;
+}
+
+cudaError_t
+launch_fix_tables (int, const FixPlan &p, const double *pos, const double *x, cudaStream_t st,
+                   Ctx *prof)
+{
+  cudaError_t e = cudaMemsetAsync (p.mx, 0, fix_mx_words (p) * sizeof (unsigned), st);
+  if (e != cudaSuccess) return e;
+  const int items = p.M[0] + p.M[1] + p.M[2] + 3;
+  k_fix_tables<<<dim3 ((p.np + TAB_P - 1) / TAB_P, (items + TAB_R - 1) / TAB_R), TAB_P * TAB_R, 0,
+                 st>>> (p, pos, x);
+  kmark (prof, st, "k_fix_tables");
+  k_fix_image<<<dim3 (p.ldT / 64, (p.nmi + IMG_M - 1) / IMG_M), 128, 0, st>>> (p, x);
+  kmark (prof, st, "k_fix_image");
+  return cudaGetLastError ();
+}
+
+cudaError_t
+launch_fix_forward (int, int version, const FixPlan &p, const FixMaps &m, int *status,
+                    cudaStream_t st, Ctx *prof)
+{
+  cudaError_t e = gemm_attrs ();
+  if (e != cudaSuccess) return e;
+  k_fix_fwd<7><<<p.nfitem, NT, Geo<7>::SMEM, st>>> (m.zf, p, status);
+  kmark (prof, st, "k_fix_fwd");
+  e = version == 0 ? kop_v<7, 0> (p, st) : (version == 1 ? kop_v<7, 1> (p, st) : kop_v<7, 2> (p, st));
+  kmark (prof, st, "k_fix_kop");
+  return e;
+}
+
+cudaError_t
+launch_fix_backward (int, int, const FixPlan &p, const FixMaps &m, int *status, cudaStream_t st,
+                     Ctx *prof)
+{
+  k_fix_gimage<<<dim3 ((p.Rp / 8 + 127) / 128, p.ncol), 128, 0, st>>> (p);
+  kmark (prof, st, "k_fix_gimage");
+  k_fix_bwd<7><<<dim3 (p.mt, p.nbitem), NT, Geo<7>::SMEM, st>>> (m.wb, p, status);
+  kmark (prof, st, "k_fix_bwd");
+  return cudaGetLastError ();
+}
+
+}  // namespace lsg

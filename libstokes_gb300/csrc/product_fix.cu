@@ -1,0 +1,408 @@
+// product_fix.cu -- the FP64 product of equal spheres at the tuned split: the
+// reciprocal sum as exact fixed-point GEMMs on the tensor cores
+// (kspace_fix.cu), the real space on a side stream beside it.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+#include <cstdlib>
+#include <cstring>
+#include <vector>
+
+#include "ewald_device.cuh"
+#include "fixk.h"
+#include "gpu_engine.h"
+#include "seq_graph.h"
+#include "stokes_gpu.h"
+
+namespace lsg {
+
+constexpr int ND = 7;
+
+struct FixState {
+  double key[16] = {0};
+  uint64_t id = 0;              // counts the set-ups (part of the graph key)
+  FixPlan p;
+  FixMaps maps;
+  double self[3] = {0, 0, 0};
+  DevBuf quart, nqm, coef, off, fitem, bitem, T, F, G, ZF, WB, mx, yp, partial, status;
+  int *h_status = nullptr;
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  SeqGraph graph;
+};
+
+// y = self x + real-space partials + reciprocal partials.  A CTA sums 32
+// consecutive elements: warp w takes every eighth partial (coalesced), the
+// eight sums meet in shared memory.
+constexpr int FC_W = 8;
+
+struct FixCombine {
+  const double *x, *pr, *pk;
+  int n, c, ncr, nck;
+  double self[3];
+  double *y;
+};
+
+__global__ void __launch_bounds__ (32 * FC_W)
+k_fix_combine (FixCombine a)
+{
+  __shared__ double s_v[FC_W][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int e = blockIdx.x * 32 + lane;
+  double v = 0.0;
+  if (e < a.n)
+    {
+      for (int k = w; k < a.nck; k += FC_W) v += a.pk[(size_t) k * a.n + e];
+      for (int k = w; k < a.ncr; k += FC_W) v += a.pr[(size_t) k * a.n + e];
+    }
+  s_v[w][lane] = v;
+  __syncthreads ();
+  if (w || e >= a.n) return;
+#pragma unroll
+  for (int k = 1; k < FC_W; k++) v += s_v[k][lane];
+  const int q = e % a.c;
+  // the self block is diagonal: the stresslet part (sm (S' - tr S' / 3) with
+  // S' the full contraction) gives sm times the five components
+  a.y[e] = fma (a.self[q < 3 ? 0 : (q < 6 ? 1 : 2)], a.x[e], v);
+}
+
+// octant points, weights and tiles of the split of ts, with libstokes' G term
+// of sys's own split (FTS; the correction described at tuned_applies)
+int
+fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
+{
+  if (!c->fix) c->fix = new FixState ();
+  FixState *f = c->fix;
+  const bool fts = sys->version == 2;
+  const double key[16] = {sys->lx, sys->ly, sys->lz, (double) sys->np, (double) sys->version,
+                          ts->xi, ts->kmax, sys->xi, fts ? sys->kmax : 0.0,
+                          fts ? (double) sys->kmaxx : 0.0, fts ? (double) sys->kmaxy : 0.0,
+                          fts ? (double) sys->kmaxz : 0.0, 1.0};
+  if (memcmp (key, f->key, sizeof key) == 0) return STOKES_GPU_OK;
+  f->key[12] = 0.0;
+  FixPlan p;
+  p.np = sys->np;
+  p.c = NCOMP (sys->version);
+  p.l[0] = sys->lx; p.l[1] = sys->ly; p.l[2] = sys->lz;
+  double k0[3];
+  int B[3];
+  const int ref[3] = {sys->kmaxx, sys->kmaxy, sys->kmaxz};
+  for (int d = 0; d < 3; d++)
+    {
+      p.il[d] = 1.0 / p.l[d];
+      k0[d] = 2.0 * M_PI / p.l[d];
+      B[d] = (int) (ts->kmax / k0[d]);
+      if (fts) B[d] = std::max (B[d], ref[d]);
+    }
+  // weights of one octant point without the direction; false: not in the set
+  const double pivol = M_PI / (sys->lx * sys->ly * sys->lz);
+  auto scalars = [&] (int a, int b, int d, FixCoef &w) {
+    const double k1 = k0[0] * a, k2 = k0[1] * b, k3 = k0[2] * d;
+    const double kk = k1 * k1 + k2 * k2 + k3 * k3, k = sqrt (kk);
+    w = FixCoef {};
+    if (kk == 0.0) return false;
+    bool in = false;
+    if (k <= ts->kmax)
+      {
+        const double k4z = kk / 4.0 / ts->xi2;
+        const double kexp = pivol * (1.0 + k4z * (1.0 + 2.0 * k4z)) / kk * exp (-k4z);
+        w.ya = 6.0 * (1.0 - kk / 3.0) * kexp;
+        w.yb = 3.0 * k * kexp;
+        w.yc = 1.5 * kk * kexp;
+        w.yg = -3.0 * (1.0 - 4.0 / 15.0 * kk) * k * kexp;
+        w.yh = 1.5 * kk * kexp;
+        w.ym = 3.0 * (1.0 - kk / 5.0) * kk * kexp;
+        in = true;
+      }
+    if (fts && a <= ref[0] && b <= ref[1] && d <= ref[2] && (sys->kmax == 0.0 || k <= sys->kmax))
+      {
+        const double k4z = kk / 4.0 / sys->xi2;
+        const double kexp = sys->pivol * (1.0 + k4z * (1.0 + 2.0 * k4z)) / kk * exp (-k4z);
+        w.yg += 6.0 * (1.0 - 4.0 / 15.0 * kk) * k * kexp;
+        in = true;
+      }
+    w.ex = k1 / k; w.ey = k2 / k; w.ez = k3 / k;
+    return in;
+  };
+  // quarters by length: the ones in use at |m1| are then (nearly) a prefix
+  struct Quarter { int m2, m3; double kk; };
+  std::vector<Quarter> qs;
+  for (int b = 0; b <= B[1]; b++)
+    for (int d = 0; d <= B[2]; d++)
+      {
+        const double k2 = k0[1] * b, k3 = k0[2] * d;
+        const bool own = k2 * k2 + k3 * k3 <= ts->kmax * ts->kmax;
+        const bool of_ref = fts && b <= ref[1] && d <= ref[2];
+        if (own || of_ref) qs.push_back ({b, d, k2 * k2 + k3 * k3});
+      }
+  std::stable_sort (qs.begin (), qs.end (),
+                    [] (const Quarter &a, const Quarter &b) { return a.kk < b.kk; });
+  std::vector<FixCoef> coef, line (qs.size () * ((size_t) B[0] + 1));
+  std::vector<int> nqm ((size_t) B[0] + 1), off ((size_t) B[0] + 2);
+  for (int a = 0; a <= B[0]; a++)
+    {
+      nqm[a] = 0;
+      for (size_t k = 0; k < qs.size (); k++)
+        {
+          FixCoef &w = line[(size_t) a * qs.size () + k];
+          if (scalars (a, qs[k].m2, qs[k].m3, w))
+            {
+              nqm[a] = (int) k + 1;
+              p.M[0] = a;
+            }
+        }
+    }
+  // a column tile covers the quarters of its smallest |m1|: prefixes that do
+  // not grow with |m1|
+  for (int a = B[0] - 1; a >= 0; a--) nqm[a] = std::max (nqm[a], nqm[a + 1]);
+  const int nq = nqm[0];
+  for (int a = 0; a <= B[0]; a++)
+    {
+      off[a] = (int) (coef.size () / 4);
+      for (int k = 0; k < nqm[a]; k++)
+        {
+          // weight of the vector in the sum over the four sign patterns: the
+          // point stands for prod (m ? 2 : 1) vectors, k and -k count alike
+          const double mult = (a ? 2.0 : 1.0) * (qs[k].m2 ? 2.0 : 1.0) * (qs[k].m3 ? 2.0 : 1.0) / 4.0;
+          for (int s = 0; s < 4; s++)
+            {
+              FixCoef w = line[(size_t) a * qs.size () + k];
+              w.ey *= s & 2 ? -1.0 : 1.0;
+              w.ez *= s & 1 ? -1.0 : 1.0;
+              w.ya *= mult; w.yb *= mult; w.yc *= mult;
+              w.yg *= mult; w.yh *= mult; w.ym *= mult;
+              coef.push_back (w);
+            }
+        }
+    }
+  off[B[0] + 1] = (int) (coef.size () / 4);
+  for (int k = 0; k < nq; k++)
+    {
+      p.M[1] = std::max (p.M[1], qs[k].m2);
+      p.M[2] = std::max (p.M[2], qs[k].m3);
+    }
+  p.nmi = 2 * p.M[0] + 1;
+  p.ncol = p.nmi * p.c;
+  p.nq = nq;
+  p.nqp = (std::max (nq, 1) + 31) / 32 * 32;
+  p.Rp = 4 * p.nqp;
+  p.ldT = (p.np + 127) / 128 * 128;
+  p.oy = p.nmi;
+  p.oz = p.oy + 2 * p.M[1] + 1;
+  p.zero = p.oz + 2 * p.M[2] + 1;
+  p.nT = p.zero + 1;
+  std::vector<int4> fitem, bitem;
+  fix_plan_items (ND, p, nqm, fitem, bitem);
+
+  std::vector<int4> quart ((size_t) p.nqp, make_int4 (p.zero, p.zero, p.zero, p.zero));
+  for (int k = 0; k < nq; k++)
+    {
+      const int b = qs[k].m2, d = qs[k].m3;
+      quart[k] = make_int4 (p.oy + (b ? 2 * b - 1 : 0), b ? p.oy + 2 * b : p.zero,
+                            p.oz + (d ? 2 * d - 1 : 0), d ? p.oz + 2 * d : p.zero);
+    }
+  cudaError_t e = cudaSuccess;
+  cudaStream_t st = c->stream;
+  auto up = [&] (DevBuf &b, const void *h, size_t bytes) {
+    if (e == cudaSuccess) e = b.ensure (std::max<size_t> (bytes, 64));
+    if (e == cudaSuccess && bytes) e = cudaMemcpyAsync (b.p, h, bytes, cudaMemcpyHostToDevice, st);
+  };
+  // no product of this context may still be using the tables of the last set-up
+  if (f->id && (e = cudaDeviceSynchronize ()) != cudaSuccess)
+    return cuda_fail (e, "FP64 product set-up");
+  up (f->quart, quart.data (), sizeof (int4) * quart.size ());
+  up (f->nqm, nqm.data (), sizeof (int) * nqm.size ());
+  up (f->off, off.data (), sizeof (int) * off.size ());
+  up (f->coef, coef.data (), sizeof (FixCoef) * coef.size ());
+  up (f->fitem, fitem.data (), sizeof (int4) * fitem.size ());
+  up (f->bitem, bitem.data (), sizeof (int4) * bitem.size ());
+  auto room = [&] (DevBuf &b, size_t bytes, bool clear) {
+    if (e == cudaSuccess) e = b.ensure (std::max<size_t> (bytes, 64));
+    if (e == cudaSuccess && clear) e = cudaMemsetAsync (b.p, 0, bytes, st);
+  };
+  // table pads, rows and columns that nothing writes stay zero
+  room (f->T, fix_bytes_T (ND, p), true);
+  room (f->F, fix_bytes_F (ND, p), false);
+  room (f->G, fix_bytes_G (ND, p), true);
+  room (f->ZF, fix_bytes_ZF (ND, p), true);
+  room (f->WB, fix_bytes_WB (ND, p), true);
+  room (f->yp, fix_bytes_yp (ND, p), false);
+  room (f->mx, fix_mx_words (p) * sizeof (unsigned), true);
+  if (!f->status.p) room (f->status, sizeof (int), true);
+  // the uploads read host vectors of this call
+  if (e == cudaSuccess) e = cudaStreamSynchronize (st);
+  if (e != cudaSuccess) return cuda_fail (e, "FP64 product set-up");
+  p.quart = (const int4 *) f->quart.p;
+  p.nqm = (const int *) f->nqm.p;
+  p.off = (const int *) f->off.p;
+  p.coef = (const FixCoef *) f->coef.p;
+  p.fitem = (const int4 *) f->fitem.p;
+  p.bitem = (const int4 *) f->bitem.p;
+  p.T = f->T.p; p.F = f->F.p; p.G = f->G.p; p.ZF = f->ZF.p; p.WB = f->WB.p;
+  p.mx = (unsigned *) f->mx.p;
+  p.yp = f->yp.p;
+  const int me = fix_maps (ND, p, &f->maps);
+  if (me) return set_error (STOKES_GPU_ECUDA, "TMA tensor maps of the FP64 product (%d)", me);
+  if (!f->h_status)
+    {
+      if ((e = cudaMallocHost (&f->h_status, sizeof (int))) != cudaSuccess)
+        return cuda_fail (e, "status");
+      *f->h_status = 0;
+    }
+  if (!f->side)
+    {
+      int lo = 0, hi = 0;
+      cudaDeviceGetStreamPriorityRange (&lo, &hi);
+      if (cudaStreamCreateWithPriority (&f->side, cudaStreamNonBlocking, lo) != cudaSuccess
+          || cudaEventCreateWithFlags (&f->ev_fork, cudaEventDisableTiming) != cudaSuccess
+          || cudaEventCreateWithFlags (&f->ev_join, cudaEventDisableTiming) != cudaSuccess)
+        return set_error (STOKES_GPU_ECUDA, "FP64 product: side stream");
+    }
+  f->self[0] = ts->self_a;
+  f->self[1] = ts->self_c;
+  f->self[2] = ts->self_m;
+  f->p = p;
+  f->id++;
+  memcpy (f->key, key, sizeof key);
+  return STOKES_GPU_OK;
+}
+
+// source chunks per target of the real-space kernel: about 32 warps per SM
+static int
+real_chunks (int np)
+{
+  return std::max (1, std::min (std::min (np, 64), (152 * 32 + np - 1) / np));
+}
+
+int
+atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cudaStream_t st,
+                bool timed)
+{
+  FixState *f = c->fix;
+  FixPlan p = f->p;
+  p.stall = g_test_gemm_stall;
+  const int np = c->np, n = np * p.c;
+  // a status word raised by a bounded device wait of the previous product
+  if (*f->h_status)
+    {
+      *f->h_status = 0;
+      cudaMemsetAsync (f->status.p, 0, sizeof (int), st);
+      return set_error (STOKES_GPU_ETIMEOUT,
+                        "a tensor-core wait of the previous FP64 product ran out");
+    }
+  const int nchunk = real_chunks (np);
+  cudaError_t e = f->partial.ensure (sizeof (double) * (size_t) nchunk * n);
+  if (e != cudaSuccess) return cuda_fail (e, "real-space scratch");
+
+  RealArgs a;
+  a.pos = d_pos;
+  a.x = d_x;
+  a.img = (const Img4 *) c->img.p;
+  a.nimg = c->nimg;
+  a.np = np;
+  a.nchunk = nchunk;
+  a.rmax2 = c->rmax2;
+  a.rmin = c->rmin;
+  a.xi = c->xi;
+  a.xisp = c->xisp;
+  a.rad = a.slipa = nullptr;
+  a.partial = (double *) f->partial.p;
+  a.open = 0;
+  a.clampfix = c->rmin > 0.0 ? 1 : 0;
+  a.xi_ref = c->xi_ref;
+  a.xisp_ref = c->xi_ref / sqrt (M_PI);
+
+  cudaEvent_t *E = phase_events (c, timed);
+  const bool overlap = (!E || E == c->ev) && !c->kprof_on;
+  auto sequence = [&] () -> int {
+    int *status = (int *) f->status.p;
+    cudaError_t e;
+    if (E) cudaEventRecord (E[0], st);
+    kmark (c, st, nullptr);
+    // the real space needs the positions only; recorded after the forward
+    // GEMM, its CTAs take what that leaves idle
+    if (overlap) cudaEventRecord (f->ev_fork, st);
+    if ((e = launch_fix_tables (ND, p, d_pos, d_x, st, c)) != cudaSuccess)
+      return cuda_fail (e, "reciprocal tables");
+    if ((e = launch_fix_forward (ND, c->version, p, f->maps, status, st, c)) != cudaSuccess)
+      return cuda_fail (e, "reciprocal space (forward)");
+    if (overlap)
+      {
+        cudaStreamWaitEvent (f->side, f->ev_fork, 0);
+        if (E) cudaEventRecord (E[1], f->side);
+        e = launch_real_fp64 (c->version, MODE_MONO, a, f->side);
+        if (E) cudaEventRecord (E[2], f->side);
+        cudaEventRecord (f->ev_join, f->side);
+        if (e != cudaSuccess) return cuda_fail (e, "real-space kernel");
+      }
+    if ((e = launch_fix_backward (ND, c->version, p, f->maps, status, st, c)) != cudaSuccess)
+      return cuda_fail (e, "reciprocal space (backward)");
+    if (overlap)
+      cudaStreamWaitEvent (st, f->ev_join, 0);
+    else
+      {
+        if (E) cudaEventRecord (E[1], st);
+        if ((e = launch_real_fp64 (c->version, MODE_MONO, a, st)) != cudaSuccess)
+          return cuda_fail (e, "real-space kernel");
+        kmark (c, st, "k_real");
+        if (E) cudaEventRecord (E[2], st);
+      }
+    FixCombine cb {d_x, (const double *) f->partial.p, (const double *) p.yp, n, p.c, nchunk,
+                   p.nbitem, {f->self[0], f->self[1], f->self[2]}, d_y};
+    k_fix_combine<<<(n + 31) / 32, 32 * FC_W, 0, st>>> (cb);
+    kmark (c, st, "k_fix_combine");
+    if (E) cudaEventRecord (E[3], st);
+    cudaMemcpyAsync (f->h_status, f->status.p, sizeof (int), cudaMemcpyDeviceToHost, st);
+    if ((e = cudaGetLastError ()) != cudaSuccess) return cuda_fail (e, "FP64 product");
+    return STOKES_GPU_OK;
+  };
+  static const bool graphs = [] {
+    const char *g = getenv ("LIBSTOKES_GB300_GRAPHS");
+    return !(g && strcmp (g, "0") == 0);
+  }();
+  uint64_t key = 1469598103934665603ull;
+  uint64_t rmin_bits;
+  memcpy (&rmin_bits, &a.rmin, sizeof rmin_bits);
+  for (uint64_t v : {f->id, (uint64_t) (uintptr_t) d_pos, (uint64_t) (uintptr_t) d_x,
+                     (uint64_t) (uintptr_t) d_y, (uint64_t) (uintptr_t) a.img, (uint64_t) a.nimg,
+                     (uint64_t) (uintptr_t) a.partial, (uint64_t) (uintptr_t) E, rmin_bits})
+    key = (key ^ v) * 1099511628211ull;
+  const bool use = graphs && !c->kprof_on && (E == nullptr || E == c->ev) && p.stall == 0;
+  const int rc = run_sequence (f->graph, key, st, E, use, sequence);
+  if (rc) return rc;
+  c->launches = 8;
+  c->timed = timed;
+  return STOKES_GPU_OK;
+}
+
+int
+fix_check_status (Ctx *c)
+{
+  FixState *f = c->fix;
+  if (!f || !f->h_status || !*f->h_status) return STOKES_GPU_OK;
+  *f->h_status = 0;
+  cudaMemsetAsync (f->status.p, 0, sizeof (int), c->stream);
+  cudaStreamSynchronize (c->stream);
+  return set_error (STOKES_GPU_ETIMEOUT, "a tensor-core wait of the FP64 product ran out");
+}
+
+void
+release_fix (Ctx *c)
+{
+  FixState *f = c->fix;
+  if (!f) return;
+  for (DevBuf *b : {&f->quart, &f->nqm, &f->coef, &f->off, &f->fitem, &f->bitem, &f->T, &f->F, &f->G, &f->ZF, &f->WB,
+                    &f->mx, &f->yp, &f->partial, &f->status})
+    b->release ();
+  f->graph.release ();
+  if (f->h_status) cudaFreeHost (f->h_status);
+  if (f->side) cudaStreamDestroy (f->side);
+  if (f->ev_fork) cudaEventDestroy (f->ev_fork);
+  if (f->ev_join) cudaEventDestroy (f->ev_join);
+  delete f;
+  c->fix = nullptr;
+}
+
+}  // namespace lsg

@@ -68,6 +68,30 @@ idesc_tf32 (uint32_t M, uint32_t N)
     | ((M >> 4) << 24);       // M / 16
 }
 
+// the same for a 64-byte swizzled tile: rows of 64 bytes (32 f16 values),
+// 8-row groups 512 bytes apart, the four 16-byte chunks of row r permuted by
+// (r / 2) % 4
+__device__ __forceinline__ uint64_t
+smem_desc_sw64 (uint32_t saddr)
+{
+  uint64_t d = 0;
+  d |= (uint64_t) ((saddr >> 4) & 0x3FFFu);
+  d |= (uint64_t) 1u << 16;                 // LBO (ignored): 16 bytes
+  d |= (uint64_t) (512u >> 4) << 32;        // SBO: 512 bytes
+  d |= (uint64_t) 1u << 46;                 // descriptor version
+  d |= (uint64_t) 4u << 61;                 // layout: 64-byte swizzle
+  return d;
+}
+
+// instruction descriptor, kind::f16: D f32, A/B f16, both K-major
+__host__ __device__ __forceinline__ uint32_t
+idesc_f16 (uint32_t M, uint32_t N)
+{
+  return (1u << 4)            // D format: f32 (A and B format 0: f16)
+    | ((N >> 3) << 17)        // N / 8
+    | ((M >> 4) << 24);       // M / 16
+}
+
 __device__ __forceinline__ uint32_t
 smem_u32 (const void *p)
 {
@@ -132,6 +156,17 @@ mma_tf32 (uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint3
     "{\n\t.reg .pred p;\n\t"
     "setp.ne.b32 p, %4, 0;\n\t"
     "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+    :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+// the same with f16 operands (K = 16 per instruction)
+__device__ __forceinline__ void
+mma_f16 (uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+{
+  asm volatile (
+    "{\n\t.reg .pred p;\n\t"
+    "setp.ne.b32 p, %4, 0;\n\t"
+    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
     :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
@@ -297,6 +332,31 @@ tmem_ld16 (uint32_t taddr, float v[16])
   asm volatile ("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int q = 0; q < 16; q++) v[q] = __uint_as_float (r[q]);
+}
+
+// the same load without the wait: v holds the columns after tmem_ld_wait (v)
+__device__ __forceinline__ void
+tmem_ld16_issue (uint32_t taddr, float v[16])
+{
+  asm volatile (
+    "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+    "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+    : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
+      "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]),
+      "=f"(v[14]), "=f"(v[15])
+    : "r"(taddr));
+}
+
+// every issued load of this thread is complete; the operands tie the loaded
+// registers to the wait
+__device__ __forceinline__ void
+tmem_ld_wait (float v[16])
+{
+  asm volatile ("tcgen05.wait::ld.sync.aligned;"
+                : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]),
+                  "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]),
+                  "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15])
+                :: "memory");
 }
 
 }  // namespace umma
