@@ -470,4 +470,20 @@ warp_sum (R v)
   return v;
 }
 
+// a signed 64-bit integer as FP64, rounded to nearest (ties away), in integer
+// arithmetic: conversions run at the FP64 rate, 1/64 of the integer one
+__device__ __forceinline__ double
+int_to_double (long long v)
+{
+  const unsigned long long sign = (unsigned long long) v & 0x8000000000000000ull;
+  unsigned long long m = v < 0 ? 0ull - (unsigned long long) v : (unsigned long long) v;
+  const int z = __clzll ((long long) m);
+  m <<= z;                                              // leading bit at 63
+  const unsigned long long r = (m >> 11) + ((m >> 10) & 1ull);
+  // r has its leading bit at 52 (or 53 after a carry), which adds to the
+  // exponent field
+  const unsigned long long bits = ((unsigned long long) (1023 + 62 - z) << 52) + r;
+  return __longlong_as_double ((long long) (v ? bits | sign : 0ull));
+}
+
 }  // namespace lsg

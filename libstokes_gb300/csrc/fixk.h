@@ -46,10 +46,13 @@ struct FixPlan {
   const FixCoef *coef = nullptr;   // octant points: [off[m1] + quarter][4 sign patterns]
   const int *off = nullptr;        // [M0 + 2] first octant point of |m1|
   void *T = nullptr;          // function table [nT][ldT]
+  uint4 *q = nullptr;         // [np] fractional coordinates, upper 32 bits
+  unsigned long long *u = nullptr;   // [np][4] the same, 64 bits
+  void *S = nullptr;          // digit strings [Rp][ldT]
   void *F = nullptr;          // structure factors [nsplit][ncol][Rp], int64
   void *G = nullptr;          // operator output [ncol][Rp]
-  void *ZF = nullptr;         // forward image [digits][ncol][ldT] f16
-  void *WB = nullptr;         // backward image [digits][ncol][Rp] f16
+  void *ZF = nullptr;         // forward image, f16 digits of [ncol][ldT]
+  void *WB = nullptr;         // backward image, f16 digits of [ncol][Rp]
   // high words of max |x_q| at [q] and of max |G| of the columns (m1, q) at
   // [16 (|m1| + 1) + q]
   unsigned *mx = nullptr;
@@ -66,6 +69,7 @@ inline size_t fix_mx_words (const FixPlan &p) { return 16 * ((size_t) p.M[0] + 2
 
 // host entry points of kspace_fix.cu; ND: digits per number, 7 (FP64)
 size_t fix_bytes_T (int nd, const FixPlan &p);
+size_t fix_bytes_S (int nd, const FixPlan &p);
 size_t fix_bytes_F (int nd, const FixPlan &p);
 size_t fix_bytes_G (int nd, const FixPlan &p);
 size_t fix_bytes_ZF (int nd, const FixPlan &p);

@@ -33,17 +33,18 @@
 // carries the rounding of its inputs, about 2^-56 of full scale each, and
 // none from the summation.
 //
-// Operands.  B comes from images [digit][column][K] of f16 by TMA.  A is
-// built in shared memory by the worker warps from the function table (int64,
-// 62 fractional bits): a 64-bit high product, one rounding shift, one add
-// that biases all digits at once, and per digit pair a byte permute, a mask
-// and an f16x2 subtraction.  Images of A would be 7 f16 planes of rows x
-// particles, re-read for every column tile.
+// Operands.  B comes from images of f16 digits by TMA.  A is kept as 64-bit
+// digit strings [row][particle], made once per product and read by both
+// GEMMs; the worker warps cut them into f16 digits in shared memory (per
+// digit pair a byte permute, a mask and an f16x2 subtraction).  As f16 images
+// A would be twice as large and needed in two orientations.
 //
-// What bounds the GEMMs: shared-memory reads of the MMAs.  A 128 x 64 x 16
-// MMA reads 6 KB (48 clocks of shared memory against 32 of tensor pipe); a
-// 32-wide K tile has 56 of them (2700 clocks) next to about 900 clocks of
-// operand stores and 250 of drain per tile, spread over 16 worker warps.
+// Shared memory rows are 128 bytes: 32 K values of an even digit and of the
+// next odd one side by side.  The rows of all even digits of B follow one
+// another, so one MMA takes a digit of A against all of them (see mma_role).
+// One MMA per digit pair (N = 64) took 78 clocks, 80 us of MMAs in the forward
+// GEMM of FTS N = 1000: it reads 6 KB of shared memory for 32 clocks of tensor
+// pipe.  Now a 16-wide K step is 13 MMAs that read 108 KB for 896 clocks.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -77,16 +78,33 @@ template <> struct Cfg<7> {
   static constexpr int DK = 4;          // tiles per drain (K = 128)
 };
 
+// Tiles of 128-byte rows: KT = 64 values of one digit, or KT = 32 values of
+// an even digit and the next one
 template <int ND>
 struct Geo {
   using C = Cfg<ND>;
-  static constexpr int ROWB = 2 * C::KT;                // bytes of a tile row
-  static constexpr uint32_t A_PLANE = TM * ROWB;
-  static constexpr uint32_t B_PLANE = C::TN * ROWB;
-  static constexpr uint32_t STAGE = ND * (A_PLANE + B_PLANE);
+  static constexpr int PAIR = 64 / C::KT;               // digits per row
+  static constexpr int NP = (ND + PAIR - 1) / PAIR;     // planes
+  static constexpr uint32_t A_PLANE = TM * 128;
+  static constexpr uint32_t B_PLANE = C::TN * 128;
+  static constexpr uint32_t STAGE = NP * (A_PLANE + B_PLANE);
   static constexpr uint32_t SMEM = STAGES * STAGE + 1024;
   static constexpr int CPT = C::TN / 4;                 // accumulator columns per worker
+  // byte offset of digit p in its row, after the plane's own offset
+  static constexpr uint32_t part (int p) { return PAIR == 2 ? (uint32_t) (p & 1) * 64u : 0u; }
+  static constexpr int plane (int p) { return p / PAIR; }
 };
+
+// element (digit p, row n, k) of an f16 image with `rows` rows of ld values
+template <int ND>
+__device__ __forceinline__ size_t
+image_off (int p, size_t rows, size_t n, size_t ld, int k)
+{
+  using G = Geo<ND>;
+  constexpr int KT = Cfg<ND>::KT;
+  const size_t row = (G::plane (p) * rows + n) * ld * G::PAIR;
+  return row + (size_t) (k / KT) * 64 + G::part (p) / 2 + k % KT;
+}
 
 struct Sync {
   uint64_t full[STAGES], empty[STAGES], acc_full, acc_empty, done, never;
@@ -169,15 +187,18 @@ scale_exp (uint32_t hw, bool &finite)
   return e - 1022;
 }
 
-// 2^(E - log) as the factor that turns results in units of 2^-log into values;
-// NaN where an input was NaN or infinite, as a sum over it would be
+// v 2^(E - frac) as FP64, E the exponent of hw; NaN where an input was NaN or
+// infinite, as a sum over it would be.  In integers, like to_fixed.
 __device__ __forceinline__ double
-unit_of (uint32_t hw, int log)
+from_fixed (long long v, uint32_t hw, int frac)
 {
   bool finite;
-  const int e = scale_exp (hw, finite) - log;
+  const int e = scale_exp (hw, finite) - frac;
   if (!finite) return __longlong_as_double (0x7ff8000000000000ll);
-  return e > -1022 ? __hiloint2double ((e + 1023) << 20, 0) : scalbn (1.0, e);
+  const double d = int_to_double (v);
+  // exponents far from the ends of the range: add e to the exponent field
+  if (e > -1022 && e < 960) return v ? __longlong_as_double (__double_as_longlong (d) + ((long long) e << 52)) : 0.0;
+  return scalbn (d, e);
 }
 
 __device__ __forceinline__ uint32_t
@@ -187,111 +208,86 @@ abs_hi (double v)
 }
 
 // ---- operand builders -----------------------------------------------------
-// byte offset of 16-byte chunk c of row r in a swizzled plane
-template <int ND>
+// byte offset of 16-byte chunk c of row r in a 128-byte swizzled plane
 __device__ __forceinline__ uint32_t
 chunk_off (int r, int c)
 {
-  if (Geo<ND>::ROWB == 64) return (uint32_t) (r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
   return (uint32_t) (r * 128 + ((c ^ (r & 7)) << 4));
 }
 
-// The A operand of a tile is built in two steps, so that the table loads of
-// the next tile are in flight while a worker waits for its stage: load()
-// reads the table entries of a thread's share into registers, store() forms
-// the products, cuts the digits and writes them to the stage.
+// The A operand of a tile is built in two steps, so that the loads of the
+// next tile are in flight while a worker waits for its stage: load() reads a
+// thread's digit strings, store() cuts them and writes the stage.
 
-// Forward: rows r0 .. r0 + 127 (32 quarters, two per warp), particles j0 ..
-// j0 + 31.  Half a warp covers the 32 particles (two per lane) of one
-// quarter, whose four rows share its four table entries.  The upper half-warp
-// takes the rows in the order 1 0 3 2, so that the two halves write different
-// 64-byte halves of a 128-byte bank line.
+// Forward: rows r0 .. r0 + 127, particles j0 .. j0 + 31.  Half a warp covers
+// the 32 particles (two per lane) of four rows; the two halves of a warp write
+// different halves of a 128-byte bank line (their rows differ by 4).
 template <int ND>
 struct BuildF {
-  const long long *T;
-  int ldT, j0;
-  int4 f;                       // table rows of the thread's quarter
-  longlong2 y[2], z[2];         // cosine and sine entries of two particles
-  __device__ __forceinline__ BuildF (const FixPlan &p, int r0, int jb)
-    : T ((const long long *) p.T), ldT (p.ldT)
+  const long long *S;
+  int ldT;
+  longlong2 v[4];
+  __device__ __forceinline__ BuildF (const FixPlan &p, int r0, int jb) : ldT (p.ldT)
   {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    f = p.quart[r0 / 4 + 2 * warp + (lane >> 4)];
-    j0 = jb + 2 * (lane & 15);
+    S = (const long long *) p.S + (size_t) (r0 + 8 * warp + 4 * (lane >> 4)) * ldT + jb
+        + 2 * (lane & 15);
   }
   __device__ __forceinline__ void load (int t)
   {
-    const size_t jo = (size_t) j0 + Cfg<ND>::KT * t;
-    y[0] = *reinterpret_cast<const longlong2 *> (T + (size_t) f.x * ldT + jo);
-    y[1] = *reinterpret_cast<const longlong2 *> (T + (size_t) f.y * ldT + jo);
-    z[0] = *reinterpret_cast<const longlong2 *> (T + (size_t) f.z * ldT + jo);
-    z[1] = *reinterpret_cast<const longlong2 *> (T + (size_t) f.w * ldT + jo);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      v[k] = __ldg (reinterpret_cast<const longlong2 *> (S + (size_t) k * ldT + Cfg<ND>::KT * t));
   }
   __device__ __forceinline__ void store (unsigned char *stage) const
   {
+    using G = Geo<ND>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int jp = lane & 15, hs = lane >> 4, qd = 2 * warp + hs;
-    // z in the order of this half-warp's rows
-    const Limbs za[2] = {limbs (hs ? z[1].x : z[0].x), limbs (hs ? z[0].x : z[1].x)};
-    const Limbs zb[2] = {limbs (hs ? z[1].y : z[0].y), limbs (hs ? z[0].y : z[1].y)};
+    const int jp = lane & 15;
 #pragma unroll
     for (int k = 0; k < 4; k++)
       {
-        const int r = 4 * qd + (k ^ hs);                // row 2 p2 + p3 of the quarter
+        const int r = 8 * warp + 4 * (lane >> 4) + k;
         uint32_t d[7];
-        digits (biased (limbs (y[k >> 1].x), za[k & 1]), biased (limbs (y[k >> 1].y), zb[k & 1]), d);
-        unsigned char *o = stage + chunk_off<ND> (r, jp >> 2) + (jp & 3) * 4;
+        digits (v[k].x, v[k].y, d);
+        // digits of odd number sit four chunks further
+        unsigned char *o0 = stage + chunk_off (r, jp >> 2) + (jp & 3) * 4;
+        unsigned char *o1 = stage + chunk_off (r, 4 + (jp >> 2)) + (jp & 3) * 4;
 #pragma unroll
         for (int q = 0; q < ND; q++)
-          *reinterpret_cast<uint32_t *> (o + q * Geo<ND>::A_PLANE) = d[q];
+          *reinterpret_cast<uint32_t *> ((q & 1 ? o1 : o0) + G::plane (q) * G::A_PLANE) = d[q];
       }
   }
 };
 
-// Backward: particles i0 .. i0 + 127, one per lane, rows 4 quart0 .. + 31, two
-// quarters (16 bytes per plane) per thread
+// Backward: particles i0 .. i0 + 127, one per lane, 32 rows, eight of them (16
+// bytes per digit) per thread
 template <int ND>
 struct BuildB {
-  const long long *T;
-  const int4 *quart;
-  int ldT, i, c;
-  long long y[2][2], z[2][2];
-  __device__ __forceinline__ BuildB (const FixPlan &p, int i0, int quart0)
-    : T ((const long long *) p.T), quart (p.quart), ldT (p.ldT)
+  const long long *S;
+  int ldT, c;
+  long long v[8];
+  __device__ __forceinline__ BuildB (const FixPlan &p, int i0, int r0) : ldT (p.ldT)
   {
-    i = i0 + (threadIdx.x & 127);
     c = threadIdx.x >> 7;
-    quart += quart0 + 2 * c;
+    S = (const long long *) p.S + (size_t) (r0 + 8 * c) * ldT + i0 + (threadIdx.x & 127);
   }
   __device__ __forceinline__ void load (int t)
   {
 #pragma unroll
-    for (int u = 0; u < 2; u++)
-      {
-        const int4 f = __ldg (quart + t * (Cfg<ND>::KT / 4) + u);
-        y[u][0] = T[(size_t) f.x * ldT + i];
-        y[u][1] = T[(size_t) f.y * ldT + i];
-        z[u][0] = T[(size_t) f.z * ldT + i];
-        z[u][1] = T[(size_t) f.w * ldT + i];
-      }
+    for (int u = 0; u < 8; u++) v[u] = __ldg (S + (size_t) (t * Cfg<ND>::KT + u) * ldT);
   }
   __device__ __forceinline__ void store (unsigned char *stage) const
   {
-    uint32_t w[ND][4];
+    using G = Geo<ND>;
+    uint32_t w[4][7];
 #pragma unroll
-    for (int u = 0; u < 4; u++)
-      {
-        uint32_t d[7];
-        const Limbs fy = limbs (y[u >> 1][u & 1]);
-        digits (biased (fy, limbs (z[u >> 1][0])), biased (fy, limbs (z[u >> 1][1])), d);
-#pragma unroll
-        for (int q = 0; q < ND; q++) w[q][u] = d[q];
-      }
-    unsigned char *o = stage + chunk_off<ND> (threadIdx.x & 127, c);
+    for (int u = 0; u < 4; u++) digits (v[2 * u], v[2 * u + 1], w[u]);
 #pragma unroll
     for (int q = 0; q < ND; q++)
-      *reinterpret_cast<uint4 *> (o + q * Geo<ND>::A_PLANE)
-        = make_uint4 (w[q][0], w[q][1], w[q][2], w[q][3]);
+      *reinterpret_cast<uint4 *> (stage + G::plane (q) * G::A_PLANE
+                                  + chunk_off (threadIdx.x & 127, (q & 1) * 4 + c))
+        = make_uint4 (w[0][q], w[1][q], w[2][q], w[3][q]);
   }
 };
 
@@ -340,9 +336,9 @@ tma_role (Sync &s, unsigned char *smem, const CUtensorMap *tb, int n0, int k0, i
       if (t >= STAGES
           && !umma::mbar_wait_or_abort (&s.empty[st], ((t / STAGES) - 1) & 1, WAIT_LIMIT, err))
         break;
-      umma::mbar_expect_tx (&s.full[st], ND * G::B_PLANE);
-      umma::tma_load_3d (smem + (size_t) st * G::STAGE + ND * G::A_PLANE, tb,
-                         k0 + Cfg<ND>::KT * t, n0, 0, &s.full[st]);
+      umma::mbar_expect_tx (&s.full[st], G::NP * G::B_PLANE);
+      umma::tma_load_3d (smem + (size_t) st * G::STAGE + G::NP * G::A_PLANE, tb,
+                         G::PAIR * (k0 + Cfg<ND>::KT * t), n0, 0, &s.full[st]);
       issued = t + 1;
     }
   // the last load of each stage must land before the shared memory goes away
@@ -352,23 +348,27 @@ tma_role (Sync &s, unsigned char *smem, const CUtensorMap *tb, int n0, int k0, i
     umma::mbar_wait_or_abort (&s.full[t % STAGES], (t / STAGES) & 1, WAIT_LIMIT, &never);
 }
 
+// TMEM columns of accumulator group g: the even groups first, then the odd
 template <int ND>
-__device__ __forceinline__ uint64_t
-tile_desc (uint32_t a)
+constexpr int
+group_col (int g)
 {
-  return Geo<ND>::ROWB == 64 ? umma::smem_desc_sw64 (a) : umma::smem_desc_sw128 (a);
+  return ((g & 1) * ((ND + 1) / 2) + g / 2) * Cfg<ND>::TN;
 }
 
-// the MMA lane: digit products by group (i + j), accumulator group g in TMEM
-// columns g TN; a new set of accumulators every DK tiles
+// the MMA lane.  The even digits of B lie one after the other as rows of the
+// tile, the odd ones likewise, and so do their groups in TMEM: one MMA of
+// digit i of A with all even (or odd) digits j <= ND - 1 - i of B adds the
+// products to groups i, i + 2, ... at once, with N up to 256.  A new set of
+// accumulators starts every DK tiles.
 template <int ND>
 __device__ __forceinline__ void
 mma_role (Sync &s, const unsigned char *smem, uint32_t tmem, int ntiles, int stall)
 {
   using G = Geo<ND>;
   using C = Cfg<ND>;
+  static_assert (G::PAIR == 2 && (ND + 1) / 2 * C::TN <= 256, "even digits in one MMA");
   volatile int *err = &s.err;
-  const uint32_t idesc = umma::idesc_f16 (TM, C::TN);
   if (stall > 0 && !umma::mbar_wait_or_abort (&s.never, 0, (uint32_t) stall, err)) ntiles = 0;
   for (int t = 0; t < ntiles; t++)
     {
@@ -379,17 +379,23 @@ mma_role (Sync &s, const unsigned char *smem, uint32_t tmem, int ntiles, int sta
         break;
       umma::fence_after_sync ();
       const uint32_t a = umma::smem_u32 (smem) + (uint32_t) st * G::STAGE;
-      const uint32_t b = a + ND * G::A_PLANE;
+      const uint32_t b = a + G::NP * G::A_PLANE;
       const uint32_t first = t % C::DK == 0 ? 1u : 0u;
 #pragma unroll
-      for (int g = 0; g < ND; g++)
+      for (int k = 0; k < C::KT / 16; k++)
 #pragma unroll
-        for (int i = 0; i <= g; i++)
+        for (int i = 0; i < ND; i++)
 #pragma unroll
-          for (int k = 0; k < C::KT / 16; k++)
-            umma::mma_f16 (tmem + (uint32_t) (g * C::TN), tile_desc<ND> (a + i * G::A_PLANE + 32 * k),
-                           tile_desc<ND> (b + (g - i) * G::B_PLANE + 32 * k), idesc,
-                           (first && i == 0 && k == 0) ? 0u : 1u);
+          for (int odd = 0; odd < 2; odd++)
+            {
+              const int nj = (ND - i + 1 - odd) / 2;        // digits j = odd, odd + 2, ...
+              if (nj == 0) continue;
+              umma::mma_f16 (tmem + (uint32_t) group_col<ND> (i + odd),
+                             umma::smem_desc_sw128 (a + G::plane (i) * G::A_PLANE + G::part (i) + 32 * k),
+                             umma::smem_desc_sw128 (b + G::part (odd) + 32 * k),
+                             umma::idesc_f16 (TM, (uint32_t) (nj * C::TN)),
+                             (first && i == 0 && k == 0) ? 0u : 1u);
+            }
       umma::mma_commit (&s.empty[st]);
       if (t % C::DK == C::DK - 1 || t == ntiles - 1) umma::mma_commit (&s.acc_full);
     }
@@ -414,12 +420,12 @@ template <> struct Acc<7> {
   {
     static_assert (CPT == 16, "one TMEM load per group");
     float f[2][16];
-    umma::tmem_ld16_issue (d, f[0]);
+    umma::tmem_ld16_issue (d + group_col<7> (0), f[0]);
 #pragma unroll
     for (int g = 0; g < 7; g++)
       {
         umma::tmem_ld_wait (f[g & 1]);
-        if (g < 6) umma::tmem_ld16_issue (d + (g + 1) * Cfg<7>::TN, f[(g + 1) & 1]);
+        if (g < 6) umma::tmem_ld16_issue (d + group_col<7> (g + 1), f[(g + 1) & 1]);
 #pragma unroll
         for (int u = 0; u < 16; u++)
           {
@@ -600,7 +606,7 @@ k_fix_bwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
     {
       Acc<ND> acc;
       acc.zero ();
-      BuildB<ND> build (p, i0, tb * (C::KT / 4));
+      BuildB<ND> build (p, i0, tb * C::KT);
       if (worker_role<ND> (s, smem, tmem, ntiles, acc, build))
         {
           // the last set is drained, so every build, load and MMA is done and
@@ -680,6 +686,15 @@ k_fix_tables (FixPlan p, const double *pos, const double *x)
       s_u[d][jl] = u;
     }
   __syncthreads ();
+  if (blockIdx.y == 0 && t < TAB_P && jb + t < p.np)
+    {
+      // the coordinates for the real space
+      const unsigned long long ux = s_u[0][t], uy = s_u[1][t], uz = s_u[2][t];
+      p.q[jb + t] = make_uint4 ((unsigned) (ux >> 32), (unsigned) (uy >> 32), (unsigned) (uz >> 32), 0u);
+      ulonglong2 *o = reinterpret_cast<ulonglong2 *> (p.u) + 2 * (size_t) (jb + t);
+      o[0] = make_ulonglong2 (ux, uy);
+      o[1] = make_ulonglong2 (uz, 0ull);
+    }
   const int item = blockIdx.y * TAB_R + t / TAB_P, j = jb + t % TAB_P;
   const int n0 = p.M[0] + 1, n1 = n0 + p.M[1] + 1, n2 = n1 + p.M[2] + 1;
   if (item < n2 && j < p.np)
@@ -700,6 +715,24 @@ k_fix_tables (FixPlan p, const double *pos, const double *x)
       atomicMax (&s_mx[e % p.c], abs_hi (x[(size_t) jb * p.c + e]));
   __syncthreads ();
   if (t < p.c) atomicMax (p.mx + t, s_mx[t]);
+}
+
+// Digit strings of the rows, S[row][particle] = f_y f_z: a thread makes the
+// four rows of a quarter for two particles
+__global__ void __launch_bounds__ (128)
+k_fix_strings (FixPlan p)
+{
+  const int j2 = blockIdx.x * 32 + (threadIdx.x & 31), qd = blockIdx.y * 4 + (threadIdx.x >> 5);
+  const longlong2 *T = (const longlong2 *) p.T;
+  const int4 f = p.quart[qd];
+  const size_t ld = p.ldT / 2;
+  const longlong2 y[2] = {T[f.x * ld + j2], T[f.y * ld + j2]};
+  const longlong2 z[2] = {T[f.z * ld + j2], T[f.w * ld + j2]};
+  longlong2 *o = (longlong2 *) p.S + (size_t) 4 * qd * ld + j2;
+#pragma unroll
+  for (int b = 0; b < 4; b++)
+    o[b * ld] = make_longlong2 (biased (limbs (y[b >> 1].x), limbs (z[b & 1].x)),
+                                biased (limbs (y[b >> 1].y), limbs (z[b & 1].y)));
 }
 
 // Forward image: digits of f_x(j) x_q(j), 64 particles and IMG_M x functions
@@ -733,11 +766,11 @@ k_fix_image (FixPlan p, const double *x)
           digits (biased (limbs (v.x), limbs (s_x[q][8 * j8 + 2 * k])),
                   biased (limbs (v.y), limbs (s_x[q][8 * j8 + 2 * k + 1])), w[k]);
         }
-      uint4 *o = reinterpret_cast<uint4 *> ((__half *) p.ZF + (size_t) (mi * p.c + q) * p.ldT + jb)
-                 + j8;
 #pragma unroll
       for (int d = 0; d < 7; d++)
-        o[(size_t) d * p.ncol * p.ldT / 8] = make_uint4 (w[0][d], w[1][d], w[2][d], w[3][d]);
+        *reinterpret_cast<uint4 *> ((__half *) p.ZF
+                                    + image_off<7> (d, p.ncol, mi * p.c + q, p.ldT, jb + 8 * j8))
+          = make_uint4 (w[0][d], w[1][d], w[2][d], w[3][d]);
     }
 }
 
@@ -854,10 +887,10 @@ k_fix_kop (FixPlan p)
 #pragma unroll
   for (int q = 0; q < C; q++)
     {
-      const R u = (R) unit_of (p.mx[q], p.fu);
+      const uint32_t hw = p.mx[q];
       const long long fc = ia[q], fs = is[q];
-      a[q] = (R) walsh4 (b == 0 ? fc : (b == 3 ? -fc : -fs), b) * u;
-      sn[q] = (R) walsh4 (b == 0 ? fs : (b == 3 ? -fs : fc), b) * u;
+      a[q] = (R) from_fixed (walsh4 (b == 0 ? fc : (b == 3 ? -fc : -fs), b), hw, p.fu);
+      sn[q] = (R) from_fixed (walsh4 (b == 0 ? fs : (b == 3 ? -fs : fc), b), hw, p.fu);
     }
   const FixCoef K = p.coef[(size_t) 4 * (p.off[m1] + (live ? qr : 0)) + b];
   const R e[3] = {(R) K.ex, (R) K.ey, (R) K.ez};
@@ -909,10 +942,10 @@ k_fix_gimage (FixPlan p)
       digits ((finite ? to_fixed (v.x, E, 55) : 0ll) + bias,
               (finite ? to_fixed (v.y, E, 55) : 0ll) + bias, w[k]);
     }
-  uint4 *o = reinterpret_cast<uint4 *> ((__half *) p.WB + (size_t) n * p.Rp) + r8;
 #pragma unroll
   for (int d = 0; d < 7; d++)
-    o[(size_t) d * p.ncol * p.Rp / 8] = make_uint4 (w[0][d], w[1][d], w[2][d], w[3][d]);
+    *reinterpret_cast<uint4 *> ((__half *) p.WB + image_off<7> (d, p.ncol, n, p.Rp, 8 * r8))
+      = make_uint4 (w[0][d], w[1][d], w[2][d], w[3][d]);
 }
 
 template <int ND, int V>
@@ -953,8 +986,10 @@ fix_bytes_F (int, const FixPlan &p)
   return sizeof (long long) * (size_t) p.nsplit * p.ncol * p.Rp;
 }
 size_t fix_bytes_G (int, const FixPlan &p) { return sizeof (double) * (size_t) p.ncol * p.Rp; }
-size_t fix_bytes_ZF (int nd, const FixPlan &p) { return 2 * (size_t) nd * p.ncol * p.ldT; }
-size_t fix_bytes_WB (int nd, const FixPlan &p) { return 2 * (size_t) nd * p.ncol * p.Rp; }
+size_t fix_bytes_S (int, const FixPlan &p) { return sizeof (long long) * (size_t) p.Rp * p.ldT; }
+static size_t image_planes () { return (size_t) Geo<7>::NP * Geo<7>::PAIR; }
+size_t fix_bytes_ZF (int, const FixPlan &p) { return 2 * image_planes () * p.ncol * p.ldT; }
+size_t fix_bytes_WB (int, const FixPlan &p) { return 2 * image_planes () * p.ncol * p.Rp; }
 size_t
 fix_bytes_yp (int, const FixPlan &p)
 {
@@ -1062,10 +1097,11 @@ fix_plan_items (int, FixPlan &p, const std::vector<int> &nqm, std::vector<int4> 
 }
 
 int
-fix_maps (int nd, const FixPlan &p, FixMaps *m)
+fix_maps (int, const FixPlan &p, FixMaps *m)
 {
-  int e = encode_planes_f16 (&m->zf, p.ZF, nd, p.ncol, p.ldT, Cfg<7>::KT, Cfg<7>::TN);
-  if (!e) e = encode_planes_f16 (&m->wb, p.WB, nd, p.ncol, p.Rp, Cfg<7>::KT, Cfg<7>::TN);
+  using G = Geo<7>;
+  int e = encode_planes_f16 (&m->zf, p.ZF, G::NP, p.ncol, (size_t) G::PAIR * p.ldT, Cfg<7>::TN);
+  if (!e) e = encode_planes_f16 (&m->wb, p.WB, G::NP, p.ncol, (size_t) G::PAIR * p.Rp, Cfg<7>::TN);
   return e;
 }
 
@@ -1079,6 +1115,8 @@ launch_fix_tables (int, const FixPlan &p, const double *pos, const double *x, cu
   k_fix_tables<<<dim3 ((p.np + TAB_P - 1) / TAB_P, (items + TAB_R - 1) / TAB_R), TAB_P * TAB_R, 0,
                  st>>> (p, pos, x);
   kmark (prof, st, "k_fix_tables");
+  k_fix_strings<<<dim3 (p.ldT / 64, p.nqp / 4), 128, 0, st>>> (p);
+  kmark (prof, st, "k_fix_strings");
   k_fix_image<<<dim3 (p.ldT / 64, (p.nmi + IMG_M - 1) / IMG_M), 128, 0, st>>> (p, x);
   kmark (prof, st, "k_fix_image");
   return cudaGetLastError ();

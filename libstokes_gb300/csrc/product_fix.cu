@@ -13,6 +13,7 @@
 #include "ewald_device.cuh"
 #include "fixk.h"
 #include "gpu_engine.h"
+#include "real_tab.h"
 #include "seq_graph.h"
 #include "stokes_gpu.h"
 
@@ -26,7 +27,12 @@ struct FixState {
   FixPlan p;
   FixMaps maps;
   double self[3] = {0, 0, 0};
-  DevBuf quart, nqm, coef, off, fitem, bitem, T, F, G, ZF, WB, mx, yp, partial, status;
+  // real space: its radial table and lattice offsets; tabled: false for
+  // splits with too many offsets, which the image-table kernel serves
+  bool tabled = false;
+  RealTabArgs real;
+  DevBuf rtab, roff, rcell, q, u;
+  DevBuf quart, nqm, coef, off, fitem, bitem, S, T, F, G, ZF, WB, mx, yp, partial, status;
   int *h_status = nullptr;
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -224,12 +230,70 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
   };
   // table pads, rows and columns that nothing writes stay zero
   room (f->T, fix_bytes_T (ND, p), true);
+  room (f->S, fix_bytes_S (ND, p), false);
   room (f->F, fix_bytes_F (ND, p), false);
   room (f->G, fix_bytes_G (ND, p), true);
   room (f->ZF, fix_bytes_ZF (ND, p), true);
   room (f->WB, fix_bytes_WB (ND, p), true);
   room (f->yp, fix_bytes_yp (ND, p), false);
   room (f->mx, fix_mx_words (p) * sizeof (unsigned), true);
+  room (f->q, sizeof (uint4) * p.np, false);
+  room (f->u, sizeof (unsigned long long) * 4 * p.np, false);
+  // real space: lattice offsets whose cell of minimum-image displacements
+  // comes within the cutoff, and the radial table
+  RealTabArgs r {};
+  const double rc = sqrt (ts->rmax2);
+  std::vector<float4> roff;
+  std::vector<int4> rcell;
+  {
+    int n[3];
+    for (int d = 0; d < 3; d++) n[d] = std::min (7, (int) ceil (rc / p.l[d] + 0.5));
+    for (int a1 = -n[0]; a1 <= n[0]; a1++)
+      for (int a2 = -n[1]; a2 <= n[1]; a2++)
+        for (int a3 = -n[2]; a3 <= n[2]; a3++)
+          {
+            const int m[3] = {a1, a2, a3};
+            double dd = 0.0;
+            for (int d = 0; d < 3; d++)
+              {
+                const double gap = std::max (0.0, (fabs ((double) m[d]) - 0.5) * p.l[d]);
+                dd += gap * gap;
+              }
+            if (dd > rc * rc * 1.0001) continue;
+            if (!a1 && !a2 && !a3) r.home = (int) roff.size ();
+            roff.push_back (make_float4 ((float) (a1 * p.l[0]), (float) (a2 * p.l[1]),
+                                         (float) (a3 * p.l[2]), 0.f));
+            rcell.push_back (make_int4 (a1, a2, a3, 0));
+          }
+  }
+  r.nimg = (int) roff.size ();
+  f->tabled = r.nimg <= REAL_TAB_MAXIMG && rc <= 7.4 * std::min (p.l[0], std::min (p.l[1], p.l[2]));
+  if (f->tabled)
+    {
+      real_tab_range (rc, &r.bin0, &r.nbin);
+      up (f->roff, roff.data (), sizeof (float4) * roff.size ());
+      up (f->rcell, rcell.data (), sizeof (int4) * rcell.size ());
+      room (f->rtab, real_tab_bytes (sys->version, r.nbin), false);
+      if (e == cudaSuccess)
+        e = launch_real_tab_build (sys->version, r.bin0, r.nbin, ts->xi, (double *) f->rtab.p, st);
+      r.np = p.np;
+      r.off = (const float4 *) f->roff.p;
+      r.cell = (const int4 *) f->rcell.p;
+      for (int d = 0; d < 3; d++)
+        {
+          r.sf[d] = (float) (p.l[d] / 4294967296.0);
+          r.s60[d] = p.l[d] / 1152921504606846976.0;
+        }
+      // FP32 distances are within 1e-6 of the exact ones
+      r.rc2 = (float) (ts->rmax2 * 1.00001);
+      r.xi = ts->xi;
+      r.xisp = ts->xi / sqrt (M_PI);
+      r.xi_ref = sys->xi;
+      r.tab = (const double *) f->rtab.p;
+      r.q = (const uint4 *) f->q.p;
+      r.u = (const unsigned long long *) f->u.p;
+    }
+  f->real = r;
   if (!f->status.p) room (f->status, sizeof (int), true);
   // the uploads read host vectors of this call
   if (e == cudaSuccess) e = cudaStreamSynchronize (st);
@@ -240,8 +304,10 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
   p.coef = (const FixCoef *) f->coef.p;
   p.fitem = (const int4 *) f->fitem.p;
   p.bitem = (const int4 *) f->bitem.p;
-  p.T = f->T.p; p.F = f->F.p; p.G = f->G.p; p.ZF = f->ZF.p; p.WB = f->WB.p;
+  p.T = f->T.p; p.S = f->S.p; p.F = f->F.p; p.G = f->G.p; p.ZF = f->ZF.p; p.WB = f->WB.p;
   p.mx = (unsigned *) f->mx.p;
+  p.q = (uint4 *) f->q.p;
+  p.u = (unsigned long long *) f->u.p;
   p.yp = f->yp.p;
   const int me = fix_maps (ND, p, &f->maps);
   if (me) return set_error (STOKES_GPU_ECUDA, "TMA tensor maps of the FP64 product (%d)", me);
@@ -292,7 +358,7 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
       return set_error (STOKES_GPU_ETIMEOUT,
                         "a tensor-core wait of the previous FP64 product ran out");
     }
-  const int nchunk = real_chunks (np);
+  const int nchunk = f->tabled ? 1 : real_chunks (np);
   cudaError_t e = f->partial.ensure (sizeof (double) * (size_t) nchunk * n);
   if (e != cudaSuccess) return cuda_fail (e, "real-space scratch");
 
@@ -314,6 +380,16 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
   a.xi_ref = c->xi_ref;
   a.xisp_ref = c->xi_ref / sqrt (M_PI);
 
+  RealTabArgs rt = f->real;
+  rt.x = d_x;
+  rt.rmin = c->rmin;
+  rt.rm2 = 4.0 * c->rmin * c->rmin;
+  rt.out = (double *) f->partial.p;
+  auto real_space = [&] (cudaStream_t rs) {
+    return f->tabled ? launch_real_tab (c->version, rt, rs)
+                     : launch_real_fp64 (c->version, MODE_MONO, a, rs);
+  };
+
   cudaEvent_t *E = phase_events (c, timed);
   const bool overlap = (!E || E == c->ev) && !c->kprof_on;
   auto sequence = [&] () -> int {
@@ -321,18 +397,18 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
     cudaError_t e;
     if (E) cudaEventRecord (E[0], st);
     kmark (c, st, nullptr);
-    // the real space needs the positions only; recorded after the forward
-    // GEMM, its CTAs take what that leaves idle
-    if (overlap) cudaEventRecord (f->ev_fork, st);
     if ((e = launch_fix_tables (ND, p, d_pos, d_x, st, c)) != cudaSuccess)
       return cuda_fail (e, "reciprocal tables");
+    // the real space needs the coordinates only; recorded after the forward
+    // GEMM, its CTAs take what that leaves idle
+    if (overlap) cudaEventRecord (f->ev_fork, st);
     if ((e = launch_fix_forward (ND, c->version, p, f->maps, status, st, c)) != cudaSuccess)
       return cuda_fail (e, "reciprocal space (forward)");
     if (overlap)
       {
         cudaStreamWaitEvent (f->side, f->ev_fork, 0);
         if (E) cudaEventRecord (E[1], f->side);
-        e = launch_real_fp64 (c->version, MODE_MONO, a, f->side);
+        e = real_space (f->side);
         if (E) cudaEventRecord (E[2], f->side);
         cudaEventRecord (f->ev_join, f->side);
         if (e != cudaSuccess) return cuda_fail (e, "real-space kernel");
@@ -344,9 +420,9 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
     else
       {
         if (E) cudaEventRecord (E[1], st);
-        if ((e = launch_real_fp64 (c->version, MODE_MONO, a, st)) != cudaSuccess)
+        if ((e = real_space (st)) != cudaSuccess)
           return cuda_fail (e, "real-space kernel");
-        kmark (c, st, "k_real");
+        kmark (c, st, f->tabled ? "k_real_tab" : "k_real");
         if (E) cudaEventRecord (E[2], st);
       }
     FixCombine cb {d_x, (const double *) f->partial.p, (const double *) p.yp, n, p.c, nchunk,
@@ -372,7 +448,7 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
   const bool use = graphs && !c->kprof_on && (E == nullptr || E == c->ev) && p.stall == 0;
   const int rc = run_sequence (f->graph, key, st, E, use, sequence);
   if (rc) return rc;
-  c->launches = 8;
+  c->launches = 9;
   c->timed = timed;
   return STOKES_GPU_OK;
 }
@@ -393,7 +469,7 @@ release_fix (Ctx *c)
 {
   FixState *f = c->fix;
   if (!f) return;
-  for (DevBuf *b : {&f->quart, &f->nqm, &f->coef, &f->off, &f->fitem, &f->bitem, &f->T, &f->F, &f->G, &f->ZF, &f->WB,
+  for (DevBuf *b : {&f->rtab, &f->roff, &f->rcell, &f->q, &f->u, &f->quart, &f->nqm, &f->coef, &f->off, &f->fitem, &f->bitem, &f->S, &f->T, &f->F, &f->G, &f->ZF, &f->WB,
                     &f->mx, &f->yp, &f->partial, &f->status})
     b->release ();
   f->graph.release ();

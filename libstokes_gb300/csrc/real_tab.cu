@@ -1,0 +1,434 @@
+// real_tab.cu -- FP64 real-space pair sum of equal spheres from a table of
+// its radial functions.
+//
+// The sum is bound by the FP64 pipe (about two lanes a clock and SM), so what
+// counts is the FP64 instructions of a pair term.  Evaluated from the closed
+// forms an FTS term takes about 970 of them: a square root, a division, erfc,
+// exp, eleven scalars and the pair tensors.  Written in the plain
+// displacement d instead of the unit vector, every coefficient is a smooth
+// function of s = d.d alone (no square root, no division), and tracelessness
+// leaves 2 (F), 5 (FT) or 10 (FTS) independent ones:
+//
+//   U = ya F + a2 (d.F) d + yb T x d - (g1 tr S + g3 dSd) d - 2 g2 S d
+//   W = yb F x d + yc T + c2 (d.T) d - 2 c2 d x (S d)
+//   E = (g1 d.F + m2 dSd + m3 tr S) I + (g3 d.F + m1 dSd + m2 tr S) d d
+//       + d V + V d + zm S,     V = g2 F - c2 T x d + m4 S d
+//   g1 = -(g3 s + 2 g2) / 3,  m2 = -(m1 s + 2 m4) / 3,  m3 = -(m2 s + zm) / 3
+//
+// (S the full contraction S' of ewald_device.cuh; its yh equals yc - xc).
+// Each is a polynomial of degree 7 in s - s_mid per bin, RT_BINS bins per
+// octave of s: 7 FMAs a function, about 200 FP64 instructions an FTS term.
+// The bin and its midpoint come from the bits of s.  The truncation of such a
+// bin is below 2^-53 of the function for powers s^-5.5 (bin half width over s
+// at most 1/128: 2^-56 times 2^10 for the binomial and 2^-7 for Chebyshev
+// nodes); the table is made on the device from the closed forms, with the
+// change of basis in double-double.
+//
+// Positions are the 64-bit fixed-point fractional coordinates of the
+// reciprocal sum, so the minimum image is the integer overflow and a
+// displacement carries one rounding, however close the pair; the conversion
+// to FP64 is done in integers.
+#include <cuda_runtime.h>
+
+#include <cmath>
+#include <vector>
+
+#include "ewald_device.cuh"
+#include "real_tab.h"
+
+namespace lsg {
+namespace {
+
+constexpr int RT_LOG = 6;                     // log2 of the bins per octave
+constexpr int RT_DEG = 8;                     // coefficients per function
+constexpr int RT_T = 128;                     // threads per CTA: one target
+constexpr int RT_W = RT_T / 32;               // warps
+constexpr int RT_SEG = 1024;                  // accepted pairs a warp lists at a time
+static_assert (32 * REAL_TAB_MAXIMG <= RT_SEG, "32 sources with every offset fit a list");
+
+template <int V> struct NFun;
+template <> struct NFun<0> { static constexpr int value = 2; };
+template <> struct NFun<1> { static constexpr int value = 5; };
+template <> struct NFun<2> { static constexpr int value = 10; };
+
+// the independent coefficients at distance r, s = r^2
+template <int V>
+__device__ __forceinline__ void
+radial (double xi, double xisp, double r, double s, double *f)
+{
+  PairScalars<double> c;
+  real_scalars_mono<V, double> (xi, xisp, r, c);
+  f[0] = c.ya;
+  f[1] = (c.xa - c.ya) / s;
+  if (V == V_F) return;
+  f[2] = c.yb / r;
+  f[3] = c.yc;
+  f[4] = (c.xc - c.yc) / s;
+  if (V == V_FT) return;
+  f[5] = c.yg / r;                                            // g2
+  f[6] = (c.xg - 2.0 * c.yg) / (r * s);                       // g3
+  f[7] = (1.5 * c.xm - 2.0 * c.ym + 0.5 * c.zm) / (s * s);    // m1
+  f[8] = (c.ym - c.zm) / s;                                   // m4
+  f[9] = c.zm;
+}
+
+__device__ __forceinline__ double
+bin_mid (int bin)
+{
+  return __hiloint2double ((bin << (20 - RT_LOG)) | (1 << (19 - RT_LOG)), 0);
+}
+
+// coefficients of one bin: values at the Chebyshev nodes, then the monomial
+// coefficients c_k = sum_n B[k][n] f(node n) / h^k by compensated sums
+struct Basis {
+  double hi[RT_DEG][RT_DEG], lo[RT_DEG][RT_DEG];
+  double node[RT_DEG];
+};
+
+template <int V>
+__global__ void __launch_bounds__ (RT_DEG * NFun<V>::value)
+k_rt_table (Basis b, int bin0, double xi, double xisp, double *tab)
+{
+  constexpr int NF = NFun<V>::value;
+  __shared__ double s_f[RT_DEG][NF];
+  const int bin = bin0 + blockIdx.x, t = threadIdx.x;
+  const double mid = bin_mid (bin);
+  // half the bin: 2^(exponent - RT_LOG - 1)
+  const double h = __hiloint2double (((bin >> RT_LOG) - RT_LOG - 1) << 20, 0);
+  if (t < RT_DEG)
+    {
+      const double s = fma (h, b.node[t], mid);
+      double f[NF];
+      radial<V> (xi, xisp, sqrt (s), s, f);
+      for (int q = 0; q < NF; q++) s_f[t][q] = f[q];
+    }
+  __syncthreads ();
+  const int q = t / RT_DEG, k = t % RT_DEG;
+  double sum = 0.0, err = 0.0;
+  for (int n = 0; n < RT_DEG; n++)
+    {
+      const double f = s_f[n][q], p = b.hi[k][n] * f, pe = fma (b.hi[k][n], f, -p);
+      const double v = sum + p, bb = v - sum;
+      err += (sum - (v - bb)) + (p - bb) + pe + b.lo[k][n] * f;
+      sum = v;
+    }
+  double c = sum + err;
+  for (int n = 0; n < k; n++) c /= h;                   // h is a power of two
+  tab[((size_t) blockIdx.x * NF + q) * RT_DEG + k] = c;
+}
+
+// y += M x_j of one pair at displacement d, s = d.d, coefficients f
+template <int V>
+__device__ __forceinline__ void
+apply (const double d[3], double s, const double *f, const double *__restrict__ x, double *y)
+{
+  const double F0 = x[0], F1 = x[1], F2 = x[2];
+  const double dF = d[0] * F0 + d[1] * F1 + d[2] * F2;
+  double along = f[1] * dF;
+  if (V == V_F)
+    {
+      y[0] += fma (f[0], F0, along * d[0]);
+      y[1] += fma (f[0], F1, along * d[1]);
+      y[2] += fma (f[0], F2, along * d[2]);
+      return;
+    }
+  const double T0 = x[3], T1 = x[4], T2 = x[5];
+  const double t0 = T1 * d[2] - T2 * d[1], t1 = T2 * d[0] - T0 * d[2], t2 = T0 * d[1] - T1 * d[0];
+  const double f0 = F1 * d[2] - F2 * d[1], f1 = F2 * d[0] - F0 * d[2], f2 = F0 * d[1] - F1 * d[0];
+  const double w = f[4] * (d[0] * T0 + d[1] * T1 + d[2] * T2);
+  y[3] = fma (w, d[0], fma (f[3], T0, fma (f[2], f0, y[3])));
+  y[4] = fma (w, d[1], fma (f[3], T1, fma (f[2], f1, y[4])));
+  y[5] = fma (w, d[2], fma (f[3], T2, fma (f[2], f2, y[5])));
+  if (V == V_FT)
+    {
+      y[0] = fma (along, d[0], fma (f[0], F0, fma (f[2], t0, y[0])));
+      y[1] = fma (along, d[1], fma (f[0], F1, fma (f[2], t1, y[1])));
+      y[2] = fma (along, d[2], fma (f[0], F2, fma (f[2], t2, y[2])));
+      return;
+    }
+  const double sxx = x[6], sxy = x[7], sxz = x[8], syz = x[9], syy = x[10];
+  const double Sxx = fma (2.0, sxx, syy), Syy = fma (2.0, syy, sxx);
+  const double s0 = Sxx * d[0] + sxy * d[1] + sxz * d[2];
+  const double s1 = sxy * d[0] + Syy * d[1] + syz * d[2];
+  const double s2 = sxz * d[0] + syz * d[1];
+  const double ss = d[0] * s0 + d[1] * s1 + d[2] * s2, tr = Sxx + Syy;
+  const double third = -1.0 / 3.0, g2 = f[5], g3 = f[6], m1 = f[7], m4 = f[8], zm = f[9];
+  const double g1 = fma (g3, s, 2.0 * g2) * third;
+  const double m2 = fma (m1, s, 2.0 * m4) * third;
+  const double m3 = fma (m2, s, zm) * third;
+  along = fma (-g1, tr, fma (-g3, ss, along));
+  const double n2 = -2.0 * g2, nc = -f[4];
+  y[0] = fma (along, d[0], fma (f[0], F0, fma (f[2], t0, fma (n2, s0, y[0]))));
+  y[1] = fma (along, d[1], fma (f[0], F1, fma (f[2], t1, fma (n2, s1, y[1]))));
+  y[2] = fma (along, d[2], fma (f[0], F2, fma (f[2], t2, fma (n2, s2, y[2]))));
+  const double h2 = 2.0 * nc;
+  y[3] = fma (h2, d[1] * s2 - d[2] * s1, y[3]);
+  y[4] = fma (h2, d[2] * s0 - d[0] * s2, y[4]);
+  y[5] = fma (h2, d[0] * s1 - d[1] * s0, y[5]);
+  const double v0 = fma (g2, F0, fma (nc, t0, m4 * s0));
+  const double v1 = fma (g2, F1, fma (nc, t1, m4 * s1));
+  const double v2 = fma (g2, F2, fma (nc, t2, m4 * s2));
+  const double dE = fma (g1, dF, fma (m2, ss, m3 * tr));
+  const double ee = fma (g3, dF, fma (m1, ss, m2 * tr));
+  // ee d d + d V + V d = d (V + ee d / 2) + (V + ee d / 2) d
+  const double he = 0.5 * ee;
+  const double w0 = fma (he, d[0], v0), w1 = fma (he, d[1], v1), w2 = fma (he, d[2], v2);
+  y[6] += fma (2.0 * d[0], w0, fma (zm, Sxx, dE));
+  y[7] = fma (d[0], w1, fma (d[1], w0, fma (zm, sxy, y[7])));
+  y[8] = fma (d[0], w2, fma (d[2], w0, fma (zm, sxz, y[8])));
+  y[9] = fma (d[1], w2, fma (d[2], w1, fma (zm, syz, y[9])));
+  y[10] += fma (2.0 * d[1], w1, fma (zm, Syy, dE));
+}
+
+// pairs the table does not serve: nearer than its first bin, or under the
+// rmin clamp (r raised to rm and e = d / r with the raised r,
+// src/ewald.c:693-699).  At a split other than the struct's own a clamped
+// pair contributes T(d / rm; s_ref(rm)) + T(d / r; s_xi(r) - s_ref(r)), the
+// change of the clamp at the struct's split.
+template <int V>
+__device__ __noinline__ void
+near_term (const RealTabArgs &a, double d0, double d1, double d2, double s, const double *x,
+           double *z)
+{
+  const double d[3] = {d0, d1, d2};
+  const double r = sqrt (s), rm = 2.0 * a.rmin;
+  GenF<V, double> g;
+  load_genf<V, double> (x, g);
+  GenU<V, double> u;
+  u.zero ();
+  PairScalars<double> c;
+  const double e[3] = {d[0] / r, d[1] / r, d[2] / r};
+  if (r < rm)
+    {
+      const double ec[3] = {d[0] / rm, d[1] / rm, d[2] / rm};
+      real_scalars_mono<V, double> (a.xi_ref, a.xi_ref * 0.56418958354775628, rm, c);
+      pair_apply<V, double> (ec, c, g, u);
+      split_diff<V, double> (a.xi_ref, a.xi, r, c);
+    }
+  else
+    real_scalars_mono<V, double> (a.xi, a.xisp, r, c);
+  pair_apply<V, double> (e, c, g, u);
+#pragma unroll
+  for (int q = 0; q < NComp<V>::value; q++) z[q] = u.v[q];
+}
+
+// v[0 .. P) summed over the warp, P a power of two <= 16: lane l ends up with
+// the sum of element l / (32 / P).  P - 1 + 5 - log2 P additions instead of
+// 5 P.
+template <int P>
+__device__ __forceinline__ double
+warp_sums (double (&v)[P], int lane)
+{
+  int o = 16;
+#pragma unroll
+  for (int n = P / 2; n >= 1; n >>= 1, o >>= 1)
+#pragma unroll
+    for (int k = 0; k < n; k++)
+      {
+        const bool up = lane & o;
+        const double keep = up ? v[k + n] : v[k], send = up ? v[k] : v[k + n];
+        v[k] = keep + __shfl_xor_sync (0xffffffffu, send, o);
+      }
+  for (; o >= 1; o >>= 1) v[0] += __shfl_xor_sync (0xffffffffu, v[0], o);
+  return v[0];
+}
+
+// One CTA per target.  Its threads test the sources (times the lattice
+// offsets of a cutoff beyond half the box) in FP32 on the upper 32 bits of
+// the fixed-point coordinates and list the accepted ones in shared memory (a
+// segment per warp, so that the order and with it the sum is reproducible);
+// then the warps take the entries of all segments 32 at a time, so that the
+// FP64 pipe only sees accepted pairs and at most one partly filled warp per
+// target and round.
+template <int V>
+__global__ void __launch_bounds__ (RT_T)
+k_real_tab (RealTabArgs a)
+{
+  constexpr int C = NComp<V>::value, NF = NFun<V>::value;
+  constexpr int P = C <= 4 ? 4 : (C <= 8 ? 8 : 16);
+  __shared__ unsigned s_list[RT_W][RT_SEG];             // source | offset << 24
+  __shared__ int s_n[RT_W];
+  __shared__ double s_y[RT_W][P];
+  const int i = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint4 qi = a.q[i];
+  const ulonglong2 ua = reinterpret_cast<const ulonglong2 *> (a.u)[2 * i];
+  const unsigned long long uz = a.u[4 * (size_t) i + 2];
+  double y[P];
+#pragma unroll
+  for (int q = 0; q < P; q++) y[q] = 0.0;
+  // sources per warp and round: all of them times the offsets fit its segment
+  const int per = RT_SEG / a.nimg / 32 * 32;
+  for (int b0 = 0; b0 < a.np; b0 += RT_W * per)
+    {
+      const int j1 = min (a.np, b0 + (warp + 1) * per);
+      int cnt = 0;
+      for (int jb = b0 + warp * per; jb < j1; jb += 32)
+        {
+          const int j = jb + lane;
+          float x0 = 0.f, x1 = 0.f, x2 = 0.f;
+          if (j < j1)
+            {
+              const uint4 qj = a.q[j];
+              x0 = (float) (int) (qj.x - qi.x) * a.sf[0];
+              x1 = (float) (int) (qj.y - qi.y) * a.sf[1];
+              x2 = (float) (int) (qj.z - qi.z) * a.sf[2];
+            }
+          for (int m = 0; m < a.nimg; m++)
+            {
+              const float4 T = a.nimg > 1 ? a.off[m] : make_float4 (0.f, 0.f, 0.f, 0.f);
+              const float dx = x0 + T.x, dy = x1 + T.y, dz = x2 + T.z;
+              const bool ok = j < j1 && (j != i || m != a.home)
+                              && dx * dx + dy * dy + dz * dz < a.rc2;
+              const unsigned got = __ballot_sync (0xffffffffu, ok);
+              if (ok)
+                s_list[warp][cnt + __popc (got & ((1u << lane) - 1u))]
+                  = (unsigned) (j - b0) | (unsigned) m << 24;
+              cnt += __popc (got);
+            }
+        }
+      if (lane == 0) s_n[warp] = cnt;
+      __syncthreads ();
+      int n = 0;
+#pragma unroll
+      for (int w = 0; w < RT_W; w++) n += s_n[w];
+      for (int k = t; k < n; k += RT_T)
+        {
+          int w = 0, at = k;
+          while (at >= s_n[w]) at -= s_n[w++];
+          const unsigned en = s_list[w][at];
+          const int j = b0 + (int) (en & 0xffffffu), m = (int) (en >> 24);
+          const ulonglong2 ub = reinterpret_cast<const ulonglong2 *> (a.u)[2 * (size_t) j];
+          const unsigned long long vz = a.u[4 * (size_t) j + 2];
+          int4 o = make_int4 (0, 0, 0, 0);
+          if (a.nimg > 1) o = a.cell[m];
+          // displacement in units of 2^-60 of the box
+          double d[3];
+          d[0] = int_to_double (((long long) (ub.x - ua.x) >> 4) + ((long long) o.x << 60)) * a.s60[0];
+          d[1] = int_to_double (((long long) (ub.y - ua.y) >> 4) + ((long long) o.y << 60)) * a.s60[1];
+          d[2] = int_to_double (((long long) (vz - uz) >> 4) + ((long long) o.z << 60)) * a.s60[2];
+          const double s = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+          const double *x = a.x + (size_t) C * j;
+          const int bin = (__double2hiint (s) >> (20 - RT_LOG)) - a.bin0;
+          if (bin < 0 || s < a.rm2)
+            {
+              // coincident points of distinct particles count as no pair
+              if (s > 0.0)
+                {
+                  double v[C];
+                  near_term<V> (a, d[0], d[1], d[2], s, x, v);
+#pragma unroll
+                  for (int q = 0; q < C; q++) y[q] += v[q];
+                }
+              continue;
+            }
+          const double z = s - bin_mid (bin + a.bin0);
+          const double2 *c = reinterpret_cast<const double2 *> (a.tab)
+                             + (size_t) min (bin, a.nbin - 1) * (NF * RT_DEG / 2);
+          double f[NF];
+#pragma unroll
+          for (int q = 0; q < NF; q++)
+            {
+              const double2 c3 = __ldg (c + 4 * q + 3), c2 = __ldg (c + 4 * q + 2),
+                            c1 = __ldg (c + 4 * q + 1), c0 = __ldg (c + 4 * q);
+              f[q] = fma (fma (fma (fma (fma (fma (fma (c3.y, z, c3.x), z, c2.y), z, c2.x), z, c1.y),
+                                    z, c1.x), z, c0.y), z, c0.x);
+            }
+          apply<V> (d, s, f, x, y);
+        }
+      __syncthreads ();
+    }
+  const double v = warp_sums<P> (y, lane);
+  if (lane % (32 / P) == 0) s_y[warp][lane / (32 / P)] = v;
+  __syncthreads ();
+  if (t < C)
+    {
+      double r = s_y[0][t];
+#pragma unroll
+      for (int w = 1; w < RT_W; w++) r += s_y[w][t];
+      a.out[(size_t) i * C + t] = r;
+    }
+}
+
+// inverse of the Vandermonde matrix of the Chebyshev nodes, as hi + lo pairs
+const Basis &
+basis ()
+{
+  static const Basis b = [] {
+    Basis r;
+    long double x[RT_DEG];
+    const long double pi = 3.14159265358979323846264338327950288L;
+    for (int n = 0; n < RT_DEG; n++)
+      {
+        r.node[n] = (double) cosl (pi * (2 * n + 1) / (2 * RT_DEG));
+        x[n] = r.node[n];                       // the nodes as they are used
+      }
+    for (int n = 0; n < RT_DEG; n++)
+      {
+        // Lagrange polynomial of node n: product of (x - x_m) / (x_n - x_m)
+        long double c[RT_DEG] = {1.0L};
+        int deg = 0;
+        for (int m = 0; m < RT_DEG; m++)
+          {
+            if (m == n) continue;
+            const long double w = 1.0L / (x[n] - x[m]);
+            deg++;
+            for (int k = deg; k >= 0; k--)
+              c[k] = ((k ? c[k - 1] : 0.0L) - (k < deg ? c[k] * x[m] : 0.0L)) * w;
+          }
+        for (int k = 0; k < RT_DEG; k++)
+          {
+            r.hi[k][n] = (double) c[k];
+            r.lo[k][n] = (double) (c[k] - (long double) r.hi[k][n]);
+          }
+      }
+    return r;
+  }();
+  return b;
+}
+
+int
+bin_of (double s)
+{
+  long long bits;
+  static_assert (sizeof bits == sizeof s, "");
+  __builtin_memcpy (&bits, &s, sizeof s);
+  return (int) (bits >> (52 - RT_LOG));
+}
+
+}  // namespace
+
+// the table covers r from 1 (half of contact) to a little past the cutoff
+void
+real_tab_range (double rc, int *bin0, int *nbin)
+{
+  *bin0 = bin_of (1.0);
+  *nbin = std::max (1, bin_of (std::max (1.0, rc * rc * 1.0001)) - *bin0 + 1);
+}
+
+size_t
+real_tab_bytes (int version, int nbin)
+{
+  const int nf = version == 0 ? 2 : (version == 1 ? 5 : 10);
+  return sizeof (double) * (size_t) nbin * nf * RT_DEG;
+}
+
+cudaError_t
+launch_real_tab_build (int version, int bin0, int nbin, double xi, double *tab, cudaStream_t st)
+{
+  const double xisp = xi / sqrt (M_PI);
+  if (version == 0) k_rt_table<0><<<nbin, RT_DEG * 2, 0, st>>> (basis (), bin0, xi, xisp, tab);
+  else if (version == 1) k_rt_table<1><<<nbin, RT_DEG * 5, 0, st>>> (basis (), bin0, xi, xisp, tab);
+  else k_rt_table<2><<<nbin, RT_DEG * 10, 0, st>>> (basis (), bin0, xi, xisp, tab);
+  return cudaGetLastError ();
+}
+
+cudaError_t
+launch_real_tab (int version, const RealTabArgs &a, cudaStream_t st)
+{
+  if (version == 0) k_real_tab<0><<<a.np, RT_T, 0, st>>> (a);
+  else if (version == 1) k_real_tab<1><<<a.np, RT_T, 0, st>>> (a);
+  else k_real_tab<2><<<a.np, RT_T, 0, st>>> (a);
+  return cudaGetLastError ();
+}
+
+}  // namespace lsg

@@ -68,21 +68,6 @@ idesc_tf32 (uint32_t M, uint32_t N)
     | ((M >> 4) << 24);       // M / 16
 }
 
-// the same for a 64-byte swizzled tile: rows of 64 bytes (32 f16 values),
-// 8-row groups 512 bytes apart, the four 16-byte chunks of row r permuted by
-// (r / 2) % 4
-__device__ __forceinline__ uint64_t
-smem_desc_sw64 (uint32_t saddr)
-{
-  uint64_t d = 0;
-  d |= (uint64_t) ((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t) 1u << 16;                 // LBO (ignored): 16 bytes
-  d |= (uint64_t) (512u >> 4) << 32;        // SBO: 512 bytes
-  d |= (uint64_t) 1u << 46;                 // descriptor version
-  d |= (uint64_t) 4u << 61;                 // layout: 64-byte swizzle
-  return d;
-}
-
 // instruction descriptor, kind::f16: D f32, A/B f16, both K-major
 __host__ __device__ __forceinline__ uint32_t
 idesc_f16 (uint32_t M, uint32_t N)

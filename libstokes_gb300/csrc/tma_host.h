@@ -71,27 +71,25 @@ encode_rows_plain (CUtensorMap *map, const float *base, unsigned long long rows,
   return r == CUDA_SUCCESS ? 0 : (int) r;
 }
 
-// A [planes][rows][cols] f16 array, row-major, cols a multiple of 8, as a
-// 3-d tensor map whose box is {box_cols, box_rows, planes} (every plane of a
-// tile in one load), rows of 64 or 128 bytes in the swizzled layout of that
-// width; reads outside [rows] x [cols] fill zeros.  0 on success.
+// A [planes][rows][cols] f16 array, row-major, cols a multiple of 64, as a
+// 3-d tensor map whose box is {64 columns (128 bytes), box_rows, planes}
+// (every plane of a tile in one load) in the 128-byte swizzled layout; reads
+// outside [rows] x [cols] fill zeros.  0 on success.
 inline int
 encode_planes_f16 (CUtensorMap *map, const void *base, unsigned long long planes,
-                   unsigned long long rows, unsigned long long cols, unsigned box_cols,
-                   unsigned box_rows)
+                   unsigned long long rows, unsigned long long cols, unsigned box_rows)
 {
   EncodeTiledFn fn = encode_fn ();
   if (!fn) return -1;
-  if (cols % 8 || ((unsigned long long) base & 15ull) || box_rows == 0 || box_rows > 256
-      || (box_cols != 32 && box_cols != 64) || planes == 0 || planes > 256)
+  if (cols % 64 || ((unsigned long long) base & 15ull) || box_rows == 0 || box_rows > 256
+      || planes == 0 || planes > 256)
     return -2;
   const cuuint64_t dims[3] = {cols, rows, planes};
   const cuuint64_t strides[2] = {cols * 2ull, rows * cols * 2ull};
-  const cuuint32_t box[3] = {box_cols, box_rows, (cuuint32_t) planes};
+  const cuuint32_t box[3] = {64u, box_rows, (cuuint32_t) planes};
   const cuuint32_t estr[3] = {1u, 1u, 1u};
   const CUresult r = fn (map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void *) base, dims, strides, box,
-                         estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                         estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : (int) r;
 }

@@ -49,13 +49,18 @@ def test_tile_edges(lib, version, n, side):
 
 @pytest.mark.parametrize("version", [0, 2])
 @pytest.mark.parametrize("box", [(14.0, 19.0, 27.0), (30.0, 12.0, 12.0), (11.0, 13.0, 31.0)])
-def test_boxes(lib, version, box):
+def test_boxes_and_unwrapped_positions(lib, version, box):
     rng = np.random.default_rng(7)
     n = 70
     pos = _positions(n, box, rng)
     x = rng.standard_normal((3, 11)[version // 2] * n)
     y, yo = _both(version, pos, box, x)
     assert rel_l2(y, yo) < 1e-12
+    # whole-box shifts of single particles leave the periodic sum as it is
+    from libstokes_gb300 import System
+    s = System(version, pos + np.asarray(box) * rng.integers(-3, 4, (n, 3)), box)
+    assert rel_l2(s.atimes(x), yo) < 1e-12
+    s.close()
 
 
 @pytest.mark.parametrize("scale", [1e-250, 1e-30, 1.0, 1e30, 1e250])
