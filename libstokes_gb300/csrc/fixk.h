@@ -48,6 +48,8 @@ struct FixPlan {
   void *T = nullptr;          // function table [nT][ldT]
   uint4 *q = nullptr;         // [np] fractional coordinates, upper 32 bits
   unsigned long long *u = nullptr;   // [np][4] the same, 64 bits
+  float *xf = nullptr;        // [np][XF_LD] x / 2^xtop in FP32
+  int *xtop = nullptr;
   void *S = nullptr;          // digit strings [Rp][ldT]
   void *F = nullptr;          // structure factors [nsplit][ncol][Rp], int64
   void *G = nullptr;          // operator output [ncol][Rp]
@@ -60,6 +62,8 @@ struct FixPlan {
   const int4 *bitem = nullptr;     // backward: column tile, first K tile, K tiles
   void *yp = nullptr;         // back-projection partials [nbitem][np][c]
 };
+
+constexpr int XF_LD = 12;     // floats per particle of xf
 
 struct FixMaps {
   CUtensorMap zf, wb;

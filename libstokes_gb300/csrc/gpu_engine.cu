@@ -337,8 +337,8 @@ upload_if_changed (DevBuf &buf, uint64_t &fp, const void *host, size_t bytes,
 // (LIBSTOKES_GB300_FP64_ETA sets eta, 0 keeps the reference's split), set up
 // by the reference's own rules on a private copy of the system.  Equal spheres
 // take the fixed-point tensor-core reciprocal sum (product_fix.cu), so eta is
-// high: 12, at most xi = 0.7.  FTS N = 1000, phi 0.3, one GB300: 9.6 ms at eta
-// 6 with the SIMT sums, 1.6 ms now (real space 1.3 ms, GEMMs 110 + 121 us).
+// high (tuned_eta).  FTS N = 1000, phi 0.3, one GB300: 9.6 ms at eta 6 with
+// the SIMT sums, 0.42 ms now (real space 197 us, GEMMs 68 + 82 us).
 // Unequal spheres keep the SIMT sums: eta 6 up to 1024 particles, 8 up to
 // 4096, 10 above.  The sum is split-invariant to rounding
 // (measured 5e-15 to 8e-15 against the reference's split) -- except under
@@ -365,10 +365,15 @@ tuned_eta (const struct stokes *sys)
   const int np = sys->np;
   if (sys->a == nullptr)
     {
-      // xi up to 0.7 (or eta 6 in a very small box): beyond, the self, real
-      // and reciprocal parts grow against their sum and cost digits
+      // real pairs grow as N^2 / eta^3, reciprocal work as N eta^3, so the two
+      // balance at an eta proportional to N^(1/6).  Measured on one GB300, best
+      // eta of 8-20: F 10, 11, 14, 18 at N = 300, 1000, 4096, 16000; FT 9, 11,
+      // 13, 15 at 300, 1000, 2048, 4096; FTS 10, 12, 14, 18 at 300, 1000,
+      // 2500, 8000.  xi up to 0.7 (or eta 6 in a very small box): beyond, the
+      // self, real and reciprocal parts grow against their sum and cost digits.
       const double l = cbrt (sys->lx * sys->ly * sys->lz);
-      return std::min (12.0, std::max (6.0, 0.7 * l));
+      const double eta = (sys->version == 2 ? 12.0 : 11.5) * pow (np / 1000.0, 1.0 / 6.0);
+      return std::max (6.0, std::min (eta, 0.7 * l));
     }
   return np <= 1024 ? 6.0 : (np <= 4096 ? 8.0 : 10.0);
 }
@@ -424,7 +429,11 @@ tuned_applies (const Ctx *c, const struct stokes *sys, bool cube)
 static const struct stokes *
 tuned_system (Ctx *c, const struct stokes *sys)
 {
-  const double eps = sys->ewald_eps > 0.0 ? sys->ewald_eps : 1e-12;
+  double eps = sys->ewald_eps > 0.0 ? sys->ewald_eps : 1e-12;
+  // FTS: the cutoff rule estimates the force term; the stresslet terms fall
+  // off later.  At a third of the tolerance the error against long double is
+  // 1.1e-15 instead of 2.3e-15 (N = 200, phi 0.3) for 0.5% more time.
+  if (sys->version == 2 && sys->a == nullptr) eps *= 0.3;
   const double eta = tuned_eta (sys);
   const double key[7] = {sys->lx, sys->ly, sys->lz, (double) sys->np, (double) sys->version,
                          eta, eps};

@@ -752,6 +752,29 @@ k_fix_image (FixPlan p, const double *x)
       s_x[q][jl] = jb + jl < p.np && finite ? to_fixed (x[(size_t) jb * p.c + e], E, 62) : 0ll;
     }
   __syncthreads ();
+  if (blockIdx.y == 0)
+    {
+      // FP32 copy for the far pairs of the real space, in units of the largest
+      // component (components that are not finite: their couplings are not,
+      // already from the reciprocal part)
+      int top = -2000;
+      for (int q = 0; q < p.c; q++)
+        {
+          bool finite;
+          const int E = scale_exp (p.mx[q], finite);
+          if (finite) top = max (top, E);
+        }
+      for (int e = t; e < 64 * p.c; e += 128)
+        {
+          const int jl = e / p.c, q = e - jl * p.c;
+          bool finite;
+          scale_exp (p.mx[q], finite);
+          if (jb + jl < p.np)
+            p.xf[(size_t) (jb + jl) * XF_LD + q]
+              = finite ? (float) scalbn (x[(size_t) jb * p.c + e], -top) : 0.f;
+        }
+      if (t == 0 && blockIdx.x == 0) *p.xtop = top;
+    }
   const long long *T = (const long long *) p.T;
   for (int e = t; e < IMG_M * p.c * 8; e += 128)
     {
@@ -777,14 +800,22 @@ k_fix_image (FixPlan p, const double *x)
 // Operators: four lanes per octant point, lane b = 2 p2 + p3 holding row b of
 // the quarter; after the transform lane sigma holds the sign pattern
 // (s2, s3) = (1 - 2 (sigma >> 1), 1 - 2 (sigma & 1)).
+// (a sign change, not a second FP64 instruction: v or -v for bit = 0, 1)
+__device__ __forceinline__ double
+flip (double v, int bit)
+{
+  return __hiloint2double (__double2hiint (v) ^ (int) ((unsigned) bit << 31), __double2loint (v));
+}
+__device__ __forceinline__ long long flip (long long v, int bit) { return bit ? -v : v; }
+
 template <typename R>
 __device__ __forceinline__ R
 walsh4 (R v, int b)
 {
   const R o = __shfl_xor_sync (0xffffffffu, v, 1);
-  v = (b & 1) ? o - v : v + o;
+  v = o + flip (v, b & 1);
   const R q = __shfl_xor_sync (0xffffffffu, v, 2);
-  return (b & 2) ? q - v : v + q;
+  return q + flip (v, b >> 1);
 }
 
 // The transverse parts of a generalised force v at direction e: F, T x e and
@@ -855,7 +886,8 @@ couple (const R e[3], const FixCoef &K, R sg, const Trans<V, R> &c, const Trans<
   y[10] = R (2) * e[1] * v[1];
 }
 
-constexpr int KOP_T = 64;               // threads per CTA: 16 octant points
+constexpr int KOP_T = 32;               // threads per CTA: 8 octant points (FP64-bound: small CTAs
+                                        // even out the SMs)
 
 template <int ND, int V>
 __global__ void __launch_bounds__ (KOP_T)

@@ -31,7 +31,7 @@ struct FixState {
   // splits with too many offsets, which the image-table kernel serves
   bool tabled = false;
   RealTabArgs real;
-  DevBuf rtab, roff, rcell, q, u;
+  DevBuf rtab, roff, rcell, q, u, xf, xtop;
   DevBuf quart, nqm, coef, off, fitem, bitem, S, T, F, G, ZF, WB, mx, yp, partial, status;
   int *h_status = nullptr;
   cudaStream_t side = nullptr;
@@ -239,6 +239,8 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
   room (f->mx, fix_mx_words (p) * sizeof (unsigned), true);
   room (f->q, sizeof (uint4) * p.np, false);
   room (f->u, sizeof (unsigned long long) * 4 * p.np, false);
+  room (f->xf, sizeof (float) * XF_LD * p.np, false);
+  room (f->xtop, sizeof (int), false);
   // real space: lattice offsets whose cell of minimum-image displacements
   // comes within the cutoff, and the radial table
   RealTabArgs r {};
@@ -275,7 +277,12 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
       up (f->rcell, rcell.data (), sizeof (int4) * rcell.size ());
       room (f->rtab, real_tab_bytes (sys->version, r.nbin), false);
       if (e == cudaSuccess)
-        e = launch_real_tab_build (sys->version, r.bin0, r.nbin, ts->xi, (double *) f->rtab.p, st);
+        {
+          r.tab = (const double *) f->rtab.p;
+          r.tabf = (const float *) (r.tab + real_tab_doubles (sys->version, r.nbin));
+          e = launch_real_tab_build (sys->version, r.bin0, r.nbin, ts->xi, (double *) r.tab,
+                                     (float *) r.tabf, st);
+        }
       r.np = p.np;
       r.off = (const float4 *) f->roff.p;
       r.cell = (const int4 *) f->rcell.p;
@@ -289,7 +296,10 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
       r.xi = ts->xi;
       r.xisp = ts->xi / sqrt (M_PI);
       r.xi_ref = sys->xi;
-      r.tab = (const double *) f->rtab.p;
+      r.far2 = (float) real_tab_far (sys->version, ts->xi);
+      r.xf = (const float *) f->xf.p;
+      r.xtop = (const int *) f->xtop.p;
+      r.xf_ld = XF_LD;
       r.q = (const uint4 *) f->q.p;
       r.u = (const unsigned long long *) f->u.p;
     }
@@ -308,6 +318,8 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
   p.mx = (unsigned *) f->mx.p;
   p.q = (uint4 *) f->q.p;
   p.u = (unsigned long long *) f->u.p;
+  p.xf = (float *) f->xf.p;
+  p.xtop = (int *) f->xtop.p;
   p.yp = f->yp.p;
   const int me = fix_maps (ND, p, &f->maps);
   if (me) return set_error (STOKES_GPU_ECUDA, "TMA tensor maps of the FP64 product (%d)", me);
@@ -384,6 +396,7 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
   rt.x = d_x;
   rt.rmin = c->rmin;
   rt.rm2 = 4.0 * c->rmin * c->rmin;
+  rt.far2 = std::max (rt.far2, (float) (rt.rm2 * 1.0001));     // clamped pairs are near ones
   rt.out = (double *) f->partial.p;
   auto real_space = [&] (cudaStream_t rs) {
     return f->tabled ? launch_real_tab (c->version, rt, rs)
@@ -469,7 +482,7 @@ release_fix (Ctx *c)
 {
   FixState *f = c->fix;
   if (!f) return;
-  for (DevBuf *b : {&f->rtab, &f->roff, &f->rcell, &f->q, &f->u, &f->quart, &f->nqm, &f->coef, &f->off, &f->fitem, &f->bitem, &f->S, &f->T, &f->F, &f->G, &f->ZF, &f->WB,
+  for (DevBuf *b : {&f->rtab, &f->roff, &f->rcell, &f->q, &f->u, &f->xf, &f->xtop, &f->quart, &f->nqm, &f->coef, &f->off, &f->fitem, &f->bitem, &f->S, &f->T, &f->F, &f->G, &f->ZF, &f->WB,
                     &f->mx, &f->yp, &f->partial, &f->status})
     b->release ();
   f->graph.release ();

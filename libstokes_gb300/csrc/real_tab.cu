@@ -24,6 +24,15 @@
 // nodes); the table is made on the device from the closed forms, with the
 // change of basis in double-double.
 //
+// Far pairs.  The functions fall off as exp(-xi^2 r^2), so beyond xi r = FAR_U
+// a pair contributes less than about 1e-9 of a near one, and single precision
+// there costs the sum less than FP64 rounding does: 6e-8 of 1e-9 at the
+// border, sqrt(300) such pairs, falling by e^-2u per 1 / xi further out, is
+// 2e-16 of a near term.  About half of the pairs within the cutoff (xi r =
+// 6.6) are far.  Only the relative error of s would be magnified (by u^2), so
+// s and its distance to the bin's middle stay FP64 (8 instructions); the
+// functions, the tensors and the sum of the far pairs are FP32.
+//
 // Positions are the 64-bit fixed-point fractional coordinates of the
 // reciprocal sum, so the minimum image is the integer overflow and a
 // displacement carries one rounding, however close the pair; the conversion
@@ -87,7 +96,7 @@ struct Basis {
 
 template <int V>
 __global__ void __launch_bounds__ (RT_DEG * NFun<V>::value)
-k_rt_table (Basis b, int bin0, double xi, double xisp, double *tab)
+k_rt_table (Basis b, int bin0, double xi, double xisp, double *tab, float *tabf)
 {
   constexpr int NF = NFun<V>::value;
   __shared__ double s_f[RT_DEG][NF];
@@ -115,16 +124,17 @@ k_rt_table (Basis b, int bin0, double xi, double xisp, double *tab)
   double c = sum + err;
   for (int n = 0; n < k; n++) c /= h;                   // h is a power of two
   tab[((size_t) blockIdx.x * NF + q) * RT_DEG + k] = c;
+  tabf[((size_t) blockIdx.x * NF + q) * RT_DEG + k] = (float) c;
 }
 
 // y += M x_j of one pair at displacement d, s = d.d, coefficients f
-template <int V>
+template <int V, typename R>
 __device__ __forceinline__ void
-apply (const double d[3], double s, const double *f, const double *__restrict__ x, double *y)
+apply (const R d[3], R s, const R *f, const R *__restrict__ x, R *y)
 {
-  const double F0 = x[0], F1 = x[1], F2 = x[2];
-  const double dF = d[0] * F0 + d[1] * F1 + d[2] * F2;
-  double along = f[1] * dF;
+  const R F0 = x[0], F1 = x[1], F2 = x[2];
+  const R dF = d[0] * F0 + d[1] * F1 + d[2] * F2;
+  R along = f[1] * dF;
   if (V == V_F)
     {
       y[0] += fma (f[0], F0, along * d[0]);
@@ -132,10 +142,10 @@ apply (const double d[3], double s, const double *f, const double *__restrict__ 
       y[2] += fma (f[0], F2, along * d[2]);
       return;
     }
-  const double T0 = x[3], T1 = x[4], T2 = x[5];
-  const double t0 = T1 * d[2] - T2 * d[1], t1 = T2 * d[0] - T0 * d[2], t2 = T0 * d[1] - T1 * d[0];
-  const double f0 = F1 * d[2] - F2 * d[1], f1 = F2 * d[0] - F0 * d[2], f2 = F0 * d[1] - F1 * d[0];
-  const double w = f[4] * (d[0] * T0 + d[1] * T1 + d[2] * T2);
+  const R T0 = x[3], T1 = x[4], T2 = x[5];
+  const R t0 = T1 * d[2] - T2 * d[1], t1 = T2 * d[0] - T0 * d[2], t2 = T0 * d[1] - T1 * d[0];
+  const R f0 = F1 * d[2] - F2 * d[1], f1 = F2 * d[0] - F0 * d[2], f2 = F0 * d[1] - F1 * d[0];
+  const R w = f[4] * (d[0] * T0 + d[1] * T1 + d[2] * T2);
   y[3] = fma (w, d[0], fma (f[3], T0, fma (f[2], f0, y[3])));
   y[4] = fma (w, d[1], fma (f[3], T1, fma (f[2], f1, y[4])));
   y[5] = fma (w, d[2], fma (f[3], T2, fma (f[2], f2, y[5])));
@@ -146,38 +156,38 @@ apply (const double d[3], double s, const double *f, const double *__restrict__ 
       y[2] = fma (along, d[2], fma (f[0], F2, fma (f[2], t2, y[2])));
       return;
     }
-  const double sxx = x[6], sxy = x[7], sxz = x[8], syz = x[9], syy = x[10];
-  const double Sxx = fma (2.0, sxx, syy), Syy = fma (2.0, syy, sxx);
-  const double s0 = Sxx * d[0] + sxy * d[1] + sxz * d[2];
-  const double s1 = sxy * d[0] + Syy * d[1] + syz * d[2];
-  const double s2 = sxz * d[0] + syz * d[1];
-  const double ss = d[0] * s0 + d[1] * s1 + d[2] * s2, tr = Sxx + Syy;
-  const double third = -1.0 / 3.0, g2 = f[5], g3 = f[6], m1 = f[7], m4 = f[8], zm = f[9];
-  const double g1 = fma (g3, s, 2.0 * g2) * third;
-  const double m2 = fma (m1, s, 2.0 * m4) * third;
-  const double m3 = fma (m2, s, zm) * third;
+  const R sxx = x[6], sxy = x[7], sxz = x[8], syz = x[9], syy = x[10];
+  const R Sxx = fma (R (2), sxx, syy), Syy = fma (R (2), syy, sxx);
+  const R s0 = Sxx * d[0] + sxy * d[1] + sxz * d[2];
+  const R s1 = sxy * d[0] + Syy * d[1] + syz * d[2];
+  const R s2 = sxz * d[0] + syz * d[1];
+  const R ss = d[0] * s0 + d[1] * s1 + d[2] * s2, tr = Sxx + Syy;
+  const R third = R (-1.0 / 3.0), g2 = f[5], g3 = f[6], m1 = f[7], m4 = f[8], zm = f[9];
+  const R g1 = fma (g3, s, R (2) * g2) * third;
+  const R m2 = fma (m1, s, R (2) * m4) * third;
+  const R m3 = fma (m2, s, zm) * third;
   along = fma (-g1, tr, fma (-g3, ss, along));
-  const double n2 = -2.0 * g2, nc = -f[4];
+  const R n2 = R (-2) * g2, nc = -f[4];
   y[0] = fma (along, d[0], fma (f[0], F0, fma (f[2], t0, fma (n2, s0, y[0]))));
   y[1] = fma (along, d[1], fma (f[0], F1, fma (f[2], t1, fma (n2, s1, y[1]))));
   y[2] = fma (along, d[2], fma (f[0], F2, fma (f[2], t2, fma (n2, s2, y[2]))));
-  const double h2 = 2.0 * nc;
+  const R h2 = R (2) * nc;
   y[3] = fma (h2, d[1] * s2 - d[2] * s1, y[3]);
   y[4] = fma (h2, d[2] * s0 - d[0] * s2, y[4]);
   y[5] = fma (h2, d[0] * s1 - d[1] * s0, y[5]);
-  const double v0 = fma (g2, F0, fma (nc, t0, m4 * s0));
-  const double v1 = fma (g2, F1, fma (nc, t1, m4 * s1));
-  const double v2 = fma (g2, F2, fma (nc, t2, m4 * s2));
-  const double dE = fma (g1, dF, fma (m2, ss, m3 * tr));
-  const double ee = fma (g3, dF, fma (m1, ss, m2 * tr));
+  const R v0 = fma (g2, F0, fma (nc, t0, m4 * s0));
+  const R v1 = fma (g2, F1, fma (nc, t1, m4 * s1));
+  const R v2 = fma (g2, F2, fma (nc, t2, m4 * s2));
+  const R dE = fma (g1, dF, fma (m2, ss, m3 * tr));
+  const R ee = fma (g3, dF, fma (m1, ss, m2 * tr));
   // ee d d + d V + V d = d (V + ee d / 2) + (V + ee d / 2) d
-  const double he = 0.5 * ee;
-  const double w0 = fma (he, d[0], v0), w1 = fma (he, d[1], v1), w2 = fma (he, d[2], v2);
-  y[6] += fma (2.0 * d[0], w0, fma (zm, Sxx, dE));
+  const R he = R (0.5) * ee;
+  const R w0 = fma (he, d[0], v0), w1 = fma (he, d[1], v1), w2 = fma (he, d[2], v2);
+  y[6] += fma (R (2) * d[0], w0, fma (zm, Sxx, dE));
   y[7] = fma (d[0], w1, fma (d[1], w0, fma (zm, sxy, y[7])));
   y[8] = fma (d[0], w2, fma (d[2], w0, fma (zm, sxz, y[8])));
   y[9] = fma (d[1], w2, fma (d[2], w1, fma (zm, syz, y[9])));
-  y[10] += fma (2.0 * d[1], w1, fma (zm, Syy, dE));
+  y[10] += fma (R (2) * d[1], w1, fma (zm, Syy, dE));
 }
 
 // pairs the table does not serve: nearer than its first bin, or under the
@@ -215,9 +225,9 @@ near_term (const RealTabArgs &a, double d0, double d1, double d2, double s, cons
 // v[0 .. P) summed over the warp, P a power of two <= 16: lane l ends up with
 // the sum of element l / (32 / P).  P - 1 + 5 - log2 P additions instead of
 // 5 P.
-template <int P>
-__device__ __forceinline__ double
-warp_sums (double (&v)[P], int lane)
+template <int P, typename R>
+__device__ __forceinline__ R
+warp_sums (R (&v)[P], int lane)
 {
   int o = 16;
 #pragma unroll
@@ -226,7 +236,7 @@ warp_sums (double (&v)[P], int lane)
     for (int k = 0; k < n; k++)
       {
         const bool up = lane & o;
-        const double keep = up ? v[k + n] : v[k], send = up ? v[k] : v[k + n];
+        const R keep = up ? v[k + n] : v[k], send = up ? v[k] : v[k + n];
         v[k] = keep + __shfl_xor_sync (0xffffffffu, send, o);
       }
   for (; o >= 1; o >>= 1) v[0] += __shfl_xor_sync (0xffffffffu, v[0], o);
@@ -247,21 +257,26 @@ k_real_tab (RealTabArgs a)
   constexpr int C = NComp<V>::value, NF = NFun<V>::value;
   constexpr int P = C <= 4 ? 4 : (C <= 8 ? 8 : 16);
   __shared__ unsigned s_list[RT_W][RT_SEG];             // source | offset << 24
-  __shared__ int s_n[RT_W];
+  __shared__ int s_n[RT_W], s_f[RT_W];                  // near entries, far entries (from the end)
   __shared__ double s_y[RT_W][P];
   const int i = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const uint4 qi = a.q[i];
   const ulonglong2 ua = reinterpret_cast<const ulonglong2 *> (a.u)[2 * i];
   const unsigned long long uz = a.u[4 * (size_t) i + 2];
   double y[P];
+  float yf[P];
 #pragma unroll
-  for (int q = 0; q < P; q++) y[q] = 0.0;
+  for (int q = 0; q < P; q++)
+    {
+      y[q] = 0.0;
+      yf[q] = 0.f;
+    }
   // sources per warp and round: all of them times the offsets fit its segment
   const int per = RT_SEG / a.nimg / 32 * 32;
   for (int b0 = 0; b0 < a.np; b0 += RT_W * per)
     {
       const int j1 = min (a.np, b0 + (warp + 1) * per);
-      int cnt = 0;
+      int cnt = 0, far = 0;
       for (int jb = b0 + warp * per; jb < j1; jb += 32)
         {
           const int j = jb + lane;
@@ -277,35 +292,51 @@ k_real_tab (RealTabArgs a)
             {
               const float4 T = a.nimg > 1 ? a.off[m] : make_float4 (0.f, 0.f, 0.f, 0.f);
               const float dx = x0 + T.x, dy = x1 + T.y, dz = x2 + T.z;
-              const bool ok = j < j1 && (j != i || m != a.home)
-                              && dx * dx + dy * dy + dz * dz < a.rc2;
-              const unsigned got = __ballot_sync (0xffffffffu, ok);
+              const float rr = dx * dx + dy * dy + dz * dz;
+              const bool ok = j < j1 && (j != i || m != a.home) && rr < a.rc2;
+              const bool out = ok && rr > a.far2;
+              const unsigned near = __ballot_sync (0xffffffffu, ok && !out);
+              const unsigned away = __ballot_sync (0xffffffffu, out), below = (1u << lane) - 1u;
               if (ok)
-                s_list[warp][cnt + __popc (got & ((1u << lane) - 1u))]
+                s_list[warp][out ? RT_SEG - 1 - far - __popc (away & below)
+                                 : cnt + __popc (near & below)]
                   = (unsigned) (j - b0) | (unsigned) m << 24;
-              cnt += __popc (got);
+              cnt += __popc (near);
+              far += __popc (away);
             }
         }
-      if (lane == 0) s_n[warp] = cnt;
+      if (lane == 0)
+        {
+          s_n[warp] = cnt;
+          s_f[warp] = far;
+        }
       __syncthreads ();
-      int n = 0;
+      int n = 0, nf = 0;
 #pragma unroll
-      for (int w = 0; w < RT_W; w++) n += s_n[w];
+      for (int w = 0; w < RT_W; w++)
+        {
+          n += s_n[w];
+          nf += s_f[w];
+        }
+      // displacement of entry en in FP64
+      auto displace = [&] (unsigned en, int j, double d[3]) {
+        const ulonglong2 ub = reinterpret_cast<const ulonglong2 *> (a.u)[2 * (size_t) j];
+        const unsigned long long vz = a.u[4 * (size_t) j + 2];
+        int4 o = make_int4 (0, 0, 0, 0);
+        if (a.nimg > 1) o = a.cell[en >> 24];
+        // in units of 2^-60 of the box
+        d[0] = int_to_double (((long long) (ub.x - ua.x) >> 4) + ((long long) o.x << 60)) * a.s60[0];
+        d[1] = int_to_double (((long long) (ub.y - ua.y) >> 4) + ((long long) o.y << 60)) * a.s60[1];
+        d[2] = int_to_double (((long long) (vz - uz) >> 4) + ((long long) o.z << 60)) * a.s60[2];
+      };
       for (int k = t; k < n; k += RT_T)
         {
           int w = 0, at = k;
           while (at >= s_n[w]) at -= s_n[w++];
           const unsigned en = s_list[w][at];
-          const int j = b0 + (int) (en & 0xffffffu), m = (int) (en >> 24);
-          const ulonglong2 ub = reinterpret_cast<const ulonglong2 *> (a.u)[2 * (size_t) j];
-          const unsigned long long vz = a.u[4 * (size_t) j + 2];
-          int4 o = make_int4 (0, 0, 0, 0);
-          if (a.nimg > 1) o = a.cell[m];
-          // displacement in units of 2^-60 of the box
+          const int j = b0 + (int) (en & 0xffffffu);
           double d[3];
-          d[0] = int_to_double (((long long) (ub.x - ua.x) >> 4) + ((long long) o.x << 60)) * a.s60[0];
-          d[1] = int_to_double (((long long) (ub.y - ua.y) >> 4) + ((long long) o.y << 60)) * a.s60[1];
-          d[2] = int_to_double (((long long) (vz - uz) >> 4) + ((long long) o.z << 60)) * a.s60[2];
+          displace (en, j, d);
           const double s = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
           const double *x = a.x + (size_t) C * j;
           const int bin = (__double2hiint (s) >> (20 - RT_LOG)) - a.bin0;
@@ -333,11 +364,51 @@ k_real_tab (RealTabArgs a)
               f[q] = fma (fma (fma (fma (fma (fma (fma (c3.y, z, c3.x), z, c2.y), z, c2.x), z, c1.y),
                                     z, c1.x), z, c0.y), z, c0.x);
             }
-          apply<V> (d, s, f, x, y);
+          apply<V, double> (d, s, f, x, y);
+        }
+      for (int k = t; k < nf; k += RT_T)
+        {
+          int w = 0, at = k;
+          while (at >= s_f[w]) at -= s_f[w++];
+          const unsigned en = s_list[w][RT_SEG - 1 - at];
+          const int j = b0 + (int) (en & 0xffffffu);
+          double d[3];
+          displace (en, j, d);
+          const double s = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+          const int bin = (__double2hiint (s) >> (20 - RT_LOG)) - a.bin0;
+          const float z = (float) (s - bin_mid (bin + a.bin0));
+          const uint4 qj = a.q[j];
+          float e[3] = {(float) (int) (qj.x - qi.x) * a.sf[0], (float) (int) (qj.y - qi.y) * a.sf[1],
+                        (float) (int) (qj.z - qi.z) * a.sf[2]};
+          if (a.nimg > 1)
+            {
+              const float4 T = a.off[en >> 24];
+              e[0] += T.x; e[1] += T.y; e[2] += T.z;
+            }
+          const float4 *c = reinterpret_cast<const float4 *> (a.tabf)
+                            + (size_t) min (bin, a.nbin - 1) * (NF * RT_DEG / 4);
+          float f[NF], xj[12];
+#pragma unroll
+          for (int q = 0; q < NF; q++)
+            {
+              const float4 c1 = __ldg (c + 2 * q + 1), c0 = __ldg (c + 2 * q);
+              f[q] = fmaf (fmaf (fmaf (fmaf (fmaf (c1.y, z, c1.x), z, c0.w), z, c0.z), z, c0.y), z, c0.x);
+            }
+          const float4 *xs = reinterpret_cast<const float4 *> (a.xf + (size_t) a.xf_ld * j);
+#pragma unroll
+          for (int q = 0; q < (C + 3) / 4; q++)
+            {
+              const float4 v = __ldg (xs + q);
+              xj[4 * q] = v.x; xj[4 * q + 1] = v.y; xj[4 * q + 2] = v.z; xj[4 * q + 3] = v.w;
+            }
+          apply<V, float> (e, e[0] * e[0] + e[1] * e[1] + e[2] * e[2], f, xj, yf);
         }
       __syncthreads ();
     }
-  const double v = warp_sums<P> (y, lane);
+  double v = warp_sums<P, double> (y, lane);
+  // the far sum, back in its unit
+  const float vf = warp_sums<P, float> (yf, lane);
+  if (vf != 0.f) v += scalbn ((double) vf, *a.xtop);
   if (lane % (32 / P) == 0) s_y[warp][lane / (32 / P)] = v;
   __syncthreads ();
   if (t < C)
@@ -409,16 +480,31 @@ size_t
 real_tab_bytes (int version, int nbin)
 {
   const int nf = version == 0 ? 2 : (version == 1 ? 5 : 10);
-  return sizeof (double) * (size_t) nbin * nf * RT_DEG;
+  return (sizeof (double) + sizeof (float)) * (size_t) nbin * nf * RT_DEG;
+}
+
+size_t
+real_tab_doubles (int version, int nbin)
+{
+  return real_tab_bytes (version, nbin) / (sizeof (double) + sizeof (float));
+}
+
+// FAR_U: 5.2 for F and FT; the stresslet functions are up to u^2 larger
+double
+real_tab_far (int version, double xi)
+{
+  const double u = version == 2 ? 5.5 : 5.2;
+  return (u / xi) * (u / xi);
 }
 
 cudaError_t
-launch_real_tab_build (int version, int bin0, int nbin, double xi, double *tab, cudaStream_t st)
+launch_real_tab_build (int version, int bin0, int nbin, double xi, double *tab, float *tabf,
+                       cudaStream_t st)
 {
   const double xisp = xi / sqrt (M_PI);
-  if (version == 0) k_rt_table<0><<<nbin, RT_DEG * 2, 0, st>>> (basis (), bin0, xi, xisp, tab);
-  else if (version == 1) k_rt_table<1><<<nbin, RT_DEG * 5, 0, st>>> (basis (), bin0, xi, xisp, tab);
-  else k_rt_table<2><<<nbin, RT_DEG * 10, 0, st>>> (basis (), bin0, xi, xisp, tab);
+  if (version == 0) k_rt_table<0><<<nbin, RT_DEG * 2, 0, st>>> (basis (), bin0, xi, xisp, tab, tabf);
+  else if (version == 1) k_rt_table<1><<<nbin, RT_DEG * 5, 0, st>>> (basis (), bin0, xi, xisp, tab, tabf);
+  else k_rt_table<2><<<nbin, RT_DEG * 10, 0, st>>> (basis (), bin0, xi, xisp, tab, tabf);
   return cudaGetLastError ();
 }
 
