@@ -26,6 +26,8 @@
 #include "engine.h"
 #include "gpu_engine.h"
 
+extern "C" void lsg_set_split (struct stokes *sys, double xi, double ewald_eps);
+
 namespace lsg {
 
 // ---------------------------------------------------------------------------
@@ -445,7 +447,7 @@ tuned_system (Ctx *c, const struct stokes *sys)
   sv->periodic = 1;
   stokes_set_np (sv, sys->np, sys->nm);
   stokes_set_l (sv, sys->lx, sys->ly, sys->lz);
-  stokes_set_xi (sv, eta / cbrt (sys->lx * sys->ly * sys->lz), eps);
+  lsg_set_split (sv, eta / cbrt (sys->lx * sys->ly * sys->lz), eps);
   c->tuned = sv;
   memcpy (c->tuned_key, key, sizeof key);
   return sv;
@@ -561,8 +563,9 @@ prepare (Ctx *c, const struct stokes *sys, bool cube, int tables)
   // 2^22 particles: the range of the fixed-point sums
   if (ts != sys && c->mode == MODE_MONO && sys->np <= (1 << 22))
     {
-      c->use_fix = true;
-      return fix_setup (c, sys, ts);
+      c->use_fix = true;          // its tables are made by the first product
+      c->fix_split = ts;
+      return STOKES_GPU_OK;
     }
   if (c->open)
     c->h_kt.clear ();

@@ -73,6 +73,7 @@ struct Ctx {
   // use_fix: the last prepare chose it
   FixState *fix = nullptr;
   bool use_fix = false;
+  const struct stokes *fix_split = nullptr;   // the tuned split of that prepare
 
   DevBuf openf;   // scratch of the mixed-precision free-space product
   DevBuf imgf;    // the images in FP32 (split-precision dense builder)
@@ -139,9 +140,6 @@ int atimes_fp64_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y
 // the same for equal spheres at the tuned split (product_fix.cu)
 int atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cudaStream_t st,
                     bool timed);
-// brings the tables of that product up to date: sys as the caller set it, ts
-// its private copy at the tuned split
-int fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts);
 int fix_check_status (Ctx *c);
 void release_fix (Ctx *c);
 void collect_times (Ctx *c);

@@ -31,8 +31,7 @@ struct FixState {
   // splits with too many offsets, which the image-table kernel serves
   bool tabled = false;
   RealTabArgs real;
-  DevBuf rtab, roff, rcell, q, u, xf, xtop;
-  DevBuf quart, nqm, coef, off, fitem, bitem, S, T, F, G, ZF, WB, mx, yp, partial, status;
+  DevBuf arena, partial, status;   // arena: every table and buffer of p and real
   int *h_status = nullptr;
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -76,7 +75,7 @@ k_fix_combine (FixCombine a)
 
 // octant points, weights and tiles of the split of ts, with libstokes' G term
 // of sys's own split (FTS; the correction described at tuned_applies)
-int
+static int
 fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
 {
   if (!c->fix) c->fix = new FixState ();
@@ -209,38 +208,6 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
       quart[k] = make_int4 (p.oy + (b ? 2 * b - 1 : 0), b ? p.oy + 2 * b : p.zero,
                             p.oz + (d ? 2 * d - 1 : 0), d ? p.oz + 2 * d : p.zero);
     }
-  cudaError_t e = cudaSuccess;
-  cudaStream_t st = c->stream;
-  auto up = [&] (DevBuf &b, const void *h, size_t bytes) {
-    if (e == cudaSuccess) e = b.ensure (std::max<size_t> (bytes, 64));
-    if (e == cudaSuccess && bytes) e = cudaMemcpyAsync (b.p, h, bytes, cudaMemcpyHostToDevice, st);
-  };
-  // no product of this context may still be using the tables of the last set-up
-  if (f->id && (e = cudaDeviceSynchronize ()) != cudaSuccess)
-    return cuda_fail (e, "FP64 product set-up");
-  up (f->quart, quart.data (), sizeof (int4) * quart.size ());
-  up (f->nqm, nqm.data (), sizeof (int) * nqm.size ());
-  up (f->off, off.data (), sizeof (int) * off.size ());
-  up (f->coef, coef.data (), sizeof (FixCoef) * coef.size ());
-  up (f->fitem, fitem.data (), sizeof (int4) * fitem.size ());
-  up (f->bitem, bitem.data (), sizeof (int4) * bitem.size ());
-  auto room = [&] (DevBuf &b, size_t bytes, bool clear) {
-    if (e == cudaSuccess) e = b.ensure (std::max<size_t> (bytes, 64));
-    if (e == cudaSuccess && clear) e = cudaMemsetAsync (b.p, 0, bytes, st);
-  };
-  // table pads, rows and columns that nothing writes stay zero
-  room (f->T, fix_bytes_T (ND, p), true);
-  room (f->S, fix_bytes_S (ND, p), false);
-  room (f->F, fix_bytes_F (ND, p), false);
-  room (f->G, fix_bytes_G (ND, p), true);
-  room (f->ZF, fix_bytes_ZF (ND, p), true);
-  room (f->WB, fix_bytes_WB (ND, p), true);
-  room (f->yp, fix_bytes_yp (ND, p), false);
-  room (f->mx, fix_mx_words (p) * sizeof (unsigned), true);
-  room (f->q, sizeof (uint4) * p.np, false);
-  room (f->u, sizeof (unsigned long long) * 4 * p.np, false);
-  room (f->xf, sizeof (float) * XF_LD * p.np, false);
-  room (f->xtop, sizeof (int), false);
   // real space: lattice offsets whose cell of minimum-image displacements
   // comes within the cutoff, and the radial table
   RealTabArgs r {};
@@ -270,57 +237,96 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
   }
   r.nimg = (int) roff.size ();
   f->tabled = r.nimg <= REAL_TAB_MAXIMG && rc <= 7.4 * std::min (p.l[0], std::min (p.l[1], p.l[2]));
-  if (f->tabled)
+  if (f->tabled) real_tab_range (rc, &r.bin0, &r.nbin);
+
+  // one allocation: host tables (uploaded in one copy), then what stays zero
+  // where nothing writes it (table pads, rows and columns), then the rest
+  std::vector<char> host;
+  size_t bytes = 0;
+  auto align = [] (size_t n) { return (n + 255) / 256 * 256; };
+  auto place = [&] (size_t n) {
+    const size_t at = bytes;
+    bytes += align (std::max<size_t> (n, 16));
+    return at;
+  };
+  auto table = [&] (const void *src, size_t n) {
+    const size_t at = place (n);
+    host.resize (bytes);
+    if (n) memcpy (host.data () + at, src, n);
+    return at;
+  };
+  const size_t o_quart = table (quart.data (), sizeof (int4) * quart.size ());
+  const size_t o_nqm = table (nqm.data (), sizeof (int) * nqm.size ());
+  const size_t o_off = table (off.data (), sizeof (int) * off.size ());
+  const size_t o_coef = table (coef.data (), sizeof (FixCoef) * coef.size ());
+  const size_t o_fit = table (fitem.data (), sizeof (int4) * fitem.size ());
+  const size_t o_bit = table (bitem.data (), sizeof (int4) * bitem.size ());
+  const size_t o_roff = table (roff.data (), sizeof (float4) * roff.size ());
+  const size_t o_rcell = table (rcell.data (), sizeof (int4) * rcell.size ());
+  const size_t zero0 = bytes;
+  const size_t o_mx = place (fix_mx_words (p) * sizeof (unsigned));
+  const size_t o_T = place (fix_bytes_T (ND, p)), o_G = place (fix_bytes_G (ND, p));
+  const size_t o_ZF = place (fix_bytes_ZF (ND, p)), o_WB = place (fix_bytes_WB (ND, p));
+  const size_t zero1 = bytes;
+  const size_t o_S = place (fix_bytes_S (ND, p)), o_F = place (fix_bytes_F (ND, p));
+  const size_t o_yp = place (fix_bytes_yp (ND, p));
+  const size_t o_q = place (sizeof (uint4) * p.np), o_u = place (sizeof (unsigned long long) * 4 * p.np);
+  const size_t o_xf = place (sizeof (float) * XF_LD * p.np), o_top = place (sizeof (int));
+  const size_t o_rt = place (f->tabled ? real_tab_bytes (sys->version, r.nbin) : 0);
+
+  cudaStream_t st = c->stream;
+  // no product of this context may still be using the tables of the last set-up
+  cudaError_t e = f->id ? cudaDeviceSynchronize () : cudaSuccess;
+  if (e == cudaSuccess) e = f->arena.ensure (bytes);
+  char *base = (char *) f->arena.p;
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync (base, host.data (), host.size (), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync (base + zero0, 0, zero1 - zero0, st);
+  if (e == cudaSuccess && !f->status.p)
     {
-      real_tab_range (rc, &r.bin0, &r.nbin);
-      up (f->roff, roff.data (), sizeof (float4) * roff.size ());
-      up (f->rcell, rcell.data (), sizeof (int4) * rcell.size ());
-      room (f->rtab, real_tab_bytes (sys->version, r.nbin), false);
-      if (e == cudaSuccess)
-        {
-          r.tab = (const double *) f->rtab.p;
-          r.tabf = (const float *) (r.tab + real_tab_doubles (sys->version, r.nbin));
-          e = launch_real_tab_build (sys->version, r.bin0, r.nbin, ts->xi, (double *) r.tab,
-                                     (float *) r.tabf, st);
-        }
-      r.np = p.np;
-      r.off = (const float4 *) f->roff.p;
-      r.cell = (const int4 *) f->rcell.p;
-      for (int d = 0; d < 3; d++)
-        {
-          r.sf[d] = (float) (p.l[d] / 4294967296.0);
-          r.s60[d] = p.l[d] / 1152921504606846976.0;
-        }
-      // FP32 distances are within 1e-6 of the exact ones
-      r.rc2 = (float) (ts->rmax2 * 1.00001);
-      r.xi = ts->xi;
-      r.xisp = ts->xi / sqrt (M_PI);
-      r.xi_ref = sys->xi;
-      r.far2 = (float) real_tab_far (sys->version, ts->xi);
-      r.xf = (const float *) f->xf.p;
-      r.xtop = (const int *) f->xtop.p;
-      r.xf_ld = XF_LD;
-      r.q = (const uint4 *) f->q.p;
-      r.u = (const unsigned long long *) f->u.p;
+      e = f->status.ensure (sizeof (int));
+      if (e == cudaSuccess) e = cudaMemsetAsync (f->status.p, 0, sizeof (int), st);
     }
-  f->real = r;
-  if (!f->status.p) room (f->status, sizeof (int), true);
-  // the uploads read host vectors of this call
+  if (e == cudaSuccess && f->tabled)
+    {
+      r.tab = (const double *) (base + o_rt);
+      r.tabf = (const float *) (r.tab + real_tab_doubles (sys->version, r.nbin));
+      e = launch_real_tab_build (sys->version, r.bin0, r.nbin, ts->xi, (double *) r.tab,
+                                 (float *) r.tabf, st);
+    }
+  // the upload reads a host vector of this call
   if (e == cudaSuccess) e = cudaStreamSynchronize (st);
   if (e != cudaSuccess) return cuda_fail (e, "FP64 product set-up");
-  p.quart = (const int4 *) f->quart.p;
-  p.nqm = (const int *) f->nqm.p;
-  p.off = (const int *) f->off.p;
-  p.coef = (const FixCoef *) f->coef.p;
-  p.fitem = (const int4 *) f->fitem.p;
-  p.bitem = (const int4 *) f->bitem.p;
-  p.T = f->T.p; p.S = f->S.p; p.F = f->F.p; p.G = f->G.p; p.ZF = f->ZF.p; p.WB = f->WB.p;
-  p.mx = (unsigned *) f->mx.p;
-  p.q = (uint4 *) f->q.p;
-  p.u = (unsigned long long *) f->u.p;
-  p.xf = (float *) f->xf.p;
-  p.xtop = (int *) f->xtop.p;
-  p.yp = f->yp.p;
+  p.quart = (const int4 *) (base + o_quart);
+  p.nqm = (const int *) (base + o_nqm);
+  p.off = (const int *) (base + o_off);
+  p.coef = (const FixCoef *) (base + o_coef);
+  p.fitem = (const int4 *) (base + o_fit);
+  p.bitem = (const int4 *) (base + o_bit);
+  p.mx = (unsigned *) (base + o_mx);
+  p.T = base + o_T; p.G = base + o_G; p.ZF = base + o_ZF; p.WB = base + o_WB;
+  p.S = base + o_S; p.F = base + o_F; p.yp = base + o_yp;
+  p.q = (uint4 *) (base + o_q);
+  p.u = (unsigned long long *) (base + o_u);
+  p.xf = (float *) (base + o_xf);
+  p.xtop = (int *) (base + o_top);
+  r.np = p.np;
+  r.off = (const float4 *) (base + o_roff);
+  r.cell = (const int4 *) (base + o_rcell);
+  for (int d = 0; d < 3; d++)
+    {
+      r.sf[d] = (float) (p.l[d] / 4294967296.0);
+      r.s60[d] = p.l[d] / 1152921504606846976.0;
+    }
+  // FP32 distances are within 1e-6 of the exact ones
+  r.rc2 = (float) (ts->rmax2 * 1.00001);
+  r.far2 = (float) real_tab_far (sys->version, ts->xi);
+  r.xi = ts->xi;
+  r.xisp = ts->xi / sqrt (M_PI);
+  r.xi_ref = sys->xi;
+  r.q = p.q; r.u = p.u; r.xf = p.xf; r.xtop = p.xtop;
+  r.xf_ld = XF_LD;
+  f->real = r;
   const int me = fix_maps (ND, p, &f->maps);
   if (me) return set_error (STOKES_GPU_ECUDA, "TMA tensor maps of the FP64 product (%d)", me);
   if (!f->h_status)
@@ -358,6 +364,8 @@ int
 atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cudaStream_t st,
                 bool timed)
 {
+  const int rs = fix_setup (c, c->sys, c->fix_split);
+  if (rs) return rs;
   FixState *f = c->fix;
   FixPlan p = f->p;
   p.stall = g_test_gemm_stall;
@@ -482,9 +490,7 @@ release_fix (Ctx *c)
 {
   FixState *f = c->fix;
   if (!f) return;
-  for (DevBuf *b : {&f->rtab, &f->roff, &f->rcell, &f->q, &f->u, &f->xf, &f->xtop, &f->quart, &f->nqm, &f->coef, &f->off, &f->fitem, &f->bitem, &f->S, &f->T, &f->F, &f->G, &f->ZF, &f->WB,
-                    &f->mx, &f->yp, &f->partial, &f->status})
-    b->release ();
+  for (DevBuf *b : {&f->arena, &f->partial, &f->status}) b->release ();
   f->graph.release ();
   if (f->h_status) cudaFreeHost (f->h_status);
   if (f->side) cudaStreamDestroy (f->side);

@@ -287,8 +287,10 @@ fill_k_table (struct stokes *sys)
   sys->nk = nk;
 }
 
-void
-stokes_set_xi (struct stokes *sys, double xi, double ewald_eps)
+/* split, self terms, cutoffs and image table; the reciprocal table too with
+ * k_table */
+static void
+set_split (struct stokes *sys, double xi, double ewald_eps, int k_table)
 {
   sys->ewald_eps = ewald_eps;
   sys->xi = xi;
@@ -362,9 +364,25 @@ stokes_set_xi (struct stokes *sys, double xi, double ewald_eps)
         }
     }
   sys->nr = nr;
+  if (!k_table) return;
   fill_k_table (sys);
   sys->flag_table = 1;
+}
+
+void
+stokes_set_xi (struct stokes *sys, double xi, double ewald_eps)
+{
+  set_split (sys, xi, ewald_eps, 1);
   stokes_gpu_note_split (sys);
+}
+
+/* Internal: the same split without the reciprocal table, for private copies
+ * whose kernels build their own (the table of a short-ranged split takes
+ * milliseconds). */
+void
+lsg_set_split (struct stokes *sys, double xi, double ewald_eps)
+{
+  set_split (sys, xi, ewald_eps, 0);
 }
 
 double
