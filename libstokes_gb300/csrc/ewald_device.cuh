@@ -486,4 +486,118 @@ int_to_double (long long v)
   return __longlong_as_double ((long long) (v ? bits | sign : 0ull));
 }
 
+// The transverse parts of a generalised force v at direction e: F, T x e and
+// S' e without their components along e.  Every reciprocal coupling acts
+// through these (a force and its derivatives drive an incompressible flow).
+template <int V, typename R> struct Trans { R f[3], t[3], s[3]; };
+
+template <int V, typename R>
+__device__ __forceinline__ void
+transverse (const R e[3], const R *x, Trans<V, R> &o)
+{
+  GenF<V, R> g;
+  load_genf<V, R> (x, g);
+  const R eF = e[0] * g.F[0] + e[1] * g.F[1] + e[2] * g.F[2];
+#pragma unroll
+  for (int d = 0; d < 3; d++) o.f[d] = fma (-eF, e[d], g.F[d]);
+  if constexpr (V >= V_FT)
+    {
+      o.t[0] = g.T[1] * e[2] - g.T[2] * e[1];
+      o.t[1] = g.T[2] * e[0] - g.T[0] * e[2];
+      o.t[2] = g.T[0] * e[1] - g.T[1] * e[0];
+    }
+  if constexpr (V == V_FTS)
+    {
+      const R s0 = g.S[0] * e[0] + g.S[2] * e[1] + g.S[3] * e[2];
+      const R s1 = g.S[2] * e[0] + g.S[1] * e[1] + g.S[4] * e[2];
+      const R s2 = g.S[3] * e[0] + g.S[4] * e[1];
+      const R es = e[0] * s0 + e[1] * s1 + e[2] * s2;
+      o.s[0] = fma (-es, e[0], s0);
+      o.s[1] = fma (-es, e[1], s1);
+      o.s[2] = fma (-es, e[2], s2);
+    }
+}
+
+// the couplings of recip_apply on transverse parts: c of the vector that
+// meets the cosine-type weights (ya, yc, yh, ym), s of the one that meets the
+// sine-type weights (yb, yg; their sign is the caller's)
+template <int V, typename R>
+__device__ __forceinline__ void
+couple (const R e[3], R ya, R yb, R yc, R yg, R yh, R ym, const Trans<V, R> &c,
+        const Trans<V, R> &s, R *y)
+{
+  R w[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++)
+    {
+      y[d] = ya * c.f[d];
+      if (V >= V_FT)
+        {
+          y[d] = fma (yb, s.t[d], y[d]);
+          w[d] = fma (yc, c.t[d], -yb * s.f[d]);
+        }
+      if (V == V_FTS)
+        {
+          y[d] = fma (R (-2) * yg, s.s[d], y[d]);
+          w[d] = fma (R (2) * yh, c.s[d], w[d]);
+        }
+    }
+  if constexpr (V >= V_FT)
+    {
+      y[3] = e[1] * w[2] - e[2] * w[1];
+      y[4] = e[2] * w[0] - e[0] * w[2];
+      y[5] = e[0] * w[1] - e[1] * w[0];
+    }
+  if constexpr (V == V_FTS)
+    {
+      R v[3];
+#pragma unroll
+      for (int d = 0; d < 3; d++) v[d] = fma (yg, s.f[d], fma (yh, c.t[d], ym * c.s[d]));
+      y[6] = R (2) * e[0] * v[0];
+      y[7] = fma (e[0], v[1], e[1] * v[0]);
+      y[8] = fma (e[0], v[2], e[2] * v[0]);
+      y[9] = fma (e[1], v[2], e[2] * v[1]);
+      y[10] = R (2) * e[1] * v[1];
+    }
+}
+
+// the transverse parts of the lane at lane ^ mask
+template <int V, typename R>
+__device__ __forceinline__ void
+swap_trans (const Trans<V, R> &a, Trans<V, R> &o, int mask)
+{
+#pragma unroll
+  for (int d = 0; d < 3; d++)
+    {
+      o.f[d] = __shfl_xor_sync (0xffffffffu, a.f[d], mask);
+      if (V >= V_FT) o.t[d] = __shfl_xor_sync (0xffffffffu, a.t[d], mask);
+      if (V == V_FTS) o.s[d] = __shfl_xor_sync (0xffffffffu, a.s[d], mask);
+    }
+}
+
+// sign change without an arithmetic instruction of the type's pipe: v or -v
+// for bit = 0, 1
+__device__ __forceinline__ double
+flip (double v, int bit)
+{
+  return __hiloint2double (__double2hiint (v) ^ (int) ((unsigned) bit << 31), __double2loint (v));
+}
+__device__ __forceinline__ float
+flip (float v, int bit)
+{
+  return __int_as_float (__float_as_int (v) ^ (int) ((unsigned) bit << 31));
+}
+__device__ __forceinline__ long long flip (long long v, int bit) { return bit ? -v : v; }
+
+// 2-bit Walsh-Hadamard transform over lanes b = 0 .. 3 of a group of four
+template <typename R>
+__device__ __forceinline__ R
+walsh4 (R v, int b)
+{
+  const R o = __shfl_xor_sync (0xffffffffu, v, 1);
+  v = o + flip (v, b & 1);
+  const R q = __shfl_xor_sync (0xffffffffu, v, 2);
+  return q + flip (v, b >> 1);
+}
+
 }  // namespace lsg

@@ -48,9 +48,9 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <queue>
 #include <vector>
 
+#include "digit_gemm.cuh"
 #include "ewald_device.cuh"
 #include "fixk.h"
 #include "gpu_engine.h"
@@ -60,14 +60,7 @@
 namespace lsg {
 namespace {
 
-constexpr int NT = 576;                 // 16 worker warps, a TMA and an MMA warp
-constexpr int NWORK = 512;
-constexpr int TMA_WARP = 16;
-constexpr int MMA_WARP = 17;
-constexpr int TM = 128;                 // MMA M
-constexpr int STAGES = 2;
-constexpr uint32_t TMEM_COLS = 512;
-constexpr uint32_t WAIT_LIMIT = 1u << 18;   // polls of up to ~20 us each
+using namespace dg;
 
 // per precision: ND digits, operators in R
 template <int ND> struct Cfg;
@@ -87,8 +80,10 @@ struct Geo {
   static constexpr int NP = (ND + PAIR - 1) / PAIR;     // planes
   static constexpr uint32_t A_PLANE = TM * 128;
   static constexpr uint32_t B_PLANE = C::TN * 128;
-  static constexpr uint32_t STAGE = NP * (A_PLANE + B_PLANE);
-  static constexpr uint32_t SMEM = STAGES * STAGE + 1024;
+  static constexpr int NS = 2;                          // stages
+  static constexpr uint32_t A_BYTES = NP * A_PLANE, B_BYTES = NP * B_PLANE;
+  static constexpr uint32_t STAGE = A_BYTES + B_BYTES;
+  static constexpr uint32_t SMEM = NS * STAGE + 1024;
   static constexpr int CPT = C::TN / 4;                 // accumulator columns per worker
   // byte offset of digit p in its row, after the plane's own offset
   static constexpr uint32_t part (int p) { return PAIR == 2 ? (uint32_t) (p & 1) * 64u : 0u; }
@@ -105,12 +100,6 @@ image_off (int p, size_t rows, size_t n, size_t ld, int k)
   const size_t row = (G::plane (p) * rows + n) * ld * G::PAIR;
   return row + (size_t) (k / KT) * 64 + G::part (p) / 2 + k % KT;
 }
-
-struct Sync {
-  uint64_t full[STAGES], empty[STAGES], acc_full, acc_empty, done, never;
-  uint32_t tslot;
-  int err;
-};
 
 // ---- fixed point ----------------------------------------------------------
 // A table entry f (62 fractional bits) as hi 2^32 + lo with lo signed
@@ -208,13 +197,6 @@ abs_hi (double v)
 }
 
 // ---- operand builders -----------------------------------------------------
-// byte offset of 16-byte chunk c of row r in a 128-byte swizzled plane
-__device__ __forceinline__ uint32_t
-chunk_off (int r, int c)
-{
-  return (uint32_t) (r * 128 + ((c ^ (r & 7)) << 4));
-}
-
 // The A operand of a tile is built in two steps, so that the loads of the
 // next tile are in flight while a worker waits for its stage: load() reads a
 // thread's digit strings, store() cuts them and writes the stage.
@@ -292,62 +274,6 @@ struct BuildB {
 };
 
 // ---- GEMM roles -----------------------------------------------------------
-__device__ __forceinline__ unsigned char *
-align1k (unsigned char *p)
-{
-  return p + ((1024u - (umma::smem_u32 (p) & 1023u)) & 1023u);
-}
-
-__device__ __forceinline__ void
-cta_setup (Sync &s)
-{
-  if (threadIdx.x < 32) umma::tmem_alloc (&s.tslot, TMEM_COLS);
-  if (threadIdx.x == 32)
-    {
-      for (int k = 0; k < STAGES; k++)
-        {
-          umma::mbar_init (&s.full[k], 1 + NWORK);
-          umma::mbar_init (&s.empty[k], 1);
-        }
-      umma::mbar_init (&s.acc_full, 1);
-      umma::mbar_init (&s.acc_empty, NWORK);
-      umma::mbar_init (&s.done, 1);
-      umma::mbar_init (&s.never, 1);
-      s.err = 0;
-      umma::fence_mbar_init ();
-    }
-  umma::fence_before_sync ();
-  __syncthreads ();
-  umma::fence_after_sync ();
-}
-
-// the TMA lane: all digit planes of the B tile at (K = k0 + KT t, column n0)
-template <int ND>
-__device__ __forceinline__ void
-tma_role (Sync &s, unsigned char *smem, const CUtensorMap *tb, int n0, int k0, int ntiles)
-{
-  using G = Geo<ND>;
-  volatile int *err = &s.err;
-  umma::tma_prefetch_desc (tb);
-  int issued = 0;
-  for (int t = 0; t < ntiles; t++)
-    {
-      const int st = t % STAGES;
-      if (t >= STAGES
-          && !umma::mbar_wait_or_abort (&s.empty[st], ((t / STAGES) - 1) & 1, WAIT_LIMIT, err))
-        break;
-      umma::mbar_expect_tx (&s.full[st], G::NP * G::B_PLANE);
-      umma::tma_load_3d (smem + (size_t) st * G::STAGE + G::NP * G::A_PLANE, tb,
-                         G::PAIR * (k0 + Cfg<ND>::KT * t), n0, 0, &s.full[st]);
-      issued = t + 1;
-    }
-  // the last load of each stage must land before the shared memory goes away
-  // (in an aborted CTA, whose workers may not arrive, the limit bounds the wait)
-  volatile int never = 0;
-  for (int t = issued > STAGES ? issued - STAGES : 0; t < issued; t++)
-    umma::mbar_wait_or_abort (&s.full[t % STAGES], (t / STAGES) & 1, WAIT_LIMIT, &never);
-}
-
 // TMEM columns of accumulator group g: the even groups first, then the odd
 template <int ND>
 constexpr int
@@ -356,52 +282,33 @@ group_col (int g)
   return ((g & 1) * ((ND + 1) / 2) + g / 2) * Cfg<ND>::TN;
 }
 
-// the MMA lane.  The even digits of B lie one after the other as rows of the
-// tile, the odd ones likewise, and so do their groups in TMEM: one MMA of
-// digit i of A with all even (or odd) digits j <= ND - 1 - i of B adds the
-// products to groups i, i + 2, ... at once, with N up to 256.  A new set of
-// accumulators starts every DK tiles.
+// the MMAs of one tile.  The even digits of B lie one after the other as rows
+// of the tile, the odd ones likewise, and so do their groups in TMEM: one MMA
+// of digit i of A with all even (or odd) digits j <= ND - 1 - i of B adds the
+// products to groups i, i + 2, ... at once, with N up to 256.
 template <int ND>
 __device__ __forceinline__ void
-mma_role (Sync &s, const unsigned char *smem, uint32_t tmem, int ntiles, int stall)
+issue_tile (uint32_t a, uint32_t tmem, bool first)
 {
   using G = Geo<ND>;
   using C = Cfg<ND>;
   static_assert (G::PAIR == 2 && (ND + 1) / 2 * C::TN <= 256, "even digits in one MMA");
-  volatile int *err = &s.err;
-  if (stall > 0 && !umma::mbar_wait_or_abort (&s.never, 0, (uint32_t) stall, err)) ntiles = 0;
-  for (int t = 0; t < ntiles; t++)
-    {
-      const int st = t % STAGES, set = t / C::DK;
-      if (!umma::mbar_wait_or_abort (&s.full[st], (t / STAGES) & 1, WAIT_LIMIT, err)) break;
-      if (t % C::DK == 0 && set > 0
-          && !umma::mbar_wait_or_abort (&s.acc_empty, (set - 1) & 1, WAIT_LIMIT, err))
-        break;
-      umma::fence_after_sync ();
-      const uint32_t a = umma::smem_u32 (smem) + (uint32_t) st * G::STAGE;
-      const uint32_t b = a + G::NP * G::A_PLANE;
-      const uint32_t first = t % C::DK == 0 ? 1u : 0u;
+  const uint32_t b = a + G::A_BYTES;
 #pragma unroll
-      for (int k = 0; k < C::KT / 16; k++)
+  for (int k = 0; k < C::KT / 16; k++)
 #pragma unroll
-        for (int i = 0; i < ND; i++)
+    for (int i = 0; i < ND; i++)
 #pragma unroll
-          for (int odd = 0; odd < 2; odd++)
-            {
-              const int nj = (ND - i + 1 - odd) / 2;        // digits j = odd, odd + 2, ...
-              if (nj == 0) continue;
-              umma::mma_f16 (tmem + (uint32_t) group_col<ND> (i + odd),
-                             umma::smem_desc_sw128 (a + G::plane (i) * G::A_PLANE + G::part (i) + 32 * k),
-                             umma::smem_desc_sw128 (b + G::part (odd) + 32 * k),
-                             umma::idesc_f16 (TM, (uint32_t) (nj * C::TN)),
-                             (first && i == 0 && k == 0) ? 0u : 1u);
-            }
-      umma::mma_commit (&s.empty[st]);
-      if (t % C::DK == C::DK - 1 || t == ntiles - 1) umma::mma_commit (&s.acc_full);
-    }
-  umma::mma_commit (&s.done);
-  volatile int never = 0;
-  umma::mbar_wait_or_abort (&s.done, 0, WAIT_LIMIT, &never);
+      for (int odd = 0; odd < 2; odd++)
+        {
+          const int nj = (ND - i + 1 - odd) / 2;        // digits j = odd, odd + 2, ...
+          if (nj == 0) continue;
+          umma::mma_f16 (tmem + (uint32_t) group_col<ND> (i + odd),
+                         umma::smem_desc_sw128 (a + G::plane (i) * G::A_PLANE + G::part (i) + 32 * k),
+                         umma::smem_desc_sw128 (b + G::part (odd) + 32 * k),
+                         umma::idesc_f16 (TM, (uint32_t) (nj * C::TN)),
+                         (first && i == 0 && k == 0) ? 0u : 1u);
+        }
 }
 
 // running sums of one worker: CPT columns of one row.  Value of a column:
@@ -411,12 +318,14 @@ template <> struct Acc<7> {
   static constexpr int CPT = Geo<7>::CPT;
   long long hi[CPT];
   float lo[CPT];
-  __device__ __forceinline__ void zero ()
+  uint32_t d;                           // TMEM address of its lanes and columns
+  __device__ __forceinline__ void zero (uint32_t tmem)
   {
+    d = tmem;
 #pragma unroll
     for (int u = 0; u < CPT; u++) { hi[u] = 0; lo[u] = 0.f; }
   }
-  __device__ __forceinline__ void drain (uint32_t d)
+  __device__ __forceinline__ void take (int, int)
   {
     static_assert (CPT == 16, "one TMEM load per group");
     float f[2][16];
@@ -444,44 +353,12 @@ template <> struct Acc<7> {
   }
 };
 
-// worker warps: build tile t + 2 once the MMAs of tile t are done; at the end
-// of a set drain first, so that the next set's MMAs start early
-template <int ND, class Build>
-__device__ __forceinline__ bool
-worker_role (Sync &s, unsigned char *smem, uint32_t tmem, int ntiles, Acc<ND> &acc, Build &build)
+// TMEM address of a worker's lanes and columns
+__device__ __forceinline__ uint32_t
+worker_tmem (uint32_t tmem, int cpt)
 {
-  using G = Geo<ND>;
-  using C = Cfg<ND>;
   const int warp = threadIdx.x >> 5;
-  volatile int *err = &s.err;
-  auto put = [&] (int t) {
-    build.store (smem + (size_t) (t % STAGES) * G::STAGE);
-    umma::fence_async_smem ();
-    umma::mbar_arrive (&s.full[t % STAGES]);
-    if (t + 1 < ntiles) build.load (t + 1);
-  };
-  if (ntiles > 0) build.load (0);
-  for (int t = 0; t < STAGES && t < ntiles; t++) put (t);
-  const uint32_t dm = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + (uint32_t) ((warp >> 2) * G::CPT);
-  for (int t = 0; t < ntiles; t++)
-    {
-      if (t % C::DK == C::DK - 1 || t == ntiles - 1)
-        {
-          if (!umma::mbar_wait_or_abort (&s.acc_full, (t / C::DK) & 1, WAIT_LIMIT, err))
-            return false;
-          umma::fence_after_sync ();
-          acc.drain (dm);
-          umma::fence_before_sync ();
-          umma::mbar_arrive (&s.acc_empty);
-        }
-      if (t + STAGES < ntiles)
-        {
-          if (!umma::mbar_wait_or_abort (&s.empty[t % STAGES], (t / STAGES) & 1, WAIT_LIMIT, err))
-            return false;
-          put (t + STAGES);
-        }
-    }
-  return true;
+  return tmem + ((uint32_t) ((warp & 3) * 32) << 16) + (uint32_t) ((warp >> 2) * cpt);
 }
 
 __device__ __forceinline__ int
@@ -499,15 +376,6 @@ first_col (const FixPlan &p, int n0, int q)
 
 constexpr int NOT_FINITE = 1 << 20;
 
-__device__ __forceinline__ void
-cta_finish (Sync &s, uint32_t tmem, int *status)
-{
-  if (threadIdx.x == 0 && s.err) atomicExch (status, 1);
-  umma::fence_before_sync ();
-  __syncthreads ();
-  if (threadIdx.x < 32) umma::tmem_dealloc (tmem, TMEM_COLS);
-}
-
 // forward: a CTA takes one item (row tile, column tile, particle slice) and
 // writes F[slice][column][row]; lanes are consecutive rows, so the stores
 // coalesce
@@ -516,6 +384,7 @@ __global__ void __launch_bounds__ (NT, 1)
 k_fix_fwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
 {
   using C = Cfg<ND>;
+  using G = Geo<ND>;
   extern __shared__ unsigned char dsm[];
   __shared__ Sync s;
   const int4 it = p.fitem[blockIdx.x];
@@ -526,29 +395,18 @@ k_fix_fwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
   const int ntiles = je > jb ? (je - jb + C::KT - 1) / C::KT : 0;
   cta_setup (s);
   const uint32_t tmem = s.tslot;
-  if (warp == TMA_WARP)
+  Acc<ND> acc;
+  acc.zero (worker_tmem (tmem, G::CPT));
+  BuildF<ND> build (p, r0, jb);
+  const BTiles bt {&tmB, G::PAIR * jb, G::PAIR * C::KT, n0, G::A_BYTES, G::B_BYTES};
+  if (run_tiles<C::DK, 1, G::NS> (s, smem, ntiles, G::STAGE, bt, p.stall, build, acc,
+                                  [=] (uint32_t a, int, bool first) { issue_tile<ND> (a, tmem, first); }))
     {
-      if (lane == 0) tma_role<ND> (s, smem, &tmB, n0, jb, ntiles);
-      __syncwarp ();
-    }
-  else if (warp == MMA_WARP)
-    {
-      if (lane == 0) mma_role<ND> (s, smem, tmem, ntiles, p.stall);
-      __syncwarp ();
-    }
-  else
-    {
-      Acc<ND> acc;
-      acc.zero ();
-      BuildF<ND> build (p, r0, jb);
-      if (worker_role<ND> (s, smem, tmem, ntiles, acc, build))
-        {
-          const int r = r0 + (warp & 3) * 32 + lane, c0 = n0 + (warp >> 2) * Geo<ND>::CPT;
-          long long *F = (long long *) p.F + (size_t) it.z * p.ncol * p.Rp + r;
+      const int r = r0 + (warp & 3) * 32 + lane, c0 = n0 + (warp >> 2) * G::CPT;
+      long long *F = (long long *) p.F + (size_t) it.z * p.ncol * p.Rp + r;
 #pragma unroll
-          for (int u = 0; u < Geo<ND>::CPT; u++)
-            if (c0 + u < p.ncol) F[(size_t) (c0 + u) * p.Rp] = acc.fixed (u, p.fu);
-        }
+      for (int u = 0; u < G::CPT; u++)
+        if (c0 + u < p.ncol) F[(size_t) (c0 + u) * p.Rp] = acc.fixed (u, p.fu);
     }
   cta_finish (s, tmem, status);
 }
@@ -564,9 +422,12 @@ __global__ void __launch_bounds__ (NT, 1)
 k_fix_bwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
 {
   using C = Cfg<ND>;
+  using G = Geo<ND>;
   constexpr int HLD = C::TN + 1;
   constexpr uint32_t H_LO = TM * HLD * sizeof (long long);
-  static_assert (H_LO + TM * HLD * sizeof (float) <= STAGES * Geo<ND>::STAGE, "parked tile");
+  constexpr uint32_t X_OFF = H_LO + TM * HLD * sizeof (float);
+  // the parked sums and the x functions of 64 columns (three components: 23)
+  static_assert (X_OFF + 23 * TM * sizeof (long long) <= G::NS * G::STAGE, "parked tile");
   extern __shared__ unsigned char dsm[];
   __shared__ Sync s;
   __shared__ int s_exp[C::TN], s_top[16];
@@ -592,43 +453,43 @@ k_fix_bwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
       for (int n = first_col (p, n0, threadIdx.x); n < ne; n += p.c) top = max (top, s_exp[n]);
       s_top[threadIdx.x] = top;
     }
-  if (warp == TMA_WARP)
-    {
-      if (lane == 0) tma_role<ND> (s, smem, &tmB, n0, tb * C::KT, ntiles);
-      __syncwarp ();
-    }
-  else if (warp == MMA_WARP)
-    {
-      if (lane == 0) mma_role<ND> (s, smem, tmem, ntiles, p.stall);
-      __syncwarp ();
-    }
-  else
-    {
-      Acc<ND> acc;
-      acc.zero ();
-      BuildB<ND> build (p, i0, tb * C::KT);
-      if (worker_role<ND> (s, smem, tmem, ntiles, acc, build))
-        {
-          // the last set is drained, so every build, load and MMA is done and
-          // the stages are free
-          const int o = ((warp & 3) * 32 + lane) * HLD + (warp >> 2) * Geo<ND>::CPT;
-          long long *Hi = reinterpret_cast<long long *> (smem) + o;
-          float *Lo = reinterpret_cast<float *> (smem + H_LO) + o;
+  {
+    Acc<ND> acc;
+    acc.zero (worker_tmem (tmem, G::CPT));
+    BuildB<ND> build (p, i0, tb * C::KT);
+    const BTiles bt {&tmB, G::PAIR * tb * C::KT, G::PAIR * C::KT, n0, G::A_BYTES, G::B_BYTES};
+    if (run_tiles<C::DK, 1, G::NS> (s, smem, ntiles, G::STAGE, bt, p.stall, build, acc,
+                                    [=] (uint32_t a, int, bool first) {
+                                      issue_tile<ND> (a, tmem, first);
+                                    }))
+      {
+        // the last set is drained, so every build, load and MMA is done and
+        // the stages are free
+        const int o = ((warp & 3) * 32 + lane) * HLD + (warp >> 2) * G::CPT;
+        long long *Hi = reinterpret_cast<long long *> (smem) + o;
+        float *Lo = reinterpret_cast<float *> (smem + H_LO) + o;
 #pragma unroll
-          for (int u = 0; u < Geo<ND>::CPT; u++)
-            {
-              Hi[u] = acc.hi[u];
-              Lo[u] = acc.lo[u];
-            }
-        }
-    }
+        for (int u = 0; u < G::CPT; u++)
+          {
+            Hi[u] = acc.hi[u];
+            Lo[u] = acc.lo[u];
+          }
+      }
+  }
   __syncthreads ();
   if (!s.err)
     {
       const long long *Hi = reinterpret_cast<const long long *> (smem);
       const float *Lo = reinterpret_cast<const float *> (smem + H_LO);
-      double *yp = (double *) p.yp + (size_t) blockIdx.y * p.np * p.c;
+      // the x functions of the tile's columns, in one pass (a load per term
+      // would wait for L2 every time)
+      const int f0 = n0 / p.c, nf = (n0 + ne - 1) / p.c - f0 + 1;
+      long long *X = reinterpret_cast<long long *> (smem + X_OFF);
       const long long *T = (const long long *) p.T;
+      for (int e = threadIdx.x; e < nf * TM; e += NT)
+        X[e] = T[(size_t) (f0 + e / TM) * p.ldT + i0 + e % TM];
+      __syncthreads ();
+      double *yp = (double *) p.yp + (size_t) blockIdx.y * p.np * p.c;
       for (int e = threadIdx.x; e < TM * p.c; e += NT)
         {
           const int q = e / TM, r = e - q * TM, i = i0 + r;
@@ -640,7 +501,7 @@ k_fix_bwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
             {
               const int sh = top - s_exp[n];
               if (sh > 62) continue;              // below the last bit
-              const long long f = T[(size_t) ((n0 + n) / p.c) * p.ldT + i] >> sh;
+              const long long f = X[((n0 + n) / p.c - f0) * TM + r] >> sh;
               y += (__int128) f * Hi[r * HLD + n];
               yl = fmaf ((float) (int) (f >> 32), Lo[r * HLD + n], yl);
             }
@@ -797,159 +658,65 @@ k_fix_image (FixPlan p, const double *x)
     }
 }
 
-// Operators: four lanes per octant point, lane b = 2 p2 + p3 holding row b of
-// the quarter; after the transform lane sigma holds the sign pattern
-// (s2, s3) = (1 - 2 (sigma >> 1), 1 - 2 (sigma & 1)).
-// (a sign change, not a second FP64 instruction: v or -v for bit = 0, 1)
-__device__ __forceinline__ double
-flip (double v, int bit)
-{
-  return __hiloint2double (__double2hiint (v) ^ (int) ((unsigned) bit << 31), __double2loint (v));
-}
-__device__ __forceinline__ long long flip (long long v, int bit) { return bit ? -v : v; }
-
-template <typename R>
-__device__ __forceinline__ R
-walsh4 (R v, int b)
-{
-  const R o = __shfl_xor_sync (0xffffffffu, v, 1);
-  v = o + flip (v, b & 1);
-  const R q = __shfl_xor_sync (0xffffffffu, v, 2);
-  return q + flip (v, b >> 1);
-}
-
-// The transverse parts of a generalised force v at direction e: F, T x e and
-// S' e without their components along e.  Every reciprocal coupling acts
-// through these (a force and its derivatives drive an incompressible flow).
-template <int V, typename R> struct Trans { R f[3], t[3], s[3]; };
-
-template <int V, typename R>
-__device__ __forceinline__ void
-transverse (const R e[3], const R *x, Trans<V, R> &o)
-{
-  GenF<V, R> g;
-  load_genf<V, R> (x, g);
-  const R eF = e[0] * g.F[0] + e[1] * g.F[1] + e[2] * g.F[2];
-#pragma unroll
-  for (int d = 0; d < 3; d++) o.f[d] = fma (-eF, e[d], g.F[d]);
-  if (V == V_F) return;
-  o.t[0] = g.T[1] * e[2] - g.T[2] * e[1];
-  o.t[1] = g.T[2] * e[0] - g.T[0] * e[2];
-  o.t[2] = g.T[0] * e[1] - g.T[1] * e[0];
-  if (V == V_FT) return;
-  const R s0 = g.S[0] * e[0] + g.S[2] * e[1] + g.S[3] * e[2];
-  const R s1 = g.S[2] * e[0] + g.S[1] * e[1] + g.S[4] * e[2];
-  const R s2 = g.S[3] * e[0] + g.S[4] * e[1];
-  const R es = e[0] * s0 + e[1] * s1 + e[2] * s2;
-  o.s[0] = fma (-es, e[0], s0);
-  o.s[1] = fma (-es, e[1], s1);
-  o.s[2] = fma (-es, e[2], s2);
-}
-
-// the couplings of recip_apply on transverse parts: c of the vector that
-// meets the cosine-type weights (ya, yc, yh, ym), s of the one that meets the
-// sine-type weights (yb, yg); the sine part enters with the factor sg
-template <int V, typename R>
-__device__ __forceinline__ void
-couple (const R e[3], const FixCoef &K, R sg, const Trans<V, R> &c, const Trans<V, R> &s, R *y)
-{
-  const R ya = (R) K.ya, yb = sg * (R) K.yb, yc = (R) K.yc, yg = sg * (R) K.yg, yh = (R) K.yh,
-          ym = (R) K.ym;
-  R w[3];
-#pragma unroll
-  for (int d = 0; d < 3; d++)
-    {
-      y[d] = ya * c.f[d];
-      if (V >= V_FT)
-        {
-          y[d] = fma (yb, s.t[d], y[d]);
-          w[d] = fma (yc, c.t[d], -yb * s.f[d]);
-        }
-      if (V == V_FTS)
-        {
-          y[d] = fma (R (-2) * yg, s.s[d], y[d]);
-          w[d] = fma (R (2) * yh, c.s[d], w[d]);
-        }
-    }
-  if (V == V_F) return;
-  y[3] = e[1] * w[2] - e[2] * w[1];
-  y[4] = e[2] * w[0] - e[0] * w[2];
-  y[5] = e[0] * w[1] - e[1] * w[0];
-  if (V == V_FT) return;
-  R v[3];
-#pragma unroll
-  for (int d = 0; d < 3; d++) v[d] = fma (yg, s.f[d], fma (yh, c.t[d], ym * c.s[d]));
-  y[6] = R (2) * e[0] * v[0];
-  y[7] = fma (e[0], v[1], e[1] * v[0]);
-  y[8] = fma (e[0], v[2], e[2] * v[0]);
-  y[9] = fma (e[1], v[2], e[2] * v[1]);
-  y[10] = R (2) * e[1] * v[1];
-}
-
-constexpr int KOP_T = 32;               // threads per CTA: 8 octant points (FP64-bound: small CTAs
+constexpr int KOP_T = 32;               // threads per CTA: 4 octant points (FP64-bound: small CTAs
                                         // even out the SMs)
 
+// Operators: eight lanes per octant point.  Lane (w, b): b = 2 p2 + p3 names
+// the row of the quarter, and after the transform the sign pattern (s2, s3) =
+// (1 - 2 (b >> 1), 1 - 2 (b & 1)); w = 0 carries the cosine sums C and makes
+// P, w = 1 the sine sums S and makes Q.  Row b enters C with its cosine column
+// for b = 0, 3 and its sine column for b = 1, 2, and S with the other one; G
+// goes back the same way, so every lane reads and writes one column set.
 template <int ND, int V>
 __global__ void __launch_bounds__ (KOP_T)
 k_fix_kop (FixPlan p)
 {
   using R = typename Cfg<ND>::R;
   constexpr int C = NComp<V>::value;
-  const int m1 = blockIdx.y, b = threadIdx.x & 3;
+  const int m1 = blockIdx.y, b = threadIdx.x & 3, w = (threadIdx.x >> 2) & 1;
   const int nqm = p.nqm[m1];
-  if ((int) (blockIdx.x * (KOP_T / 4)) >= nqm) return;
-  const int qr = blockIdx.x * (KOP_T / 4) + threadIdx.x / 4;
+  if ((int) (blockIdx.x * (KOP_T / 8)) >= nqm) return;
+  const int qr = blockIdx.x * (KOP_T / 8) + threadIdx.x / 8;
   const bool live = qr < nqm;
   const int row = 4 * (live ? qr : 0) + b;
-  const int colc = (m1 ? 2 * m1 - 1 : 0) * C, cols = 2 * m1 * C;
-  // a: this row's part of the cosine sums, s: of the sine sums
-  long long ia[C], is[C];
+  const bool sine = (b == 0 || b == 3) == (w == 1);     // this lane's columns
+  const bool neg = b == 3 || (w == 0 && b != 0);        // and their sign
+  const bool have = live && !(sine && m1 == 0);
+  const int col = (sine ? 2 * m1 : (m1 ? 2 * m1 - 1 : 0)) * C;
+  long long f[C];
 #pragma unroll
-  for (int q = 0; q < C; q++) ia[q] = is[q] = 0;
-  for (int s = 0; s < p.nsplit; s++)
-    {
-      const long long *F = (const long long *) p.F + (size_t) s * p.ncol * p.Rp + row;
+  for (int q = 0; q < C; q++) f[q] = 0;
+  if (have)
+#pragma unroll 2
+    for (int s = 0; s < p.nsplit; s++)
+      {
+        const long long *F = (const long long *) p.F + ((size_t) s * p.ncol + col) * p.Rp + row;
 #pragma unroll
-      for (int q = 0; q < C; q++) ia[q] += F[(size_t) (colc + q) * p.Rp];
-      if (m1)
-#pragma unroll
-        for (int q = 0; q < C; q++) is[q] += F[(size_t) (cols + q) * p.Rp];
-    }
-  R a[C], sn[C];
+        for (int q = 0; q < C; q++) f[q] += F[(size_t) q * p.Rp];
+      }
+  R x[C];
 #pragma unroll
   for (int q = 0; q < C; q++)
-    {
-      const uint32_t hw = p.mx[q];
-      const long long fc = ia[q], fs = is[q];
-      a[q] = (R) from_fixed (walsh4 (b == 0 ? fc : (b == 3 ? -fc : -fs), b), hw, p.fu);
-      sn[q] = (R) from_fixed (walsh4 (b == 0 ? fs : (b == 3 ? -fs : fc), b), hw, p.fu);
-    }
+    x[q] = (R) from_fixed (walsh4 (neg ? -f[q] : f[q], b), p.mx[q], p.fu);
   const FixCoef K = p.coef[(size_t) 4 * (p.off[m1] + (live ? qr : 0)) + b];
   const R e[3] = {(R) K.ex, (R) K.ey, (R) K.ez};
-  Trans<V, R> tc, ts;
-  transverse<V, R> (e, a, tc);
-  transverse<V, R> (e, sn, ts);
-  R P[C], Q[C];
-  couple<V, R> (e, K, R (-1), tc, ts, P);
-  couple<V, R> (e, K, R (1), ts, tc, Q);
-  R *G = (R *) p.G + row;
+  Trans<V, R> own, other;
+  transverse<V, R> (e, x, own);
+  swap_trans<V, R> (own, other, 4);
+  // P = A C - B S, Q = A S + B C
+  R g[C];
+  const R sg = w ? R (1) : R (-1);
+  couple<V, R> (e, (R) K.ya, sg * (R) K.yb, (R) K.yc, sg * (R) K.yg, (R) K.yh, (R) K.ym, own, other, g);
+  R *G = (R *) p.G + (size_t) col * p.Rp + row;
 #pragma unroll
   for (int q = 0; q < C; q++)
     {
-      const R wp = walsh4 (P[q], b), wq = walsh4 (Q[q], b);
-      // the cosine and the sine column of this row
-      const R gc = b == 0 ? wp : (b == 3 ? -wp : wq);
-      const R gs = b == 0 ? wq : (b == 3 ? -wq : -wp);
+      const R v = walsh4 (g[q], b);
       uint32_t mx = 0u;
-      if (live)
+      if (have)
         {
-          G[(size_t) (colc + q) * p.Rp] = gc;
-          mx = abs_hi ((double) gc);
-          if (m1)
-            {
-              G[(size_t) (cols + q) * p.Rp] = gs;
-              mx = max (mx, abs_hi ((double) gs));
-            }
+          G[(size_t) q * p.Rp] = neg ? -v : v;
+          mx = abs_hi ((double) v);
         }
       mx = __reduce_max_sync (0xffffffffu, mx);
       if ((threadIdx.x & 31) == 0 && mx) atomicMax (p.mx + 16 * (m1 + 1) + q, mx);
@@ -984,7 +751,7 @@ template <int ND, int V>
 cudaError_t
 kop_v (const FixPlan &p, cudaStream_t st)
 {
-  k_fix_kop<ND, V><<<dim3 (4 * p.nqp / KOP_T, p.M[0] + 1), KOP_T, 0, st>>> (p);
+  k_fix_kop<ND, V><<<dim3 (8 * p.nqp / KOP_T, p.M[0] + 1), KOP_T, 0, st>>> (p);
   return cudaGetLastError ();
 }
 
@@ -1031,25 +798,7 @@ fix_bytes_yp (int, const FixPlan &p)
 // The time of a set of CTAs (their K tiles, longest first) on one CTA per SM,
 // in K tiles; a CTA's start and end cost about START tiles (measured: a
 // 4-tile forward CTA takes as long as 7 tiles of a long one).
-constexpr int SMS = 152, START = 3;
-
-static long long
-makespan (std::vector<int> &len, int copies)
-{
-  std::sort (len.begin (), len.end (), [] (int a, int b) { return a > b; });
-  std::priority_queue<long long, std::vector<long long>, std::greater<long long>> free;
-  for (int k = 0; k < SMS; k++) free.push (0);
-  long long last = 0;
-  for (int l : len)
-    for (int k = 0; k < copies; k++)
-      {
-        const long long t = free.top () + l + START;
-        free.pop ();
-        free.push (t);
-        last = std::max (last, t);
-      }
-  return last;
-}
+constexpr int START = 3;               // start and end of a CTA, in K tiles
 
 // Work items of the two GEMMs.  A column tile needs the quarters that its
 // smallest |m1| uses (nqm): the forward has no item for row tiles past them,
@@ -1103,7 +852,7 @@ fix_plan_items (int, FixPlan &p, const std::vector<int> &nqm, std::vector<int4> 
           for (int z = 0; z < n; z++) len.push_back ((k + n - 1) / n);
         }
       if (s > 1 && len.size () > 96) break;
-      const long long t = makespan (len, p.mt);
+      const long long t = makespan (len, p.mt, START);
       if (best < 0 || t < best)
         {
           best = t;

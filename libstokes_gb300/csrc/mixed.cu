@@ -2,7 +2,7 @@
 // <= 1e-6 against the FP64 path).
 //
 // The sum is re-split so that most of the work moves to where GB300 is fast:
-//  * split: xi = eta / V^(1/3) with eta ~ 10 (libstokes uses xi = sqrt(pi)/L),
+//  * split: xi = eta / V^(1/3) with eta 8-18 (libstokes uses xi = sqrt(pi)/L),
 //    cutoffs from libstokes' own error estimators at tolerance eps_m; the
 //    real-space cutoff stays below half the box, so the real-space sum is a
 //    minimum-image all-pairs sum;
@@ -10,9 +10,9 @@
 //    exact integer subtractions and the periodic wrap is the integer
 //    overflow, so pair geometry costs no FP64 and loses no digits;
 //  * real space: FP32 pair terms (erfcf/expf), compacted per warp;
-//  * reciprocal space: structure factors C(k), S(k) over half of k space with
-//    e^{ik.r} built from per-particle FP64-accurate phase tables (stored FP32),
-//    FP32 accumulation; back-projection y_i = 2 sum_k cos P + sin Q;
+//  * reciprocal space: 24-bit fixed-point GEMMs over products of real functions
+//    of x, y and z (kspace_mix.cu); for unequal radii structure factors C(k),
+//    S(k) over half of k space with e^{ik.r} from per-particle phase tables;
 //  * FP64: the self term, the split constants and the final combination.
 #include <cuda_runtime.h>
 
@@ -21,14 +21,12 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
-#include <unordered_map>
 #include <vector>
 
 #include "ewald_device.cuh"
 #include "gpu_engine.h"
 #include "mixed.h"
 #include "stokes_gpu.h"
-#include "tc_umma.cuh"
 
 extern "C" void lsg_ewald_cutoffs (double xi, double eps, double lmin, double lmax,
                                    double *rmax_out, double *kmax_out);
@@ -43,19 +41,24 @@ cuda_ok (cudaError_t e, const char *what)
 
 struct MixedState {
   uint64_t fp = 0;
+  bool made = false;     // a split has been made, for fp
+  bool kt_made = false;  // and its half-space list is on the device (kt)
   double xi = 0, rc = 0, kc = 0, eta = 0, eps = 0;
   int M[3] = {0, 0, 0};
   int nkh = 0;
   int nk_split = 0;      // rows of the re-tuned split; the rest: reference G term
   double selfc[3] = {0, 0, 0};
   std::vector<MixK> h_k;
-  DevBuf kt, qpos, tab, xf, pq, part_real, part_rec, selfbuf, status, sf, rowm, rot;
-  DevBuf img_zf, img_wb;        // GEMM B-operand images (kspace_tc.cu)
-  DevBuf tyz;                   // particle-major y, z phases (the GEMMs' A operands)
+  DevBuf kt, qpos, tab, xf, pq, part_real, part_rec, selfbuf, status, rot;
   DevBuf img;                   // real-space lattice offsets (float4)
   int nimg = 1;
-  KMaps maps;
-  uint64_t img_key = 0;         // buffers and plan the maps and zeroed pads belong to
+  // tensor-core reciprocal sum (kspace_mix.cu): plan, TMA maps and one
+  // allocation for its tables and buffers, made for the split mix_fp; mix_id
+  // counts the set-ups
+  MixPlan mp {};
+  MixMaps maps;
+  DevBuf mix;
+  uint64_t mix_fp = 0, mix_id = 0;
   // the real-space kernel runs on this side stream, concurrently with the
   // reciprocal chain (low priority: it fills the SMs the chain leaves idle)
   cudaStream_t side = nullptr;
@@ -63,10 +66,8 @@ struct MixedState {
   // the recorded launch sequence (run_mixed_sequence)
   cudaGraphExec_t gexec = nullptr;
   uint64_t gkey = 0, gcand = 0;
-  int nrow = 0;          // (m2, m3) rows of the tensor-core contraction
   int *h_status = nullptr;      // pinned copy of the kernels' status word
   bool tensor = true;           // reciprocal space on the tensor cores
-  KGemm plan;
   uint64_t self_fp = 0;
   int self_np = 0;
   int nchunk_r = 1, nchunk_k = 1;
@@ -102,34 +103,17 @@ struct PrepArgs {
   uint32_t *qpos;       // [np][4] fixed-point x, y, z (+ pad)
   float2 *tab;          // [ntab][np]
   float *xf;            // [np][cpad(c)]
-  float *zf;            // forward GEMM image ZF (tensor-core path) or NULL
-  size_t zplane;        // floats per ZF plane
-  int kf;               // floats per ZF row
-  float2 *tyz;          // particle-major y, z phases for both signs of m (or NULL)
-  int wyz, M1, M2;
 };
 
 constexpr int PREP_P = 32;       // particles per mk_prep CTA
 constexpr int PREP_ROWS = 4;     // table rows per mk_prep CTA (one entry per thread)
-constexpr int PREP_CMAX = 11;    // components per particle at most
-
-// floor(v) mod 2^32 for |v| < 2^62: the 32-bit fixed-point coordinate, the
-// periodic wrap being the modulo
-__device__ __forceinline__ uint32_t
-fixq (double v)
-{
-  return (uint32_t) (unsigned long long) __double2ll_rd (v);
-}
 
 // Fixed-point positions (wrapped to the primary cell, Lees-Edwards aware),
 // x in FP32 and the per-axis phase tables tab[m][j] = e^{2 pi i m u_d(j)}.
 // u_d is the particle's fractional coordinate on axis d as a 32-bit fixed
 // point q_d, so m u_d mod 1 is the exact integer product m q_d mod 2^32; on
 // a sheared lattice the flow-axis phase coordinate is u_x - (shift/lx) u_g.
-// With a ZF image (the tensor-core path) the CTA also writes, for its
-// flow-axis rows m1, Z = t0[m1] x_q as TF32 hi/lo pairs in the forward
-// GEMM's sign pattern: image row (m1, re, q) = (Re Z, -Im Z), (m1, im, q) =
-// (Im Z, Re Z) at column pair j.
+// For the SIMT reciprocal sums; the tensor-core path has mk_prep_tc.
 // CTA (blockIdx.x, blockIdx.y): PREP_P particles x PREP_ROWS table rows, one
 // entry per thread; the few FP64 operations per particle are repeated by
 // each row group.
@@ -137,21 +121,16 @@ __global__ void __launch_bounds__ (128)
 mk_prep (PrepArgs a)
 {
   __shared__ uint32_t s_q[4][PREP_P];
-  __shared__ float s_x[PREP_P * PREP_CMAX];
   const int t = threadIdx.x;
   const int jb = blockIdx.x * PREP_P;
-  {
-    const size_t e0 = (size_t) jb * a.c;
-    const int nx = PREP_P * a.c;
-    const int cp = (a.c + 3) & ~3;
-    for (int e = t; e < nx; e += blockDim.x)
-      {
-        const float v = (e0 + e < (size_t) a.np * a.c) ? (float) a.x[e0 + e] : 0.f;
-        s_x[e] = v;
-        if (blockIdx.y == 0 && e0 + e < (size_t) a.np * a.c)
-          a.xf[(size_t) (jb + e / a.c) * cp + e % a.c] = v;
-      }
-  }
+  if (blockIdx.y == 0)
+    {
+      const size_t e0 = (size_t) jb * a.c;
+      const int cp = (a.c + 3) & ~3;
+      for (int e = t; e < PREP_P * a.c; e += blockDim.x)
+        if (e0 + e < (size_t) a.np * a.c)
+          a.xf[(size_t) (jb + e / a.c) * cp + e % a.c] = (float) a.x[e0 + e];
+    }
   if (t < PREP_P)
     {
       const int j = jb + t;
@@ -179,56 +158,14 @@ mk_prep (PrepArgs a)
       s_q[0][t] = qu; s_q[1][t] = q1; s_q[2][t] = q2;
     }
   __syncthreads ();
-  // row group y takes rows y, y + G, y + 2 G, y + 3 G (G = gridDim.y), so the
-  // flow-axis rows, which also write ZF, spread over the groups; thread
-  // (rr, jl) computes entry (row rr of the group, particle jl)
-  __shared__ float2 s_ph[PREP_ROWS][PREP_P];
-  const int G = gridDim.y;
-  {
-    const int rr = t / PREP_P, jl = t % PREP_P, j = jb + jl;
-    const int row = (int) blockIdx.y + rr * G;
-    if (row < a.ntab && j < a.np)
-      {
-        const int d = row < a.m0end ? 0 : (row < a.m1end ? 1 : 2);
-        const uint32_t m = (uint32_t) (row - (d == 0 ? 0 : (d == 1 ? a.m0end : a.m1end)));
-        const float2 ph = phase_of (a.rot, m * s_q[d][jl]);
-        a.tab[(size_t) row * a.np + j] = ph;
-        if (d != 0 && a.tyz)
-          {
-            float2 *ty = a.tyz + (size_t) j * a.wyz + (d == 1 ? a.M1 : 2 * a.M1 + 1 + a.M2);
-            ty[(int) m] = ph;
-            ty[-(int) m] = make_float2 (ph.x, -ph.y);
-          }
-        s_ph[rr][jl] = ph;
-      }
-  }
-  if (!a.zf) return;
-  __syncthreads ();
-  // Z = t0[m1] x_q as TF32 hi / lo pairs for the flow-axis rows of this
-  // group, one (row, component, particle) entry per thread at a time (the
-  // particle fastest: neighbouring threads store neighbouring columns)
-  int nz = 0;                                  // flow-axis rows of the group
-  while (nz < PREP_ROWS && (int) blockIdx.y + nz * G < a.m0end) nz++;
-  for (int e = t; e < nz * PREP_P * a.c; e += blockDim.x)
+  // thread (rr, jl) computes entry (row y + rr G, particle jl), G = gridDim.y
+  const int rr = t / PREP_P, jl = t % PREP_P, j = jb + jl;
+  const int row = (int) blockIdx.y + rr * gridDim.y;
+  if (row < a.ntab && j < a.np)
     {
-      const int rr = e / (PREP_P * a.c), rem = e - rr * PREP_P * a.c;
-      const int q = rem / PREP_P, jl = rem - q * PREP_P, j = jb + jl;
-      if (j >= a.np) continue;
-      const int m = (int) blockIdx.y + rr * G;
-      const float2 ph = s_ph[rr][jl];
-      const float xq = s_x[jl * a.c + q];
-      const float u = ph.x * xq, v = ph.y * xq;
-      for (int part = 0; part < 2; part++)
-        {
-          const float p0 = part ? v : u, p1 = part ? u : -v;
-          uint32_t h0, l0, h1, l1;
-          umma::split_tf32 (p0, h0, l0);
-          umma::split_tf32 (p1, h1, l1);
-          float2 *o = reinterpret_cast<float2 *> (
-                        a.zf + (((size_t) m * 2 + part) * a.c + q) * a.kf) + j;
-          o[0] = make_float2 (__uint_as_float (h0), __uint_as_float (h1));
-          o[a.zplane / 2] = make_float2 (__uint_as_float (l0), __uint_as_float (l1));
-        }
+      const int d = row < a.m0end ? 0 : (row < a.m1end ? 1 : 2);
+      const uint32_t m = (uint32_t) (row - (d == 0 ? 0 : (d == 1 ? a.m0end : a.m1end)));
+      a.tab[(size_t) row * a.np + j] = phase_of (a.rot, m * s_q[d][jl]);
     }
 }
 
@@ -1069,25 +1006,26 @@ env_double (const char *name, double dflt)
 }
 
 // default split parameter eta = xi V^(1/3), minimum image, by version and
-// system size.  Measured on one GB300 (FTS at phi 0.3, FT 0.25, F 0.2) with
-// the real space recorded after the forward GEMM; an eta below the smallest
-// minimum-image split is raised to it, so small values all time the same:
-//   FTS  N <= 512: 8 (N = 512 49.0 us against 52.5 with images at 10);
-//        N <= 4096: 10 (N = 4096 273 us against 283 with images at 11);
-//        above: 11 (N = 8192 726 us against 936 with images at 13)
-//   FT   N = 1025-8192: 9 (N = 4096 171 us against 233 at 12; N = 8192
-//        444 against 614 at 14)
-//   F    N = 1025-4096: 9 (N = 2048 69.6 us against 75.2 at 12); above 12
-//        (N = 16384 1131 us against 1189 at 9)
-//   N <= 1024: the time is flat over eta 7-11 for all three
+// system size.  Measured on one GB300 (FTS at phi 0.3, FT 0.25, F 0.2); an
+// eta below the smallest minimum-image split is raised to it, so small values
+// time the same there.  The reciprocal GEMMs cost little against the real
+// space of a large system, so eta grows with N:
+//   N <= 2048   flat over 8-11 (FTS N = 1000 67.1 us at 8, 69.8 at 12)
+//   FTS  N = 4096 237 us at 12 (241 at 8, 249 at 14); N = 8192 599 at 14 (672
+//        at 10); N = 12001 1056 at 14 (1179 at 11); N = 20000 2386 at 18 (2763
+//        at 12)
+//   FT   N = 4096 158 at 8-10 (169 at 12); N = 8000 391 at 9 and at 13; N =
+//        16000 1071 at 16 (1172 at 12); N = 30000 2441 at 18 (2780 at 16)
+//   F    N = 8192 324 at 8-12 (332 at 14); N = 16000 868 at 16 (965 at 12); N =
+//        40000 2960 at 18 (3793 at 16)
+// (From 16 on, three cutoffs fit in the box and the cell list is used.)
 static double
 default_eta (int version, int np)
 {
   if (np <= 256) return 8.0;
-  if (version == 2) return np <= 512 ? 8.0 : (np <= 4096 ? 10.0 : 11.0);
-  if (np <= 1024) return 10.0;
-  if (version == 1) return np <= 8192 ? 9.0 : 10.0;
-  return np <= 4096 ? 9.0 : 12.0;
+  if (np <= 2048) return 9.0;
+  if (version == 2) return np <= 6144 ? 12.0 : (np <= 16384 ? 14.0 : 18.0);
+  return np <= 8192 ? 9.0 : (np <= 16384 ? 16.0 : 18.0);
 }
 
 // eta when lattice images are asked for (LIBSTOKES_GB300_MIXED_IMAGES=1)
@@ -1134,7 +1072,8 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
           fp = (fp ^ b) * 1099511628211ull;
         }
     }
-  if (fp == m->fp && m->kt.p) return STOKES_GPU_OK;
+  if (fp == m->fp && m->made) return STOKES_GPU_OK;
+  m->made = false;
   m->poly = poly;
   m->amax = amax;
 
@@ -1188,7 +1127,6 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
     if (e == cudaSuccess)
       e = cudaMemcpyAsync (m->img.p, hi.data (), sizeof (float4) * hi.size (),
                            cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
     if (e != cudaSuccess) return cuda_fail (e, "mixed real-space images");
     m->nimg = (int) hi.size ();
   }
@@ -1211,52 +1149,61 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
   const int B3 = (int) (kc / k0z) + 1 + (sys->shear_mode == 2 ? (int) ceil (fabs (sl) * B1) : 0);
   m->h_k.clear ();
   int M[3] = {0, 0, 0};
+  const double kc2 = kc * kc * (1.0 + 1e-14);
+  // exp(-k^2 / 4 xi^2) is a product over the axes: (B1 + 1) (2 B2 + 2 B3 + 3)
+  // exponentials instead of one per vector
+  std::vector<double> e2 (2 * B2 + 1), e3 (2 * B3 + 1);
   for (int m1 = 0; m1 <= B1; m1++)
-    for (int m2 = -B2; m2 <= B2; m2++)
-      for (int m3 = -B3; m3 <= B3; m3++)
-        {
-          // half space: m1 > 0, or m1 == 0 and (m2 > 0 or (m2 == 0 and m3 > 0))
-          if (m1 == 0 && (m2 < 0 || (m2 == 0 && m3 <= 0))) continue;
-          const double k1 = k0x * m1;
-          double k2 = k0y * m2, k3 = k0z * m3;
-          if (sys->shear_mode == 1) k2 = k0y * ((double) m2 - sl * (double) m1);
-          else if (sys->shear_mode == 2) k3 = k0z * ((double) m3 - sl * (double) m1);
-          const double kk = k1 * k1 + k2 * k2 + k3 * k3;
-          const double k = sqrt (kk);
-          if (k > kc) continue;
-          const double k4z = kk / 4.0 / xi2;
-          const double kexp = pivol * (1.0 + k4z * (1.0 + 2.0 * k4z)) / kk * exp (-k4z);
-          MixK r;
-          memset (&r, 0, sizeof r);
-          r.m1 = m1; r.m2 = m2; r.m3 = m3;
-          r.ex = (float) (k1 / k); r.ey = (float) (k2 / k); r.ez = (float) (k3 / k);
-          if (poly)
-            {
-              // the per-k factors of the unequal-radius weights
-              // (mk_backproj_poly); G with the xi-independent sign
-              r.ya = (float) kexp;
-              r.yb = (float) k;
-              r.yc = (float) kk;
-              r.yg = (float) -kexp;
-              r.yh = r.ym = 0.f;
-            }
-          else
-            {
-              r.ya = (float) (6.0 * (1.0 - kk / 3.0) * kexp);
-              r.yb = (float) (3.0 * k * kexp);
-              r.yc = (float) (1.5 * kk * kexp);
-              // G coupling with the sign that makes real + reciprocal
-              // independent of xi (the opposite of libstokes'
-              // src/ewald.c:1060-1066)
-              r.yg = (float) (-3.0 * (1.0 - 4.0 / 15.0 * kk) * k * kexp);
-              r.yh = (float) (1.5 * kk * kexp);
-              r.ym = (float) (3.0 * (1.0 - kk / 5.0) * kk * kexp);
-            }
-          m->h_k.push_back (r);
-          M[0] = std::max (M[0], abs (m1));
-          M[1] = std::max (M[1], abs (m2));
-          M[2] = std::max (M[2], abs (m3));
-        }
+    {
+      const double k1 = k0x * m1;
+      const double s2 = sys->shear_mode == 1 ? sl * m1 : 0.0, s3 = sys->shear_mode == 2 ? sl * m1 : 0.0;
+      auto gauss = [&] (double k) { return exp (-k * k / 4.0 / xi2); };
+      for (int m2 = -B2; m2 <= B2; m2++) e2[m2 + B2] = gauss (k1) * gauss (k0y * ((double) m2 - s2));
+      for (int m3 = -B3; m3 <= B3; m3++) e3[m3 + B3] = gauss (k0z * ((double) m3 - s3));
+      for (int m2 = -B2; m2 <= B2; m2++)
+        for (int m3 = -B3; m3 <= B3; m3++)
+          {
+            // half space: m1 > 0, or m1 == 0 and (m2 > 0 or (m2 == 0 and m3 > 0))
+            if (m1 == 0 && (m2 < 0 || (m2 == 0 && m3 <= 0))) continue;
+            const double k2 = k0y * ((double) m2 - s2), k3 = k0z * ((double) m3 - s3);
+            const double kk = k1 * k1 + k2 * k2 + k3 * k3;
+            if (kk > kc2) continue;
+            const double k = sqrt (kk);
+            if (k > kc) continue;
+            const double k4z = kk / 4.0 / xi2;
+            const double kexp = pivol * (1.0 + k4z * (1.0 + 2.0 * k4z)) / kk * (e2[m2 + B2] * e3[m3 + B3]);
+            MixK r;
+            memset (&r, 0, sizeof r);
+            r.m1 = m1; r.m2 = m2; r.m3 = m3;
+            r.ex = (float) (k1 / k); r.ey = (float) (k2 / k); r.ez = (float) (k3 / k);
+            if (poly)
+              {
+                // the per-k factors of the unequal-radius weights
+                // (mk_backproj_poly); G with the xi-independent sign
+                r.ya = (float) kexp;
+                r.yb = (float) k;
+                r.yc = (float) kk;
+                r.yg = (float) -kexp;
+                r.yh = r.ym = 0.f;
+              }
+            else
+              {
+                r.ya = (float) (6.0 * (1.0 - kk / 3.0) * kexp);
+                r.yb = (float) (3.0 * k * kexp);
+                r.yc = (float) (1.5 * kk * kexp);
+                // G coupling with the sign that makes real + reciprocal
+                // independent of xi (the opposite of libstokes'
+                // src/ewald.c:1060-1066)
+                r.yg = (float) (-3.0 * (1.0 - 4.0 / 15.0 * kk) * k * kexp);
+                r.yh = (float) (1.5 * kk * kexp);
+                r.ym = (float) (3.0 * (1.0 - kk / 5.0) * kk * kexp);
+              }
+            m->h_k.push_back (r);
+            M[0] = std::max (M[0], abs (m1));
+            M[1] = std::max (M[1], abs (m2));
+            M[2] = std::max (M[2], abs (m3));
+          }
+    }
   m->nk_split = (int) m->h_k.size ();
   // libstokes' FTS result depends on its own xi through the sign of its
   // reciprocal G term: y_ref = y_xi_invariant + 2 G_ref(xi_ref), where G_ref is
@@ -1265,12 +1212,13 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
   if (sys->version == 2)
     {
       const double rxi2 = sys->xi2;
-      auto kkey = [] (int a, int b, int c) {
-        return ((int64_t) a << 42) ^ ((int64_t) (b + (1 << 20)) << 21) ^ (int64_t) (c + (1 << 20));
-      };
-      std::unordered_map<int64_t, int> own;
+      // position of each vector of the split in h_k, by its indexes
+      const int X1 = M[0], X2 = M[1], X3 = M[2], W2 = 2 * X2 + 1, W3 = 2 * X3 + 1;
+      if (X1 > MX_MTAB || X2 > MX_MTAB || X3 > MX_MTAB)
+        return set_error (STOKES_GPU_ETOOBIG, "mixed split: |m| above %d", MX_MTAB);
+      std::vector<int> own ((size_t) (X1 + 1) * W2 * W3, -1);
       for (int k = 0; k < m->nk_split; k++)
-        own.emplace (kkey (m->h_k[k].m1, m->h_k[k].m2, m->h_k[k].m3), k);
+        own[((size_t) m->h_k[k].m1 * W2 + m->h_k[k].m2 + X2) * W3 + m->h_k[k].m3 + X3] = k;
       for (int m1 = 0; m1 <= sys->kmaxx; m1++)
         for (int m2 = -sys->kmaxy; m2 <= sys->kmaxy; m2++)
           for (int m3 = -sys->kmaxz; m3 <= sys->kmaxz; m3++)
@@ -1302,10 +1250,11 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
               // the operator is linear in its coefficients, so a k vector of
               // the split's own list takes the term into its yg; each (m1,
               // m2, m3) then appears once, which the GEMM path relies on
-              const auto hit = own.find (kkey (m1, m2, m3));
-              if (hit != own.end ())
+              const bool inside = m1 <= X1 && abs (m2) <= X2 && abs (m3) <= X3;
+              const int hit = inside ? own[((size_t) m1 * W2 + m2 + X2) * W3 + m3 + X3] : -1;
+              if (hit >= 0)
                 {
-                  m->h_k[(size_t) hit->second].yg += r.yg;
+                  m->h_k[(size_t) hit].yg += r.yg;
                   continue;
                 }
               m->h_k.push_back (r);
@@ -1318,37 +1267,148 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
     return set_error (STOKES_GPU_ETOOBIG, "mixed split: |m| above %d", MX_MTAB);
   m->M[0] = M[0]; m->M[1] = M[1]; m->M[2] = M[2];
   m->nkh = (int) m->h_k.size ();
-  // rows of the tensor-core contraction: the (m2, m3) combinations in use,
-  // in (m2, m3) order
-  std::vector<int> rowid ((size_t) (2 * M[1] + 1) * (2 * M[2] + 1), -1);
-  for (const MixK &k : m->h_k) rowid[(size_t) (k.m2 + M[1]) * (2 * M[2] + 1) + (k.m3 + M[2])] = 0;
-  std::vector<int2> rows;
-  for (int a = -M[1]; a <= M[1]; a++)
-    for (int b = -M[2]; b <= M[2]; b++)
-      {
-        int &id = rowid[(size_t) (a + M[1]) * (2 * M[2] + 1) + (b + M[2])];
-        if (id < 0) continue;
-        id = (int) rows.size ();
-        rows.push_back (make_int2 (a, b));
-      }
-  for (MixK &k : m->h_k) k.r = rowid[(size_t) (k.m2 + M[1]) * (2 * M[2] + 1) + (k.m3 + M[2])];
-  m->nrow = (int) rows.size ();
-  cudaError_t e = m->rowm.ensure (sizeof (int2) * (rows.empty () ? 1 : rows.size ()));
-  if (e == cudaSuccess && !rows.empty ())
-    e = cudaMemcpyAsync (m->rowm.p, rows.data (), sizeof (int2) * rows.size (),
-                         cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
-  if (e != cudaSuccess) return cuda_fail (e, "mixed row table");
-  e = m->kt.ensure (sizeof (MixK) * (m->nkh > 0 ? m->nkh : 1));
-  if (e != cudaSuccess) return cuda_fail (e, "mixed k table");
-  if (m->nkh)
-    {
-      e = cudaMemcpyAsync (m->kt.p, m->h_k.data (), sizeof (MixK) * m->nkh,
-                           cudaMemcpyHostToDevice, c->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
-      if (e != cudaSuccess) return cuda_fail (e, "mixed k table");
-    }
+  m->kt_made = false;
   m->fp = fp;
+  m->made = true;
+  return STOKES_GPU_OK;
+}
+
+// the half-space list on the device, for the SIMT and unequal-radii kernels
+static int
+upload_k (Ctx *c, MixedState *m)
+{
+  if (m->kt_made) return STOKES_GPU_OK;
+  cudaError_t e = m->kt.ensure (sizeof (MixK) * std::max (m->nkh, 1));
+  if (e == cudaSuccess && m->nkh)
+    e = cudaMemcpyAsync (m->kt.p, m->h_k.data (), sizeof (MixK) * m->nkh, cudaMemcpyHostToDevice,
+                         c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
+  if (e != cudaSuccess) return cuda_fail (e, "mixed k table");
+  m->kt_made = true;
+  return STOKES_GPU_OK;
+}
+
+// plan, tables and buffers of the tensor-core reciprocal sum for the split of
+// m (its half-space list h_k)
+static int
+mix_setup (Ctx *c, MixedState *m)
+{
+  if (m->mix_fp == m->fp && m->mix.p) return STOKES_GPU_OK;
+  MixPlan p {};
+  p.np = c->np;
+  p.cf = p.cb = NCOMP (c->version);
+  for (int d = 0; d < 3; d++) p.M[d] = m->M[d];
+  p.nmi = 2 * p.M[0] + 1;
+  p.ncolf = p.nmi * p.cf;
+  p.ncolb = p.nmi * p.cb;
+  // quarters (|m2|, |m3|) in use, by length: the ones in use at |m1| are then
+  // (nearly, on a sheared lattice) a prefix
+  const int W = p.M[2] + 1;
+  std::vector<char> used ((size_t) (p.M[1] + 1) * W, 0);
+  for (const MixK &k : m->h_k) used[(size_t) abs (k.m2) * W + abs (k.m3)] = 1;
+  const struct stokes *sys = c->sys;
+  std::vector<std::pair<double, int>> order;
+  for (int b = 0; b <= p.M[1]; b++)
+    for (int d = 0; d <= p.M[2]; d++)
+      if (used[(size_t) b * W + d])
+        order.push_back ({(b / sys->ly) * (b / sys->ly) + (d / sys->lz) * (d / sys->lz), b * W + d});
+  std::stable_sort (order.begin (), order.end ());
+  p.nq = (int) order.size ();
+  p.nqp = (std::max (p.nq, 1) + 31) / 32 * 32;
+  p.Rp = 4 * p.nqp;
+  p.ldT = (p.np + 127) / 128 * 128;
+  p.oy = p.nmi;
+  p.oz = p.oy + 2 * p.M[1] + 1;
+  p.zero = p.oz + 2 * p.M[2] + 1;
+  p.nT = p.zero + 1;
+  std::vector<int> at ((size_t) (p.M[1] + 1) * W, -1);
+  std::vector<int4> quart ((size_t) p.nqp, make_int4 (p.zero, p.zero, p.zero, p.zero));
+  for (int k = 0; k < p.nq; k++)
+    {
+      const int b = order[k].second / W, d = order[k].second % W;
+      at[order[k].second] = k;
+      quart[k] = make_int4 (p.oy + (b ? 2 * b - 1 : 0), b ? p.oy + 2 * b : p.zero,
+                            p.oz + (d ? 2 * d - 1 : 0), d ? p.oz + 2 * d : p.zero);
+    }
+  // quarters of each |m1|, as prefixes that do not grow with |m1| (a column
+  // tile covers the quarters of its smallest |m1|)
+  std::vector<int> nqm ((size_t) p.M[0] + 1, 0), off ((size_t) p.M[0] + 2, 0);
+  for (const MixK &k : m->h_k)
+    nqm[k.m1] = std::max (nqm[k.m1], at[(size_t) abs (k.m2) * W + abs (k.m3)] + 1);
+  for (int a = p.M[0] - 1; a >= 0; a--) nqm[a] = std::max (nqm[a], nqm[a + 1]);
+  for (int a = 0; a <= p.M[0]; a++) off[a + 1] = off[a] + nqm[a];
+  // weights by sign pattern: each half-space vector (m1 >= 0) is one pattern
+  // of its octant point; patterns that name the same vector (m2 or m3 zero)
+  // get it once
+  std::vector<MixCoef> coef ((size_t) 4 * off[p.M[0] + 1]);
+  if (!coef.empty ()) memset (coef.data (), 0, sizeof (MixCoef) * coef.size ());
+  for (const MixK &k : m->h_k)
+    {
+      const int q = at[(size_t) abs (k.m2) * W + abs (k.m3)];
+      MixCoef &w = coef[(size_t) 4 * (off[k.m1] + q) + 2 * (k.m2 < 0) + (k.m3 < 0)];
+      w.ex = k.ex; w.ey = k.ey; w.ez = k.ez;
+      w.ya = k.ya; w.yb = k.yb; w.yc = k.yc; w.yg = k.yg; w.yh = k.yh; w.ym = k.ym;
+    }
+  std::vector<int4> fitem, bitem;
+  mix_plan_items (p, nqm, fitem, bitem);
+  // one allocation: host tables (one copy), what stays zero where nothing
+  // writes it (table pads, rows and columns), the rest
+  std::vector<char> host;
+  host.reserve (sizeof (int4) * (quart.size () + fitem.size () + bitem.size ())
+                + sizeof (MixCoef) * coef.size () + 8 * (nqm.size () + off.size ()) + 2048);
+  size_t bytes = 0;
+  auto place = [&] (size_t n) {
+    const size_t o = bytes;
+    bytes += (std::max<size_t> (n, 16) + 255) / 256 * 256;
+    return o;
+  };
+  auto table = [&] (const void *src, size_t n) {
+    const size_t o = place (n);
+    host.resize (bytes);
+    if (n) memcpy (host.data () + o, src, n);
+    return o;
+  };
+  const size_t o_quart = table (quart.data (), sizeof (int4) * quart.size ());
+  const size_t o_nqm = table (nqm.data (), sizeof (int) * nqm.size ());
+  const size_t o_off = table (off.data (), sizeof (int) * off.size ());
+  const size_t o_coef = table (coef.data (), sizeof (MixCoef) * coef.size ());
+  const size_t o_fit = table (fitem.data (), sizeof (int4) * fitem.size ());
+  const size_t o_bit = table (bitem.data (), sizeof (int4) * bitem.size ());
+  const size_t zero0 = bytes;
+  const size_t o_T = place (sizeof (int) * (size_t) p.nT * p.ldT);
+  const size_t o_ZF = place (mix_zf_bytes (p)), o_WB = place (mix_wb_bytes (p));
+  const size_t o_ws = place (sizeof (float) * mix_ws_floats (p));
+  const size_t zero1 = bytes;
+  const size_t o_zs = place (sizeof (float) * mix_zs_floats (p));
+  const size_t o_F = place (sizeof (float) * (size_t) p.nsplit * p.ncolf * p.Rp);
+  const size_t o_yp = place (sizeof (float) * (size_t) p.nbitem * p.np * p.cb);
+  // no product of this context may still be using the tables of the last set-up
+  cudaError_t e = m->mix_id ? cudaDeviceSynchronize () : cudaSuccess;
+  if (e == cudaSuccess) e = m->mix.ensure (bytes);
+  char *base = (char *) m->mix.p;
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync (base, host.data (), host.size (), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync (base + zero0, 0, zero1 - zero0, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
+  if (e != cudaSuccess) return cuda_fail (e, "mixed reciprocal set-up");
+  p.quart = (const int4 *) (base + o_quart);
+  p.nqm = (const int *) (base + o_nqm);
+  p.off = (const int *) (base + o_off);
+  p.coef = (const MixCoef *) (base + o_coef);
+  p.fitem = (const int4 *) (base + o_fit);
+  p.bitem = (const int4 *) (base + o_bit);
+  p.T = (int *) (base + o_T);
+  p.ZF = base + o_ZF;
+  p.WB = base + o_WB;
+  p.ws = (float *) (base + o_ws);
+  p.zs = (float *) (base + o_zs);
+  p.F = (float *) (base + o_F);
+  p.yp = (float *) (base + o_yp);
+  const int me = mix_maps (p, &m->maps);
+  if (me) return set_error (STOKES_GPU_ECUDA, "TMA tensor maps of the mixed product (%d)", me);
+  m->mp = p;
+  m->mix_id++;
+  m->mix_fp = m->fp;
   return STOKES_GPU_OK;
 }
 
@@ -1371,7 +1431,7 @@ run_mixed_sequence (Ctx *c, MixedState *m, const double *d_pos, const double *d_
   }();
   // the context's own phase events record from inside the graph (event
   // record nodes); a profiling window's ring of events changes per product
-  bool use = enabled && !c->kprof_on && (E == nullptr || E == c->ev) && m->plan.stall == 0;
+  bool use = enabled && !c->kprof_on && (E == nullptr || E == c->ev) && m->mp.stall == 0;
   if (use)
     {
       cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1382,16 +1442,15 @@ run_mixed_sequence (Ctx *c, MixedState *m, const double *d_pos, const double *d_
   uint64_t key = 1469598103934665603ull;
   auto mix = [&] (uint64_t v) { key = (key ^ v) * 1099511628211ull; };
   mix (m->fp);
-  mix (m->img_key);
+  mix (m->mix_id);
   mix ((uint64_t) m->tensor);
   mix ((uint64_t) m->nchunk_r);
   mix ((uint64_t) m->real_g);
   mix ((uint64_t) m->nc[0] * 1000003ull + (uint64_t) m->nc[1] * 1009ull + (uint64_t) m->nc[2]);
   mix ((uint64_t) m->nchunk_k);
   const void *ptrs[] = {d_pos, d_x, d_y, m->kt.p, m->qpos.p, m->tab.p, m->xf.p, m->pq.p,
-                        m->part_real.p, m->part_rec.p, m->selfbuf.p, m->status.p, m->sf.p,
-                        m->rowm.p, m->rot.p, m->img_zf.p, m->img_wb.p, m->h_status, m->tyz.p,
-                        m->img.p, m->sq.p, m->cstart.p, m->prad.p, m->pqa.p, m->pself.p};
+                        m->part_real.p, m->part_rec.p, m->selfbuf.p, m->status.p,
+                        m->rot.p, m->mix.p, m->h_status, m->img.p, m->sq.p, m->cstart.p, m->prad.p, m->pqa.p, m->pself.p};
   for (const void *p : ptrs) mix ((uint64_t) (uintptr_t) p);
   mix ((uint64_t) (uintptr_t) E);
   // a captured cudaEventRecord is only a dependency, not a record: around a
@@ -1494,18 +1553,16 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
   }
   const size_t off1 = (size_t) (m->M[0] + 1) * np;
   const size_t off2 = off1 + (size_t) (m->M[1] + 1) * np;
-  PhaseTables pt{(const float2 *) m->tab.p, off1, off2, m->M[0], m->M[1], m->M[2], np,
-                 (const uint4 *) m->qpos.p, (const float4 *) m->rot.p};
   {
     // reciprocal space on the tensor cores unless LIBSTOKES_GB300_KSPACE=simt
     const char *ks = getenv ("LIBSTOKES_GB300_KSPACE");   // read per call: tests switch it
-    m->plan = kgemm_plan (c->version, pt, (const int2 *) m->rowm.p, m->nrow);
-    m->plan.stall = g_test_gemm_stall;
-    m->tensor = !(ks && strcmp (ks, "simt") == 0) && !m->poly && m->nkh > 0
-                && kgemm_fits (m->plan);
+    m->tensor = !(ks && strcmp (ks, "simt") == 0) && !m->poly && m->nkh > 0;
+    rc = m->tensor ? mix_setup (c, m) : upload_k (c, m);
+    if (rc) return rc;
+    m->mp.stall = g_test_gemm_stall;
   }
   if (m->tensor)
-    m->nchunk_k = kgemm_ypart_chunks (m->plan);
+    m->nchunk_k = m->mp.nbitem;
   else
     {
       m->nchunk_k = std::max (1, std::min (64, (152 * 48 + np - 1) / np));
@@ -1537,8 +1594,8 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
         return set_error (STOKES_GPU_ECUDA, "mixed product: side stream");
     }
   if ((e = m->qpos.ensure (sizeof (uint32_t) * 4 * np)) != cudaSuccess) return cuda_fail (e, "qpos");
-  if ((e = m->tab.ensure (sizeof (float2) * (size_t) ntab * np)) != cudaSuccess) return cuda_fail (e, "phase tables");
-  m->plan.t.tab = (const float2 *) m->tab.p;
+  if (!m->tensor && (e = m->tab.ensure (sizeof (float2) * (size_t) ntab * np)) != cudaSuccess)
+    return cuda_fail (e, "phase tables");
   if ((e = m->xf.ensure (sizeof (float) * (size_t) cpad (C) * np)) != cudaSuccess) return cuda_fail (e, "xf");
   if (m->nc[0])
     {
@@ -1549,25 +1606,13 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
                                      (int) sizeof (int) * 32 * CELL_MAX)) != cudaSuccess)
         return cuda_fail (e, "cell kernel attribute");
     }
-  if (m->tensor)
-    {
-      if ((e = m->sf.ensure (sizeof (float) * kgemm_sf_floats (m->plan))) != cudaSuccess) return cuda_fail (e, "structure factors");
-      if ((e = m->img_zf.ensure (sizeof (float) * kgemm_zf_floats (m->plan))) != cudaSuccess) return cuda_fail (e, "image ZF");
-      if ((e = m->img_wb.ensure (sizeof (float) * kgemm_wb_floats (m->plan))) != cudaSuccess) return cuda_fail (e, "image WB");
-      m->plan.ZF = (float *) m->img_zf.p;
-      m->plan.WB = (float *) m->img_wb.p;
-      m->plan.sf = (float *) m->sf.p;
-      const int wyz = (2 * m->M[1] + 1) + (2 * m->M[2] + 1);
-      if ((e = m->tyz.ensure (sizeof (float2) * (size_t) wyz * np)) != cudaSuccess)
-        return cuda_fail (e, "phase table (particle-major)");
-      m->plan.t.tyz = (const float2 *) m->tyz.p;
-      m->plan.t.wyz = wyz;
-    }
-  else if ((e = m->pq.ensure (sizeof (float) * (m->poly ? 4 : 2) * C
-                               * (size_t) (m->nkh > 0 ? m->nkh : 1))) != cudaSuccess)
+  if (!m->tensor
+      && (e = m->pq.ensure (sizeof (float) * (m->poly ? 4 : 2) * C
+                            * (size_t) (m->nkh > 0 ? m->nkh : 1))) != cudaSuccess)
     return cuda_fail (e, "pq");
   if ((e = m->part_real.ensure (sizeof (float) * (size_t) m->nchunk_r * np * C)) != cudaSuccess) return cuda_fail (e, "real partials");
-  if ((e = m->part_rec.ensure (sizeof (float) * (size_t) m->nchunk_k * np * C)) != cudaSuccess) return cuda_fail (e, "k partials");
+  if (!m->tensor && (e = m->part_rec.ensure (sizeof (float) * (size_t) m->nchunk_k * np * C)) != cudaSuccess)
+    return cuda_fail (e, "k partials");
   // the self block as a C x C matrix, rebuilt when the split changes; with
   // unequal radii the unit block, scaled per particle by its self terms
   if (m->fp != m->self_fp || !m->selfbuf.p)
@@ -1630,64 +1675,48 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
       if (e != cudaSuccess) return cuda_fail (e, "rotations");
     }
 
-  m->plan.t.qpos = (const uint4 *) m->qpos.p;
-  m->plan.t.rot = (const float4 *) m->rot.p;
-  if (m->tensor)
-    {
-      // the pads of ZF and the (row, m1) slots of WB that no k vector owns
-      // stay zero; zeroed, and the TMA maps encoded, when the split or the
-      // buffers change
-      uint64_t key = m->fp * 1000003ull;
-      for (const void *p : {(const void *) m->img_zf.p, (const void *) m->img_wb.p,
-                            (const void *) m->sf.p})
-        key = (key ^ (uint64_t) (uintptr_t) p) * 1099511628211ull;
-      if (key != m->img_key)
-        {
-          e = cudaMemsetAsync (m->img_zf.p, 0, sizeof (float) * kgemm_zf_floats (m->plan), st);
-          if (e == cudaSuccess)
-            e = cudaMemsetAsync (m->img_wb.p, 0, sizeof (float) * kgemm_wb_floats (m->plan), st);
-          if (e != cudaSuccess) return cuda_fail (e, "GEMM images");
-          const int me = kgemm_maps (m->plan, (float *) m->sf.p, &m->maps);
-          if (me) return set_error (STOKES_GPU_ECUDA, "TMA tensor maps of the GEMM images (%d)", me);
-          m->img_key = key;
-        }
-    }
-
   cudaEvent_t *E = phase_events (c, timed);
   // the launch sequence of one product (kernels, copies and stream events);
   // recorded into a CUDA graph once the same configuration repeats
   auto sequence = [&] () -> int {
     if (E) cudaEventRecord (E[0], st);
     kmark (c, st, nullptr);
-    PrepArgs pa;
-    pa.pos = d_pos; pa.x = d_x; pa.np = np; pa.c = C;
-    {
-      const double two32 = 4294967296.0;
-      pa.sx = two32 / sys->lx; pa.sy = two32 / sys->ly; pa.sz = two32 / sys->lz;
-    }
-    pa.shift = sys->shear_shift;
-    pa.sl = sys->shear_shift / sys->lx;
-    pa.shear_mode = sys->shear_mode;
-    pa.ntab = ntab;
-    pa.m0end = m->M[0] + 1;
-    pa.m1end = m->M[0] + m->M[1] + 2;
-    pa.rot = (const float4 *) m->rot.p;
-    pa.qpos = (uint32_t *) m->qpos.p; pa.tab = (float2 *) m->tab.p; pa.xf = (float *) m->xf.p;
-    pa.zf = m->tensor ? m->plan.ZF : nullptr;
-    pa.zplane = m->plan.pZF;
-    pa.kf = m->plan.KF;
-    pa.tyz = m->tensor ? (float2 *) m->tyz.p : nullptr;
-    pa.wyz = (2 * m->M[1] + 1) + (2 * m->M[2] + 1);
-    pa.M1 = m->M[1];
-    pa.M2 = m->M[2];
-    mk_prep<<<dim3 ((np + PREP_P - 1) / PREP_P, (ntab + PREP_ROWS - 1) / PREP_ROWS), 128, 0, st>>> (pa);
+    const double two32 = 4294967296.0;
+    if (m->tensor)
+      {
+        MixPrep pa {};
+        pa.pos = d_pos; pa.x = d_x; pa.np = np; pa.c = C;
+        pa.sx = two32 / sys->lx; pa.sy = two32 / sys->ly; pa.sz = two32 / sys->lz;
+        pa.shift = sys->shear_shift;
+        pa.sl = sys->shear_shift / sys->lx;
+        pa.shear_mode = sys->shear_mode;
+        pa.rot = (const float4 *) m->rot.p;
+        pa.qpos = (uint32_t *) m->qpos.p;
+        pa.xf = (float *) m->xf.p;
+        pa.p = m->mp;
+        if ((e = launch_mix_prep (pa, st)) != cudaSuccess) return cuda_fail (e, "mk_prep");
+      }
+    else
+      {
+        PrepArgs pa;
+        pa.pos = d_pos; pa.x = d_x; pa.np = np; pa.c = C;
+        pa.sx = two32 / sys->lx; pa.sy = two32 / sys->ly; pa.sz = two32 / sys->lz;
+        pa.shift = sys->shear_shift;
+        pa.sl = sys->shear_shift / sys->lx;
+        pa.shear_mode = sys->shear_mode;
+        pa.ntab = ntab;
+        pa.m0end = m->M[0] + 1;
+        pa.m1end = m->M[0] + m->M[1] + 2;
+        pa.rot = (const float4 *) m->rot.p;
+        pa.qpos = (uint32_t *) m->qpos.p; pa.tab = (float2 *) m->tab.p; pa.xf = (float *) m->xf.p;
+        mk_prep<<<dim3 ((np + PREP_P - 1) / PREP_P, (ntab + PREP_ROWS - 1) / PREP_ROWS), 128, 0, st>>> (pa);
+      }
     kmark (c, st, "mk_prep");
 
     RealMixArgs ra;
     memset (&ra, 0, sizeof ra);
     ra.qpos = (const uint32_t *) m->qpos.p; ra.xf = (const float *) m->xf.p;
     ra.np = np; ra.G = m->real_g;
-    const double two32 = 4294967296.0;
     ra.scale[0] = (float) (sys->lx / two32);
     ra.scale[1] = (float) (sys->ly / two32);
     ra.scale[2] = (float) (sys->lz / two32);
@@ -1784,7 +1813,7 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
     cb.x = d_x;
     cb.pr = (const float *) m->part_real.p;
     cb.ncr = m->nchunk_r;
-    cb.pk = (const float *) m->part_rec.p;
+    cb.pk = m->tensor ? m->mp.yp : (const float *) m->part_rec.p;
     cb.nck = m->nchunk_k;
     cb.S = (const double *) m->selfbuf.p;
     cb.selfp = m->poly ? (const double *) m->pself.p : nullptr;
@@ -1795,8 +1824,8 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
     // then the real-space partials, the back-projection and the final sum
     if (fused)
       {
-        if ((e = launch_kspace_forward (c->version, m->plan, m->maps, ka.kt, m->nkh,
-                                        (int *) m->status.p, st, c)) != cudaSuccess)
+        if ((e = launch_mix_forward (c->version, m->mp, m->maps, (int *) m->status.p, st, c))
+            != cudaSuccess)
           return cuda_fail (e, "reciprocal space (tensor cores)");
         if (overlap) fork_real ();
       }
@@ -1833,8 +1862,7 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
         if (E) cudaEventRecord (E[2], st);
       }
     if (fused
-        && (e = launch_kspace_backward (c->version, m->plan, m->maps, (float *) m->part_rec.p,
-                                        (int *) m->status.p, st, c)) != cudaSuccess)
+        && (e = launch_mix_backward (m->mp, m->maps, (int *) m->status.p, st, c)) != cudaSuccess)
       return cuda_fail (e, "reciprocal space (tensor cores)");
     // the real-space partials must be complete before the combine
     if (overlap) cudaStreamWaitEvent (st, m->ev_join, 0);
@@ -1872,8 +1900,8 @@ release_mixed (Ctx *c)
   if (!c->mixed) return;
   MixedState *m = c->mixed;
   for (DevBuf *b : {&m->kt, &m->qpos, &m->tab, &m->xf, &m->pq, &m->part_real, &m->part_rec,
-                    &m->selfbuf, &m->status, &m->sf, &m->rowm, &m->rot, &m->img_zf,
-                    &m->img_wb, &m->tyz, &m->img, &m->sq, &m->cstart})
+                    &m->selfbuf, &m->status, &m->rot, &m->mix, &m->img, &m->sq, &m->cstart,
+                    &m->prad, &m->pqa, &m->pself})
     b->release ();
   if (m->h_status) cudaFreeHost (m->h_status);
   if (m->gexec) cudaGraphExecDestroy (m->gexec);

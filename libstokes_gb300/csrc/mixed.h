@@ -1,5 +1,5 @@
 // mixed.h -- data shared by the mixed-precision host code (mixed.cu) and its
-// reciprocal-space tensor-core kernels (kspace_tc.cu).
+// reciprocal-space tensor-core kernels (kspace_mix.cu).
 #pragma once
 
 #include <cuda.h>
@@ -7,32 +7,24 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <vector>
+
 namespace lsg {
 
-// one half-space reciprocal vector (64 bytes); r: its (m2, m3) row of the
-// tensor-core contraction
+// floor(v) mod 2^32 for |v| < 2^62: the 32-bit fixed-point coordinate, the
+// periodic wrap being the modulo
+__device__ __forceinline__ uint32_t
+fixq (double v)
+{
+  return (uint32_t) (unsigned long long) __double2ll_rd (v);
+}
+
+// one half-space reciprocal vector (64 bytes)
 struct __align__ (16) MixK {
-  int m1, m2, m3, r;
+  int m1, m2, m3, pad;
   float ex, ey, ez;
   float ya, yb, yc, yg, yh, ym;
   float f0, f1, f2;
-};
-
-// per-axis phase tables e^{2 pi i m u_j}: tab[off_d + m * np + j], m = 0..M_d;
-// qpos: the 32-bit fixed-point fractional coordinates the tables come from
-// (x, y, z, pad per particle); rot: the 1024 rotations of phase_of
-struct PhaseTables {
-  const float2 *tab;
-  size_t off1, off2;
-  int M0, M1, M2;
-  int np;
-  const uint4 *qpos;
-  const float4 *rot;
-  // particle-major y and z phases for both signs of m: tyz[j wyz + M1 + m2]
-  // = e^{2 pi i m2 u_y(j)}, tyz[j wyz + (2 M1 + 1) + M2 + m3] = e^{2 pi i m3
-  // u_z(j)}, wyz = (2 M1 + 1) + (2 M2 + 1)
-  const float2 *tyz;
-  int wyz;
 };
 
 // e^{2 pi i p / 2^32} to FP32 accuracy from a fixed-point phase p (turns x
@@ -57,94 +49,78 @@ phase_of (const float4 *rot, uint32_t p)
   return make_float2 (re, im);
 }
 
-// e^{2 pi i p / 2^32} without a table: the nearest quarter turn q (exact:
-// a swap and sign change) and sin, cos of the remaining angle |x| <= pi / 4
-// by their Taylor series to x^11 and x^12 in nested (Horner) form; x is
-// formed from the exact integer remainder with a two-part 2 pi / 2^32.  The
-// truncation errors are below 1e-11; FP32 rounding leaves about 1e-7 at most
-// (8.5e-8 measured over 3e6 random phases, 2e-8 on average).  No memory
-// access, so it suits kernels whose lanes would otherwise gather from a table.
-__device__ __forceinline__ float2
-phase_poly (uint32_t p)
-{
-  const uint32_t q = (p + (1u << 29)) >> 30;             // nearest quarter turn
-  const int32_t r = (int32_t) (p - (q << 30));           // |r| <= 2^29
-  const float ch = 1.4629180792671596e-09f;               // 2 pi / 2^32 = ch + cl
-  const float cl = -4.0709404e-17f;
-  const float rh = (float) (r & ~0xFF), rl = (float) (r & 0xFF);
-  const float x = fmaf (rh, ch, fmaf (rl, ch, rh * cl));
-  const float x2 = x * x;
-  float sn = fmaf (-x2, 1.0f / 110.0f, 1.0f);
-  sn = fmaf (-x2 * (1.0f / 72.0f), sn, 1.0f);
-  sn = fmaf (-x2 * (1.0f / 42.0f), sn, 1.0f);
-  sn = fmaf (-x2 * (1.0f / 20.0f), sn, 1.0f);
-  sn = fmaf (-x2 * (1.0f / 6.0f), sn, 1.0f);
-  sn *= x;
-  float cs = fmaf (-x2, 1.0f / 132.0f, 1.0f);
-  cs = fmaf (-x2 * (1.0f / 90.0f), cs, 1.0f);
-  cs = fmaf (-x2 * (1.0f / 56.0f), cs, 1.0f);
-  cs = fmaf (-x2 * (1.0f / 30.0f), cs, 1.0f);
-  cs = fmaf (-x2 * (1.0f / 12.0f), cs, 1.0f);
-  cs = fmaf (-x2 * 0.5f, cs, 1.0f);
-  switch (q & 3u)
-    {
-    case 0: return make_float2 (cs, sn);
-    case 1: return make_float2 (-sn, cs);
-    case 2: return make_float2 (-cs, -sn);
-    default: return make_float2 (sn, -cs);
-    }
-}
+// weights of one reciprocal vector on the tensor-core path: direction and the
+// six scalars of recip_apply
+struct __align__ (16) MixCoef {
+  float ex, ey, ez, ya, yb, yc, yg, yh, ym, p0, p1, p2;
+};
 
-// plan of the separable tensor-core reciprocal sum (kspace_tc.cu).  The k
-// vectors of the list are (m1, row) with row = one (m2, m3) combination that
-// occurs in it; R rows, n1 = M0 + 1 values of m1.  The B operands of the
-// GEMMs are images [2 planes: TF32 hi, lo][rows][K] in FP32 (K contiguous):
-//   ZF [NZ][KF]  rows (m1, re|im, q): t0[m1](j) x_q(j) in the forward sign pattern
-//   WB [NZ][KB]  rows (m1, re|im, q): the k operators W in the backward pattern
-// The A operands (the row phases T_r(j)) are built in shared memory by the
-// GEMM kernels themselves.
-struct KGemm {
-  PhaseTables t;
-  const int2 *rowm;       // (m2, m3) of each row, R entries
-  int R, Rk, Rp;          // rows; padded to 16 (backward K) and 32 (partials)
-  int c;                  // components per particle (3, 6, 11)
-  int n1;                 // M0 + 1
-  int nrt;                // forward row tiles of 128 rows
-  int gf, ntile_f, nf;    // m1 per forward column tile, tiles, MMA N
-  int jper, nsplit;       // particles per forward K slice, number of slices
-  int gb, ntile_b, nb;    // m1 per backward column tile, tiles, MMA N
-  int mtiles;             // 128-particle row tiles of the backward GEMM
-  int rper, ksplit;       // rows per backward K slice, number of slices
-  int ldT;                // particles padded to a multiple of 16
-  int KF, KB, NZ;         // K extents (floats) of the images, rows of ZF and WB
-  float *ZF, *WB;
-  size_t pZF, pWB;        // plane strides (floats)
-  float *sf;              // forward partials [nsplit][n1][c][re|im][Rp]
+// plan of the tensor-core reciprocal sum (kspace_mix.cu).  Functions of an
+// axis: index 0 is 1, 2 m - 1 is cos 2 pi m u, 2 m is sin 2 pi m u.
+//   quarter  one (|m2|, |m3|) of the k list, sorted by length
+//   row      4 quarter + 2 p2 + p3, p = 0 cosine, 1 sine: f_y f_z
+//   column   mi c + q, mi the x function index, q one of c components (cf
+//            forward, cb backward)
+struct MixPlan {
+  int np, M[3];
+  int cf, cb;             // components per x function, forward and backward
+  int nmi, ncolf, ncolb;  // x functions 2 M[0] + 1; columns
+  int nq, nqp, Rp;        // quarters; padded to 32; rows 4 nqp
+  int ldT;                // particles padded to 128
+  int oy, oz, zero, nT;   // table rows: x from 0, y, z, the zero row, total
+  int tnf, nctf, ldf;     // forward columns per tile, tiles, padded columns
+  int tnb, nctb, ldb;     // backward
+  int mt;                 // 128-particle tiles
+  int jper, nsplit;       // particles per forward slice, slices
+  int nfitem, nbitem;     // work items
   int stall;              // > 0 (tests only): the MMA lane first waits that many
                           // polls on an mbarrier that nothing arrives at
+  const int4 *quart;      // [nqp] table rows of (cos y, sin y, cos z, sin z)
+  const int *nqm;         // [M0 + 1] quarters in use at |m1|
+  const int *off;         // [M0 + 2] first octant point of |m1|
+  const MixCoef *coef;    // [octant points][4 sign patterns]
+  const int4 *fitem;      // forward: row tile, column tile, particle slice
+  const int4 *bitem;      // backward: column tile, first K tile, K tiles
+  int *T;                 // function table [nT][ldT], 30 fractional bits
+  float *zs;              // units of ZF, [ldT / 128][ldf]
+  float *ws;              // units of WB, [Rp / 128][ldb]
+  void *ZF, *WB;          // images, f16 digits [3][columns][ldT or Rp]
+  float *F;               // structure factors [nsplit][ncolf][Rp]
+  float *yp;              // back-projection partials [nbitem][np][cb]
 };
 
-// TMA descriptors of the two images (128-byte swizzled boxes of 32 K values)
-// and of the forward partials sf (boxes of 128 rows x one m1's columns)
-struct KMaps {
-  CUtensorMap zf, wb, sf;
+// TMA descriptors of the two images
+struct MixMaps {
+  CUtensorMap zf, wb;
 };
 
-KGemm kgemm_plan (int version, PhaseTables t, const int2 *rowm, int R);
-bool kgemm_fits (const KGemm &g);
-size_t kgemm_sf_floats (const KGemm &g);      // partial structure factors
-size_t kgemm_zf_floats (const KGemm &g);      // image sizes, both planes
-size_t kgemm_wb_floats (const KGemm &g);
-size_t kgemm_ypart_floats (const KGemm &g);   // partial y, [ksplit][ntile_b][np][c]
-int kgemm_ypart_chunks (const KGemm &g);       // ksplit * ntile_b
-int kgemm_maps (const KGemm &g, float *sf, KMaps *m);   // 0 on success
+struct MixPrep {
+  const double *pos, *x;
+  int np, c;
+  double sx, sy, sz;      // 2^32 / L_d
+  double shift, sl;       // Lees-Edwards shift (flow axis x), shift / lx
+  int shear_mode;
+  const float4 *rot;      // rotations of phase_of
+  const float *qa;        // unequal radii: squared radii
+  uint32_t *qpos;         // [np][4] fixed-point x, y, z (+ pad)
+  float *xf;              // [np][c padded to 4]
+  MixPlan p;
+};
 
-// forward GEMM -> per-k operators (image WB); then the backward GEMM into
-// ypart.  The image ZF is written beforehand by mk_prep.
+void mix_plan_items (MixPlan &p, const std::vector<int> &nqm, std::vector<int4> &fwd,
+                     std::vector<int4> &bwd);
+size_t mix_zf_bytes (const MixPlan &p);
+size_t mix_wb_bytes (const MixPlan &p);
+size_t mix_zs_floats (const MixPlan &p);
+size_t mix_ws_floats (const MixPlan &p);
+int mix_maps (const MixPlan &p, MixMaps *m);      // 0 on success
+
+// prep -> forward GEMM and operators -> backward GEMM into yp
 struct Ctx;
-cudaError_t launch_kspace_forward (int version, const KGemm &g, const KMaps &maps, const MixK *kt,
-                                   int nk, int *status, cudaStream_t st, Ctx *prof);
-cudaError_t launch_kspace_backward (int version, const KGemm &g, const KMaps &maps, float *ypart,
-                                    int *status, cudaStream_t st, Ctx *prof);
+cudaError_t launch_mix_prep (const MixPrep &a, cudaStream_t st);
+cudaError_t launch_mix_forward (int version, const MixPlan &p, const MixMaps &m, int *status,
+                                cudaStream_t st, Ctx *prof);
+cudaError_t launch_mix_backward (const MixPlan &p, const MixMaps &m, int *status, cudaStream_t st,
+                                 Ctx *prof);
 
 }  // namespace lsg

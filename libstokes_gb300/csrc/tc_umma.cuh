@@ -83,14 +83,6 @@ smem_u32 (const void *p)
   return (uint32_t) __cvta_generic_to_shared (p);
 }
 
-__device__ __forceinline__ uint32_t
-to_tf32 (float x)
-{
-  uint32_t r;
-  asm volatile ("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
-
 // TF32 rounding of an FP32 bit pattern, to nearest with ties away from zero
 // (the rounding of cvt.rna.tf32.f32): add half a TF32 unit to the magnitude
 // bits and clear the 13 bits below TF32's mantissa; a carry moves into the
@@ -108,13 +100,6 @@ split_tf32 (float x, uint32_t &hi, uint32_t &lo)
 {
   hi = rna_tf32_bits (__float_as_uint (x));
   lo = rna_tf32_bits (__float_as_uint (x - __uint_as_float (hi)));
-}
-
-// an L1 prefetch of the line holding p (no register result)
-__device__ __forceinline__ void
-prefetch_l1 (const void *p)
-{
-  asm volatile ("prefetch.global.L1 [%0];" :: "l"(p));
 }
 
 // TMEM allocation by one full warp; the column address lands in *slot
@@ -144,14 +129,19 @@ mma_tf32 (uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint3
     :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-// the same with f16 operands (K = 16 per instruction)
+// the same with f16 operands (K = 16 per instruction), called by a whole
+// converged warp: one elected lane issues it.  The descriptors are then warp
+// uniform and live in uniform registers; issued from a branch on one lane each
+// MMA first moved them there (about 115 clocks an MMA instead of the 32 to 96
+// that the tensor pipe takes).
 __device__ __forceinline__ void
 mma_f16 (uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
 {
   asm volatile (
-    "{\n\t.reg .pred p;\n\t"
+    "{\n\t.reg .pred p, q;\n\t"
+    "elect.sync _|q, 0xffffffff;\n\t"
     "setp.ne.b32 p, %4, 0;\n\t"
-    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+    "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
     :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
@@ -160,6 +150,16 @@ __device__ __forceinline__ void
 mma_commit (uint64_t *mbar)
 {
   asm volatile ("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                :: "r"(smem_u32 (mbar)) : "memory");
+}
+
+// the same from a whole converged warp (the lane that mma_f16 elects)
+__device__ __forceinline__ void
+mma_commit_warp (uint64_t *mbar)
+{
+  asm volatile ("{\n\t.reg .pred q;\n\t"
+                "elect.sync _|q, 0xffffffff;\n\t"
+                "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
                 :: "r"(smem_u32 (mbar)) : "memory");
 }
 
@@ -250,30 +250,6 @@ tma_load_3d (void *dst, const void *tmap, int c0, int c1, int c2, uint64_t *mbar
     " [%0], [%1, {%2, %3, %4}], [%5];"
     :: "r"(smem_u32 (dst)), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32 (mbar))
     : "memory");
-}
-
-// 2-d tiled TMA store of one box from shared memory (128-byte aligned, the
-// box's rows back to back) to coordinates (c0, c1); parts of the box outside
-// the tensor are not written.  Completes asynchronously: commit the group and
-// wait before the shared memory is reused.
-__device__ __forceinline__ void
-tma_store_2d (const void *tmap, const void *src, int c0, int c1)
-{
-  asm volatile ("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-                :: "l"(tmap), "r"(smem_u32 (src)), "r"(c0), "r"(c1) : "memory");
-}
-
-__device__ __forceinline__ void
-bulk_commit ()
-{
-  asm volatile ("cp.async.bulk.commit_group;" ::: "memory");
-}
-
-// wait until every committed bulk store has finished reading shared memory
-__device__ __forceinline__ void
-bulk_wait_read ()
-{
-  asm volatile ("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
 __device__ __forceinline__ void
