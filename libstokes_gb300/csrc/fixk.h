@@ -17,6 +17,18 @@ struct __align__ (16) FixCoef {
   double ex, ey, ez, ya, yb, yc, yg, yh, ym, pad;
 };
 
+// Columns and rows of the dense builder (dense_fix.cu): the functions along y
+// and z of a class have one parity each, so its K rows are products of these
+// alone, in blocks of 2 x 2 (|m2|, |m3|), and its columns are (|m1|, q), q a
+// pair moment of the class.  Components whose bit in `odd` is set go with
+// sin(2 pi m1 x), the others with the cosine.
+struct FixClass {
+  int col0, ncol, nc;         // first column (a tile's), columns, components
+  int row0, nblk, nq0;        // first row of S, blocks, first entry in nqm
+  int odd;
+  int slot0, nslot;           // its slots of partial results
+};
+
 // Plan of one reciprocal sum.  The k vectors are (m1, m2, m3) with m1 along x;
 // an octant point is (|m1|, |m2|, |m3|).  Everything is expanded in products
 // of real functions: function index 0 of an axis is 1, 2 m - 1 is
@@ -60,7 +72,10 @@ struct FixPlan {
   unsigned *mx = nullptr;
   const int4 *fitem = nullptr;     // forward: row tile, column tile, particle slice
   const int4 *bitem = nullptr;     // backward: column tile, first K tile, K tiles
-  void *yp = nullptr;         // back-projection partials [nbitem][np][c]
+  void *yp = nullptr;         // back-projection partials [nbitem][np][c]; dense [slot][16][ldT]
+
+  // dense builder: four classes; "particles" are the pairs of a chunk
+  FixClass cls[4];
 };
 
 constexpr int XF_LD = 12;     // floats per particle of xf
@@ -69,7 +84,12 @@ struct FixMaps {
   CUtensorMap zf, wb;
 };
 
-inline size_t fix_mx_words (const FixPlan &p) { return 16 * ((size_t) p.M[0] + 2); }
+// words of mx (a class of the dense builder; 16 (|m1| + 1) + component)
+__host__ __device__ inline size_t
+fix_mx_words (const FixPlan &p)
+{
+  return 16 * ((size_t) p.M[0] + 2);
+}
 
 // host entry points of kspace_fix.cu; ND: digits per number, 7 (FP64)
 size_t fix_bytes_T (int nd, const FixPlan &p);
@@ -91,5 +111,18 @@ cudaError_t launch_fix_forward (int nd, int version, const FixPlan &p, const Fix
                                 cudaStream_t st, Ctx *prof);
 cudaError_t launch_fix_backward (int nd, int version, const FixPlan &p, const FixMaps &m,
                                  int *status, cudaStream_t st, Ctx *prof);
+
+// dense builder: columns, items and maps of its classes (cls[] holds nc, nblk
+// and odd; nqm blocks in use by class and |m1|)
+void fix_plan_dense (FixPlan &p, const std::vector<int> &nqm, std::vector<int4> &items);
+int fix_map_wb (const FixPlan &p, FixMaps *m);
+// function table of np positions (no strings or images)
+cudaError_t launch_fix_functions (const FixPlan &p, const double *pos, cudaStream_t st);
+// digits of G into the backward image
+cudaError_t launch_fix_dense_image (const FixPlan &p, cudaStream_t st);
+// partial moments of the pairs of `ntile` 8 x 8 tiles (tile[]: row, column of
+// the tile) from the function table of the particles
+cudaError_t launch_fix_dense (const FixPlan &particles, const FixPlan &p, const FixMaps &m,
+                              const int2 *tile, int ntile, int *status, cudaStream_t st, Ctx *prof);
 
 }  // namespace lsg

@@ -143,6 +143,7 @@ free_ctx (Ctx *c)
   cudaStreamDestroy (c->stream);
   release_mixed (c);
   release_fix (c);
+  release_dense (c);
   release_vjp_mixed (c);
   if (c->tuned) stokes_free (c->tuned);
   if (c->dense) stokes_free (c->dense);
@@ -511,6 +512,7 @@ prepare (Ctx *c, const struct stokes *sys, bool cube, int tables)
   c->sys = sys;
   c->cube = cube;
   c->use_fix = false;
+  c->use_dense = false;
   c->version = sys->version;
   c->np = sys->np;
   c->mode = sys->slip ? MODE_SLIP : (sys->a ? MODE_POLY : MODE_MONO);
@@ -529,10 +531,18 @@ prepare (Ctx *c, const struct stokes *sys, bool cube, int tables)
   // the free-space products (FP64 and mixed) read the particle table and the
   // FP64 set-up of the open system
   if (tables < 0) tables = c->precision == STOKES_GPU_MIXED && !c->open ? 0 : 1;
-  // the dense builder pays for every k vector once per pair: it keeps the
-  // reference's split, which is light in reciprocal space
+  // the dense builders of unequal radii, slip, sheared boxes and the cube
+  // list pay for every k vector once per pair: they keep the reference's
+  // split, which is light in reciprocal space
   const bool dense = tables == 2;
   if (dense) tables = 1;
+  if (dense && c->tune && c->precision == STOKES_GPU_FP64 && !cube && !c->open && sys->periodic
+      && c->mode == MODE_MONO && sys->shear_mode == 0 && sys->np > 0 && split_is_as_set (sys)
+      && dense_fix_applies (c, sys))
+    {
+      c->use_dense = true;        // its tables are made by the first build
+      return STOKES_GPU_OK;
+    }
   if (!tables)
     {
       // the particle table only (radii for the BD interactions); equal
@@ -984,6 +994,7 @@ matrix_pairs_dev (Ctx *c, const struct stokes *sys, const double *d_pos, double 
 int
 matrix_dev (Ctx *c, const double *d_pos, double *d_mat, cudaStream_t st)
 {
+  if (c->use_dense) return matrix_fix_dev (c, d_pos, d_mat, st);
   if (c->sys && dense_pairs_apply (c, c->sys)) return matrix_pairs_dev (c, c->sys, d_pos, d_mat, st);
   const int np = c->np;
   cudaError_t e;
@@ -1087,6 +1098,7 @@ matrix_host (struct stokes *sys, double *mat, bool cube)
   e = cudaMemcpyAsync (mat, c->mat.p, sizeof (double) * n * n, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
   if (e != cudaSuccess) return cuda_fail (e, "matrix");
+  if (c->use_dense && (rc = dense_check_status (c)) != 0) return rc;
   float t = 0.f;
   cudaEventElapsedTime (&t, c->ev[0], c->ev[3]);
   sys->cpu1 = t;
@@ -1123,6 +1135,7 @@ atimes_matrix_host (struct stokes *sys, const double *x, double *y, bool cube)
   e = cudaMemcpyAsync (y, c->y.p, sizeof (double) * n, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
   if (e != cudaSuccess) return cuda_fail (e, "atimes_3all_matrix");
+  if (c->use_dense && (rc = dense_check_status (c)) != 0) return rc;
   return STOKES_GPU_OK;
 }
 

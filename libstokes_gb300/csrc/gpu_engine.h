@@ -20,6 +20,7 @@ struct DevBuf {
 };
 
 struct MixedState;   // mixed-precision state (mixed.cu)
+struct DenseState;   // FP64 dense builder on the tensor cores (dense_fix.cu)
 struct FixState;     // FP64 product with the fixed-point reciprocal sum (product_fix.cu)
 
 struct Ctx {
@@ -74,6 +75,9 @@ struct Ctx {
   FixState *fix = nullptr;
   bool use_fix = false;
   const struct stokes *fix_split = nullptr;   // the tuned split of that prepare
+  // the FP64 dense builder of equal spheres (dense_fix.cu), likewise
+  DenseState *dfix = nullptr;
+  bool use_dense = false;
 
   DevBuf openf;   // scratch of the mixed-precision free-space product
   DevBuf imgf;    // the images in FP32 (split-precision dense builder)
@@ -142,6 +146,11 @@ int atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
                     bool timed);
 int fix_check_status (Ctx *c);
 void release_fix (Ctx *c);
+// the dense matrix of equal spheres in FP64 (dense_fix.cu)
+bool dense_fix_applies (const Ctx *c, const struct stokes *sys);
+int matrix_fix_dev (Ctx *c, const double *d_pos, double *d_mat, cudaStream_t st);
+int dense_check_status (Ctx *c);
+void release_dense (Ctx *c);
 void collect_times (Ctx *c);
 cudaEvent_t *phase_events (Ctx *c, bool timed);
 // record a kernel-profiling mark on st when the window is open

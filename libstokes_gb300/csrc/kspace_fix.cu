@@ -367,11 +367,11 @@ col_m (const FixPlan &p, int n)
   return (n / p.c + 1) / 2;              // |m1| of column n
 }
 
-// first column of component q in the tile that starts at column n0
+// first column of component q, of c, in the tile that starts at column n0
 __device__ __forceinline__ int
-first_col (const FixPlan &p, int n0, int q)
+first_col (int c, int n0, int q)
 {
-  return (q + p.c - n0 % p.c) % p.c;
+  return (q + c - n0 % c) % c;
 }
 
 constexpr int NOT_FINITE = 1 << 20;
@@ -417,17 +417,20 @@ k_fix_fwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
 // 128-bit integers (an FP64 operation on the 128 x 64 tile takes the FP64 pipe
 // 4096 clocks, a 64 x 64 bit product of integers about a tenth): the columns'
 // different units 2^E come in as a right shift of the table entry.
-template <int ND>
+//
+// DENSE: the moments of 128 pairs, columns and rows by class (FixClass).
+template <int ND, bool DENSE>
 __global__ void __launch_bounds__ (NT, 1)
-k_fix_bwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
+k_fix_bwd (const __grid_constant__ CUtensorMap tmB, const __grid_constant__ FixPlan p, int *status)
 {
   using C = Cfg<ND>;
   using G = Geo<ND>;
   constexpr int HLD = C::TN + 1;
   constexpr uint32_t H_LO = TM * HLD * sizeof (long long);
   constexpr uint32_t X_OFF = H_LO + TM * HLD * sizeof (float);
-  // the parked sums and the x functions of 64 columns (three components: 23)
-  static_assert (X_OFF + 23 * TM * sizeof (long long) <= G::NS * G::STAGE, "parked tile");
+  // the parked sums and the x functions of 64 columns (a class of one
+  // component: 64)
+  static_assert (X_OFF + 64 * TM * sizeof (long long) <= G::NS * G::STAGE, "parked tile");
   extern __shared__ unsigned char dsm[];
   __shared__ Sync s;
   __shared__ int s_exp[C::TN], s_top[16];
@@ -435,28 +438,41 @@ k_fix_bwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int4 it = p.bitem[blockIdx.y];
   const int i0 = blockIdx.x * TM, n0 = it.x * C::TN;
-  const int ne = min (C::TN, p.ncol - n0);
+  // columns n of the tile are column nb + n of the list (x function or |m1|,
+  // component), nc components each
+  int cl = 0, nb = n0, nc = p.c, ncol = p.ncol, row0 = 0;
+  const unsigned *mx = p.mx;
+  if constexpr (DENSE)
+    {
+      while (cl < 3 && n0 >= p.cls[cl + 1].col0) cl++;
+      nb = n0 - p.cls[cl].col0;
+      nc = p.cls[cl].nc;
+      ncol = p.cls[cl].ncol;
+      row0 = p.cls[cl].row0;
+      mx += cl * fix_mx_words (p);
+    }
+  const int ne = min (C::TN, ncol - nb);
   if ((int) threadIdx.x < ne)
     {
-      const int n = n0 + threadIdx.x;
+      const int n = nb + threadIdx.x, m1 = DENSE ? n / nc : (n / nc + 1) / 2;
       bool finite;
-      const int E = scale_exp (p.mx[16 * (col_m (p, n) + 1) + n % p.c], finite);
+      const int E = scale_exp (mx[16 * (m1 + 1) + n % nc], finite);
       s_exp[threadIdx.x] = finite ? E : NOT_FINITE;
     }
   const int tb = it.y, ntiles = it.z;
   cta_setup (s);
   const uint32_t tmem = s.tslot;
   // the largest unit of each component
-  if ((int) threadIdx.x < p.c)
+  if ((int) threadIdx.x < nc)
     {
       int top = -2000;
-      for (int n = first_col (p, n0, threadIdx.x); n < ne; n += p.c) top = max (top, s_exp[n]);
+      for (int n = first_col (nc, nb, threadIdx.x); n < ne; n += nc) top = max (top, s_exp[n]);
       s_top[threadIdx.x] = top;
     }
   {
     Acc<ND> acc;
     acc.zero (worker_tmem (tmem, G::CPT));
-    BuildB<ND> build (p, i0, tb * C::KT);
+    BuildB<ND> build (p, i0, row0 + tb * C::KT);
     const BTiles bt {&tmB, G::PAIR * tb * C::KT, G::PAIR * C::KT, n0, G::A_BYTES, G::B_BYTES};
     if (run_tiles<C::DK, 1, G::NS> (s, smem, ntiles, G::STAGE, bt, p.stall, build, acc,
                                     [=] (uint32_t a, int, bool first) {
@@ -483,33 +499,48 @@ k_fix_bwd (const __grid_constant__ CUtensorMap tmB, FixPlan p, int *status)
       const float *Lo = reinterpret_cast<const float *> (smem + H_LO);
       // the x functions of the tile's columns, in one pass (a load per term
       // would wait for L2 every time)
-      const int f0 = n0 / p.c, nf = (n0 + ne - 1) / p.c - f0 + 1;
+      const int f0 = nb / nc, nf = (nb + ne - 1) / nc - f0 + 1;
       long long *X = reinterpret_cast<long long *> (smem + X_OFF);
       const long long *T = (const long long *) p.T;
-      for (int e = threadIdx.x; e < nf * TM; e += NT)
-        X[e] = T[(size_t) (f0 + e / TM) * p.ldT + i0 + e % TM];
+      // DENSE: function k of |m1| = f0 + k / 2 where a class has both parities
+      const int odd = DENSE ? p.cls[cl].odd : 0;
+      const bool both = DENSE && odd != 0 && odd != (1 << nc) - 1;
+      const int np2 = both ? 2 : 1;
+      for (int e = threadIdx.x; e < np2 * nf * TM; e += NT)
+        {
+          int f = f0 + e / TM;
+          if constexpr (DENSE)
+            {
+              const int m1 = f0 + (e / TM) / np2, sine = both ? (e / TM) & 1 : odd & 1;
+              f = sine ? (m1 ? 2 * m1 : p.zero) : (m1 ? 2 * m1 - 1 : 0);
+            }
+          X[e] = T[(size_t) f * p.ldT + i0 + e % TM];
+        }
       __syncthreads ();
-      double *yp = (double *) p.yp + (size_t) blockIdx.y * p.np * p.c;
-      for (int e = threadIdx.x; e < TM * p.c; e += NT)
+      for (int e = threadIdx.x; e < TM * nc; e += NT)
         {
           const int q = e / TM, r = e - q * TM, i = i0 + r;
-          if (i >= p.np) continue;
+          if (!DENSE && i >= p.np) continue;
           const int top = s_top[q];
           __int128 y = 0;
           float yl = 0.f;
-          for (int n = first_col (p, n0, q); n < ne; n += p.c)
+          for (int n = first_col (nc, nb, q); n < ne; n += nc)
             {
               const int sh = top - s_exp[n];
               if (sh > 62) continue;              // below the last bit
-              const long long f = X[((n0 + n) / p.c - f0) * TM + r] >> sh;
+              const int k = DENSE ? np2 * ((nb + n) / nc - f0) + (both ? odd >> q & 1 : 0)
+                                  : (nb + n) / nc - f0;
+              const long long f = X[k * TM + r] >> sh;
               y += (__int128) f * Hi[r * HLD + n];
               yl = fmaf ((float) (int) (f >> 32), Lo[r * HLD + n], yl);
             }
           // y: 62 + 38 fractional bits, yl: 30 + 38
           const double v = (double) (long long) (y >> 64) * 0x1p-36
                            + (double) (unsigned long long) y * 0x1p-100 + (double) yl * 0x1p-68;
-          yp[(size_t) i * p.c + q] = top == NOT_FINITE ? __longlong_as_double (0x7ff8000000000000ll)
-                                                       : scalbn (v, top);
+          double *o = (double *) p.yp;
+          if constexpr (DENSE) o += ((size_t) it.w * 16 + q) * p.ldT + i;
+          else o += ((size_t) blockIdx.y * p.np + i) * p.c + q;
+          *o = top == NOT_FINITE ? __longlong_as_double (0x7ff8000000000000ll) : scalbn (v, top);
         }
     }
   cta_finish (s, tmem, status);
@@ -724,13 +755,32 @@ k_fix_kop (FixPlan p)
 }
 
 // Backward image: digits of G, eight rows per thread
+template <bool DENSE>
 __global__ void __launch_bounds__ (128)
-k_fix_gimage (FixPlan p)
+k_fix_gimage (const __grid_constant__ FixPlan p)
 {
   const int n = blockIdx.y, r8 = blockIdx.x * 128 + threadIdx.x;
-  if (8 * r8 >= 4 * p.nqm[col_m (p, n)]) return;
+  int m1, rows;
+  const unsigned *mx = p.mx;
+  if constexpr (DENSE)
+    {
+      int cl = 0;
+      while (cl < 3 && n >= p.cls[cl + 1].col0) cl++;
+      const int nl = n - p.cls[cl].col0, nc = p.cls[cl].nc;
+      if (nl >= p.cls[cl].ncol) return;
+      m1 = nl / nc;
+      rows = 4 * p.nqm[p.cls[cl].nq0 + m1];
+      mx += cl * fix_mx_words (p) + 16 * (m1 + 1) + nl % nc;
+    }
+  else
+    {
+      m1 = col_m (p, n);
+      rows = 4 * p.nqm[m1];
+      mx += 16 * (m1 + 1) + n % p.c;
+    }
+  if (8 * r8 >= rows) return;
   bool finite;
-  const int E = scale_exp (p.mx[16 * (col_m (p, n) + 1) + n % p.c], finite);
+  const int E = scale_exp (*mx, finite);
   const double *g = (const double *) p.G + (size_t) n * p.Rp + 8 * r8;
   uint32_t w[4][7];
 #pragma unroll
@@ -745,6 +795,48 @@ k_fix_gimage (FixPlan p)
   for (int d = 0; d < 7; d++)
     *reinterpret_cast<uint4 *> ((__half *) p.WB + image_off<7> (d, p.ncol, n, p.Rp, 8 * r8))
       = make_uint4 (w[0][d], w[1][d], w[2][d], w[3][d]);
+}
+
+// ---- dense builder --------------------------------------------------------
+// f g with 62 fractional bits, both with 62
+__device__ __forceinline__ long long
+mul62 (Limbs f, Limbs g)
+{
+  const long long cross = (long long) f.hi * g.lo + (long long) f.lo * g.hi;
+  return (((long long) f.hi * g.hi) << 2) + (cross >> 30);
+}
+
+// Function table of the displacements r_j - r_i of an 8 x 8 tile of pairs, by
+// the addition theorem from the functions of the particles in integers: a
+// thread makes the functions of one pair for one (axis, m) in four.  (sincospi
+// of every pair would be 60 FP64 instructions a value.)
+constexpr int PT = 64;                  // pairs of a tile
+__global__ void __launch_bounds__ (4 * PT)
+k_fix_pair_tables (const __grid_constant__ FixPlan a, const __grid_constant__ FixPlan p,
+                   const int2 *tile)
+{
+  const int2 ij = tile[blockIdx.x];
+  const int t = threadIdx.x & (PT - 1);
+  const int i = 8 * ij.x + (t >> 3), j = 8 * ij.y + (t & 7);
+  const long long *A = (const long long *) a.T;
+  long long *T = (long long *) p.T + (size_t) blockIdx.x * PT + t;
+  const int n0 = p.M[0] + 1, n1 = n0 + p.M[1] + 1, n2 = n1 + p.M[2] + 1;
+  for (int item = blockIdx.y * 4 + (threadIdx.x >> 6); item < n2; item += 4 * gridDim.y)
+    {
+      const int d = item < n0 ? 0 : (item < n1 ? 1 : 2);
+      const int m = item - (d == 0 ? 0 : (d == 1 ? n0 : n1));
+      const int row = (d == 0 ? 0 : (d == 1 ? p.oy : p.oz)) + (m ? 2 * m - 1 : 0);
+      if (m == 0)
+        {
+          T[(size_t) row * p.ldT] = 1ll << 62;
+          continue;
+        }
+      const long long *r = A + (size_t) row * a.ldT;
+      const Limbs ci = limbs (r[i]), si = limbs (r[a.ldT + i]);
+      const Limbs cj = limbs (r[j]), sj = limbs (r[a.ldT + j]);
+      T[(size_t) row * p.ldT] = mul62 (cj, ci) + mul62 (sj, si);
+      T[(size_t) (row + 1) * p.ldT] = mul62 (sj, ci) - mul62 (cj, si);
+    }
 }
 
 template <int ND, int V>
@@ -766,7 +858,10 @@ gemm_attrs ()
   if ((e = cudaFuncSetAttribute (k_fix_fwd<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int) Geo<7>::SMEM)) != cudaSuccess)
     return e;
-  if ((e = cudaFuncSetAttribute (k_fix_bwd<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if ((e = cudaFuncSetAttribute (k_fix_bwd<7, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int) Geo<7>::SMEM)) != cudaSuccess)
+    return e;
+  if ((e = cudaFuncSetAttribute (k_fix_bwd<7, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int) Geo<7>::SMEM)) != cudaSuccess)
     return e;
   attr_dev = dev;
@@ -799,6 +894,45 @@ fix_bytes_yp (int, const FixPlan &p)
 // in K tiles; a CTA's start and end cost about START tiles (measured: a
 // 4-tile forward CTA takes as long as 7 tiles of a long one).
 constexpr int START = 3;               // start and end of a CTA, in K tiles
+
+// backward items (column tile, first K tile, K tiles) from the K tiles of each
+// column tile, for mt tiles of 128 particles: slices of about equal length
+static void
+slice_rows (const std::vector<int> &tiles, int mt, std::vector<int4> &items)
+{
+  long long best = -1;
+  int slice = 1;
+  const int most = *std::max_element (tiles.begin (), tiles.end ());
+  for (int s = 1; s <= 24; s++)
+    {
+      const int l = std::max (1, (most + s - 1) / s);
+      if (s > 1 && l < 4) break;
+      std::vector<int> len;
+      for (int k : tiles)
+        {
+          const int n = std::max (1, (k + l - 1) / l);
+          for (int z = 0; z < n; z++) len.push_back ((k + n - 1) / n);
+        }
+      if (s > 1 && len.size () > 96) break;
+      const long long t = makespan (len, mt, START);
+      if (best < 0 || t < best)
+        {
+          best = t;
+          slice = l;
+        }
+    }
+  items.clear ();
+  for (size_t ct = 0; ct < tiles.size (); ct++)
+    {
+      const int k = tiles[ct], n = std::max (1, (k + slice - 1) / slice);
+      for (int z = 0; z < n; z++)
+        {
+          const int a = (int) ((long long) k * z / n), b = (int) ((long long) k * (z + 1) / n);
+          items.push_back (make_int4 ((int) ct, a, b - a, 0));
+        }
+    }
+  std::stable_sort (items.begin (), items.end (), [] (const int4 &a, const int4 &b) { return a.z > b.z; });
+}
 
 // Work items of the two GEMMs.  A column tile needs the quarters that its
 // smallest |m1| uses (nqm): the forward has no item for row tiles past them,
@@ -837,39 +971,8 @@ fix_plan_items (int, FixPlan &p, const std::vector<int> &nqm, std::vector<int4> 
     for (int ct = 0; ct < p.nct; ct++)
       for (int rt = 0; rt * TM < rows[ct]; rt++) fwd.push_back (make_int4 (rt, ct, z, 0));
   p.nfitem = (int) fwd.size ();
-  // backward: row slices of about equal length
-  best = -1;
-  int slice = 1;
-  const int most = (rows[0] + C::KT - 1) / C::KT;
-  for (int s = 1; s <= 24; s++)
-    {
-      const int l = (most + s - 1) / s;
-      if (s > 1 && l < 4) break;
-      std::vector<int> len;
-      for (int ct = 0; ct < p.nct; ct++)
-        {
-          const int k = (rows[ct] + C::KT - 1) / C::KT, n = (k + l - 1) / l;
-          for (int z = 0; z < n; z++) len.push_back ((k + n - 1) / n);
-        }
-      if (s > 1 && len.size () > 96) break;
-      const long long t = makespan (len, p.mt, START);
-      if (best < 0 || t < best)
-        {
-          best = t;
-          slice = l;
-        }
-    }
-  bwd.clear ();
-  for (int ct = 0; ct < p.nct; ct++)
-    {
-      const int k = (rows[ct] + C::KT - 1) / C::KT, n = std::max (1, (k + slice - 1) / slice);
-      for (int z = 0; z < n; z++)
-        {
-          const int a = (int) ((long long) k * z / n), b = (int) ((long long) k * (z + 1) / n);
-          bwd.push_back (make_int4 (ct, a, b - a, 0));
-        }
-    }
-  std::stable_sort (bwd.begin (), bwd.end (), [] (const int4 &a, const int4 &b) { return a.z > b.z; });
+  for (int &r : rows) r = (r + C::KT - 1) / C::KT;
+  slice_rows (rows, p.mt, bwd);
   p.nbitem = (int) bwd.size ();
   // |F| <= np in units of its component, and the operators add four of them
   int lg = 0;
@@ -920,9 +1023,88 @@ cudaError_t
 launch_fix_backward (int, int, const FixPlan &p, const FixMaps &m, int *status, cudaStream_t st,
                      Ctx *prof)
 {
-  k_fix_gimage<<<dim3 ((p.Rp / 8 + 127) / 128, p.ncol), 128, 0, st>>> (p);
+  k_fix_gimage<false><<<dim3 ((p.Rp / 8 + 127) / 128, p.ncol), 128, 0, st>>> (p);
   kmark (prof, st, "k_fix_gimage");
-  k_fix_bwd<7><<<dim3 (p.mt, p.nbitem), NT, Geo<7>::SMEM, st>>> (m.wb, p, status);
+  k_fix_bwd<7, false><<<dim3 (p.mt, p.nbitem), NT, Geo<7>::SMEM, st>>> (m.wb, p, status);
+  kmark (prof, st, "k_fix_bwd");
+  return cudaGetLastError ();
+}
+
+// ---------------------------------------------------------------------------
+// dense builder
+// ---------------------------------------------------------------------------
+void
+fix_plan_dense (FixPlan &p, const std::vector<int> &nqm, std::vector<int4> &items)
+{
+  using C = Cfg<7>;
+  p.ncol = 0;
+  int row0 = 0, most = 1;
+  for (FixClass &c : p.cls)
+    {
+      c.col0 = p.ncol;
+      c.ncol = (p.M[0] + 1) * c.nc;
+      p.ncol += (c.ncol + C::TN - 1) / C::TN * C::TN;
+      c.row0 = row0;
+      const int rows = (4 * c.nblk + C::KT - 1) / C::KT * C::KT;
+      row0 += rows;
+      most = std::max (most, rows);
+    }
+  p.nqp = row0 / 4;
+  p.Rp = most;
+  p.nct = p.ncol / C::TN;
+  p.mt = p.ldT / TM;
+  std::vector<int> tiles (p.nct);
+  for (const FixClass &c : p.cls)
+    for (int n = 0; n < c.ncol; n += C::TN)
+      tiles[(c.col0 + n) / C::TN] = (4 * nqm[c.nq0 + n / c.nc] + C::KT - 1) / C::KT;
+  slice_rows (tiles, p.mt, items);
+  p.nbitem = (int) items.size ();
+  int slot = 0;
+  for (FixClass &c : p.cls)
+    {
+      c.slot0 = slot;
+      for (int4 &it : items)
+        if (it.x * C::TN >= c.col0 && it.x * C::TN < c.col0 + c.ncol) it.w = slot++;
+      c.nslot = slot - c.slot0;
+    }
+}
+
+int
+fix_map_wb (const FixPlan &p, FixMaps *m)
+{
+  using G = Geo<7>;
+  return encode_planes_f16 (&m->wb, p.WB, G::NP, p.ncol, (size_t) G::PAIR * p.Rp, Cfg<7>::TN);
+}
+
+cudaError_t
+launch_fix_functions (const FixPlan &p, const double *pos, cudaStream_t st)
+{
+  const int items = p.M[0] + p.M[1] + p.M[2] + 3;
+  k_fix_tables<<<dim3 ((p.np + TAB_P - 1) / TAB_P, (items + TAB_R - 1) / TAB_R), TAB_P * TAB_R, 0,
+                 st>>> (p, pos, nullptr);
+  return cudaGetLastError ();
+}
+
+cudaError_t
+launch_fix_dense_image (const FixPlan &p, cudaStream_t st)
+{
+  k_fix_gimage<true><<<dim3 ((p.Rp / 8 + 127) / 128, p.ncol), 128, 0, st>>> (p);
+  return cudaGetLastError ();
+}
+
+cudaError_t
+launch_fix_dense (const FixPlan &particles, const FixPlan &p, const FixMaps &m, const int2 *tile,
+                  int ntile, int *status, cudaStream_t st, Ctx *prof)
+{
+  cudaError_t e = gemm_attrs ();
+  if (e != cudaSuccess) return e;
+  const int items = p.M[0] + p.M[1] + p.M[2] + 3;
+  k_fix_pair_tables<<<dim3 (ntile, (items + 15) / 16), 4 * PT, 0, st>>> (particles, p, tile);
+  kmark (prof, st, "k_fix_pair_tables");
+  k_fix_strings<<<dim3 (ntile, p.nqp / 4), 128, 0, st>>> (p);
+  kmark (prof, st, "k_fix_strings");
+  k_fix_bwd<7, true><<<dim3 ((ntile * PT + TM - 1) / TM, p.nbitem), NT, Geo<7>::SMEM, st>>> (m.wb, p,
+                                                                                            status);
   kmark (prof, st, "k_fix_bwd");
   return cudaGetLastError ();
 }

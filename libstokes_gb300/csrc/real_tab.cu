@@ -43,49 +43,16 @@
 #include <vector>
 
 #include "ewald_device.cuh"
+#include "radial.cuh"
 #include "real_tab.h"
 
 namespace lsg {
 namespace {
 
-constexpr int RT_LOG = 6;                     // log2 of the bins per octave
-constexpr int RT_DEG = 8;                     // coefficients per function
 constexpr int RT_T = 128;                     // threads per CTA: one target
 constexpr int RT_W = RT_T / 32;               // warps
 constexpr int RT_SEG = 1024;                  // accepted pairs a warp lists at a time
 static_assert (32 * REAL_TAB_MAXIMG <= RT_SEG, "32 sources with every offset fit a list");
-
-template <int V> struct NFun;
-template <> struct NFun<0> { static constexpr int value = 2; };
-template <> struct NFun<1> { static constexpr int value = 5; };
-template <> struct NFun<2> { static constexpr int value = 10; };
-
-// the independent coefficients at distance r, s = r^2
-template <int V>
-__device__ __forceinline__ void
-radial (double xi, double xisp, double r, double s, double *f)
-{
-  PairScalars<double> c;
-  real_scalars_mono<V, double> (xi, xisp, r, c);
-  f[0] = c.ya;
-  f[1] = (c.xa - c.ya) / s;
-  if (V == V_F) return;
-  f[2] = c.yb / r;
-  f[3] = c.yc;
-  f[4] = (c.xc - c.yc) / s;
-  if (V == V_FT) return;
-  f[5] = c.yg / r;                                            // g2
-  f[6] = (c.xg - 2.0 * c.yg) / (r * s);                       // g3
-  f[7] = (1.5 * c.xm - 2.0 * c.ym + 0.5 * c.zm) / (s * s);    // m1
-  f[8] = (c.ym - c.zm) / s;                                   // m4
-  f[9] = c.zm;
-}
-
-__device__ __forceinline__ double
-bin_mid (int bin)
-{
-  return __hiloint2double ((bin << (20 - RT_LOG)) | (1 << (19 - RT_LOG)), 0);
-}
 
 // coefficients of one bin: values at the Chebyshev nodes, then the monomial
 // coefficients c_k = sum_n B[k][n] f(node n) / h^k by compensated sums
@@ -352,18 +319,8 @@ k_real_tab (RealTabArgs a)
                 }
               continue;
             }
-          const double z = s - bin_mid (bin + a.bin0);
-          const double2 *c = reinterpret_cast<const double2 *> (a.tab)
-                             + (size_t) min (bin, a.nbin - 1) * (NF * RT_DEG / 2);
           double f[NF];
-#pragma unroll
-          for (int q = 0; q < NF; q++)
-            {
-              const double2 c3 = __ldg (c + 4 * q + 3), c2 = __ldg (c + 4 * q + 2),
-                            c1 = __ldg (c + 4 * q + 1), c0 = __ldg (c + 4 * q);
-              f[q] = fma (fma (fma (fma (fma (fma (fma (c3.y, z, c3.x), z, c2.y), z, c2.x), z, c1.y),
-                                    z, c1.x), z, c0.y), z, c0.x);
-            }
+          table_radial<NF> (a.tab, s, bin, a.bin0, a.nbin, f);
           apply<V, double> (d, s, f, x, y);
         }
       for (int k = t; k < nf; k += RT_T)
