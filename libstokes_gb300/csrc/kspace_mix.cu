@@ -44,6 +44,7 @@
 #include "ewald_device.cuh"
 #include "gpu_engine.h"
 #include "mixed.h"
+#include "pdl.cuh"
 #include "tma_host.h"
 
 namespace lsg {
@@ -130,10 +131,10 @@ struct BuildF {
 #pragma unroll
     for (int u = 0; u < 2; u++)
       {
-        v[u][0] = __ldg (reinterpret_cast<const int2 *> (T + (size_t) f[u].x * ldT + jo));
-        v[u][1] = __ldg (reinterpret_cast<const int2 *> (T + (size_t) f[u].y * ldT + jo));
-        v[u][2] = __ldg (reinterpret_cast<const int2 *> (T + (size_t) f[u].z * ldT + jo));
-        v[u][3] = __ldg (reinterpret_cast<const int2 *> (T + (size_t) f[u].w * ldT + jo));
+        v[u][0] = *reinterpret_cast<const int2 *> (T + (size_t) f[u].x * ldT + jo);
+        v[u][1] = *reinterpret_cast<const int2 *> (T + (size_t) f[u].y * ldT + jo);
+        v[u][2] = *reinterpret_cast<const int2 *> (T + (size_t) f[u].z * ldT + jo);
+        v[u][3] = *reinterpret_cast<const int2 *> (T + (size_t) f[u].w * ldT + jo);
       }
   }
   __device__ __forceinline__ void store (unsigned char *stage) const
@@ -172,10 +173,10 @@ struct BuildB {
     for (int u = 0; u < 4; u++)
       {
         const int4 f = __ldg (quart + t * (KT / 4) + u);
-        v[u][0] = __ldg (T + (size_t) f.x * ldT + i);
-        v[u][1] = __ldg (T + (size_t) f.y * ldT + i);
-        v[u][2] = __ldg (T + (size_t) f.z * ldT + i);
-        v[u][3] = __ldg (T + (size_t) f.w * ldT + i);
+        v[u][0] = T[(size_t) f.x * ldT + i];
+        v[u][1] = T[(size_t) f.y * ldT + i];
+        v[u][2] = T[(size_t) f.z * ldT + i];
+        v[u][3] = T[(size_t) f.w * ldT + i];
       }
   }
   __device__ __forceinline__ void store (unsigned char *stage) const
@@ -244,7 +245,7 @@ struct Sums {
   __device__ __forceinline__ void take (int set, int)
   {
     const float u0 = unit;
-    if (set + 1 < sets) unit = __ldg (units + (size_t) (set + 1) * ld);
+    if (set + 1 < sets) unit = units[(size_t) (set + 1) * ld];
 #pragma unroll
     for (int h = 0; h < 2; h++)
       {
@@ -285,7 +286,7 @@ gemm_cta (Sync &s, unsigned char *smem, const CUtensorMap *tmB, int tn, int n0, 
   acc.tmem = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + (uint32_t) acc.col;
   const int mine = acc.col + (lane & 15) + 64 * (lane >> 4);
   acc.units = units + min (mine, tn - 1);
-  acc.unit = acc.sets > 0 ? __ldg (acc.units) : 0.f;
+  acc.unit = acc.sets > 0 ? *acc.units : 0.f;
   const BTiles bt {tmB, k0, KT, n0, A_BYTES, b_bytes (tn)};
   return run_tiles<DK, 1, NS> (s, smem, ntiles, stage_bytes (tn), bt, stall, build, acc,
                                [=] (uint32_t a, int, bool first) { issue_tile (a, tmem, tn, first); });
@@ -310,9 +311,11 @@ k_sfac_gemm (const __grid_constant__ CUtensorMap tmB, MixPlan p, int *status)
   unsigned char *smem = align1k (dsm);
   const int jb = it.z * p.jper, je = min (p.ldT, jb + p.jper);
   const int ntiles = je > jb ? (je - jb) / KT : 0;
+  chain_next ();
   cta_setup (s);
   const uint32_t tmem = s.tslot;
   BuildF build (p, r0, jb);
+  chain_wait ();
   Sums acc;
   if (gemm_cta (s, smem, &tmB, p.tnf, n0, jb, ntiles, p.stall,
                 p.zs + (size_t) (jb / KB) * p.ldf + n0, p.ldf, build, acc))
@@ -349,7 +352,20 @@ k_bp_gemm (const __grid_constant__ CUtensorMap tmB, MixPlan p, int *status)
   const uint32_t tmem = s.tslot;
   BuildB build (p, i0, k0);
   Sums acc;
-  float *H = reinterpret_cast<float *> (smem);
+  float *H = reinterpret_cast<float *> (smem), *X = H + TM * HLD;
+  const int c = p.cb, ne = min (p.tnb, p.ncolb - n0), f0 = n0 / c, nf = (n0 + ne - 1) / c - f0 + 1;
+  chain_wait ();
+  // the x functions of the tile's columns, read ahead (a load per term of the
+  // epilogue waited for L2 every time: 10 us at FTS N = 1000)
+  constexpr int XW = 32 * WORKERS, XMAX = (44 * TM + XW - 1) / XW;
+  int xr[XMAX];
+  if ((int) threadIdx.x < XW)
+#pragma unroll
+    for (int k = 0; k < XMAX; k++)
+      {
+        const int e = (int) threadIdx.x + XW * k;
+        xr[k] = e < nf * TM ? p.T[(size_t) (f0 + e / TM) * p.ldT + i0 + e % TM] : 0;
+      }
   if (gemm_cta (s, smem, &tmB, p.tnb, n0, k0, it.z, p.stall, p.ws + (size_t) (k0 / KB) * p.ldb + n0,
                 p.ldb, build, acc))
     {
@@ -362,17 +378,13 @@ k_bp_gemm (const __grid_constant__ CUtensorMap tmB, MixPlan p, int *status)
         for (int u = 0; u < 16; u++)
           if (acc.col + 64 * h < p.tnb)
             H[((warp & 3) * 32 + lane) * HLD + acc.col + 64 * h + u] = acc.v[h][u];
+#pragma unroll
+      for (int k = 0; k < XMAX; k++)
+        if ((int) threadIdx.x + XW * k < nf * TM) X[threadIdx.x + XW * k] = (float) xr[k];
     }
   __syncthreads ();
   if (!s.err)
     {
-      // the x functions of the tile's columns, in one pass (a load per term
-      // waited for L2 every time: 10 us at FTS N = 1000)
-      const int c = p.cb, ne = min (p.tnb, p.ncolb - n0), f0 = n0 / c, nf = (n0 + ne - 1) / c - f0 + 1;
-      float *X = H + TM * HLD;
-      for (int e = threadIdx.x; e < nf * TM; e += NT)
-        X[e] = (float) p.T[(size_t) (f0 + e / TM) * p.ldT + i0 + e % TM];
-      __syncthreads ();
       float *yp = p.yp + (size_t) blockIdx.y * p.np * c;
       for (int e = threadIdx.x; e < TM * c; e += NT)
         {
@@ -413,20 +425,13 @@ mk_prep_tc (MixPrep a)
   const MixPlan &p = a.p;
   const int t = threadIdx.x, jb = blockIdx.x * PREP_P, G = gridDim.y;
   const bool lead = blockIdx.y == 0;
-  if (t < CMAX) s_mx[t] = 0u;
-  __syncthreads ();
+  chain_next ();
   for (int e = t; e < PREP_P * a.c; e += PREP_T)
     {
       const int jl = e / a.c, q = e - jl * a.c, j = jb + jl;
       const float v = j < a.np ? (float) a.x[(size_t) j * a.c + q] : 0.f;
       s_x[q][jl] = v;
-      atomicMax (&s_mx[q], __float_as_uint (v) & 0x7fffffffu);
-      if (p.cf > a.c)
-        {
-          const float w = j < a.np ? a.qa[j] * v : 0.f;
-          s_x[a.c + q][jl] = w;
-          atomicMax (&s_mx[a.c + q], __float_as_uint (w) & 0x7fffffffu);
-        }
+      if (p.cf > a.c) s_x[a.c + q][jl] = j < a.np ? a.qa[j] * v : 0.f;
       if (lead && j < a.np) a.xf[(size_t) j * ((a.c + 3) & ~3) + q] = v;
     }
   if (t < PREP_P)
@@ -454,12 +459,23 @@ mk_prep_tc (MixPrep a)
       s_q[0][t] = qu; s_q[1][t] = q1; s_q[2][t] = q2;
     }
   __syncthreads ();
-  if (t < p.cf)
+  // the units: one warp per component (atomics on a handful of words took 2 us)
+  for (int q = t >> 5; q < p.cf; q += PREP_T / 32)
     {
-      float inv;
-      unit_of (s_mx[t], inv);
-      s_inv[t] = inv;
+      uint32_t mx = 0u;
+#pragma unroll
+      for (int k = 0; k < PREP_P / 32; k++)
+        mx = max (mx, __float_as_uint (s_x[q][(t & 31) + 32 * k]) & 0x7fffffffu);
+      mx = __reduce_max_sync (0xffffffffu, mx);
+      if ((t & 31) == 0)
+        {
+          float inv;
+          unit_of (mx, inv);
+          s_mx[q] = mx;
+          s_inv[q] = inv;
+        }
     }
+  if (lead) __syncthreads ();
   if (lead)
     for (int n = t; n < p.ldf; n += PREP_T)
       {
@@ -624,6 +640,7 @@ k_kop (MixPlan p)
   constexpr int C = NComp<V>::value;
   __shared__ uint32_t s_mx[C][2];
   const int nqm = p.nqm[blockIdx.y];
+  chain_next ();
   if ((int) (blockIdx.x * (KOP_T / 8)) >= nqm) return;
   const KopLane l (nqm);
   const MixCoef K = p.coef[(size_t) 4 * (p.off[l.m1] + (l.live ? l.qr : 0)) + l.b];
@@ -645,13 +662,17 @@ k_kop (MixPlan p)
 // ---------------------------------------------------------------------------
 constexpr int START = 4;                // start and end of a CTA, in K tiles
 
-// columns per tile: a multiple of 16 up to 128 that leaves the fewest unused
+// columns per tile: a multiple of 16 up to `most` that leaves the fewest unused
 int
-tile_cols (int ncol)
+tile_cols (int ncol, int most)
 {
-  const int nt = (ncol + TN_MAX - 1) / TN_MAX;
+  const int nt = (ncol + most - 1) / most;
   return (((ncol + nt - 1) / nt) + 15) / 16 * 16;
 }
+
+// time of a tile of tn columns, of one of 128: the build of A stays, B, the
+// MMAs, the drain and the epilogue go with tn
+double tile_time (int tn) { return (64.0 + tn) / 192.0; }
 
 }  // namespace
 
@@ -663,28 +684,23 @@ void
 mix_plan_items (MixPlan &p, const std::vector<int> &nqm, std::vector<int4> &fwd,
                 std::vector<int4> &bwd)
 {
-  p.tnf = tile_cols (p.ncolf);
-  p.tnb = tile_cols (p.ncolb);
-  p.nctf = (p.ncolf + p.tnf - 1) / p.tnf;
-  p.nctb = (p.ncolb + p.tnb - 1) / p.tnb;
-  p.ldf = p.nctf * p.tnf;
-  p.ldb = p.nctb * p.tnb;
   p.mt = (p.np + TM - 1) / TM;
-  std::vector<int> rf (p.nctf), rb (p.nctb);
+  const int kb = p.ldT / KB;
+  p.tnf = tile_cols (p.ncolf, TN_MAX);
+  p.nctf = (p.ncolf + p.tnf - 1) / p.tnf;
+  std::vector<int> rf (p.nctf), rb;
   long long act = 0;
   for (int ct = 0; ct < p.nctf; ct++)
     {
       rf[ct] = (4 * nqm[col_m (ct * p.tnf, p.cf)] + TM - 1) / TM;
       act += rf[ct];
     }
-  for (int ct = 0; ct < p.nctb; ct++) rb[ct] = (4 * nqm[col_m (ct * p.tnb, p.cb)] + KB - 1) / KB;
-  long long best = -1;
-  const int kb = p.ldT / KB;
+  double best = -1;
   for (int ns = 1; ns <= std::min (16, kb); ns++)
     {
       const int per = (kb + ns - 1) / ns, used = (kb + per - 1) / per;
       // each slice is one more set of sums for the operator kernel
-      const long long t = (act * used + SMS - 1) / SMS * (DK * per + START) + used / 4;
+      const double t = (double) ((act * used + SMS - 1) / SMS) * (DK * per + START) + used / 4.0;
       if (best < 0 || t < best)
         {
           best = t;
@@ -692,30 +708,44 @@ mix_plan_items (MixPlan &p, const std::vector<int> &nqm, std::vector<int4> &fwd,
           p.nsplit = used;
         }
     }
+  p.ldf = p.nctf * p.tnf;
   fwd.clear ();
   for (int z = 0; z < p.nsplit; z++)
     for (int ct = 0; ct < p.nctf; ct++)
       for (int rt = 0; rt < rf[ct]; rt++) fwd.push_back (make_int4 (rt, ct, z, 0));
   p.nfitem = (int) fwd.size ();
+  // backward: in a small system narrower tiles, more of them, end sooner (FTS N
+  // = 200 48.6 -> 45.1 us a product, N = 600 61 -> 57.5); a larger one needs the
+  // SMs that they take for the real space beside it (F N = 2048 65.3 -> 68.5)
   best = -1;
   int slice = 1;
-  for (int s = 1; s <= std::max (1, rb[0]); s++)
+  for (int most = TN_MAX; most >= (p.np <= 1024 ? 32 : TN_MAX); most /= 2)
     {
-      const int l = (rb[0] + s - 1) / s;
-      std::vector<int> len;
-      for (int ct = 0; ct < p.nctb; ct++)
+      const int tn = tile_cols (p.ncolb, most), nct = (p.ncolb + tn - 1) / tn;
+      std::vector<int> sets (nct);
+      for (int ct = 0; ct < nct; ct++) sets[ct] = (4 * nqm[col_m (ct * tn, p.cb)] + KB - 1) / KB;
+      for (int s = 1; s <= std::max (1, sets[0]); s++)
         {
-          const int n = std::max (1, (rb[ct] + l - 1) / l);
-          for (int z = 0; z < n; z++) len.push_back (DK * ((rb[ct] + n - 1) / n));
-        }
-      if (s > 1 && len.size () > 64) break;
-      const long long t = makespan (len, p.mt, START) + (long long) len.size () / 8;
-      if (best < 0 || t < best)
-        {
-          best = t;
-          slice = l;
+          const int l = (sets[0] + s - 1) / s;
+          std::vector<int> len;
+          for (int k : sets)
+            {
+              const int n = std::max (1, (k + l - 1) / l);
+              for (int z = 0; z < n; z++) len.push_back (DK * ((k + n - 1) / n));
+            }
+          if (s > 1 && len.size () > 64) break;
+          const double t = (double) makespan (len, p.mt, START) * tile_time (tn) + len.size () / 24.0;
+          if (best < 0 || t < best)
+            {
+              best = t;
+              slice = l;
+              p.tnb = tn;
+              p.nctb = nct;
+              rb = sets;
+            }
         }
     }
+  p.ldb = p.nctb * p.tnb;
   bwd.clear ();
   for (int ct = 0; ct < p.nctb; ct++)
     {
@@ -764,8 +794,10 @@ gemm_attrs ()
 cudaError_t
 launch_mix_prep (const MixPrep &a, cudaStream_t st)
 {
-  const int items = a.p.M[0] + a.p.M[1] + a.p.M[2] + 3;
-  mk_prep_tc<<<dim3 (a.p.ldT / PREP_P, (items + PREP_I - 1) / PREP_I), PREP_T, 0, st>>> (a);
+  // fewer items a CTA while that leaves SMs idle
+  const int items = a.p.M[0] + a.p.M[1] + a.p.M[2] + 3, tiles = a.p.ldT / PREP_P;
+  const int g = std::max ((items + PREP_I - 1) / PREP_I, std::min (items, SMS / tiles));
+  mk_prep_tc<<<dim3 (tiles, g), PREP_T, 0, st>>> (a);
   return cudaGetLastError ();
 }
 
@@ -775,7 +807,8 @@ launch_mix_forward (int version, const MixPlan &p, const MixMaps &m, int *status
 {
   cudaError_t e = gemm_attrs ();
   if (e != cudaSuccess) return e;
-  k_sfac_gemm<<<p.nfitem, NT, SMEM_DYN, st>>> (m.zf, p, status);
+  e = launch_chained (k_sfac_gemm, p.nfitem, NT, SMEM_DYN, st, m.zf, p, status);
+  if (e != cudaSuccess) return e;
   kmark (prof, st, "k_sfac_gemm");
   const dim3 g (p.nqp / (KOP_T / 8), p.M[0] + 1);
   if (version == 0) k_kop<0><<<g, KOP_T, 0, st>>> (p);
@@ -788,9 +821,10 @@ launch_mix_forward (int version, const MixPlan &p, const MixMaps &m, int *status
 cudaError_t
 launch_mix_backward (const MixPlan &p, const MixMaps &m, int *status, cudaStream_t st, Ctx *prof)
 {
-  k_bp_gemm<<<dim3 (p.mt, p.nbitem), NT, SMEM_DYN, st>>> (m.wb, p, status);
+  const cudaError_t e = launch_chained (k_bp_gemm, dim3 (p.mt, p.nbitem), NT, SMEM_DYN, st, m.wb, p,
+                                        status);
   kmark (prof, st, "k_bp_gemm");
-  return cudaGetLastError ();
+  return e;
 }
 
 }  // namespace lsg

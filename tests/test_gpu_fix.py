@@ -154,3 +154,21 @@ def test_bounded_wait_is_reported(lib):
         lib.stokes_gpu_test_stall_waits(0, 0)
     assert np.array_equal(s.atimes(x), y)
     s.close()
+
+
+@pytest.mark.parametrize("version,n,side", [(0, 2, 9.0), (1, 2, 9.0), (1, 64, 14.0), (2, 129, 19.5),
+                                            (0, 513, 30.0), (2, 300, 26.0)])
+def test_new_inputs_every_time(version, n, side):
+    """The kernels of a product overlap their starts: each has to read what the
+    ones before it wrote in this product, not what an earlier one left."""
+    from libstokes_gb300 import System
+    rng = np.random.default_rng(70 + n)
+    box = (side, side, side)
+    s, f = (System(version, _positions(n, box, rng), box) for _ in range(2))
+    for _ in range(6):
+        pos, x = _positions(n, box, rng), rng.standard_normal((3, 6, 11)[version] * n)
+        s.set_pos(pos)
+        f.set_pos(pos)
+        assert rel_l2(s.atimes(x), f.atimes(x, notbl=True)) < 1e-12
+    s.close()
+    f.close()

@@ -101,3 +101,22 @@ def test_non_finite(bad):
     y64, ymx = _both(0, _positions(130, box, rng), box, x.ravel())
     assert np.isnan(ymx).all() == np.isnan(y64).all()
     assert not np.isfinite(ymx).any()
+
+
+@pytest.mark.parametrize("version,n,side", [(0, 2, 9.0), (1, 2, 9.0), (1, 64, 14.0), (2, 129, 19.5),
+                                            (0, 513, 30.0), (2, 900, 36.0)])
+def test_new_inputs_every_time(version, n, side):
+    """The kernels of a product overlap their starts: each has to read what the
+    ones before it wrote in this product, not what an earlier one left."""
+    from libstokes_gb300 import MIXED, System
+    rng = np.random.default_rng(70 + n)
+    box = (side, side, side)
+    s, f = (System(version, _positions(n, box, rng), box) for _ in range(2))
+    s.set_precision(MIXED)
+    for _ in range(8):
+        pos, x = _positions(n, box, rng), rng.standard_normal((3, 6, 11)[version] * n)
+        s.set_pos(pos)
+        f.set_pos(pos)
+        assert rel_l2(s.atimes(x), f.atimes(x, notbl=True)) < TOL
+    s.close()
+    f.close()
