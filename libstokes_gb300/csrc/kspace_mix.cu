@@ -38,6 +38,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "digit_gemm.cuh"
@@ -336,7 +337,9 @@ k_sfac_gemm (const __grid_constant__ CUtensorMap tmB, MixPlan p, int *status)
 
 // backward: a CTA takes 128 particles and one item (column tile, first K
 // tile, K tiles); the sums are parked in the freed stages and reduced over
-// the x functions of the tile into the item's partial y
+// the x functions of the tile into the item's partial y.  POLY: the columns of
+// k_kop_poly, each with its power of the particle's radius.
+template <bool POLY>
 __global__ void __launch_bounds__ (NT, 1)
 k_bp_gemm (const __grid_constant__ CUtensorMap tmB, MixPlan p, int *status)
 {
@@ -353,7 +356,7 @@ k_bp_gemm (const __grid_constant__ CUtensorMap tmB, MixPlan p, int *status)
   BuildB build (p, i0, k0);
   Sums acc;
   float *H = reinterpret_cast<float *> (smem), *X = H + TM * HLD;
-  const int c = p.cb, ne = min (p.tnb, p.ncolb - n0), f0 = n0 / c, nf = (n0 + ne - 1) / c - f0 + 1;
+  const int cb = p.cb, ne = min (p.tnb, p.ncolb - n0), f0 = n0 / cb, nf = (n0 + ne - 1) / cb - f0 + 1;
   chain_wait ();
   // the x functions of the tile's columns, read ahead (a load per term of the
   // epilogue waited for L2 every time: 10 us at FTS N = 1000)
@@ -385,14 +388,39 @@ k_bp_gemm (const __grid_constant__ CUtensorMap tmB, MixPlan p, int *status)
   __syncthreads ();
   if (!s.err)
     {
+      const int c = p.c;
       float *yp = p.yp + (size_t) blockIdx.y * p.np * c;
       for (int e = threadIdx.x; e < TM * c; e += NT)
         {
           const int q = e / TM, r = e - q * TM, i = i0 + r;
           if (i >= p.np) continue;
-          float y = 0.f;
-          for (int n = (q + c - n0 % c) % c; n < ne; n += c)
-            y = fmaf (X[((n0 + n) / c - f0) * TM + r], H[r * HLD + n], y);
+          // sum of column k of the functions
+          auto column = [&] (int k) {
+            float y = 0.f;
+            for (int n = (k + cb - n0 % cb) % cb; n < ne; n += cb)
+              y = fmaf (X[((n0 + n) / cb - f0) * TM + r], H[r * HLD + n], y);
+            return y;
+          };
+          float y;
+          if constexpr (!POLY)
+            y = column (q);
+          else
+            {
+              const float a = p.rad[i], a2 = a * a;
+              if (c == 3) y = a * fmaf (a2, column (3 + q), column (q));
+              else
+                {
+                  // a^2 and a^3; then a (U) and, for FTS, a^4 (U, E), a^5 (E)
+                  y = a2 * fmaf (a, column (c + 3 + q), column (3 + q));
+                  if (q < 3) y = fmaf (a, column (q), y);
+                  if (c == 11 && (q < 3 || q >= 6))
+                    {
+                      float z = column (q < 3 ? 25 + q : 22 + q);
+                      if (q >= 6) z = fmaf (a, column (27 + q), z);
+                      y = fmaf (a2 * a2, z, y);
+                    }
+                }
+            }
           yp[(size_t) i * c + q] = y * 0x1p-30f;
         }
     }
@@ -657,6 +685,89 @@ k_kop (MixPlan p)
   put_rows<C> (p, l, 0, g, s_mx);
 }
 
+// Unequal radii.  With a the target's radius and X, Xq the sums of x_j and a_j^2
+// x_j, the weights of a pair are polynomials in a: the forward columns are X and
+// Xq (2 c per function), the backward ones U, W, E by power of a
+//   a    U              6 X, -k^2 Xq (A)
+//   a^2  U, W, E        B and G at a = 0
+//   a^3  U, W, E        -k^2 X (A); C, H and M at a = 0
+//   a^4  U, E           G
+//   a^5  E              M
+// in this order (F: a and a^3; FT: a, a^2, a^3).  K.ya is the Ewald factor, K.yb
+// and K.yc are k and k^2, K.yg the factor of G.
+template <int V>
+__global__ void __launch_bounds__ (KOP_T)
+k_kop_poly (MixPlan p)
+{
+  constexpr int C = NComp<V>::value;
+  __shared__ uint32_t s_mx[11][2];
+  const int nqm = p.nqm[blockIdx.y];
+  chain_next ();
+  if ((int) (blockIdx.x * (KOP_T / 8)) >= nqm) return;
+  const KopLane l (nqm);
+  const MixCoef K = p.coef[(size_t) 4 * (p.off[l.m1] + (l.live ? l.qr : 0)) + l.b];
+  const float e[3] = {K.ex, K.ey, K.ez};
+  const float ax = K.ya, kk = K.yc, sg = l.w ? 1.f : -1.f, b3 = sg * 3.f * K.yb * ax, gk = sg * K.yb * K.yg;
+  Trans<V, float> xo, xs, qo, qs;       // of X and Xq: this lane's sums, the other's
+  {
+    float x[C];
+    sums<C> (p, l, 0, x);
+    transverse<V, float> (e, x, xo);
+    swap_trans<V, float> (xo, xs, 4);
+    sums<C> (p, l, C, x);
+    transverse<V, float> (e, x, qo);
+    swap_trans<V, float> (qo, qs, 4);
+  }
+  float g[C], h[C];
+  auto put = [&] (int first, auto n, int from) {
+    constexpr int N = decltype (n)::value;
+    float v[N];
+#pragma unroll
+    for (int q = 0; q < N; q++) v[q] = g[N == 8 && q >= 3 ? q + 3 : from + q];
+    put_rows<N> (p, l, first, v, s_mx);
+  };
+  using std::integral_constant;
+  // a
+#pragma unroll
+  for (int d = 0; d < 3; d++) g[d] = ax * fmaf (-kk, qo.f[d], 6.f * xo.f[d]);
+  put (0, integral_constant<int, 3> (), 0);
+  if constexpr (V == V_F)
+    {
+#pragma unroll
+      for (int d = 0; d < 3; d++) g[d] = -kk * ax * xo.f[d];
+      put (3, integral_constant<int, 3> (), 0);
+    }
+  else
+    {
+      // a^2
+      couple<V, float> (e, 0.f, b3, 0.f, 3.f * gk, 0.f, 0.f, xo, xs, g);
+      if constexpr (V == V_FTS)
+        {
+          couple<V, float> (e, 0.f, 0.f, 0.f, -0.5f * kk * gk, 0.f, 0.f, qo, qs, h);
+#pragma unroll
+          for (int q = 0; q < C; q++) g[q] += h[q];
+        }
+      put (3, integral_constant<int, C> (), 0);
+      // a^3
+      couple<V, float> (e, -kk * ax, 0.f, 1.5f * kk * ax, 0.f, 1.5f * kk * ax, 3.f * kk * ax, xo, xs, g);
+      if constexpr (V == V_FTS)
+        {
+          couple<V, float> (e, 0.f, 0.f, 0.f, 0.f, 0.f, -0.3f * kk * kk * ax, qo, qs, h);
+#pragma unroll
+          for (int q = 0; q < C; q++) g[q] += h[q];
+        }
+      put (C + 3, integral_constant<int, C> (), 0);
+      if constexpr (V == V_FTS)
+        {
+          // a^4, a^5
+          couple<V, float> (e, 0.f, 0.f, 0.f, -0.3f * kk * gk, 0.f, 0.f, xo, xs, g);
+          put (25, integral_constant<int, 8> (), 0);
+          couple<V, float> (e, 0.f, 0.f, 0.f, 0.f, 0.f, -0.3f * kk * kk * ax, xo, xs, g);
+          put (33, integral_constant<int, 5> (), 6);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -760,6 +871,7 @@ mix_plan_items (MixPlan &p, const std::vector<int> &nqm, std::vector<int4> &fwd,
   p.nbitem = (int) bwd.size ();
 }
 
+int mix_poly_columns (int version) { return version == 0 ? 6 : (version == 1 ? 15 : 38); }
 size_t mix_zf_bytes (const MixPlan &p) { return 2 * (size_t) ND * p.ncolf * p.ldT; }
 size_t mix_wb_bytes (const MixPlan &p) { return 2 * (size_t) ND * p.ncolb * p.Rp; }
 size_t mix_zs_floats (const MixPlan &p) { return (size_t) (p.ldT / KB) * p.ldf; }
@@ -784,9 +896,10 @@ gemm_attrs ()
   if ((e = cudaFuncSetAttribute (k_sfac_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int) SMEM_DYN)) != cudaSuccess)
     return e;
-  if ((e = cudaFuncSetAttribute (k_bp_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int) SMEM_DYN)) != cudaSuccess)
-    return e;
+  for (auto bp : {k_bp_gemm<false>, k_bp_gemm<true>})
+    if ((e = cudaFuncSetAttribute (bp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) SMEM_DYN))
+        != cudaSuccess)
+      return e;
   attr_dev = dev;
   return cudaSuccess;
 }
@@ -811,7 +924,13 @@ launch_mix_forward (int version, const MixPlan &p, const MixMaps &m, int *status
   if (e != cudaSuccess) return e;
   kmark (prof, st, "k_sfac_gemm");
   const dim3 g (p.nqp / (KOP_T / 8), p.M[0] + 1);
-  if (version == 0) k_kop<0><<<g, KOP_T, 0, st>>> (p);
+  if (p.rad)
+    {
+      if (version == 0) k_kop_poly<0><<<g, KOP_T, 0, st>>> (p);
+      else if (version == 1) k_kop_poly<1><<<g, KOP_T, 0, st>>> (p);
+      else k_kop_poly<2><<<g, KOP_T, 0, st>>> (p);
+    }
+  else if (version == 0) k_kop<0><<<g, KOP_T, 0, st>>> (p);
   else if (version == 1) k_kop<1><<<g, KOP_T, 0, st>>> (p);
   else k_kop<2><<<g, KOP_T, 0, st>>> (p);
   kmark (prof, st, "k_kop");
@@ -821,9 +940,9 @@ launch_mix_forward (int version, const MixPlan &p, const MixMaps &m, int *status
 cudaError_t
 launch_mix_backward (const MixPlan &p, const MixMaps &m, int *status, cudaStream_t st, Ctx *prof)
 {
-  const cudaError_t e = launch_chained (k_bp_gemm, dim3 (p.mt, p.nbitem), NT, SMEM_DYN, st, m.wb, p,
-                                        status);
-  kmark (prof, st, "k_bp_gemm");
+  const cudaError_t e = launch_chained (p.rad ? k_bp_gemm<true> : k_bp_gemm<false>, dim3 (p.mt, p.nbitem),
+                                        NT, SMEM_DYN, st, m.wb, p, status);
+  kmark (prof, st, p.rad ? "mk_backproj_poly" : "k_bp_gemm");
   return e;
 }
 

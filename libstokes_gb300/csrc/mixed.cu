@@ -1041,6 +1041,34 @@ default_eta_images (int np)
   return 13.0;
 }
 
+// Small systems are latency-bound: the chain of the two GEMMs and their tables
+// takes 38-50 us however few the particles.  They take the SIMT kernels at a
+// split with few k vectors and lattice images in real space (eta 4; 3.5 to 5 are
+// within a few us).  Measured, SIMT at eta 4 against the GEMMs, us a product:
+//   F    N = 64 24.6 / 38.6, 250 28.8 / 42.5, 400 37.0 / 42.4, 700 68 / 43
+//   FT   N = 64 22.7 / 40.4, 333 37.0 / 42.5, 500 45.2 / 44.6
+//   FTS  N = 64 24.7 / 41.5, 250 37.0 / 49.7, 400 52.6 / 50.8
+//   unequal radii: F 400 39 / 49, FT 333 43 / 51, FTS 250 45 / 67
+// A long box would need many images of its short sides.
+// LIBSTOKES_GB300_KSPACE=tc keeps the GEMMs, =simt the SIMT kernels.
+static bool
+small_system (const struct stokes *sys)
+{
+  const double lmin = fmin (sys->lx, fmin (sys->ly, sys->lz));
+  const double lmax = fmax (sys->lx, fmax (sys->ly, sys->lz));
+  const int most = sys->version == 0 ? 512 : (sys->version == 1 ? 400 : 256);
+  return sys->np <= most && lmax <= 2.0 * lmin;
+}
+
+static bool
+use_gemms (const struct stokes *sys)
+{
+  const char *ks = getenv ("LIBSTOKES_GB300_KSPACE");   // read per call: tests switch it
+  if (ks && strcmp (ks, "simt") == 0) return false;
+  if (ks && strcmp (ks, "tc") == 0) return true;
+  return !small_system (sys);
+}
+
 // choose xi, cutoffs and the half-space k list of the mixed split
 static int
 mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
@@ -1053,10 +1081,13 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
   // the back-projection, lattice images were faster at no measured size
   // (FTS N = 256-512 level at eta 8; N = 4096 283 against 273 us; N = 8192
   // and 16384 level at eta 11, where the cutoff is below half the box)
-  bool images = env_double ("LIBSTOKES_GB300_MIXED_IMAGES", 0.0) != 0.0;
+  // the exception are small systems on the SIMT path (small_system)
+  const bool small = small_system (sys) && !use_gemms (sys);
+  bool images = env_double ("LIBSTOKES_GB300_MIXED_IMAGES", small ? 1.0 : 0.0) != 0.0;
   double eta = env_double ("LIBSTOKES_GB300_MIXED_ETA",
-                           images ? default_eta_images (sys->np)
-                                  : default_eta (sys->version, sys->np));
+                           small ? 4.0
+                                 : (images ? default_eta_images (sys->np)
+                                           : default_eta (sys->version, sys->np)));
   uint64_t fp = mix_fingerprint (sys, eta + (images ? 1000.0 : 0.0), eps);
   const bool poly = c->mode == MODE_POLY;
   double amax = 1.0;
@@ -1296,7 +1327,9 @@ mix_setup (Ctx *c, MixedState *m)
   if (m->mix_fp == m->fp && m->mix.p) return STOKES_GPU_OK;
   MixPlan p {};
   p.np = c->np;
-  p.cf = p.cb = NCOMP (c->version);
+  p.c = NCOMP (c->version);
+  p.cf = m->poly ? 2 * p.c : p.c;
+  p.cb = m->poly ? mix_poly_columns (c->version) : p.c;
   for (int d = 0; d < 3; d++) p.M[d] = m->M[d];
   p.nmi = 2 * p.M[0] + 1;
   p.ncolf = p.nmi * p.cf;
@@ -1381,7 +1414,7 @@ mix_setup (Ctx *c, MixedState *m)
   const size_t zero1 = bytes;
   const size_t o_zs = place (sizeof (float) * mix_zs_floats (p));
   const size_t o_F = place (sizeof (float) * (size_t) p.nsplit * p.ncolf * p.Rp);
-  const size_t o_yp = place (sizeof (float) * (size_t) p.nbitem * p.np * p.cb);
+  const size_t o_yp = place (sizeof (float) * (size_t) p.nbitem * p.np * p.c);
   // no product of this context may still be using the tables of the last set-up
   cudaError_t e = m->mix_id ? cudaDeviceSynchronize () : cudaSuccess;
   if (e == cudaSuccess) e = m->mix.ensure (bytes);
@@ -1554,9 +1587,7 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
   const size_t off1 = (size_t) (m->M[0] + 1) * np;
   const size_t off2 = off1 + (size_t) (m->M[1] + 1) * np;
   {
-    // reciprocal space on the tensor cores unless LIBSTOKES_GB300_KSPACE=simt
-    const char *ks = getenv ("LIBSTOKES_GB300_KSPACE");   // read per call: tests switch it
-    m->tensor = !(ks && strcmp (ks, "simt") == 0) && !m->poly && m->nkh > 0;
+    m->tensor = use_gemms (sys) && m->nkh > 0;
     rc = m->tensor ? mix_setup (c, m) : upload_k (c, m);
     if (rc) return rc;
     m->mp.stall = g_test_gemm_stall;
@@ -1693,6 +1724,8 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
         pa.rot = (const float4 *) m->rot.p;
         pa.qpos = (uint32_t *) m->qpos.p;
         pa.xf = (float *) m->xf.p;
+        pa.qa = m->poly ? (const float *) m->pqa.p : nullptr;
+        m->mp.rad = m->poly ? (const float *) m->prad.p : nullptr;
         pa.p = m->mp;
         if ((e = launch_mix_prep (pa, st)) != cudaSuccess) return cuda_fail (e, "mk_prep");
       }

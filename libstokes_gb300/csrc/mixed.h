@@ -59,11 +59,13 @@ struct __align__ (16) MixCoef {
 // axis: index 0 is 1, 2 m - 1 is cos 2 pi m u, 2 m is sin 2 pi m u.
 //   quarter  one (|m2|, |m3|) of the k list, sorted by length
 //   row      4 quarter + 2 p2 + p3, p = 0 cosine, 1 sine: f_y f_z
-//   column   mi c + q, mi the x function index, q one of c components (cf
-//            forward, cb backward)
+//   column   mi c + q, mi the x function index, q one of c = cf (forward) or cb
+//            (backward) components
 struct MixPlan {
   int np, M[3];
-  int cf, cb;             // components per x function, forward and backward
+  int c;                  // vector components
+  int cf, cb;             // columns per x function, forward and backward (c; unequal
+                          // radii: see k_kop_poly)
   int nmi, ncolf, ncolb;  // x functions 2 M[0] + 1; columns
   int nq, nqp, Rp;        // quarters; padded to 32; rows 4 nqp
   int ldT;                // particles padded to 128
@@ -86,7 +88,8 @@ struct MixPlan {
   float *ws;              // units of WB, [Rp / 128][ldb]
   void *ZF, *WB;          // images, f16 digits [3][columns][ldT or Rp]
   float *F;               // structure factors [nsplit][ncolf][Rp]
-  float *yp;              // back-projection partials [nbitem][np][cb]
+  float *yp;              // back-projection partials [nbitem][np][c]
+  const float *rad;       // unequal radii (NULL: unit spheres)
 };
 
 // TMA descriptors of the two images
@@ -109,6 +112,8 @@ struct MixPrep {
 
 void mix_plan_items (MixPlan &p, const std::vector<int> &nqm, std::vector<int4> &fwd,
                      std::vector<int4> &bwd);
+// backward columns per x function of unequal radii
+int mix_poly_columns (int version);
 size_t mix_zf_bytes (const MixPlan &p);
 size_t mix_wb_bytes (const MixPlan &p);
 size_t mix_zs_floats (const MixPlan &p);

@@ -14,6 +14,16 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-6
 
 
+@pytest.fixture(autouse=True, params=["tc", ""])
+def path(request, monkeypatch):
+    """The GEMMs at every size, and what the library takes by itself (small
+    systems: the SIMT kernels at a split with lattice images)."""
+    if request.param:
+        monkeypatch.setenv("LIBSTOKES_GB300_KSPACE", request.param)
+    else:
+        monkeypatch.delenv("LIBSTOKES_GB300_KSPACE", raising=False)
+
+
 def _positions(n, box, rng):
     m = int(np.ceil(n ** (1 / 3)))
     g = np.stack(np.meshgrid(*(np.arange(m),) * 3, indexing="ij"), -1).reshape(-1, 3)
@@ -118,5 +128,25 @@ def test_new_inputs_every_time(version, n, side):
         s.set_pos(pos)
         f.set_pos(pos)
         assert rel_l2(s.atimes(x), f.atimes(x, notbl=True)) < TOL
+    s.close()
+    f.close()
+
+
+# unequal radii: columns by power of the radius, around the tiles
+@pytest.mark.parametrize("version", [0, 1, 2])
+@pytest.mark.parametrize("n,side", [(63, 16.0), (129, 19.5), (513, 31.0)])
+def test_unequal_radii(version, n, side):
+    from libstokes_gb300 import MIXED, System
+    rng = np.random.default_rng(90 + n + version)
+    box = (side, 0.9 * side, 1.1 * side)
+    radius = rng.uniform(0.4, 1.0, n)
+    pos = _positions(n, box, rng)
+    s, f = System(version, pos, box), System(version, pos, box)
+    s.set_radius(radius)
+    f.set_radius(radius)
+    s.set_precision(MIXED)
+    for _ in range(4):
+        x = rng.standard_normal((3, 6, 11)[version] * n)
+        assert rel_l2(s.atimes(x), f.atimes(x)) < TOL
     s.close()
     f.close()
