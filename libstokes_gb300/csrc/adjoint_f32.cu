@@ -147,7 +147,7 @@ struct VjpArgs {
   const VjpK *kt;
   int nk;
   float *wu;                // [nk][4 c]: W re, W im, U re, U im
-  float *dbox;              // [nk][3] or NULL
+  double *dbox;             // [CTAs of kva_wu][3] partial sums, or NULL
   float *part;              // [nchunk][np][6]
   int nchunk;
   float *grad;              // [kchunks][np][3]
@@ -283,8 +283,9 @@ __global__ void __launch_bounds__ (128)
 kva_wu (VjpArgs a, const float *sfp, int nslices)
 {
   constexpr int C = NComp<V>::value;
-  const int k = blockIdx.x * 128 + threadIdx.x;
-  if (k >= a.nk) return;
+  const int kt = blockIdx.x * 128 + threadIdx.x;
+  const bool live = kt < a.nk;
+  const int k = live ? kt : 0;         // (idle threads redo vector 0, and write nothing)
   float cf[C], sf[C], cg[C], sg[C];
 #pragma unroll
   for (int q = 0; q < C; q++) cf[q] = sf[q] = cg[q] = sg[q] = 0.f;
@@ -321,10 +322,11 @@ kva_wu (VjpArgs a, const float *sfp, int nslices)
       recip_apply<V, float> (e, K.ya, K.yb, K.yc, 0.f, 0.f, 0.f, gs, gc, Q);
 #pragma unroll
       for (int q = 0; q < C; q++)
-        {
-          o[2 * C * which + q] = P.v[q];
-          o[2 * C * which + C + q] = Q.v[q];
-        }
+        if (live)
+          {
+            o[2 * C * which + q] = P.v[q];
+            o[2 * C * which + C + q] = Q.v[q];
+          }
     }
   if (!a.dbox) return;
   // the op as a function of the box lengths: k = 2 pi m / l, pi / V
@@ -361,14 +363,21 @@ kva_wu (VjpArgs a, const float *sfp, int nslices)
   Q.zero ();
   recip_apply<V, DF> (ed, ya, yb, yc, DF (0.0), DF (0.0), DF (0.0), gc, gms, P);
   recip_apply<V, DF> (ed, ya, yb, yc, DF (0.0), DF (0.0), DF (0.0), gs, gc, Q);
-  // Re conj(S_g) . dW = Cg . dP + Sg . dQ
+  // Re conj(S_g) . dW = Cg . dP + Sg . dQ, summed over the CTA in FP64 (the
+  // list of 3 nk terms took the host longer than the kernels)
+  __shared__ double s_d[4][3];
   for (int c = 0; c < 3; c++)
     {
       float sacc = 0.f;
 #pragma unroll
       for (int q = 0; q < C; q++) sacc = fmaf (cg[q], P.v[q].d[c], fmaf (sg[q], Q.v[q].d[c], sacc));
-      a.dbox[(size_t) 3 * k + c] = sacc;
+      const double v = warp_sum (live ? (double) sacc : 0.0);
+      if ((threadIdx.x & 31) == 0) s_d[threadIdx.x >> 5][c] = v;
     }
+  __syncthreads ();
+  if (threadIdx.x < 3)
+    a.dbox[(size_t) 3 * blockIdx.x + threadIdx.x]
+      = (s_d[0][threadIdx.x] + s_d[1][threadIdx.x]) + (s_d[2][threadIdx.x] + s_d[3][threadIdx.x]);
 }
 
 // per particle l and a slice of k: sum_k k Im[e^{-ik.r_l} (g_l . W_k + f_l . U_k)],
@@ -609,6 +618,8 @@ struct VjpState {
   int nk = 0;
   std::vector<VjpK> hk;
   uint64_t uploaded = 0;        // split whose k table and rotations are on the device
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   DevBuf q, gf, gcm, p32, tab, kt, wu, dbox, part, grad, rot, g, f, pos, dldr, blk, sfp;
 };
 
@@ -734,7 +745,7 @@ vjp_mixed_v (Ctx *c, const struct stokes *sys, VjpState *s, const double *g, con
                   std::make_pair (&s->tab, sizeof (float2) * (size_t) ntab * np),
                   std::make_pair (&s->kt, sizeof (VjpK) * std::max (nk, 1)),
                   std::make_pair (&s->wu, sizeof (float) * 4 * C * std::max (nk, 1)),
-                  std::make_pair (&s->dbox, sizeof (float) * 3 * std::max (nk, 1)),
+                  std::make_pair (&s->dbox, sizeof (double) * 3 * (size_t) (nk / 128 + 1)),
                   std::make_pair (&s->part, sizeof (float) * 6 * (size_t) nchunk * np),
                   std::make_pair (&s->grad, sizeof (float) * 3 * (size_t) kchunks * np),
                   std::make_pair (&s->rot, sizeof (float) * 4 * 1024),
@@ -798,7 +809,7 @@ vjp_mixed_v (Ctx *c, const struct stokes *sys, VjpState *s, const double *g, con
   a.kt = (const VjpK *) s->kt.p;
   a.nk = nk;
   a.wu = (float *) s->wu.p;
-  a.dbox = dLdbox ? (float *) s->dbox.p : nullptr;
+  a.dbox = dLdbox ? (double *) s->dbox.p : nullptr;
   a.part = (float *) s->part.p;
   a.nchunk = nchunk;
   a.grad = (float *) s->grad.p;
@@ -807,8 +818,24 @@ vjp_mixed_v (Ctx *c, const struct stokes *sys, VjpState *s, const double *g, con
   kva_prep<V><<<(np + 127) / 128, 128, 0, st>>> (a);
   kmark (c, st, "kva_prep");
   const long long warps = (long long) np * nchunk;
-  kva_real<V><<<(int) ((warps + AR_W - 1) / AR_W), AR_W * 32, 0, st>>> (a);
+  // the real space needs the tables only: beside the reciprocal sums, unless
+  // the kernels are timed one by one
+  const bool overlap = nk > 0 && !c->kprof_on;
+  cudaStream_t rs = st;
+  if (overlap)
+    {
+      if (!s->side
+          && (cudaStreamCreateWithFlags (&s->side, cudaStreamNonBlocking) != cudaSuccess
+              || cudaEventCreateWithFlags (&s->fork, cudaEventDisableTiming) != cudaSuccess
+              || cudaEventCreateWithFlags (&s->join, cudaEventDisableTiming) != cudaSuccess))
+        return set_error (STOKES_GPU_ECUDA, "mixed VJP: side stream");
+      rs = s->side;
+      cudaEventRecord (s->fork, st);
+      cudaStreamWaitEvent (rs, s->fork, 0);
+    }
+  kva_real<V><<<(int) ((warps + AR_W - 1) / AR_W), AR_W * 32, 0, rs>>> (a);
   kmark (c, st, "kva_real");
+  if (overlap) cudaEventRecord (s->join, rs);
   if (nk > 0)
     {
       const int nsl = (np + SF_P - 1) / SF_P;
@@ -819,18 +846,20 @@ vjp_mixed_v (Ctx *c, const struct stokes *sys, VjpState *s, const double *g, con
       kva_bp<V><<<dim3 ((np + BP_T - 1) / BP_T, kchunks), BP_T, 0, st>>> (a);
       kmark (c, st, "kva_bp");
     }
+  if (overlap) cudaStreamWaitEvent (st, s->join, 0);
   const int nblk = (np + FIN_P - 1) / FIN_P;
   kva_final<<<nblk, FIN_T, 0, st>>> (a);
   kmark (c, st, "kva_final");
   if ((e = cudaGetLastError ()) != cudaSuccess) return cuda_fail (e, "mixed VJP kernels");
   std::vector<double> blk ((size_t) 6 * nblk);
-  std::vector<float> db ((size_t) 3 * std::max (nk, 1), 0.f);
+  const int nkb = (nk + 127) / 128;
+  std::vector<double> db ((size_t) 3 * std::max (nkb, 1), 0.0);
   e = cudaMemcpyAsync (dLdr, s->dldr.p, sizeof (double) * 3 * np, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync (blk.data (), s->blk.p, sizeof (double) * blk.size (),
                          cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess && nk > 0 && dLdbox)
-    e = cudaMemcpyAsync (db.data (), s->dbox.p, sizeof (float) * 3 * nk, cudaMemcpyDeviceToHost, st);
+    e = cudaMemcpyAsync (db.data (), s->dbox.p, sizeof (double) * 3 * nkb, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize (st);
   if (e != cudaSuccess) return cuda_fail (e, "mixed VJP results");
   if (dLdbox)
@@ -846,7 +875,7 @@ vjp_mixed_v (Ctx *c, const struct stokes *sys, VjpState *s, const double *g, con
       for (int k = 0; k < 3; k++)
         {
           double opd = 0.0;
-          for (int q = 0; q < nk; q++) opd += db[3 * (size_t) q + k];
+          for (int q = 0; q < nkb; q++) opd += db[3 * (size_t) q + k];
           dLdbox[k] = bx[k] + 2.0 * opd - phase[k] / L[k];
         }
     }
@@ -890,6 +919,9 @@ release_vjp_mixed (const Ctx *c)
                     &s->part, &s->grad, &s->rot, &s->g, &s->f, &s->pos, &s->dldr, &s->blk,
                     &s->sfp})
     b->release ();
+  if (s->side) cudaStreamDestroy (s->side);
+  if (s->fork) cudaEventDestroy (s->fork);
+  if (s->join) cudaEventDestroy (s->join);
   delete s;
 }
 

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "ewald_device.cuh"
 #include "gpu_engine.h"
 #include "stokes_bd.h"
 
@@ -214,11 +215,14 @@ k_bd_lj (int nm, int np, int c, const double *pos, double lx, double ly, double 
 
 // EV_LJ of this library's BD engine: the nearest image (Lees-Edwards aware;
 // the overlap range is below half the box) and the force along the image
-// vector.  CTA of LJ_T targets; the sources pass through shared memory in
-// tiles of LJ_T as FP32 positions for a pre-test on the wrapped distance
-// (with a margin); the few pairs that pass it are evaluated in FP64 from
-// the global positions.  An open system takes the plain difference.
-constexpr int LJ_T = 128;
+// vector.  One warp per target, its lanes over the sources, which pass through
+// shared memory in tiles of LJ_T as FP32 positions for a pre-test on the
+// wrapped distance (with a margin); the few pairs that pass it are evaluated
+// in FP64 from the global positions, and the lanes' sums added by shuffles.  An
+// open system takes the plain difference.  (One thread per target left all but
+// a few SMs idle: N = 1000 110 us a call.)
+constexpr int LJ_T = 256;
+constexpr int LJ_W = LJ_T / 32;          // targets per CTA
 
 __global__ void __launch_bounds__ (LJ_T)
 k_bd_lj_engine (int nm, int np, int c, const double *pos, double lx, double ly, double lz,
@@ -226,7 +230,7 @@ k_bd_lj_engine (int nm, int np, int c, const double *pos, double lx, double ly, 
                 const double *lje, const double *ljr0, int open, double *f)
 {
   __shared__ float s_p[LJ_T][4];
-  const int i = blockIdx.x * LJ_T + threadIdx.x;
+  const int lane = threadIdx.x & 31, i = blockIdx.x * LJ_W + (threadIdx.x >> 5);
   const bool live = i < nm;
   const int ii = live ? i : 0;
   const double xi = pos[3 * ii], yi = pos[3 * ii + 1], zi = pos[3 * ii + 2];
@@ -250,7 +254,7 @@ k_bd_lj_engine (int nm, int np, int c, const double *pos, double lx, double ly, 
       __syncthreads ();
       if (!live) continue;
       const int nt = min (LJ_T, np - j0);
-      for (int t = 0; t < nt; t++)
+      for (int t = lane; t < nt; t += 32)
         {
           const int j = j0 + t;
           float sx = fxi - s_p[t][0], sy = fyi - s_p[t][1], sz = fzi - s_p[t][2];
@@ -308,7 +312,10 @@ k_bd_lj_engine (int nm, int np, int c, const double *pos, double lx, double ly, 
           fz += fr * z / r;
         }
     }
-  if (!live) return;
+  fx = warp_sum (fx);
+  fy = warp_sum (fy);
+  fz = warp_sum (fz);
+  if (!live || lane) return;
   f[(size_t) i * c] += fx;
   f[(size_t) i * c + 1] += fy;
   f[(size_t) i * c + 2] += fz;
@@ -627,7 +634,7 @@ bd_forces (stokes_gpu_bd *b, const double *d_pos, double fact)
                                             b->lj_arrays ? (const double *) b->ljr0.p : nullptr,
                                             s->periodic == 0, (double *) b->f.p);
   else if (b->p.lj_e != 0.0 || b->lj_arrays)
-    k_bd_lj_engine<<<(b->nm + LJ_T - 1) / LJ_T, LJ_T, 0, st>>> (
+    k_bd_lj_engine<<<(b->nm + LJ_W - 1) / LJ_W, LJ_T, 0, st>>> (
       b->nm, b->np, b->C, d_pos, s->lx, s->ly, s->lz, s->shear_mode, s->shear_shift,
       s->a ? (const double *) b->c->pp.p : nullptr, b->p.lj_e, b->p.lj_r0,
       b->lj_arrays ? (const double *) b->lje.p : nullptr,
