@@ -26,6 +26,7 @@
 #include "ewald_device.cuh"
 #include "gpu_engine.h"
 #include "mixed.h"
+#include "radial.cuh"
 #include "stokes_gpu.h"
 
 extern "C" void lsg_ewald_cutoffs (double xi, double eps, double lmin, double lmax,
@@ -73,7 +74,7 @@ struct MixedState {
   int nchunk_r = 1, nchunk_k = 1;
   int real_g = 1;               // warps per target of mk_real
   int nc[3] = {0, 0, 0};        // cell list of mk_real (nc[0] == 0: no cells)
-  DevBuf sq, cstart;
+  DevBuf sq, xs, cstart;
   // unequal radii: radii and their squares (FP32), the per-particle self
   // terms at the split (FP64, [np][3]), for the split they were made at
   bool poly = false;
@@ -205,6 +206,7 @@ struct RealMixArgs {
   const float4 *img;     // lattice offsets added to the minimum-image difference
   int nimg;              // 1 (the zero offset) while the cutoff is below half the box
   // cell list (NULL cstart: every particle is a candidate source)
+  const float *xsrc;     // x in the order of mk_real's sources (xf or, with cells, in cell order)
   const uint4 *sq;       // particles in cell order: (q_x, q_y, q_z, particle index)
   const int *cstart;     // [ncell + 1] first slot of each cell in sq
   int nc[3];             // cells per axis (cell side >= rc / 2)
@@ -263,24 +265,31 @@ mix_term (const RealMixArgs &a, float4 d, float ai, GenU<V, float> &t)
   constexpr int C = NComp<V>::value, CP = cpad (C);
   // x_j as float4 loads of the padded copy
   float xj[CP];
-  const float4 *src = reinterpret_cast<const float4 *> (a.xf + (size_t) CP * j);
+  const float4 *src = reinterpret_cast<const float4 *> (a.xsrc + (size_t) CP * j);
 #pragma unroll
   for (int k = 0; k < CP / 4; k++)
     {
       const float4 v = __ldg (src + k);
       xj[4 * k] = v.x; xj[4 * k + 1] = v.y; xj[4 * k + 2] = v.z; xj[4 * k + 3] = v.w;
     }
-  GenF<V, float> g;
-  load_genf<V, float> (xj, g);
   const float e[3] = {d.x * ri, d.y * ri, d.z * ri};
-  PairScalars<float> s;
-  if (POLY)
-    // unequal radii (rmin = 0): the SD-form scalars of the pair's radii,
-    // scaled by the target's (src/ewald.c:204-359, :383-420)
-    real_scalars_poly<V, float> (a.xi, a.xisp, r, ai, __ldg (a.rad + j), ai, s);
+  if constexpr (POLY)
+    {
+      // unequal radii (rmin = 0): the SD-form scalars of the pair's radii,
+      // scaled by the target's (src/ewald.c:204-359, :383-420)
+      GenF<V, float> g;
+      load_genf<V, float> (xj, g);
+      PairScalars<float> s;
+      const int p = a.cstart ? (int) a.sq[j].w : j;
+      real_scalars_poly<V, float> (a.xi, a.xisp, r, ai, __ldg (a.rad + p), ai, s);
+      pair_apply<V, float> (e, s, g, t);
+    }
   else
-    real_scalars_mono_ri<V, float> (a.xi, a.xisp, r, ri, s);
-  pair_apply<V, float> (e, s, g, t);
+    {
+      float f[NFun<V>::value];
+      radial_f32<V> (a.xi, a.xisp, r, ri, f);
+      apply_radial<V, float> (e, 1.0f, f, xj, t.v);
+    }
 }
 
 // error-free sum of two values: a + b = s + e exactly
@@ -357,7 +366,7 @@ mk_real (RealMixArgs a)
         if (sj < s1)
           {
             const uint4 qj = cells ? a.sq[sj] : reinterpret_cast<const uint4 *> (a.qpos)[sj];
-            j = cells ? (int) qj.w : sj;
+            j = sj;             // (a.xsrc is in the order of the sources)
             min_image (a, qi, qj, d0x, d0y, d0z);
           }
         if (a.nimg == 1)
@@ -544,6 +553,15 @@ mk_clamp (RealMixArgs a)
       const float v = warp_sum (acc[q]);
       if (lane == 0) a.out_clamp[(size_t) i * C + q] = v;
     }
+}
+
+// x in cell order (n4 float4 a particle): the pairs of a target's queue then
+// read neighbouring entries
+__global__ void __launch_bounds__ (256)
+mk_cell_x (const uint4 *sq, const float4 *xf, int np, int n4, float4 *xs)
+{
+  const int t = blockIdx.x * 256 + threadIdx.x;
+  if (t < np * n4) xs[t] = xf[(size_t) sq[t / n4].w * n4 + t % n4];
 }
 
 // The cell list of mk_real: particles sorted by cell, stably (in particle
@@ -1483,7 +1501,7 @@ run_mixed_sequence (Ctx *c, MixedState *m, const double *d_pos, const double *d_
   mix ((uint64_t) m->nchunk_k);
   const void *ptrs[] = {d_pos, d_x, d_y, m->kt.p, m->qpos.p, m->tab.p, m->xf.p, m->pq.p,
                         m->part_real.p, m->part_rec.p, m->selfbuf.p, m->status.p,
-                        m->rot.p, m->mix.p, m->h_status, m->img.p, m->sq.p, m->cstart.p, m->prad.p, m->pqa.p, m->pself.p};
+                        m->rot.p, m->mix.p, m->h_status, m->img.p, m->sq.p, m->xs.p, m->cstart.p, m->prad.p, m->pqa.p, m->pself.p};
   for (const void *p : ptrs) mix ((uint64_t) (uintptr_t) p);
   mix ((uint64_t) (uintptr_t) E);
   // a captured cudaEventRecord is only a dependency, not a record: around a
@@ -1631,7 +1649,9 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
   if (m->nc[0])
     {
       const int ncell = m->nc[0] * m->nc[1] * m->nc[2];
-      if ((e = m->sq.ensure (sizeof (uint4) * np)) != cudaSuccess) return cuda_fail (e, "cell order");
+      if ((e = m->sq.ensure (sizeof (uint4) * np)) != cudaSuccess
+          || (e = m->xs.ensure (sizeof (float) * cpad (C) * np)) != cudaSuccess)
+        return cuda_fail (e, "cell order");
       if ((e = m->cstart.ensure (sizeof (int) * (ncell + 1))) != cudaSuccess) return cuda_fail (e, "cell starts");
       if ((e = cudaFuncSetAttribute (mk_cells, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int) sizeof (int) * 32 * CELL_MAX)) != cudaSuccess)
@@ -1748,7 +1768,7 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
 
     RealMixArgs ra;
     memset (&ra, 0, sizeof ra);
-    ra.qpos = (const uint32_t *) m->qpos.p; ra.xf = (const float *) m->xf.p;
+    ra.qpos = (const uint32_t *) m->qpos.p; ra.xf = ra.xsrc = (const float *) m->xf.p;
     ra.np = np; ra.G = m->real_g;
     ra.scale[0] = (float) (sys->lx / two32);
     ra.scale[1] = (float) (sys->ly / two32);
@@ -1776,6 +1796,7 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
     if (m->nc[0])
       {
         ra.sq = (const uint4 *) m->sq.p;
+        ra.xsrc = (const float *) m->xs.p;
         ra.cstart = (const int *) m->cstart.p;
         for (int d = 0; d < 3; d++) ra.nc[d] = m->nc[d];
       }
@@ -1793,6 +1814,9 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
           mk_cells<<<1, CELL_THREADS, sizeof (int) * 32 * ncell, rs>>> (
             (const uint4 *) m->qpos.p, np, m->nc[0], m->nc[1], m->nc[2], (int *) m->cstart.p,
             (uint4 *) m->sq.p);
+          const int cp = cpad (C);
+          mk_cell_x<<<(np * (cp / 4) + 255) / 256, 256, 0, rs>>> (
+            (const uint4 *) m->sq.p, (const float4 *) m->xf.p, np, cp / 4, (float4 *) m->xs.p);
           kmark (c, rs, "mk_cells");
         }
       if (m->poly)
@@ -1933,7 +1957,7 @@ release_mixed (Ctx *c)
   if (!c->mixed) return;
   MixedState *m = c->mixed;
   for (DevBuf *b : {&m->kt, &m->qpos, &m->tab, &m->xf, &m->pq, &m->part_real, &m->part_rec,
-                    &m->selfbuf, &m->status, &m->rot, &m->mix, &m->img, &m->sq, &m->cstart,
+                    &m->selfbuf, &m->status, &m->rot, &m->mix, &m->img, &m->sq, &m->xs, &m->cstart,
                     &m->prad, &m->pqa, &m->pself})
     b->release ();
   if (m->h_status) cudaFreeHost (m->h_status);

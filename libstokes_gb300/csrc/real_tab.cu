@@ -94,69 +94,6 @@ k_rt_table (Basis b, int bin0, double xi, double xisp, double *tab, float *tabf)
   tabf[((size_t) blockIdx.x * NF + q) * RT_DEG + k] = (float) c;
 }
 
-// y += M x_j of one pair at displacement d, s = d.d, coefficients f
-template <int V, typename R>
-__device__ __forceinline__ void
-apply (const R d[3], R s, const R *f, const R *__restrict__ x, R *y)
-{
-  const R F0 = x[0], F1 = x[1], F2 = x[2];
-  const R dF = d[0] * F0 + d[1] * F1 + d[2] * F2;
-  R along = f[1] * dF;
-  if (V == V_F)
-    {
-      y[0] += fma (f[0], F0, along * d[0]);
-      y[1] += fma (f[0], F1, along * d[1]);
-      y[2] += fma (f[0], F2, along * d[2]);
-      return;
-    }
-  const R T0 = x[3], T1 = x[4], T2 = x[5];
-  const R t0 = T1 * d[2] - T2 * d[1], t1 = T2 * d[0] - T0 * d[2], t2 = T0 * d[1] - T1 * d[0];
-  const R f0 = F1 * d[2] - F2 * d[1], f1 = F2 * d[0] - F0 * d[2], f2 = F0 * d[1] - F1 * d[0];
-  const R w = f[4] * (d[0] * T0 + d[1] * T1 + d[2] * T2);
-  y[3] = fma (w, d[0], fma (f[3], T0, fma (f[2], f0, y[3])));
-  y[4] = fma (w, d[1], fma (f[3], T1, fma (f[2], f1, y[4])));
-  y[5] = fma (w, d[2], fma (f[3], T2, fma (f[2], f2, y[5])));
-  if (V == V_FT)
-    {
-      y[0] = fma (along, d[0], fma (f[0], F0, fma (f[2], t0, y[0])));
-      y[1] = fma (along, d[1], fma (f[0], F1, fma (f[2], t1, y[1])));
-      y[2] = fma (along, d[2], fma (f[0], F2, fma (f[2], t2, y[2])));
-      return;
-    }
-  const R sxx = x[6], sxy = x[7], sxz = x[8], syz = x[9], syy = x[10];
-  const R Sxx = fma (R (2), sxx, syy), Syy = fma (R (2), syy, sxx);
-  const R s0 = Sxx * d[0] + sxy * d[1] + sxz * d[2];
-  const R s1 = sxy * d[0] + Syy * d[1] + syz * d[2];
-  const R s2 = sxz * d[0] + syz * d[1];
-  const R ss = d[0] * s0 + d[1] * s1 + d[2] * s2, tr = Sxx + Syy;
-  const R third = R (-1.0 / 3.0), g2 = f[5], g3 = f[6], m1 = f[7], m4 = f[8], zm = f[9];
-  const R g1 = fma (g3, s, R (2) * g2) * third;
-  const R m2 = fma (m1, s, R (2) * m4) * third;
-  const R m3 = fma (m2, s, zm) * third;
-  along = fma (-g1, tr, fma (-g3, ss, along));
-  const R n2 = R (-2) * g2, nc = -f[4];
-  y[0] = fma (along, d[0], fma (f[0], F0, fma (f[2], t0, fma (n2, s0, y[0]))));
-  y[1] = fma (along, d[1], fma (f[0], F1, fma (f[2], t1, fma (n2, s1, y[1]))));
-  y[2] = fma (along, d[2], fma (f[0], F2, fma (f[2], t2, fma (n2, s2, y[2]))));
-  const R h2 = R (2) * nc;
-  y[3] = fma (h2, d[1] * s2 - d[2] * s1, y[3]);
-  y[4] = fma (h2, d[2] * s0 - d[0] * s2, y[4]);
-  y[5] = fma (h2, d[0] * s1 - d[1] * s0, y[5]);
-  const R v0 = fma (g2, F0, fma (nc, t0, m4 * s0));
-  const R v1 = fma (g2, F1, fma (nc, t1, m4 * s1));
-  const R v2 = fma (g2, F2, fma (nc, t2, m4 * s2));
-  const R dE = fma (g1, dF, fma (m2, ss, m3 * tr));
-  const R ee = fma (g3, dF, fma (m1, ss, m2 * tr));
-  // ee d d + d V + V d = d (V + ee d / 2) + (V + ee d / 2) d
-  const R he = R (0.5) * ee;
-  const R w0 = fma (he, d[0], v0), w1 = fma (he, d[1], v1), w2 = fma (he, d[2], v2);
-  y[6] += fma (R (2) * d[0], w0, fma (zm, Sxx, dE));
-  y[7] = fma (d[0], w1, fma (d[1], w0, fma (zm, sxy, y[7])));
-  y[8] = fma (d[0], w2, fma (d[2], w0, fma (zm, sxz, y[8])));
-  y[9] = fma (d[1], w2, fma (d[2], w1, fma (zm, syz, y[9])));
-  y[10] += fma (R (2) * d[1], w1, fma (zm, Syy, dE));
-}
-
 // pairs the table does not serve: nearer than its first bin, or under the
 // rmin clamp (r raised to rm and e = d / r with the raised r,
 // src/ewald.c:693-699).  At a split other than the struct's own a clamped
@@ -321,7 +258,7 @@ k_real_tab (RealTabArgs a)
             }
           double f[NF];
           table_radial<NF> (a.tab, s, bin, a.bin0, a.nbin, f);
-          apply<V, double> (d, s, f, x, y);
+          apply_radial<V, double> (d, s, f, x, y);
         }
       for (int k = t; k < nf; k += RT_T)
         {
@@ -358,7 +295,7 @@ k_real_tab (RealTabArgs a)
               const float4 v = __ldg (xs + q);
               xj[4 * q] = v.x; xj[4 * q + 1] = v.y; xj[4 * q + 2] = v.z; xj[4 * q + 3] = v.w;
             }
-          apply<V, float> (e, e[0] * e[0] + e[1] * e[1] + e[2] * e[2], f, xj, yf);
+          apply_radial<V, float> (e, e[0] * e[0] + e[1] * e[1] + e[2] * e[2], f, xj, yf);
         }
       __syncthreads ();
     }
