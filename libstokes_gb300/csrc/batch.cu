@@ -36,6 +36,7 @@
 #include "ewald_device.cuh"
 #include "gpu_engine.h"
 #include "mixed.h"
+#include "radial.cuh"
 #include "stokes_gpu.h"
 
 extern "C" void lsg_ewald_cutoffs (double xi, double eps, double lmin, double lmax,
@@ -80,12 +81,15 @@ find_sys (const int *cum, int nsys, long long t)
 struct BatchArgs {
   const BSys *sys;
   int nsys;
+  const int *cum_b;        // groups of BP_N particles
   const int *cum_p, *cum_r, *cum_k;     // particles, real warps, k warps
   const double *pos, *x;
   double *y;
   uint32_t *qpos;
   float2 *tab;
   float *xf;
+  const short4 *km;        // (m1, m2, m3) of kt
+  int tab_smem;            // table rows of a particle that mb_bp stages at most
   const MixK *kt;
   float *pq, *pr;
   const float4 *img;                    // per system: image vectors (x, y, z, 0)
@@ -178,16 +182,23 @@ template <int V>
 __device__ __forceinline__ void
 bterm (const BSys &S, const float *xf, int j, float dx, float dy, float dz, GenU<V, float> &acc)
 {
-  float r = sqrtf (dx * dx + dy * dy + dz * dz);
-  const float rm = 2.0f * S.rmin;
-  if (r < rm) r = rm;
-  const float ri = 1.0f / r;
+  constexpr int C = NComp<V>::value;
+  const float rr = dx * dx + dy * dy + dz * dz, rm = 2.0f * S.rmin;
+  // 1 / r from the reciprocal square root with one Newton step (1 ulp)
+  float ri = rsqrtf (rr);
+  ri = ri * fmaf (-0.5f * rr, ri * ri, 1.5f);
+  float r = rr * ri;
+  if (r < rm)
+    {
+      r = rm;
+      ri = 1.0f / rm;
+    }
   const float e[3] = {dx * ri, dy * ri, dz * ri};
-  PairScalars<float> sc;
-  real_scalars_mono<V, float> (S.xi, S.xisp, r, sc);
-  GenF<V, float> g;
-  load_genf<V, float> (xf + S.x_off + (size_t) NComp<V>::value * j, g);
-  pair_apply<V, float> (e, sc, g, acc);
+  float f[NFun<V>::value], x[C];
+#pragma unroll
+  for (int q = 0; q < C; q++) x[q] = xf[S.x_off + (size_t) C * j + q];
+  radial_f32<V> (S.xi, S.xisp, r, ri, f);
+  apply_radial<V, float> (e, 1.0f, f, x, acc.v);
 }
 
 template <int V>
@@ -207,42 +218,49 @@ mb_real_warp (const BatchArgs &a, const BSys &S, int i, int chunk, float (*s_d)[
   for (int jb = j0; jb < j1; jb += 32)
     {
       const int j = jb + lane;
-      bool ok = false;
-      float dx = 0.f, dy = 0.f, dz = 0.f;
       float d0x = 0.f, d0y = 0.f, d0z = 0.f;
       if (j < j1) bmin_image (S, qi, qp[j], d0x, d0y, d0z);
       // the minimum image and, when the cutoff exceeds half the box, the
-      // lattice images around it
-      for (int m = 0; m < S.nimg; m++)
+      // lattice images around it: this lane's accepted ones as a bit mask, 32
+      // at a time, then one of each lane's per round into the queue (a ballot
+      // and a queue test per image took most of the time)
+      for (int m0 = 0; m0 < S.nimg; m0 += 32)
         {
-          const float4 T = a.img[S.img_off + m];
-          bool ok = false;
-          float dx = 0.f, dy = 0.f, dz = 0.f;
-          if (j < j1)
+          const float4 *img = a.img + S.img_off + m0;
+          const int n = min (32, S.nimg - m0);
+          unsigned mask = 0u;
+#pragma unroll 4
+          for (int m = 0; m < n; m++)
             {
-              dx = d0x + T.x;
-              dy = d0y + T.y;
-              dz = d0z + T.z;
+              const float4 T = __ldg (img + m);
+              const float dx = d0x + T.x, dy = d0y + T.y, dz = d0z + T.z;
               const float rr = dx * dx + dy * dy + dz * dz;
-              ok = (rr > 0.f) && (rr < S.rc2);
+              if (rr > 0.f && rr < S.rc2) mask |= 1u << m;
             }
-          const unsigned b = __ballot_sync (0xffffffffu, ok);
-          if (ok)
+          if (j >= j1) mask = 0u;
+          for (;;)
             {
-              const int slot = qn + __popc (b & lt);
-              s_d[slot][0] = dx;
-              s_d[slot][1] = dy;
-              s_d[slot][2] = dz;
-              s_j[slot] = j;
-            }
-          qn += __popc (b);
-          __syncwarp ();
-          if (qn >= 32)
-            {
-              const int slot = qn - 32 + lane;
-              bterm<V> (S, a.xf, s_j[slot], s_d[slot][0], s_d[slot][1], s_d[slot][2], acc);
-              qn -= 32;
+              const unsigned b = __ballot_sync (0xffffffffu, mask != 0u);
+              if (b == 0u) break;
+              if (mask)
+                {
+                  const float4 T = __ldg (img + __ffs (mask) - 1);
+                  const int slot = qn + __popc (b & lt);
+                  s_d[slot][0] = d0x + T.x;
+                  s_d[slot][1] = d0y + T.y;
+                  s_d[slot][2] = d0z + T.z;
+                  s_j[slot] = j;
+                  mask &= mask - 1u;
+                }
+              qn += __popc (b);
               __syncwarp ();
+              if (qn >= 32)
+                {
+                  const int slot = qn - 32 + lane;
+                  bterm<V> (S, a.xf, s_j[slot], s_d[slot][0], s_d[slot][1], s_d[slot][2], acc);
+                  qn -= 32;
+                  __syncwarp ();
+                }
             }
         }
     }
@@ -350,69 +368,92 @@ mb_sfac (BatchArgs a)
 
 // one warp per (system, particle): y_i = self x_i + sum real partials
 // + 2 sum_k cos(k.r_i) P + sin(k.r_i) Q
+// Back-projection: one warp per BP_N particles of a system, its lanes over the
+// k vectors, so that their loads serve BP_N particles (one particle a warp with
+// its table read from global memory waited for L2 most of the time: 215 us of a
+// 64-system product, 140 with the table alone in shared memory)
+constexpr int BP_N = 4;
 template <int V>
 __device__ __forceinline__ void
-mb_bp_warp (const BatchArgs &a, const BSys &S, int i)
+mb_bp_warp (const BatchArgs &a, const BSys &S, int i0, float2 *s_t)
 {
   constexpr int C = NComp<V>::value;
   const int lane = threadIdx.x & 31;
-  const float2 *t0 = a.tab + S.tab_off, *t1 = t0 + (size_t) (S.M0 + 1) * S.np,
-               *t2 = t1 + (size_t) (S.M1 + 1) * S.np;
+  // the particles' functions in shared memory, [row][particle]
+  const float2 *row = a.tab + S.tab_off;
+  const int nt = S.M0 + S.M1 + S.M2 + 3;
+  const bool staged = nt <= a.tab_smem;
+  if (staged)
+    for (int e = lane; e < nt * BP_N; e += 32)
+      s_t[e] = row[(size_t) (e / BP_N) * S.np + min (i0 + e % BP_N, S.np - 1)];
+  __syncwarp ();
+  const float2 *t0 = staged ? s_t : row + i0;
+  const size_t ld = staged ? BP_N : S.np;
+  const float2 *t1 = t0 + (S.M0 + 1) * ld, *t2 = t1 + (S.M1 + 1) * ld;
+  const int n = min (BP_N, S.np - i0);
   const float *pq = a.pq + S.pq_off;
-  float acc[C];
+  float acc[BP_N][C];
 #pragma unroll
-  for (int q = 0; q < C; q++) acc[q] = 0.f;
+  for (int u = 0; u < BP_N; u++)
+#pragma unroll
+    for (int q = 0; q < C; q++) acc[u][q] = 0.f;
   for (int k = lane; k < S.nkh; k += 32)
     {
-      const int4 m = *reinterpret_cast<const int4 *> (&a.kt[S.k_off + k].m1);
-      float2 p0 = t0[(size_t) (m.x < 0 ? -m.x : m.x) * S.np + i];
-      float2 p1 = t1[(size_t) (m.y < 0 ? -m.y : m.y) * S.np + i];
-      float2 p2 = t2[(size_t) (m.z < 0 ? -m.z : m.z) * S.np + i];
-      if (m.x < 0) p0.y = -p0.y;
-      if (m.y < 0) p1.y = -p1.y;
-      if (m.z < 0) p2.y = -p2.y;
-      const float2 p01 = make_float2 (p0.x * p1.x - p0.y * p1.y, p0.x * p1.y + p0.y * p1.x);
-      const float2 ph = make_float2 (p01.x * p2.x - p01.y * p2.y, p01.x * p2.y + p01.y * p2.x);
+      const short4 m = a.km[S.k_off + k];                   // m1 >= 0
+      float P[C], Q[C];
 #pragma unroll
       for (int q = 0; q < C; q++)
-        acc[q] = fmaf (ph.x, pq[(size_t) q * S.nkh + k],
-                       fmaf (ph.y, pq[(size_t) (C + q) * S.nkh + k], acc[q]));
-    }
+        {
+          P[q] = pq[(size_t) q * S.nkh + k];
+          Q[q] = pq[(size_t) (C + q) * S.nkh + k];
+        }
+      const float2 *f0 = t0 + m.x * ld, *f1 = t1 + abs (m.y) * ld, *f2 = t2 + abs (m.z) * ld;
+      const float s1 = m.y < 0 ? -1.f : 1.f, s2 = m.z < 0 ? -1.f : 1.f;
 #pragma unroll
-  for (int q = 0; q < C; q++) acc[q] = warp_sum (acc[q]);
-  if (lane != 0) return;
-  // self (FP64) + real partials + 2 reciprocal
-  PairScalars<double> sc;
-  sc.xa = sc.ya = S.selfc[0];
-  sc.xc = sc.yc = S.selfc[1];
-  sc.xm = sc.ym = sc.zm = S.selfc[2];
-  sc.yb = sc.xg = sc.yg = sc.yh = 0.0;
-  const double e[3] = {0.0, 0.0, 0.0};
-  GenF<V, double> g;
-  load_genf<V, double> (a.x + S.x_off + (size_t) C * i, g);
-  GenU<V, double> ys;
-  ys.zero ();
-  pair_apply<V, double> (e, sc, g, ys);
+      for (int u = 0; u < BP_N; u++)
+        {
+          const int v = staged ? u : min (u, n - 1);
+          const float2 p0 = f0[v];
+          float2 p1 = f1[v], p2 = f2[v];
+          p1.y *= s1;
+          p2.y *= s2;
+          const float2 p01 = make_float2 (p0.x * p1.x - p0.y * p1.y, p0.x * p1.y + p0.y * p1.x);
+          const float2 ph = make_float2 (p01.x * p2.x - p01.y * p2.y, p01.x * p2.y + p01.y * p2.x);
 #pragma unroll
-  for (int q = 0; q < C; q++)
-    {
-      double r = 0.0;
-      for (int ch = 0; ch < S.nchunk; ch++)
-        r += (double) a.pr[S.pr_off + ((size_t) ch * S.np + i) * C + q];
-      a.y[S.x_off + (size_t) C * i + q] = ys.v[q] + r + 2.0 * (double) acc[q];
+          for (int q = 0; q < C; q++) acc[u][q] = fmaf (ph.x, P[q], fmaf (ph.y, Q[q], acc[u][q]));
+        }
     }
+  // self + real partials + 2 reciprocal in FP64, a lane per component
+  float mine = 0.f;
+#pragma unroll
+  for (int u = 0; u < BP_N; u++)
+#pragma unroll
+    for (int q = 0; q < C; q++)
+      {
+        const float v = warp_sum (acc[u][q]);
+        if (lane == u * C + q) mine = v;
+      }
+  if (lane >= n * C) return;
+  const int i = i0 + lane / C, q = lane % C;
+  const size_t at = S.x_off + (size_t) C * i + q;
+  double r = 0.0;
+  for (int ch = 0; ch < S.nchunk; ch++)
+    r += (double) a.pr[S.pr_off + ((size_t) ch * S.np + i) * C + q];
+  a.y[at] = fma (S.selfc[q < 3 ? 0 : 1], a.x[at], fma (2.0, (double) mine, r));
 }
 
 __global__ void
 mb_bp (BatchArgs a)
 {
+  extern __shared__ float2 s_bp[];         // [warps][tab_smem][BP_N]
+  float2 *s_t = s_bp + (size_t) (threadIdx.x >> 5) * a.tab_smem * BP_N;
   const long long w = (long long) blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= a.cum_p[a.nsys]) return;
-  const int s = find_sys (a.cum_p, a.nsys, w);
+  if (w >= a.cum_b[a.nsys]) return;
+  const int s = find_sys (a.cum_b, a.nsys, w);
   const BSys S = a.sys[s];
-  const int i = (int) (w - a.cum_p[s]);
-  if (S.version == 0) mb_bp_warp<0> (a, S, i);
-  else mb_bp_warp<1> (a, S, i);
+  const int i = BP_N * (int) (w - a.cum_b[s]);
+  if (S.version == 0) mb_bp_warp<0> (a, S, i, s_t);
+  else mb_bp_warp<1> (a, S, i, s_t);
 }
 
 }  // namespace lsg
@@ -429,9 +470,14 @@ struct stokes_gpu_batch {
   std::vector<int> p_off, x_off;
   // mixed
   std::vector<lsg::BSys> h_sys;
-  std::vector<int> h_cum_p, h_cum_r, h_cum_k;
+  std::vector<int> h_cum_p, h_cum_r, h_cum_k, h_cum_b;
   std::vector<lsg::MixK> h_k;
   std::vector<float4> h_img;
+  std::vector<short4> h_km;
+  int tab_max = 0;
+  cudaStream_t real = nullptr;          // the real space beside the sums over k
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  lsg::DevBuf d_km;
   lsg::DevBuf d_sys, d_cum, d_pos, d_x, d_y, d_qpos, d_tab, d_xf, d_kt, d_pq, d_pr, d_img;
   int tab_tot = 0, k_tot = 0, pq_tot = 0, pr_tot = 0;
   int chunk_mult = 1, real_wpb = 4;     // autotuned
@@ -471,8 +517,11 @@ batch_setup_mixed (stokes_gpu_batch *b)
 {
   b->h_sys.assign (b->nsys, BSys{});
   b->h_k.clear ();
+  b->h_km.clear ();
+  b->tab_max = 0;
   b->h_img.clear ();
   b->h_cum_p.assign (b->nsys + 1, 0);
+  b->h_cum_b.assign (b->nsys + 1, 0);
   b->h_cum_k.assign (b->nsys + 1, 0);
   int tab = 0, pq = 0;
   const double eps = 3e-8;  // the single-system mixed split's truncation
@@ -564,6 +613,7 @@ batch_setup_mixed (stokes_gpu_batch *b)
               r.yb = (float) (3.0 * k * kexp);
               r.yc = (float) (1.5 * kk * kexp);
               b->h_k.push_back (r);
+              b->h_km.push_back (make_short4 ((short) m1, (short) m2, (short) m3, 0));
               M[0] = std::max (M[0], m1);
               M[1] = std::max (M[1], abs (m2));
               M[2] = std::max (M[2], abs (m3));
@@ -572,9 +622,11 @@ batch_setup_mixed (stokes_gpu_batch *b)
       S.M0 = M[0]; S.M1 = M[1]; S.M2 = M[2];
       S.tab_off = tab;
       tab += (M[0] + M[1] + M[2] + 3) * S.np;
+      b->tab_max = std::max (b->tab_max, M[0] + M[1] + M[2] + 3);
       S.pq_off = pq;
       pq += 2 * S.c * std::max (S.nkh, 1);
       b->h_cum_p[s + 1] = b->h_cum_p[s] + S.np;
+      b->h_cum_b[s + 1] = b->h_cum_b[s] + (S.np + BP_N - 1) / BP_N;
       b->h_cum_k[s + 1] = b->h_cum_k[s] + S.nkh;
     }
   b->tab_tot = tab;
@@ -605,10 +657,11 @@ batch_upload_mixed (stokes_gpu_batch *b)
 {
   cudaError_t e = cudaSuccess;
   const int ns = b->nsys;
-  std::vector<int> cum ((size_t) 3 * (ns + 1));
+  std::vector<int> cum ((size_t) 4 * (ns + 1));
   std::copy (b->h_cum_p.begin (), b->h_cum_p.end (), cum.begin ());
   std::copy (b->h_cum_r.begin (), b->h_cum_r.end (), cum.begin () + (ns + 1));
   std::copy (b->h_cum_k.begin (), b->h_cum_k.end (), cum.begin () + 2 * (ns + 1));
+  std::copy (b->h_cum_b.begin (), b->h_cum_b.end (), cum.begin () + 3 * (ns + 1));
   auto up = [&] (DevBuf &d, const void *h, size_t bytes) {
     if (e == cudaSuccess) e = d.ensure (bytes ? bytes : 16);
     if (e == cudaSuccess && bytes)
@@ -617,6 +670,7 @@ batch_upload_mixed (stokes_gpu_batch *b)
   up (b->d_sys, b->h_sys.data (), sizeof (BSys) * ns);
   up (b->d_cum, cum.data (), sizeof (int) * cum.size ());
   up (b->d_kt, b->h_k.data (), sizeof (MixK) * b->h_k.size ());
+  up (b->d_km, b->h_km.data (), sizeof (short4) * b->h_km.size ());
   up (b->d_img, b->h_img.data (), sizeof (float4) * b->h_img.size ());
   if (e == cudaSuccess) e = b->d_qpos.ensure (sizeof (uint32_t) * 4 * (size_t) b->nptot);
   if (e == cudaSuccess) e = b->d_tab.ensure (sizeof (float2) * (size_t) std::max (b->tab_tot, 1));
@@ -637,6 +691,7 @@ batch_args (stokes_gpu_batch *b)
   a.cum_p = cum;
   a.cum_r = cum + (b->nsys + 1);
   a.cum_k = cum + 2 * (b->nsys + 1);
+  a.cum_b = cum + 3 * (b->nsys + 1);
   a.pos = (const double *) b->d_pos.p;
   a.x = (const double *) b->d_x.p;
   a.y = (double *) b->d_y.p;
@@ -644,6 +699,8 @@ batch_args (stokes_gpu_batch *b)
   a.tab = (float2 *) b->d_tab.p;
   a.xf = (float *) b->d_xf.p;
   a.kt = (const MixK *) b->d_kt.p;
+  a.km = (const short4 *) b->d_km.p;
+  a.tab_smem = b->tab_max <= 180 ? b->tab_max : 0;     // 8 warps of BP_N, up to 45 KB
   a.pq = (float *) b->d_pq.p;
   a.pr = (float *) b->d_pr.p;
   a.img = (const float4 *) b->d_img.p;
@@ -659,10 +716,18 @@ batch_launch_mixed (stokes_gpu_batch *b, cudaStream_t st)
   const int wpb = b->real_wpb;
   const size_t smem = (size_t) wpb * MB_QCAP * (3 * sizeof (float) + sizeof (int));
   const long long rw = b->h_cum_r[b->nsys];
-  mb_real<<<(int) ((rw + wpb - 1) / wpb), wpb * 32, smem, st>>> (a);
   const long long kw = b->h_cum_k[b->nsys];
+  // the pair sums and the sums over k need the tables only; the
+  // back-projection adds both
+  cudaError_t e = cudaEventRecord (b->ev_fork, st);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent (b->real, b->ev_fork, 0);
+  if (e != cudaSuccess) return e;
+  mb_real<<<(int) ((rw + wpb - 1) / wpb), wpb * 32, smem, b->real>>> (a);
   if (kw > 0) mb_sfac<<<(int) ((kw + 7) / 8), 256, 0, st>>> (a);
-  mb_bp<<<(b->nptot + 7) / 8, 256, 0, st>>> (a);
+  e = cudaEventRecord (b->ev_join, b->real);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent (st, b->ev_join, 0);
+  if (e != cudaSuccess) return e;
+  mb_bp<<<(b->h_cum_b[b->nsys] + 7) / 8, 256, sizeof (float2) * 8 * BP_N * a.tab_smem, st>>> (a);
   return cudaGetLastError ();
 }
 
@@ -826,6 +891,9 @@ stokes_gpu_batch_create (struct stokes **systems, int nsys, int precision,
       b->nxtot += NCOMP (sys->version) * sys->np;
     }
   cudaError_t e = cudaStreamCreateWithFlags (&b->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags (&b->real, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags (&b->ev_fork, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags (&b->ev_join, cudaEventDisableTiming);
   if (e == cudaSuccess) e = b->d_pos.ensure (sizeof (double) * 3 * (size_t) b->nptot);
   if (e == cudaSuccess) e = b->d_x.ensure (sizeof (double) * (size_t) b->nxtot);
   if (e == cudaSuccess) e = b->d_y.ensure (sizeof (double) * (size_t) b->nxtot);
@@ -886,9 +954,13 @@ stokes_gpu_batch_destroy (stokes_gpu_batch *b)
   for (cudaStream_t s : b->side) cudaStreamDestroy (s);
   for (cudaEvent_t e : b->side_ev) cudaEventDestroy (e);
   for (DevBuf *d : {&b->d_sys, &b->d_cum, &b->d_pos, &b->d_x, &b->d_y, &b->d_qpos, &b->d_tab,
-                    &b->d_xf, &b->d_kt, &b->d_pq, &b->d_pr, &b->d_img})
+                    &b->d_xf, &b->d_kt, &b->d_pq, &b->d_pr, &b->d_img,
+                    &b->d_km})
     d->release ();
   if (b->stream) cudaStreamDestroy (b->stream);
+  if (b->real) cudaStreamDestroy (b->real);
+  if (b->ev_fork) cudaEventDestroy (b->ev_fork);
+  if (b->ev_join) cudaEventDestroy (b->ev_join);
   delete b;
   return STOKES_GPU_OK;
 }

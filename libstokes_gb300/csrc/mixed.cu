@@ -302,10 +302,7 @@ two_sum (float a, float b, float &s, float &e)
 }
 
 constexpr int RG_WARPS = 8;      // warps per CTA of mk_real
-constexpr int RG_QCAP = 192;     // queue entries per warp (the reduction reuses them)
-constexpr int RG_MAXIMG = 4;     // lattice offsets tested per candidate in one pass
-// a pass adds at most 32 RG_MAXIMG entries to at most 31 left over
-static_assert (31 + 32 * RG_MAXIMG <= RG_QCAP, "mk_real queue too small");
+constexpr int RG_QCAP = 64;      // queue entries per warp: 32 are added to at most 31 left over
 
 // The real-space sum of the mixed split: G warps per target particle.  Each
 // warp takes a share of the candidate sources (a slice of all particles, or
@@ -379,44 +376,40 @@ mk_real (RealMixArgs a)
             qn += __popc (b);
           }
         else
-          for (int m0 = 0; m0 < a.nimg; m0 += RG_MAXIMG)
+          // this lane's accepted offsets as a bit mask, 32 at a time, then one
+          // of each lane's per round into the queue
+          for (int m0 = 0; m0 < a.nimg; m0 += 32)
             {
-              // this lane's accepted offsets m0 .. m0 + 3 as a bit mask, then
-              // a warp prefix sum of the counts places them
+              const int n = min (32, a.nimg - m0);
               unsigned mask = 0u;
-              if (sj < s1)
-#pragma unroll
-                for (int k = 0; k < RG_MAXIMG; k++)
-                  {
-                    if (m0 + k >= a.nimg) break;
-                    const float4 T = a.img[m0 + k];
-                    const float dx = d0x + T.x, dy = d0y + T.y, dz = d0z + T.z;
-                    const float rr = dx * dx + dy * dy + dz * dz;
-                    if (rr > 0.f && rr < a.rc2 && !(a.clampfix && rr < a.rm2)) mask |= 1u << k;
-                  }
-              const int cnt = __popc (mask);
-              int pre = cnt;
-#pragma unroll
-              for (int o = 1; o < 32; o <<= 1)
+#pragma unroll 4
+              for (int k = 0; k < n; k++)
                 {
-                  const int v = __shfl_up_sync (0xffffffffu, pre, o);
-                  if (lane >= o) pre += v;
-                }
-              int slot = qn + pre - cnt;
-              while (mask)
-                {
-                  const int k = __ffs (mask) - 1;
-                  mask &= mask - 1u;
                   const float4 T = a.img[m0 + k];
-                  q[slot++] = make_float4 (d0x + T.x, d0y + T.y, d0z + T.z, __int_as_float (j));
+                  const float dx = d0x + T.x, dy = d0y + T.y, dz = d0z + T.z;
+                  const float rr = dx * dx + dy * dy + dz * dz;
+                  if (rr > 0.f && rr < a.rc2 && !(a.clampfix && rr < a.rm2)) mask |= 1u << k;
                 }
-              qn += __shfl_sync (0xffffffffu, pre, 31);
-              __syncwarp ();
-              while (qn >= 32)
+              if (sj >= s1) mask = 0u;
+              for (;;)
                 {
-                  mix_term<V, POLY> (a, q[qn - 32 + lane], ai, sum);
-                  qn -= 32;
+                  const unsigned b = __ballot_sync (0xffffffffu, mask != 0u);
+                  if (b == 0u) break;
+                  if (mask)
+                    {
+                      const float4 T = a.img[m0 + __ffs (mask) - 1];
+                      q[qn + __popc (b & lt)]
+                        = make_float4 (d0x + T.x, d0y + T.y, d0z + T.z, __int_as_float (j));
+                      mask &= mask - 1u;
+                    }
+                  qn += __popc (b);
                   __syncwarp ();
+                  if (qn >= 32)
+                    {
+                      mix_term<V, POLY> (a, q[qn - 32 + lane], ai, sum);
+                      qn -= 32;
+                      __syncwarp ();
+                    }
                 }
             }
         __syncwarp ();
