@@ -140,6 +140,8 @@ free_ctx (Ctx *c)
   for (int q = 0; q < 4; q++) cudaEventDestroy (c->ev[q]);
   for (int q = 0; q < 2; q++) cudaEventDestroy (c->join[q]);
   if (c->hpos) cudaFreeHost (c->hpos);
+  if (c->hx.p) cudaFreeHost (c->hx.p);
+  if (c->hy.p) cudaFreeHost (c->hy.p);
   cudaStreamDestroy (c->stream);
   release_mixed (c);
   release_fix (c);
@@ -796,6 +798,32 @@ mapped_positions (Ctx *c, const struct stokes *sys)
   return c->hpos_dev;
 }
 
+// A pinned, mapped buffer of the context for a vector of a small mixed host
+// call: copying it on the host and letting the device read or write it there
+// is quicker than a copy of pageable memory, which waits twice (FT N = 333 65
+// -> 54 us a call).  Larger vectors are not staged, nor those of FP64 products,
+// whose kernels read x several times (F N = 64 83 us, 89 with a staged copy).
+constexpr size_t STAGE_MAX = 256 * 1024;
+
+static bool
+host_stage (Ctx::Stage &s, size_t bytes)
+{
+  if (bytes > STAGE_MAX) return false;
+  if (s.bytes >= bytes) return true;
+  if (s.p) cudaFreeHost (s.p);
+  s = Ctx::Stage {};
+  if (cudaHostAlloc ((void **) &s.p, bytes, cudaHostAllocMapped) != cudaSuccess)
+    {
+      cudaGetLastError ();
+      s.p = nullptr;
+      return false;
+    }
+  s.dev = (double *) mapped_host (s.p);
+  if (!s.dev) return false;
+  s.bytes = bytes;
+  return true;
+}
+
 int
 atimes_host (struct stokes *sys, const double *x, double *y, bool cube)
 {
@@ -813,21 +841,38 @@ atimes_host (struct stokes *sys, const double *x, double *y, bool cube)
   // through their device mapping -- over the CPU-GPU link -- without a
   // staging copy and its latency: y always (each element is written once),
   // x on the mixed paths, which read it twice (the FP64 kernels read x once
-  // per reciprocal vector or pair and take a device copy); other host
-  // memory goes through device copies
-  const double *d_x = c->precision == STOKES_GPU_MIXED ? (const double *) mapped_host (x) : nullptr;
-  double *d_y = (double *) mapped_host (y);
+  // per reciprocal vector or pair and take a device copy); small vectors of
+  // mixed products in other host memory pass through the context's pinned
+  // buffers, the others through device copies
+  const bool mixed = c->precision == STOKES_GPU_MIXED;
+  const size_t nb = sizeof (double) * n;
+  const double *d_x = mixed ? (const double *) mapped_host (x) : nullptr;
+  double *d_y = (double *) mapped_host (y), *y_stage = nullptr;
   if (!d_x)
     {
-      if ((e = c->x.ensure (sizeof (double) * n)) != cudaSuccess) return cuda_fail (e, "x");
-      cudaMemcpyAsync (c->x.p, x, sizeof (double) * n, cudaMemcpyHostToDevice, c->stream);
-      d_x = (const double *) c->x.p;
+      if (mixed && host_stage (c->hx, nb))
+        {
+          memcpy (c->hx.p, x, nb);
+          d_x = c->hx.dev;
+        }
+      else
+        {
+          if ((e = c->x.ensure (nb)) != cudaSuccess) return cuda_fail (e, "x");
+          cudaMemcpyAsync (c->x.p, x, nb, cudaMemcpyHostToDevice, c->stream);
+          d_x = (const double *) c->x.p;
+        }
     }
   if (!d_y)
     {
-      if ((e = c->y.ensure (sizeof (double) * n)) != cudaSuccess) return cuda_fail (e, "y");
+      if (mixed && host_stage (c->hy, nb))
+        {
+          d_y = c->hy.dev;
+          y_stage = c->hy.p;
+        }
+      else if ((e = c->y.ensure (nb)) != cudaSuccess)
+        return cuda_fail (e, "y");
     }
-  const double *d_pos = c->precision == STOKES_GPU_MIXED ? mapped_positions (c, sys) : nullptr;
+  const double *d_pos = mixed ? mapped_positions (c, sys) : nullptr;
   if (!d_pos)
     {
       cudaMemcpyAsync (c->pos.p, sys->pos, sizeof (double) * 3 * np, cudaMemcpyHostToDevice,
@@ -844,6 +889,7 @@ atimes_host (struct stokes *sys, const double *x, double *y, bool cube)
   if (c->precision == STOKES_GPU_MIXED && !c->open && (rc = mixed_check_status (c)) != 0)
     return rc;
   if (c->use_fix && (rc = fix_check_status (c)) != 0) return rc;
+  if (y_stage) memcpy (y, y_stage, nb);
   collect_times (c);
   sys->cpu1 = c->times[0];
   sys->cpu2 = c->times[1];

@@ -94,6 +94,11 @@ struct Ctx {
 
   // pinned, mapped mirror of sys->pos for the host entry points of the
   // mixed paths, whose kernels read the positions once
+  // pinned buffers that small host calls pass x and y through (host_stage)
+  struct Stage {
+    double *p = nullptr, *dev = nullptr;      // its host and device addresses
+    size_t bytes = 0;
+  } hx, hy;
   double *hpos = nullptr;
   const double *hpos_dev = nullptr;   // its device address
   size_t hpos_bytes = 0;
