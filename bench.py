@@ -314,8 +314,6 @@ def matrix_measure(lib, abi, L, torch, dev, pos, Lbox):
     ms = e0.elapsed_time(e1)
     nbytes = 8.0 * n * n
     peak = measured_peaks().get("hbm_gbs")
-    P = C.c_longlong()
-    abi.check(lib.stokes_gpu_count_real_terms_dense(s.sp, C.byref(P)))
     # the split-precision builder (FP32 terms, FP64 entries) on the same
     # system, and its largest entry error against the FP64 matrix
     s.set_precision(abi.MIXED)
@@ -337,13 +335,12 @@ def matrix_measure(lib, abi, L, torch, dev, pos, Lbox):
     return {"workload": f"matrix_fts_n{w['n']}_phi{w['phi']:.2f}", "precision": "fp64",
             "ms": ms, "bytes": nbytes, "achieved_gbs": gbs, "hbm_peak_gbs": peak,
             "hbm_frac": gbs / peak if peak else None,
-            "pair_image_terms": P.value, "terms_per_s": P.value / (ms * 1e-3),
             "mixed": {"ms": ms32, "achieved_gbs": nbytes / (ms32 * 1e-3) / 1e9,
                       "hbm_frac": (nbytes / (ms32 * 1e-3) / 1e9) / peak if peak else None,
                       "max_err_over_max_entry": err32,
                       "precision": "FP32 terms, FP64 entries (k_matrix_pairs)"},
-            "bound": "fp64-pipe: every pair-image term of the reference split "
-                     "(xi = sqrt(pi)/L, eps 1e-12) builds an 11 x 11 block in FP64"}
+            "bound": "start and integer epilogue of the moment GEMM's CTAs (four K tiles "
+                     "each), then the FP64 pipe in the real-space moments"}
 
 
 def lub_measure(lib, abi, L, torch, dev, reps: int = 20):
@@ -848,10 +845,10 @@ def roofline_of(lib, abi, sysm, version, n, c, kernels_ms, precision, name, work
         flops = 4.0 * units
         if name.startswith("k_"):
             bound = "tensor"
-            peak = peaks.get("bf16_tflops", 1900.0) / 2.0
-            psrc = ("TF32 dense rate taken as half the measured bf16 GEMM rate "
-                    "(MEASURED_PEAKS.json bf16_tflops / 2); the 3xTF32 split executes 3x "
-                    "the algorithmic count and the m1 >= 0 box about 2x more")
+            peak = peaks.get("bf16_tflops", 1900.0)
+            psrc = ("measured bf16 GEMM rate (MEASURED_PEAKS.json bf16_tflops); operands "
+                    "are three 8-bit digits in f16, six digit products per algorithmic one, "
+                    "over one octant of k space")
         else:
             bound = "fp32-pipe"
             pk = C.c_double()

@@ -180,8 +180,8 @@ int stokes_gpu_last_launches (const struct stokes *sys, int *count);
 
 /* number of real-space (i, j, image) terms with 0 < r^2 <= rmax2 -- the
  * unit count of the real-space roofline -- at the split of the FP64
- * product (the tuned split where it applies) and at that of the dense
- * builder (the reference's split) */
+ * product (the tuned split where it applies) and at the reference's split
+ * (that of the dense builder for unequal radii, slip and shear) */
 int stokes_gpu_count_real_terms (struct stokes *sys, long long *count);
 int stokes_gpu_count_real_terms_dense (struct stokes *sys, long long *count);
 

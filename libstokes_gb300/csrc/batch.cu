@@ -796,7 +796,13 @@ batch_run (stokes_gpu_batch *b, float *ms)
   cudaEventDestroy (e0);
   cudaEventDestroy (e1);
   if (ms) *ms = t;
-  return e == cudaSuccess ? STOKES_GPU_OK : cuda_fail (e, "batch product");
+  if (e != cudaSuccess) return cuda_fail (e, "batch product");
+  // FP64: a bounded wait of a system's tensor-core kernels that ran out
+  if (b->precision != STOKES_GPU_MIXED)
+    for (int k = 0; k < b->nsys; k++)
+      if (Ctx *c = get_ctx (b->sys[k], false))
+        if (const int rc = fix_check_status (c)) return rc;
+  return STOKES_GPU_OK;
 }
 
 // time a few splits, then real-space chunkings and CTA sizes, keep the fastest

@@ -330,9 +330,9 @@ k_dense_tile (const __grid_constant__ DenseArgs a)
           const int4 o = a.cell[en >> 6];
           const unsigned long long *ui = a.u + 4 * (size_t) ei, *uj = a.u + 4 * (size_t) ej;
           double d[3], c[NF];
-          d[0] = int_to_double (((long long) (uj[0] - ui[0]) >> 4) + ((long long) o.x << 60)) * a.s60[0];
-          d[1] = int_to_double (((long long) (uj[1] - ui[1]) >> 4) + ((long long) o.y << 60)) * a.s60[1];
-          d[2] = int_to_double (((long long) (uj[2] - ui[2]) >> 4) + ((long long) o.z << 60)) * a.s60[2];
+          d[0] = int_to_double (image_diff (ui[0], uj[0]) + ((long long) o.x << 60)) * a.s60[0];
+          d[1] = int_to_double (image_diff (ui[1], uj[1]) + ((long long) o.y << 60)) * a.s60[1];
+          d[2] = int_to_double (image_diff (ui[2], uj[2]) + ((long long) o.z << 60)) * a.s60[2];
           const double s = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
           const int bin = radial_bin (s, a.bin0);
           if (s == 0.0)

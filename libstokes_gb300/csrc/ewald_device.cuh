@@ -470,6 +470,18 @@ warp_sum (R v)
   return v;
 }
 
+// b - a of two 64-bit fractional coordinates in units of 2^-60 of the box, at
+// the image that their upper halves give: near half a box the difference of all
+// 64 bits can lie at the other image than the FP32 test of the pair, which sees
+// the upper halves, and a lattice offset listed there would not belong to it
+__device__ __forceinline__ long long
+image_diff (unsigned long long a, unsigned long long b)
+{
+  const int w = (int) ((unsigned) (b >> 32) - (unsigned) (a >> 32));
+  const long long lo = (long long) (unsigned) b - (long long) (unsigned) a;
+  return ((long long) w << 28) + (lo >> 4);
+}
+
 // a signed 64-bit integer as FP64, rounded to nearest (ties away), in integer
 // arithmetic: conversions run at the FP64 rate, 1/64 of the integer one
 __device__ __forceinline__ double

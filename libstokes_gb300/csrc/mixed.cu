@@ -11,8 +11,9 @@
 //    overflow, so pair geometry costs no FP64 and loses no digits;
 //  * real space: FP32 pair terms (erfcf/expf), compacted per warp;
 //  * reciprocal space: 24-bit fixed-point GEMMs over products of real functions
-//    of x, y and z (kspace_mix.cu); for unequal radii structure factors C(k),
-//    S(k) over half of k space with e^{ik.r} from per-particle phase tables;
+//    of x, y and z (kspace_mix.cu); small systems: structure factors C(k), S(k)
+//    over half of k space with e^{ik.r} from per-particle phase tables, at a
+//    lower split with lattice images (small_system);
 //  * FP64: the self term, the split constants and the final combination.
 #include <cuda_runtime.h>
 

@@ -229,9 +229,9 @@ k_real_tab (RealTabArgs a)
         int4 o = make_int4 (0, 0, 0, 0);
         if (a.nimg > 1) o = a.cell[en >> 24];
         // in units of 2^-60 of the box
-        d[0] = int_to_double (((long long) (ub.x - ua.x) >> 4) + ((long long) o.x << 60)) * a.s60[0];
-        d[1] = int_to_double (((long long) (ub.y - ua.y) >> 4) + ((long long) o.y << 60)) * a.s60[1];
-        d[2] = int_to_double (((long long) (vz - uz) >> 4) + ((long long) o.z << 60)) * a.s60[2];
+        d[0] = int_to_double (image_diff (ua.x, ub.x) + ((long long) o.x << 60)) * a.s60[0];
+        d[1] = int_to_double (image_diff (ua.y, ub.y) + ((long long) o.y << 60)) * a.s60[1];
+        d[2] = int_to_double (image_diff (uz, vz) + ((long long) o.z << 60)) * a.s60[2];
       };
       for (int k = t; k < n; k += RT_T)
         {

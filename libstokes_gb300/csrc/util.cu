@@ -67,7 +67,11 @@ count_terms (struct stokes *sys, int tables, long long *count)
   if (!count) return set_error (STOKES_GPU_EINVAL, "NULL count");
   Ctx *c = get_ctx (sys, true);
   if (!c) return set_error (STOKES_GPU_ECUDA, "cannot create a CUDA stream");
+  // 2: the reference's split, whatever builder the system would take
+  const bool tune = c->tune;
+  if (tables == 2) c->tune = false;
   int rc = prepare (c, sys, false, tables);
+  c->tune = tune;
   if (rc) return rc;
   cudaError_t e;
   if ((e = c->pos.ensure (sizeof (double) * 3 * sys->np)) != cudaSuccess) return cuda_fail (e, "pos");
@@ -96,7 +100,7 @@ stokes_gpu_count_real_terms (struct stokes *sys, long long *count)
   return count_terms (sys, 1, count);
 }
 
-// terms of the dense builder's split (the reference's)
+// terms of the reference's split, that of the builder k_matrix
 int
 stokes_gpu_count_real_terms_dense (struct stokes *sys, long long *count)
 {

@@ -38,10 +38,10 @@ def test_oracle(lib, version, n, side):
     s.close()
 
 
-# 137 particles: 171 tiles, two chunks; unequal sides
+# 201 particles: 351 tiles, two chunks; unequal sides
 @pytest.mark.parametrize("version", [0, 1, 2])
 @pytest.mark.parametrize("n,box", [(64, (17.0, 17.0, 17.0)), (45, (12.0, 22.0, 16.0)),
-                                   (40, (26.0, 11.0, 13.0)), (137, (21.0, 24.0, 20.0))])
+                                   (40, (26.0, 11.0, 13.0)), (201, (24.0, 27.0, 22.0))])
 def test_cube_builder(lib, version, n, box):
     from libstokes_gb300 import System
     rng = np.random.default_rng(n + version)
@@ -108,4 +108,43 @@ def test_bounded_waits(lib):
     finally:
         lib.stokes_gpu_test_stall_waits(0, 0)
     assert np.array_equal(s.matrix(), m)
+    s.close()
+
+
+def test_count_of_reference_terms(lib):
+    """The term count is that of the reference's split, also where the builder
+    takes a split of its own."""
+    import ctypes as C
+    from libstokes_gb300 import System, check
+    rng = np.random.default_rng(9)
+    s = System(2, _positions(40, (14.0, 14.0, 14.0), rng), (14.0, 14.0, 14.0))
+    counts = []
+    for _ in range(2):
+        p = C.c_longlong()
+        check(lib.stokes_gpu_count_real_terms_dense(s.sp, C.byref(p)))
+        counts.append(p.value)
+        s.matrix()
+    v = 4.0 / 3.0 * np.pi * s.s.rmax2 ** 1.5 / 14.0 ** 3
+    assert counts[0] == counts[1] and 0.9 < counts[0] / (40 * 40 * v) < 1.1
+    s.close()
+
+
+def _fcc(n, side, rng):
+    m = 1
+    while 4 * m ** 3 < n:
+        m += 1
+    base = np.array([[0, 0, 0], [0, .5, .5], [.5, 0, .5], [.5, .5, 0]])
+    g = np.stack(np.meshgrid(*(np.arange(m),) * 3, indexing="ij"), -1).reshape(-1, 1, 3)
+    sites = ((g + base) * side / m).reshape(-1, 3)
+    return sites[rng.permutation(len(sites))[:n]] + rng.uniform(0, side, 3)
+
+
+@pytest.mark.parametrize("version", [0, 1, 2])
+@pytest.mark.parametrize("n,side", [(32, 9.0), (112, 11.1), (112, 13.0), (120, 15.0)])
+def test_lattice_positions(lib, version, n, side):
+    """Many pairs exactly half a box apart."""
+    from libstokes_gb300 import System
+    rng = np.random.default_rng(n + version)
+    s = System(version, _fcc(n, side, rng), (side, side, side))
+    assert rel_l2(s.matrix(), s.matrix(notbl=True)) < 1e-12
     s.close()

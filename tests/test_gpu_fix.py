@@ -172,3 +172,28 @@ def test_new_inputs_every_time(version, n, side):
         assert rel_l2(s.atimes(x), f.atimes(x, notbl=True)) < 1e-12
     s.close()
     f.close()
+
+
+def _fcc(n, side, rng):
+    m = 1
+    while 4 * m ** 3 < n:
+        m += 1
+    base = np.array([[0, 0, 0], [0, .5, .5], [.5, 0, .5], [.5, .5, 0]])
+    g = np.stack(np.meshgrid(*(np.arange(m),) * 3, indexing="ij"), -1).reshape(-1, 1, 3)
+    sites = ((g + base) * side / m).reshape(-1, 3)
+    return sites[rng.permutation(len(sites))[:n]] + rng.uniform(0, side, 3)
+
+
+@pytest.mark.parametrize("version", [0, 1, 2])
+@pytest.mark.parametrize("n,side", [(32, 8.9), (112, 11.1), (112, 13.0), (120, 11.2), (256, 18.0)])
+def test_lattice_positions(lib, version, n, side):
+    """Spheres on a lattice: many pairs exactly half a box apart, where both
+    images count and rounding decides which one is the nearest."""
+    from libstokes_gb300 import System
+    rng = np.random.default_rng(n + version)
+    box = (side, side, side)
+    pos = _fcc(n, side, rng)
+    s = System(version, pos, box)
+    x = rng.standard_normal((3, 6, 11)[version] * n)
+    assert rel_l2(s.atimes(x), s.atimes(x, notbl=True)) < 1e-12
+    s.close()

@@ -150,3 +150,49 @@ def test_unequal_radii(version, n, side):
         assert rel_l2(s.atimes(x), f.atimes(x)) < TOL
     s.close()
     f.close()
+
+
+@pytest.mark.parametrize("version,equal", [(0, True), (2, True), (1, False)])
+def test_cells(version, equal, monkeypatch):
+    """The cell list of the real space (here forced by a high split), whose
+    sources, their vectors and radii come in cell order."""
+    from libstokes_gb300 import MIXED, System
+    monkeypatch.setenv("LIBSTOKES_GB300_MIXED_ETA", "17")
+    rng = np.random.default_rng(95)
+    n, box = 701, (38.0, 42.0, 40.0)
+    pos, radius = _positions(n, box, rng), rng.uniform(0.5, 1.0, n)
+    s, f = System(version, pos, box), System(version, pos, box)
+    if not equal:
+        s.set_radius(radius)
+        f.set_radius(radius)
+    s.set_precision(MIXED)
+    for _ in range(3):
+        x = rng.standard_normal((3, 6, 11)[version] * n)
+        assert rel_l2(s.atimes(x), f.atimes(x)) < TOL
+    s.close()
+    f.close()
+
+
+def _fcc(n, side, rng):
+    m = 1
+    while 4 * m ** 3 < n:
+        m += 1
+    base = np.array([[0, 0, 0], [0, .5, .5], [.5, 0, .5], [.5, .5, 0]])
+    g = np.stack(np.meshgrid(*(np.arange(m),) * 3, indexing="ij"), -1).reshape(-1, 1, 3)
+    sites = ((g + base) * side / m).reshape(-1, 3)
+    return sites[rng.permutation(len(sites))[:n]] + rng.uniform(0, side, 3)
+
+
+@pytest.mark.parametrize("version", [0, 1, 2])
+@pytest.mark.parametrize("n,side", [(32, 8.9), (112, 11.1), (256, 18.0), (530, 24.0)])
+def test_lattice_positions(version, n, side):
+    """Many pairs exactly half a box apart."""
+    from libstokes_gb300 import MIXED, System
+    rng = np.random.default_rng(n + version)
+    box = (side, side, side)
+    s = System(version, _fcc(n, side, rng), box)
+    x = rng.standard_normal((3, 6, 11)[version] * n)
+    y = s.atimes(x, notbl=True)
+    s.set_precision(MIXED)
+    assert rel_l2(s.atimes(x), y) < TOL
+    s.close()
