@@ -217,6 +217,7 @@ struct RealMixArgs {
   float rm2;
   float xi_ref, xisp_ref;
   float *out_clamp;      // [np][c]: mk_clamp's sums (a third combine chunk)
+  int nclamp;            // lattice offsets that can bring a pair under the clamp
 };
 
 // minimum-image displacement r_j - r_i from fixed-point positions
@@ -516,9 +517,11 @@ mk_clamp (RealMixArgs a)
       const uint4 qj = reinterpret_cast<const uint4 *> (a.qpos)[j];
       float d0x, d0y, d0z;
       min_image (a, qi, qj, d0x, d0y, d0z);
-      for (int m = 0; m < a.nimg; m++)
+      // within half the box only the minimum image can be under the clamp
+      for (int m = 0; m < a.nclamp; m++)
         {
-          const float4 T = a.img[m];
+          float4 T = make_float4 (0.f, 0.f, 0.f, 0.f);
+          if (a.nclamp > 1) T = a.img[m];
           const float dx = d0x + T.x, dy = d0y + T.y, dz = d0z + T.z;
           const float rr = dx * dx + dy * dy + dz * dz;
           if (!(rr > 0.f && rr < a.rm2)) continue;
@@ -1061,6 +1064,9 @@ default_eta_images (int np)
 //   FT   N = 64 22.7 / 40.4, 333 37.0 / 42.5, 500 45.2 / 44.6
 //   FTS  N = 64 24.7 / 41.5, 250 37.0 / 49.7, 400 52.6 / 50.8
 //   unequal radii: F 400 39 / 49, FT 333 43 / 51, FTS 250 45 / 67
+// Under the rmin clamp its kernel (mk_clamp) follows the real space, so F turns
+// earlier: a BD step of 33 products N = 250 1412 / 1493 us, 350 1718 / 1476; FT
+// 330 1545 / 1640, 400 1705 / 1700.
 // A long box would need many images of its short sides.
 // LIBSTOKES_GB300_KSPACE=tc keeps the GEMMs, =simt the SIMT kernels.
 static bool
@@ -1068,7 +1074,7 @@ small_system (const struct stokes *sys)
 {
   const double lmin = fmin (sys->lx, fmin (sys->ly, sys->lz));
   const double lmax = fmax (sys->lx, fmax (sys->ly, sys->lz));
-  const int most = sys->version == 0 ? 512 : (sys->version == 1 ? 400 : 256);
+  const int most = sys->version == 0 ? (sys->rmin > 0.0 ? 256 : 512) : (sys->version == 1 ? 400 : 256);
   return sys->np <= most && lmax <= 2.0 * lmin;
 }
 
@@ -1781,6 +1787,7 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
     ra.slipa = nullptr;
     ra.clampfix = sys->rmin > 0.0 ? 1 : 0;
     ra.rm2 = (float) (4.0 * sys->rmin * sys->rmin);
+    ra.nclamp = 2.0 * sys->rmin < 0.5 * fmin (sys->lx, fmin (sys->ly, sys->lz)) ? 1 : m->nimg;
     ra.out_clamp = (float *) m->part_real.p + (size_t) 2 * np * C;
     ra.xi_ref = (float) sys->xi;
     ra.xisp_ref = (float) (sys->xi / sqrt (M_PI));
