@@ -592,8 +592,8 @@ struct DenseState {
   FixMaps maps;
   DenseArgs a;
   int tiles = 0, chunk = 0;     // tiles in all; of a chunk
-  DevBuf arena, status;
-  int *h_status = nullptr;
+  DevBuf arena;
+  int *h_status = nullptr, *d_status = nullptr;
 };
 
 // Split of the builder: eta = xi V^(1/3).  The GEMM's work grows as eta^3, the
@@ -829,16 +829,7 @@ dense_setup (Ctx *c, const struct stokes *sys)
   if (e == cudaSuccess)
     e = cudaMemcpyAsync (base, host.data (), host.size (), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemsetAsync (base + zero0, 0, zero1 - zero0, st);
-  if (e == cudaSuccess && !f->status.p)
-    {
-      e = f->status.ensure (sizeof (int));
-      if (e == cudaSuccess) e = cudaMemsetAsync (f->status.p, 0, sizeof (int), st);
-    }
-  if (e == cudaSuccess && !f->h_status)
-    {
-      e = cudaMallocHost (&f->h_status, sizeof (int));
-      if (e == cudaSuccess) *f->h_status = 0;
-    }
+  if (e == cudaSuccess) e = status_word (&f->h_status, &f->d_status);
   if (e != cudaSuccess) return cuda_fail (e, "dense builder set-up");
   p.quart = (const int4 *) (base + o_quart);
   p.nqm = (const int *) (base + o_nqm);
@@ -950,13 +941,12 @@ matrix_fix_dev (Ctx *c, const double *d_pos, double *d_mat, cudaStream_t st)
   if (*f->h_status)
     {
       *f->h_status = 0;
-      cudaMemsetAsync (f->status.p, 0, sizeof (int), st);
       return set_error (STOKES_GPU_ETIMEOUT,
                         "a tensor-core wait of the previous dense builder ran out");
     }
   FixPlan p = f->p;
   p.stall = g_test_gemm_stall;
-  int *status = (int *) f->status.p;
+  int *status = f->d_status;
   kmark (c, st, nullptr);
   cudaError_t e = launch_fix_functions (f->base, d_pos, st);
   if (e != cudaSuccess) return cuda_fail (e, "function tables");
@@ -976,7 +966,6 @@ matrix_fix_dev (Ctx *c, const double *d_pos, double *d_mat, cudaStream_t st)
       if (e != cudaSuccess) return cuda_fail (e, "matrix kernel");
       launches += 4;
     }
-  cudaMemcpyAsync (f->h_status, f->status.p, sizeof (int), cudaMemcpyDeviceToHost, st);
   c->launches = launches;
   return STOKES_GPU_OK;
 }
@@ -988,8 +977,6 @@ dense_check_status (Ctx *c)
   DenseState *f = c->dfix;
   if (!f || !f->h_status || !*f->h_status) return STOKES_GPU_OK;
   *f->h_status = 0;
-  cudaMemsetAsync (f->status.p, 0, sizeof (int), c->stream);
-  cudaStreamSynchronize (c->stream);
   return set_error (STOKES_GPU_ETIMEOUT, "a tensor-core wait of the dense builder ran out");
 }
 
@@ -999,7 +986,6 @@ release_dense (Ctx *c)
   DenseState *f = c->dfix;
   if (!f) return;
   f->arena.release ();
-  f->status.release ();
   if (f->ts) stokes_free (f->ts);
   if (f->h_status) cudaFreeHost (f->h_status);
   delete f;

@@ -80,7 +80,12 @@ cta_setup (Sync &s)
 __device__ __forceinline__ void
 cta_finish (Sync &s, uint32_t tmem, int *status)
 {
-  if (threadIdx.x == 0 && s.err) atomicExch (status, 1);
+  if (threadIdx.x == 0 && s.err)
+    {
+      // (pinned host memory, see status_word)
+      *(volatile int *) status = 1;
+      __threadfence_system ();
+    }
   umma::fence_before_sync ();
   __syncthreads ();
   if (threadIdx.x < 32) umma::tmem_dealloc (tmem, TMEM_COLS);

@@ -798,6 +798,20 @@ mapped_positions (Ctx *c, const struct stokes *sys)
   return c->hpos_dev;
 }
 
+cudaError_t
+status_word (int **host, int **dev)
+{
+  if (*host) return cudaSuccess;
+  cudaError_t e = cudaHostAlloc ((void **) host, sizeof (int), cudaHostAllocMapped);
+  if (e != cudaSuccess)
+    {
+      *host = nullptr;
+      return e;
+    }
+  **host = 0;
+  return cudaHostGetDevicePointer ((void **) dev, *host, 0);
+}
+
 // A pinned, mapped buffer of the context for a vector of a small mixed host
 // call: copying it on the host and letting the device read or write it there
 // is quicker than a copy of pageable memory, which waits twice (FT N = 333 65

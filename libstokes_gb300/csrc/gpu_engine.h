@@ -158,6 +158,10 @@ int dense_check_status (Ctx *c);
 void release_dense (Ctx *c);
 void collect_times (Ctx *c);
 cudaEvent_t *phase_events (Ctx *c, bool timed);
+// a status word that kernels raise when a bounded wait runs out: pinned host
+// memory that they write in place, so that a product needs no copy to report it
+// (a copy engine's turn at its end, 2-6 us)
+cudaError_t status_word (int **host, int **dev);
 // record a kernel-profiling mark on st when the window is open
 void kmark (Ctx *c, cudaStream_t st, const char *name);
 

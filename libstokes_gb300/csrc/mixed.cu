@@ -51,7 +51,7 @@ struct MixedState {
   int nk_split = 0;      // rows of the re-tuned split; the rest: reference G term
   double selfc[3] = {0, 0, 0};
   std::vector<MixK> h_k;
-  DevBuf kt, qpos, tab, xf, pq, part_real, part_rec, selfbuf, status, rot;
+  DevBuf kt, qpos, tab, xf, pq, part_real, part_rec, selfbuf, rot;
   DevBuf img;                   // real-space lattice offsets (float4)
   int nimg = 1;
   // tensor-core reciprocal sum (kspace_mix.cu): plan, TMA maps and one
@@ -68,7 +68,7 @@ struct MixedState {
   // the recorded launch sequence (run_mixed_sequence)
   cudaGraphExec_t gexec = nullptr;
   uint64_t gkey = 0, gcand = 0;
-  int *h_status = nullptr;      // pinned copy of the kernels' status word
+  int *h_status = nullptr, *d_status = nullptr;    // the kernels' status word (status_word)
   bool tensor = true;           // reciprocal space on the tensor cores
   uint64_t self_fp = 0;
   int self_np = 0;
@@ -1500,7 +1500,7 @@ run_mixed_sequence (Ctx *c, MixedState *m, const double *d_pos, const double *d_
   mix ((uint64_t) m->nc[0] * 1000003ull + (uint64_t) m->nc[1] * 1009ull + (uint64_t) m->nc[2]);
   mix ((uint64_t) m->nchunk_k);
   const void *ptrs[] = {d_pos, d_x, d_y, m->kt.p, m->qpos.p, m->tab.p, m->xf.p, m->pq.p,
-                        m->part_real.p, m->part_rec.p, m->selfbuf.p, m->status.p,
+                        m->part_real.p, m->part_rec.p, m->selfbuf.p,
                         m->rot.p, m->mix.p, m->h_status, m->img.p, m->sq.p, m->xs.p, m->cstart.p, m->prad.p, m->pqa.p, m->pself.p};
   for (const void *p : ptrs) mix ((uint64_t) (uintptr_t) p);
   mix ((uint64_t) (uintptr_t) E);
@@ -1621,18 +1621,11 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
   if (m->h_status && *m->h_status)
     {
       *m->h_status = 0;
-      cudaMemsetAsync (m->status.p, 0, sizeof (int), st);
       return set_error (STOKES_GPU_ETIMEOUT,
                         "a tensor-core wait of the previous mixed product ran out");
     }
   cudaError_t e;
-  if (!m->h_status)
-    {
-      if ((e = cudaMallocHost (&m->h_status, sizeof (int))) != cudaSuccess) return cuda_fail (e, "status");
-      *m->h_status = 0;
-      if ((e = m->status.ensure (sizeof (int))) != cudaSuccess) return cuda_fail (e, "status");
-      cudaMemsetAsync (m->status.p, 0, sizeof (int), st);
-    }
+  if ((e = status_word (&m->h_status, &m->d_status)) != cudaSuccess) return cuda_fail (e, "status");
   if (!m->side)
     {
       int lo = 0, hi = 0;
@@ -1882,7 +1875,7 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
     // then the real-space partials, the back-projection and the final sum
     if (fused)
       {
-        if ((e = launch_mix_forward (c->version, m->mp, m->maps, (int *) m->status.p, st, c))
+        if ((e = launch_mix_forward (c->version, m->mp, m->maps, m->d_status, st, c))
             != cudaSuccess)
           return cuda_fail (e, "reciprocal space (tensor cores)");
         if (overlap) fork_real ();
@@ -1920,15 +1913,13 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
         if (E) cudaEventRecord (E[2], st);
       }
     if (fused
-        && (e = launch_mix_backward (m->mp, m->maps, (int *) m->status.p, st, c)) != cudaSuccess)
+        && (e = launch_mix_backward (m->mp, m->maps, m->d_status, st, c)) != cudaSuccess)
       return cuda_fail (e, "reciprocal space (tensor cores)");
     // the real-space partials must be complete before the combine
     if (overlap) cudaStreamWaitEvent (st, m->ev_join, 0);
     mk_combine<<<(np * C + CMB_OUT - 1) / CMB_OUT, CMB_OUT * CMB_WARPS, 0, st>>> (cb);
     kmark (c, st, "mk_combine");
     if (E) cudaEventRecord (E[3], st);
-    if (m->tensor)
-      cudaMemcpyAsync (m->h_status, m->status.p, sizeof (int), cudaMemcpyDeviceToHost, st);
     e = cudaGetLastError ();
     if (e != cudaSuccess) return cuda_fail (e, "mixed kernels");
     return STOKES_GPU_OK;
@@ -1947,8 +1938,6 @@ mixed_check_status (Ctx *c)
   MixedState *m = c->mixed;
   if (!m || !m->h_status || !*m->h_status) return STOKES_GPU_OK;
   *m->h_status = 0;
-  cudaMemsetAsync (m->status.p, 0, sizeof (int), c->stream);
-  cudaStreamSynchronize (c->stream);
   return set_error (STOKES_GPU_ETIMEOUT, "a tensor-core wait of the mixed product ran out");
 }
 
@@ -1958,7 +1947,7 @@ release_mixed (Ctx *c)
   if (!c->mixed) return;
   MixedState *m = c->mixed;
   for (DevBuf *b : {&m->kt, &m->qpos, &m->tab, &m->xf, &m->pq, &m->part_real, &m->part_rec,
-                    &m->selfbuf, &m->status, &m->rot, &m->mix, &m->img, &m->sq, &m->xs, &m->cstart,
+                    &m->selfbuf, &m->rot, &m->mix, &m->img, &m->sq, &m->xs, &m->cstart,
                     &m->prad, &m->pqa, &m->pself})
     b->release ();
   if (m->h_status) cudaFreeHost (m->h_status);

@@ -31,8 +31,8 @@ struct FixState {
   // splits with too many offsets, which the image-table kernel serves
   bool tabled = false;
   RealTabArgs real;
-  DevBuf arena, partial, status;   // arena: every table and buffer of p and real
-  int *h_status = nullptr;
+  DevBuf arena, partial;   // arena: every table and buffer of p and real
+  int *h_status = nullptr, *d_status = nullptr;
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   SeqGraph graph;
@@ -282,11 +282,6 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
   if (e == cudaSuccess)
     e = cudaMemcpyAsync (base, host.data (), host.size (), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemsetAsync (base + zero0, 0, zero1 - zero0, st);
-  if (e == cudaSuccess && !f->status.p)
-    {
-      e = f->status.ensure (sizeof (int));
-      if (e == cudaSuccess) e = cudaMemsetAsync (f->status.p, 0, sizeof (int), st);
-    }
   if (e == cudaSuccess && f->tabled)
     {
       r.tab = (const double *) (base + o_rt);
@@ -329,12 +324,7 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
   f->real = r;
   const int me = fix_maps (ND, p, &f->maps);
   if (me) return set_error (STOKES_GPU_ECUDA, "TMA tensor maps of the FP64 product (%d)", me);
-  if (!f->h_status)
-    {
-      if ((e = cudaMallocHost (&f->h_status, sizeof (int))) != cudaSuccess)
-        return cuda_fail (e, "status");
-      *f->h_status = 0;
-    }
+  if ((e = status_word (&f->h_status, &f->d_status)) != cudaSuccess) return cuda_fail (e, "status");
   if (!f->side)
     {
       int lo = 0, hi = 0;
@@ -374,7 +364,6 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
   if (*f->h_status)
     {
       *f->h_status = 0;
-      cudaMemsetAsync (f->status.p, 0, sizeof (int), st);
       return set_error (STOKES_GPU_ETIMEOUT,
                         "a tensor-core wait of the previous FP64 product ran out");
     }
@@ -414,7 +403,7 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
   cudaEvent_t *E = phase_events (c, timed);
   const bool overlap = (!E || E == c->ev) && !c->kprof_on;
   auto sequence = [&] () -> int {
-    int *status = (int *) f->status.p;
+    int *status = f->d_status;
     cudaError_t e;
     if (E) cudaEventRecord (E[0], st);
     kmark (c, st, nullptr);
@@ -451,7 +440,6 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
     k_fix_combine<<<(n + 31) / 32, 32 * FC_W, 0, st>>> (cb);
     kmark (c, st, "k_fix_combine");
     if (E) cudaEventRecord (E[3], st);
-    cudaMemcpyAsync (f->h_status, f->status.p, sizeof (int), cudaMemcpyDeviceToHost, st);
     if ((e = cudaGetLastError ()) != cudaSuccess) return cuda_fail (e, "FP64 product");
     return STOKES_GPU_OK;
   };
@@ -480,8 +468,6 @@ fix_check_status (Ctx *c)
   FixState *f = c->fix;
   if (!f || !f->h_status || !*f->h_status) return STOKES_GPU_OK;
   *f->h_status = 0;
-  cudaMemsetAsync (f->status.p, 0, sizeof (int), c->stream);
-  cudaStreamSynchronize (c->stream);
   return set_error (STOKES_GPU_ETIMEOUT, "a tensor-core wait of the FP64 product ran out");
 }
 
@@ -490,7 +476,7 @@ release_fix (Ctx *c)
 {
   FixState *f = c->fix;
   if (!f) return;
-  for (DevBuf *b : {&f->arena, &f->partial, &f->status}) b->release ();
+  for (DevBuf *b : {&f->arena, &f->partial}) b->release ();
   f->graph.release ();
   if (f->h_status) cudaFreeHost (f->h_status);
   if (f->side) cudaStreamDestroy (f->side);
