@@ -104,7 +104,7 @@ void fix_plan_items (int nd, FixPlan &p, const std::vector<int> &nqm, std::vecto
 int fix_maps (int nd, const FixPlan &p, FixMaps *m);
 struct Ctx;
 // y partials of the reciprocal sum from positions and x (device), in order
-// on st; *status is raised when a bounded wait ran out
+// on st; p.mx is zero at the start; *status is raised when a bounded wait ran out
 cudaError_t launch_fix_tables (int nd, const FixPlan &p, const double *pos, const double *x,
                                cudaStream_t st, Ctx *prof);
 cudaError_t launch_fix_forward (int nd, int version, const FixPlan &p, const FixMaps &m, int *status,

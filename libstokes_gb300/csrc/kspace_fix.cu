@@ -993,8 +993,6 @@ cudaError_t
 launch_fix_tables (int, const FixPlan &p, const double *pos, const double *x, cudaStream_t st,
                    Ctx *prof)
 {
-  cudaError_t e = cudaMemsetAsync (p.mx, 0, fix_mx_words (p) * sizeof (unsigned), st);
-  if (e != cudaSuccess) return e;
   const int items = p.M[0] + p.M[1] + p.M[2] + 3;
   k_fix_tables<<<dim3 ((p.np + TAB_P - 1) / TAB_P, (items + TAB_R - 1) / TAB_R), TAB_P * TAB_R, 0,
                  st>>> (p, pos, x);

@@ -36,6 +36,7 @@ struct FixState {
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   SeqGraph graph;
+  bool clean = false;           // the maxima (FixPlan::mx) are zero: set-up or a whole product
 };
 
 // y = self x + real-space partials + reciprocal partials.  A CTA sums 32
@@ -48,6 +49,8 @@ struct FixCombine {
   int n, c, ncr, nck;
   double self[3];
   double *y;
+  unsigned *mx;         // the maxima of the product, cleared for the next one
+  int nmx;
 };
 
 __global__ void __launch_bounds__ (32 * FC_W)
@@ -56,6 +59,8 @@ k_fix_combine (FixCombine a)
   __shared__ double s_v[FC_W][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int e = blockIdx.x * 32 + lane;
+  if (blockIdx.x == 0)
+    for (int k = threadIdx.x; k < a.nmx; k += 32 * FC_W) a.mx[k] = 0u;
   double v = 0.0;
   if (e < a.n)
     {
@@ -338,6 +343,7 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
   f->self[1] = ts->self_c;
   f->self[2] = ts->self_m;
   f->p = p;
+  f->clean = true;
   f->id++;
   memcpy (f->key, key, sizeof key);
   return STOKES_GPU_OK;
@@ -436,7 +442,8 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
         if (E) cudaEventRecord (E[2], st);
       }
     FixCombine cb {d_x, (const double *) f->partial.p, (const double *) p.yp, n, p.c, nchunk,
-                   p.nbitem, {f->self[0], f->self[1], f->self[2]}, d_y};
+                   p.nbitem, {f->self[0], f->self[1], f->self[2]}, d_y, p.mx,
+                   (int) fix_mx_words (p)};
     k_fix_combine<<<(n + 31) / 32, 32 * FC_W, 0, st>>> (cb);
     kmark (c, st, "k_fix_combine");
     if (E) cudaEventRecord (E[3], st);
@@ -455,8 +462,15 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
                      (uint64_t) (uintptr_t) a.partial, (uint64_t) (uintptr_t) E, rmin_bits})
     key = (key ^ v) * 1099511628211ull;
   const bool use = graphs && !c->kprof_on && (E == nullptr || E == c->ev) && p.stall == 0;
+  // the last kernel of a product clears the maxima for the next one (a memset
+  // of its own takes 2 us more); after a product that was not all launched
+  // they are cleared here
+  if (!f->clean)
+    cudaMemsetAsync (p.mx, 0, fix_mx_words (p) * sizeof (unsigned), st);
+  f->clean = false;
   const int rc = run_sequence (f->graph, key, st, E, use, sequence);
   if (rc) return rc;
+  f->clean = true;
   c->launches = 9;
   c->timed = timed;
   return STOKES_GPU_OK;
