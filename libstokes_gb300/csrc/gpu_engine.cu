@@ -812,11 +812,12 @@ status_word (int **host, int **dev)
   return cudaHostGetDevicePointer ((void **) dev, *host, 0);
 }
 
-// A pinned, mapped buffer of the context for a vector of a small mixed host
-// call: copying it on the host and letting the device read or write it there
+// A pinned, mapped buffer of the context for a vector of a small host call: copying it on the host and letting the device read or write it there
 // is quicker than a copy of pageable memory, which waits twice (FT N = 333 65
-// -> 54 us a call).  Larger vectors are not staged, nor those of FP64 products,
-// whose kernels read x several times (F N = 64 83 us, 89 with a staged copy).
+// -> 54 us a call).  Larger vectors are not staged.  FP64 kernels read x and the
+// positions several times: one kernel copies both from the pinned buffers
+// (k_gather; F N = 64 84 -> 78 us), where two copies took the copy engine's turn
+// each (89).
 constexpr size_t STAGE_MAX = 256 * 1024;
 
 static bool
@@ -838,6 +839,17 @@ host_stage (Ctx::Stage &s, size_t bytes)
   return true;
 }
 
+// two vectors of pinned host memory into device memory
+__global__ void __launch_bounds__ (256)
+k_gather (const double *a, double *da, int na, const double *b, double *db, int nb)
+{
+  for (int t = blockIdx.x * 256 + threadIdx.x; t < na + nb; t += gridDim.x * 256)
+    {
+      if (t < na) da[t] = a[t];
+      else db[t - na] = b[t - na];
+    }
+}
+
 int
 atimes_host (struct stokes *sys, const double *x, double *y, bool cube)
 {
@@ -855,30 +867,30 @@ atimes_host (struct stokes *sys, const double *x, double *y, bool cube)
   // through their device mapping -- over the CPU-GPU link -- without a
   // staging copy and its latency: y always (each element is written once),
   // x on the mixed paths, which read it twice (the FP64 kernels read x once
-  // per reciprocal vector or pair and take a device copy); small vectors of
-  // mixed products in other host memory pass through the context's pinned
-  // buffers, the others through device copies
+  // per reciprocal vector or pair and take a device copy); small vectors in
+  // other host memory pass through the context's pinned buffers, larger ones
+  // through device copies
   const bool mixed = c->precision == STOKES_GPU_MIXED;
   const size_t nb = sizeof (double) * n;
   const double *d_x = mixed ? (const double *) mapped_host (x) : nullptr;
   double *d_y = (double *) mapped_host (y), *y_stage = nullptr;
   if (!d_x)
     {
-      if (mixed && host_stage (c->hx, nb))
+      if (host_stage (c->hx, nb))
         {
           memcpy (c->hx.p, x, nb);
           d_x = c->hx.dev;
         }
-      else
+      if (!d_x || !mixed)
         {
           if ((e = c->x.ensure (nb)) != cudaSuccess) return cuda_fail (e, "x");
-          cudaMemcpyAsync (c->x.p, x, nb, cudaMemcpyHostToDevice, c->stream);
-          d_x = (const double *) c->x.p;
+          // (with the positions below)
+          if (!d_x) cudaMemcpyAsync (c->x.p, x, nb, cudaMemcpyHostToDevice, c->stream);
         }
     }
   if (!d_y)
     {
-      if (mixed && host_stage (c->hy, nb))
+      if (host_stage (c->hy, nb))
         {
           d_y = c->hy.dev;
           y_stage = c->hy.p;
@@ -886,13 +898,25 @@ atimes_host (struct stokes *sys, const double *x, double *y, bool cube)
       else if ((e = c->y.ensure (nb)) != cudaSuccess)
         return cuda_fail (e, "y");
     }
-  const double *d_pos = mixed ? mapped_positions (c, sys) : nullptr;
-  if (!d_pos)
+  const bool staged = !mixed && d_x;
+  const double *d_pos = mixed || staged ? mapped_positions (c, sys) : nullptr;
+  if (!d_pos || staged)
     {
-      cudaMemcpyAsync (c->pos.p, sys->pos, sizeof (double) * 3 * np, cudaMemcpyHostToDevice,
-                       c->stream);
+      if (d_pos)
+        {
+          const int n3 = 3 * np;
+          k_gather<<<std::min (152, (n + n3 + 255) / 256), 256, 0, c->stream>>> (
+            d_x, (double *) c->x.p, n, d_pos, (double *) c->pos.p, n3);
+          d_x = nullptr;
+        }
+      else
+        cudaMemcpyAsync (c->pos.p, sys->pos, sizeof (double) * 3 * np, cudaMemcpyHostToDevice,
+                         c->stream);
       d_pos = (const double *) c->pos.p;
     }
+  if (!mixed && d_x)                    // staged, but the positions could not be mapped
+    cudaMemcpyAsync (c->x.p, c->hx.p, nb, cudaMemcpyHostToDevice, c->stream);
+  if (!mixed || !d_x) d_x = (const double *) c->x.p;
   rc = atimes_dev (c, d_pos, d_x, d_y ? d_y : (double *) c->y.p, c->stream, true);
   if (rc) return rc;
   e = d_y ? cudaSuccess
