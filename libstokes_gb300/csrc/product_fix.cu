@@ -34,7 +34,7 @@ struct FixState {
   DevBuf arena, partial;   // arena: every table and buffer of p and real
   int *h_status = nullptr, *d_status = nullptr;
   cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_end = nullptr;
   SeqGraph graph;
   bool clean = false;           // the maxima (FixPlan::mx) are zero: set-up or a whole product
 };
@@ -336,7 +336,8 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
       cudaDeviceGetStreamPriorityRange (&lo, &hi);
       if (cudaStreamCreateWithPriority (&f->side, cudaStreamNonBlocking, lo) != cudaSuccess
           || cudaEventCreateWithFlags (&f->ev_fork, cudaEventDisableTiming) != cudaSuccess
-          || cudaEventCreateWithFlags (&f->ev_join, cudaEventDisableTiming) != cudaSuccess)
+          || cudaEventCreateWithFlags (&f->ev_join, cudaEventDisableTiming) != cudaSuccess
+          || cudaEventCreateWithFlags (&f->ev_end, cudaEventDisableTiming) != cudaSuccess)
         return set_error (STOKES_GPU_ECUDA, "FP64 product: side stream");
     }
   f->self[0] = ts->self_a;
@@ -408,10 +409,10 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
 
   cudaEvent_t *E = phase_events (c, timed);
   const bool overlap = (!E || E == c->ev) && !c->kprof_on;
-  auto sequence = [&] () -> int {
+  auto sequence = [&] (bool recording) -> int {
     int *status = f->d_status;
     cudaError_t e;
-    if (E) cudaEventRecord (E[0], st);
+    if (E && !recording) cudaEventRecord (E[0], st);
     kmark (c, st, nullptr);
     if ((e = launch_fix_tables (ND, p, d_pos, d_x, st, c)) != cudaSuccess)
       return cuda_fail (e, "reciprocal tables");
@@ -423,10 +424,17 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
     if (overlap)
       {
         cudaStreamWaitEvent (f->side, f->ev_fork, 0);
-        if (E) cudaEventRecord (E[1], f->side);
+        // nodes of the graph, so that every replay measures its real space
+        const unsigned ext = recording ? cudaEventRecordExternal : cudaEventRecordDefault;
+        if (E) cudaEventRecordWithFlags (E[1], f->side, ext);
         e = real_space (f->side);
-        if (E) cudaEventRecord (E[2], f->side);
         cudaEventRecord (f->ev_join, f->side);
+        // beside the last kernel, which does not wait for it
+        if (E)
+          {
+            cudaEventRecordWithFlags (E[2], f->side, ext);
+            cudaEventRecord (f->ev_end, f->side);
+          }
         if (e != cudaSuccess) return cuda_fail (e, "real-space kernel");
       }
     if ((e = launch_fix_backward (ND, c->version, p, f->maps, status, st, c)) != cudaSuccess)
@@ -446,7 +454,8 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
                    (int) fix_mx_words (p)};
     k_fix_combine<<<(n + 31) / 32, 32 * FC_W, 0, st>>> (cb);
     kmark (c, st, "k_fix_combine");
-    if (E) cudaEventRecord (E[3], st);
+    if (E && overlap) cudaStreamWaitEvent (st, f->ev_end, 0);
+    if (E && !recording) cudaEventRecord (E[3], st);
     if ((e = cudaGetLastError ()) != cudaSuccess) return cuda_fail (e, "FP64 product");
     return STOKES_GPU_OK;
   };
@@ -496,6 +505,7 @@ release_fix (Ctx *c)
   if (f->side) cudaStreamDestroy (f->side);
   if (f->ev_fork) cudaEventDestroy (f->ev_fork);
   if (f->ev_join) cudaEventDestroy (f->ev_join);
+  if (f->ev_end) cudaEventDestroy (f->ev_end);
   delete f;
   c->fix = nullptr;
 }

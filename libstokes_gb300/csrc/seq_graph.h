@@ -19,13 +19,14 @@ struct SeqGraph {
   }
 };
 
-// Runs `sequence` (the launches of one product on st, returning a status)
-// directly the first time a configuration `key` appears, records it into a
+// Runs `sequence (recording)` (the launches of one product on st, returning a
+// status) directly the first time a configuration `key` appears, records it into a
 // graph (stream capture) the second time and replays that from then on.  The
 // key covers everything the recorded nodes hold: pointers, sizes, events.
 // Nothing is recorded while st is itself being captured by the caller.  A
 // captured cudaEventRecord is only a dependency, so the start and end events
-// E[0], E[3] (may be NULL) are recorded around a replay.
+// E[0], E[3] (E may be NULL) are recorded around a replay, and while `recording`
+// the sequence makes event nodes of the others (cudaEventRecordExternal).
 template <class Seq>
 int
 run_sequence (SeqGraph &g, uint64_t key, cudaStream_t st, cudaEvent_t *E, bool use, Seq &&sequence)
@@ -36,22 +37,22 @@ run_sequence (SeqGraph &g, uint64_t key, cudaStream_t st, cudaEvent_t *E, bool u
       if (cudaStreamIsCapturing (st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
         use = false;
     }
-  if (!use) return sequence ();
+  if (!use) return sequence (false);
   if (!g.exec || key != g.key)
     {
       if (key != g.cand)
         {
           g.cand = key;
-          return sequence ();
+          return sequence (false);
         }
       if (g.exec) cudaGraphExecDestroy (g.exec);
       g.exec = nullptr;
       if (cudaStreamBeginCapture (st, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
         {
           cudaGetLastError ();
-          return sequence ();
+          return sequence (false);
         }
-      const int rc = sequence ();
+      const int rc = sequence (true);
       cudaGraph_t gr = nullptr;
       cudaError_t e = cudaStreamEndCapture (st, &gr);
       if (!rc && e == cudaSuccess && gr) e = cudaGraphInstantiate (&g.exec, gr, 0);
@@ -61,7 +62,7 @@ run_sequence (SeqGraph &g, uint64_t key, cudaStream_t st, cudaEvent_t *E, bool u
         {
           g.exec = nullptr;
           cudaGetLastError ();
-          return sequence ();                  // not recorded: launch directly
+          return sequence (false);             // not recorded: launch directly
         }
       g.key = key;
     }
