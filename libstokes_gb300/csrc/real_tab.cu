@@ -39,6 +39,7 @@
 // to FP64 is done in integers.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -383,12 +384,16 @@ real_tab_doubles (int version, int nbin)
   return real_tab_bytes (version, nbin) / (sizeof (double) + sizeof (float));
 }
 
-// FAR_U: 5.2 for F and FT; the stresslet functions are up to u^2 larger
+// FAR_U: 5.2 for F and FT; the stresslet functions are up to u^2 larger.  Never
+// below the first bin of the table (s = 1, real_tab_range), which a split with
+// xi > 5.2 reaches (a box of about one radius): the far loop takes the table
+// for all of its pairs.  1e-4 above it, since the far pairs are told by FP32
+// distances, within 1e-6 of the exact ones.
 double
 real_tab_far (int version, double xi)
 {
   const double u = version == 2 ? 5.5 : 5.2;
-  return (u / xi) * (u / xi);
+  return std::max (1.0001, (u / xi) * (u / xi));
 }
 
 cudaError_t
