@@ -781,6 +781,19 @@ batch_capture (stokes_gpu_batch *b)
   return e == cudaSuccess ? STOKES_GPU_OK : cuda_fail (e, "batch graph");
 }
 
+// after the batch's stream was synchronised; FP64: a bounded wait of a system's
+// tensor-core kernels that ran out (every system's word is cleared)
+static int
+batch_check_status (stokes_gpu_batch *b)
+{
+  int rc = STOKES_GPU_OK;
+  if (b->precision != STOKES_GPU_MIXED)
+    for (int k = 0; k < b->nsys; k++)
+      if (Ctx *c = get_ctx (b->sys[k], false))
+        if (const int r = check_status (c)) rc = r;
+  return rc;
+}
+
 static int
 batch_run (stokes_gpu_batch *b, float *ms)
 {
@@ -797,12 +810,7 @@ batch_run (stokes_gpu_batch *b, float *ms)
   cudaEventDestroy (e1);
   if (ms) *ms = t;
   if (e != cudaSuccess) return cuda_fail (e, "batch product");
-  // FP64: a bounded wait of a system's tensor-core kernels that ran out
-  if (b->precision != STOKES_GPU_MIXED)
-    for (int k = 0; k < b->nsys; k++)
-      if (Ctx *c = get_ctx (b->sys[k], false))
-        if (const int rc = fix_check_status (c)) return rc;
-  return STOKES_GPU_OK;
+  return batch_check_status (b);
 }
 
 // time a few splits, then real-space chunkings and CTA sizes, keep the fastest
@@ -944,6 +952,7 @@ stokes_gpu_batch_create (struct stokes **systems, int nsys, int precision,
       if (!rc) rc = batch_launch_fp64 (b, b->stream);
       if (!rc && cudaStreamSynchronize (b->stream) != cudaSuccess)
         rc = set_error (STOKES_GPU_ECUDA, "batch warm-up failed");
+      if (!rc) rc = batch_check_status (b);
     }
   if (!rc) rc = batch_capture (b);
   if (rc) { stokes_gpu_batch_destroy (b); return rc; }
@@ -1197,6 +1206,7 @@ stokes_gpu_batch_bd (stokes_gpu_batch *b, double peclet, double dt, int n_cheb, 
             e = cudaMemcpyAsync (w.data (), Y, sizeof (double) * n, cudaMemcpyDeviceToHost, st);
           if (e == cudaSuccess) e = cudaStreamSynchronize (st);
           if (e != cudaSuccess) return cuda_fail (e, "batch Lanczos");
+          if (const int rc = batch_check_status (b)) return rc;
           for (int s = 0; s < ns; s++)
             {
               if (j >= steps[s]) continue;
@@ -1339,7 +1349,7 @@ stokes_gpu_batch_bd (stokes_gpu_batch *b, double peclet, double dt, int n_cheb, 
       e = cudaStreamSynchronize (st);
       if (e == cudaSuccess && pos_out)
         e = cudaMemcpy (pos_out, pos, sizeof (double) * 3 * npt, cudaMemcpyDeviceToHost);
-      if (e != cudaSuccess) rc = cuda_fail (e, "batch BD");
+      rc = e == cudaSuccess ? batch_check_status (b) : cuda_fail (e, "batch BD");
     }
   for (DevBuf *d : {&d_esys, &d_pxo, &d_c, &d_v, &d_pos0, &d_k}) d->release ();
   return rc;

@@ -465,6 +465,7 @@ bd_error (stokes_gpu_bd *b, const double *d_pos, double *err)
   cudaMemcpyAsync (b->h_dots + 2, d, 2 * sizeof (double), cudaMemcpyDeviceToHost, st);
   cudaError_t e = cudaStreamSynchronize (st);
   if (e != cudaSuccess) return cuda_fail (e, "Chebyshev error");
+  if ((rc = check_status (b->c))) return rc;
   const double zz = b->h_dots[0], yyv = b->h_dots[2];
   // a non-positive z.Mz means the noise left the bounds' interval: infinite
   // error, which makes the caller re-estimate the bounds
@@ -559,6 +560,8 @@ lanczos_extremes (stokes_gpu_bd *b, int m, unsigned long long stream,
       be.push_back (beta);
       k_bd_scale<<<gridn (n), 256, 0, st>>> (n, w, 1.0 / beta, V + (size_t) (j + 1) * n);
     }
+  // (the stream is synchronised after every operator)
+  if (const int rc = check_status (b->c)) return rc;
   *lmin = tridiag_extreme (al, be, false);
   *lmax = tridiag_extreme (al, be, true);
   return STOKES_GPU_OK;
@@ -711,7 +714,7 @@ bd_sync_pos_to_sys (stokes_gpu_bd *b)
   cudaError_t e = cudaMemcpyAsync (b->sys->pos, b->x.p, sizeof (double) * 3 * b->np,
                                    cudaMemcpyDeviceToHost, b->c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize (b->c->stream);
-  return e == cudaSuccess ? STOKES_GPU_OK : cuda_fail (e, "positions");
+  return e == cudaSuccess ? check_status (b->c) : cuda_fail (e, "positions");
 }
 
 }  // namespace lsg
@@ -870,7 +873,7 @@ stokes_gpu_bd_noise (stokes_gpu_bd *b, const double *y, double *z, double *err)
   cudaError_t e = cudaMemcpyAsync (z, b->z.p, sizeof (double) * b->n, cudaMemcpyDeviceToHost,
                                    b->c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize (b->c->stream);
-  return e == cudaSuccess ? STOKES_GPU_OK : cuda_fail (e, "noise");
+  return e == cudaSuccess ? check_status (b->c) : cuda_fail (e, "noise");
 }
 
 int
@@ -899,7 +902,7 @@ stokes_gpu_bd_run (stokes_gpu_bd *b, double t, int nsteps)
       if (rc) return rc;
     }
   cudaError_t e = cudaStreamSynchronize (b->c->stream);
-  return e == cudaSuccess ? STOKES_GPU_OK : cuda_fail (e, "BD run");
+  return e == cudaSuccess ? check_status (b->c) : cuda_fail (e, "BD run");
 }
 
 int
@@ -1247,6 +1250,7 @@ BD_calc_FB (struct BD_params *BD, double *z)
                                    cudaMemcpyDeviceToHost, b->c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize (b->c->stream);
   if (e != cudaSuccess) dropin_die (fn, cudaGetErrorString (e));
+  check_rc (check_status (b->c), fn);
   // particle order -> [F part, T part] (src/brownian.c:1851-1871)
   const int nm = sys->nm;
   if (sys->version == 0)
@@ -1354,6 +1358,7 @@ redo_scale:
   e = cudaMemcpyAsync (x, dnew, sizeof (double) * 3 * nm, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize (st);
   if (e != cudaSuccess) dropin_die (fn, cudaGetErrorString (e));
+  check_rc (check_status (b->c), fn);
   b->steps += 1;
   return dt_local;
 }

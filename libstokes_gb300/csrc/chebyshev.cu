@@ -180,7 +180,7 @@ chebyshev_eval_atimes (int ncheb, const double *a, int n, const double *y, doubl
               cudaError_t e = cudaMemcpyAsync (z, d_z, sizeof (double) * n,
                                                cudaMemcpyDeviceToHost, c->stream);
               if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
-              if (e != cudaSuccess) rc = cuda_fail (e, "Chebyshev");
+              rc = e == cudaSuccess ? check_status (c) : cuda_fail (e, "Chebyshev");
             }
         }
       if (rc) dropin_failed ("chebyshev_eval_atimes", z, n > 0 ? (size_t) n : 0);

@@ -798,6 +798,16 @@ mapped_positions (Ctx *c, const struct stokes *sys)
   return c->hpos_dev;
 }
 
+int
+check_status (Ctx *c)
+{
+  // every word is cleared, the first failure is reported
+  const int rc[3] = {fix_check_status (c), mixed_check_status (c), dense_check_status (c)};
+  for (int r : rc)
+    if (r) return r;
+  return STOKES_GPU_OK;
+}
+
 cudaError_t
 status_word (int **host, int **dev)
 {
@@ -924,9 +934,7 @@ atimes_host (struct stokes *sys, const double *x, double *y, bool cube)
   if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
   if (e != cudaSuccess) return cuda_fail (e, "atimes");
   // a bounded wait of this product's tensor-core kernels that ran out
-  if (c->precision == STOKES_GPU_MIXED && !c->open && (rc = mixed_check_status (c)) != 0)
-    return rc;
-  if (c->use_fix && (rc = fix_check_status (c)) != 0) return rc;
+  if ((rc = check_status (c)) != 0) return rc;
   if (y_stage) memcpy (y, y_stage, nb);
   collect_times (c);
   sys->cpu1 = c->times[0];
@@ -1182,7 +1190,7 @@ matrix_host (struct stokes *sys, double *mat, bool cube)
   e = cudaMemcpyAsync (mat, c->mat.p, sizeof (double) * n * n, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
   if (e != cudaSuccess) return cuda_fail (e, "matrix");
-  if (c->use_dense && (rc = dense_check_status (c)) != 0) return rc;
+  if ((rc = check_status (c)) != 0) return rc;
   float t = 0.f;
   cudaEventElapsedTime (&t, c->ev[0], c->ev[3]);
   sys->cpu1 = t;
@@ -1219,7 +1227,7 @@ atimes_matrix_host (struct stokes *sys, const double *x, double *y, bool cube)
   e = cudaMemcpyAsync (y, c->y.p, sizeof (double) * n, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
   if (e != cudaSuccess) return cuda_fail (e, "atimes_3all_matrix");
-  if (c->use_dense && (rc = dense_check_status (c)) != 0) return rc;
+  if ((rc = check_status (c)) != 0) return rc;
   return STOKES_GPU_OK;
 }
 

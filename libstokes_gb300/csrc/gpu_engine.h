@@ -181,6 +181,9 @@ void release_vjp_mixed (const Ctx *c);
 // (and the status word cleared) when a bounded wait of its tensor-core
 // kernels ran out, else STOKES_GPU_OK
 int mixed_check_status (Ctx *c);
+// the same for whatever products and dense builds c made: every call that
+// synchronises and hands back results of its own products ends with it
+int check_status (Ctx *c);
 
 // failure-injection settings of stokes_gpu_test_stall_waits (util.cu): polls
 // of an extra wait of the k-space GEMMs' MMA lane on an mbarrier that nothing

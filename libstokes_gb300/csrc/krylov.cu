@@ -828,7 +828,7 @@ solve_own (struct stokes *sys, int op, bool force_open, const double *b, double 
     {
       e = cudaMemcpyAsync (x, K.x.p, sizeof (double) * n, cudaMemcpyDeviceToHost, st);
       if (e == cudaSuccess) e = cudaStreamSynchronize (st);
-      if (e != cudaSuccess) rc = cuda_fail (e, "solution");
+      rc = e == cudaSuccess ? check_status (c) : cuda_fail (e, "solution");
     }
   c->force_open = false;
   return rc;
