@@ -124,6 +124,7 @@ get_ctx (const struct stokes *sys, bool create)
   if (cudaStreamCreateWithFlags (&c->stream, cudaStreamNonBlocking) != cudaSuccess)
     { delete c; return nullptr; }
   for (int q = 0; q < 4; q++) cudaEventCreate (&c->ev[q]);
+  cudaEventCreateWithFlags (&c->used, cudaEventDisableTiming);
   for (int q = 0; q < 2; q++) cudaEventCreateWithFlags (&c->join[q], cudaEventDisableTiming);
   const char *env = getenv ("LIBSTOKES_GB300_PRECISION");
   c->precision = (env && strcmp (env, "mixed") == 0) ? STOKES_GPU_MIXED : STOKES_GPU_FP64;
@@ -138,6 +139,7 @@ free_ctx (Ctx *c)
   for (cudaEvent_t e : c->kprof_ev) cudaEventDestroy (e);
   for (DevBuf *b : c->all_buffers ()) b->release ();
   for (int q = 0; q < 4; q++) cudaEventDestroy (c->ev[q]);
+  if (c->used) cudaEventDestroy (c->used);
   for (int q = 0; q < 2; q++) cudaEventDestroy (c->join[q]);
   if (c->hpos) cudaFreeHost (c->hpos);
   if (c->hx.p) cudaFreeHost (c->hx.p);
@@ -314,13 +316,36 @@ build_particles (const struct stokes *sys, int mode, std::vector<double> &pp, bo
     }
 }
 
+void
+note_use (Ctx *c, cudaStream_t st)
+{
+  if (st == c->stream) return;          // ordered with the uploads there
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing (st, &cs) != cudaSuccess)
+    cudaGetLastError ();
+  if (cs != cudaStreamCaptureStatusNone)
+    c->captured = true;
+  else if (cudaEventRecord (c->used, st) == cudaSuccess)
+    c->used_set = true;
+}
+
+cudaError_t
+wait_products (Ctx *c)
+{
+  if (c->captured) return cudaDeviceSynchronize ();
+  const cudaError_t e = cudaStreamSynchronize (c->stream);
+  return e == cudaSuccess && c->used_set ? cudaEventSynchronize (c->used) : e;
+}
+
 static int
-upload_if_changed (DevBuf &buf, uint64_t &fp, const void *host, size_t bytes,
-                   cudaStream_t st, const char *what)
+upload_if_changed (Ctx *c, DevBuf &buf, uint64_t &fp, const void *host, size_t bytes,
+                   const char *what)
 {
   const uint64_t h = fnv (host, bytes, fnv (&bytes, sizeof bytes));
   if (h == fp && buf.p) return STOKES_GPU_OK;
-  cudaError_t e = buf.ensure (bytes > 0 ? bytes : 64);
+  const cudaStream_t st = c->stream;
+  cudaError_t e = wait_products (c);
+  if (e == cudaSuccess) e = buf.ensure (bytes > 0 ? bytes : 64);
   if (e != cudaSuccess) return cuda_fail (e, what);
   if (bytes)
     {
@@ -551,8 +576,8 @@ prepare (Ctx *c, const struct stokes *sys, bool cube, int tables)
       // spheres without slip need none
       if (c->mode == MODE_MONO) return STOKES_GPU_OK;
       build_particles (sys, c->mode, c->h_pp, c->open);
-      return upload_if_changed (c->pp, c->fp_pp, c->h_pp.data (), sizeof (double) * c->h_pp.size (),
-                                c->stream, "particle table");
+      return upload_if_changed (c, c->pp, c->fp_pp, c->h_pp.data (),
+                                sizeof (double) * c->h_pp.size (), "particle table");
     }
   // the system whose split the FP64 tables follow
   const struct stokes *ts = sys;
@@ -569,8 +594,8 @@ prepare (Ctx *c, const struct stokes *sys, bool cube, int tables)
   else
     build_images (ts, cube, c->h_img);
   c->nimg = (int) c->h_img.size ();
-  rc = upload_if_changed (c->img, c->fp_img, c->h_img.data (), sizeof (Img4) * c->h_img.size (),
-                          c->stream, "image table");
+  rc = upload_if_changed (c, c->img, c->fp_img, c->h_img.data (), sizeof (Img4) * c->h_img.size (),
+                          "image table");
   if (rc) return rc;
   // 2^22 particles: the range of the fixed-point sums
   if (ts != sys && c->mode == MODE_MONO && sys->np <= (1 << 22))
@@ -587,15 +612,13 @@ prepare (Ctx *c, const struct stokes *sys, bool cube, int tables)
       if (ts != sys && sys->version == 2) g_correction (sys, c->h_kt);
     }
   c->nk = (int) (c->h_kt.size () / KT_STRIDE);
-  rc = upload_if_changed (c->kt, c->fp_kt, c->h_kt.data (), sizeof (double) * c->h_kt.size (),
-                          c->stream, "reciprocal table");
+  rc = upload_if_changed (c, c->kt, c->fp_kt, c->h_kt.data (), sizeof (double) * c->h_kt.size (),
+                          "reciprocal table");
   if (rc) return rc;
   // self terms at the split of the tables (radii: the system's own)
   build_particles (sys, c->mode, c->h_pp, c->open, ts);
-  rc = upload_if_changed (c->pp, c->fp_pp, c->h_pp.data (), sizeof (double) * c->h_pp.size (),
-                          c->stream, "particle table");
-  if (rc) return rc;
-  return STOKES_GPU_OK;
+  return upload_if_changed (c, c->pp, c->fp_pp, c->h_pp.data (), sizeof (double) * c->h_pp.size (),
+                            "particle table");
 }
 
 // ---------------------------------------------------------------------------
@@ -617,6 +640,7 @@ int
 atimes_fp64_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
                  cudaStream_t st, bool timed)
 {
+  const UseMark mark {c, st};
   if (c->use_fix) return atimes_fix_dev (c, d_pos, d_x, d_y, st, timed);
   const int np = c->np, C = NCOMP (c->version);
   const int nchunk = choose_nchunk (np);
@@ -972,7 +996,7 @@ dense_pairs_apply (const Ctx *c, const struct stokes *sys)
 
 // the private copy at the dense split and its half-space tables
 static int
-dense_tables (Ctx *c, const struct stokes *sys, cudaStream_t st)
+dense_tables (Ctx *c, const struct stokes *sys)
 {
   // truncation: 1e-6 in libstokes' cutoff rule leaves about 7e-8 of the
   // largest entry (measured against eps 1e-14 on the FP64 oracle)
@@ -1014,15 +1038,15 @@ dense_tables (Ctx *c, const struct stokes *sys, cudaStream_t st)
         }
       c->dense_nk = (int) (c->h_dkt.size () / KT_STRIDE);
     }
-  return upload_if_changed (c->dkt, c->fp_dkt, c->h_dkt.data (),
-                            sizeof (double) * c->h_dkt.size (), st, "dense reciprocal table");
+  return upload_if_changed (c, c->dkt, c->fp_dkt, c->h_dkt.data (),
+                            sizeof (double) * c->h_dkt.size (), "dense reciprocal table");
 }
 
 static int
 matrix_pairs_dev (Ctx *c, const struct stokes *sys, const double *d_pos, double *d_mat,
                   cudaStream_t st)
 {
-  int rc = dense_tables (c, sys, st);
+  int rc = dense_tables (c, sys);
   if (rc) return rc;
   const int np = c->np, nk = c->dense_nk;
   const struct stokes *sv = c->dense;
@@ -1086,6 +1110,7 @@ matrix_pairs_dev (Ctx *c, const struct stokes *sys, const double *d_pos, double 
 int
 matrix_dev (Ctx *c, const double *d_pos, double *d_mat, cudaStream_t st)
 {
+  const UseMark mark {c, st};
   if (c->use_dense) return matrix_fix_dev (c, d_pos, d_mat, st);
   if (c->sys && dense_pairs_apply (c, c->sys)) return matrix_pairs_dev (c, c->sys, d_pos, d_mat, st);
   const int np = c->np;

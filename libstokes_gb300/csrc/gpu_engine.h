@@ -30,6 +30,12 @@ struct Ctx {
   cudaEvent_t join[2] = {};   // orders the context's stream inside the legacy default stream
   int precision = 0;
 
+  // the end of the last product or build on another stream than `stream`
+  // (note_use, wait_products); captured: one was recorded into a graph of the
+  // caller's, whose replays are not seen here
+  cudaEvent_t used = nullptr;
+  bool used_set = false, captured = false;
+
   // geometry of the last prepared system
   const struct stokes *sys = nullptr;
   int version = 0, np = 0, mode = 0;
@@ -164,6 +170,17 @@ cudaEvent_t *phase_events (Ctx *c, bool timed);
 cudaError_t status_word (int **host, int **dev);
 // record a kernel-profiling mark on st when the window is open
 void kmark (Ctx *c, cudaStream_t st, const char *name);
+
+// Tables and buffers of a context are read by products that may still be queued
+// on a stream of the caller's: what overwrites or frees them waits first
+// (wait_products), and every function that launches such work marks its end.
+cudaError_t wait_products (Ctx *c);
+void note_use (Ctx *c, cudaStream_t st);
+struct UseMark {
+  Ctx *c;
+  cudaStream_t st;
+  ~UseMark () { note_use (c, st); }
+};
 
 // mixed-precision path (mixed.cu)
 int atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,

@@ -1123,6 +1123,12 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
     }
   if (fp == m->fp && m->made) return STOKES_GPU_OK;
   m->made = false;
+  // products queued on a caller's stream read the offsets, the k list and the
+  // buffers of the split before
+  {
+    const cudaError_t e = wait_products (c);
+    if (e != cudaSuccess) return cuda_fail (e, "mixed split");
+  }
   m->poly = poly;
   m->amax = amax;
 
@@ -1176,6 +1182,9 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
     if (e == cudaSuccess)
       e = cudaMemcpyAsync (m->img.p, hi.data (), sizeof (float4) * hi.size (),
                            cudaMemcpyHostToDevice, c->stream);
+    // the product may run on another stream (nothing else need be uploaded: a
+    // return to the split of the reciprocal tables makes none)
+    if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
     if (e != cudaSuccess) return cuda_fail (e, "mixed real-space images");
     m->nimg = (int) hi.size ();
   }
@@ -1567,6 +1576,7 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
   if (c->open)
     return set_error (STOKES_GPU_EINVAL,
                       "mixed precision serves periodic systems; the free-space operator runs in FP64");
+  const UseMark mark {c, st};
   if (!c->mixed) c->mixed = new MixedState ();
   MixedState *m = c->mixed;
   const struct stokes *sys = c->sys;

@@ -170,6 +170,7 @@ int
 atimes_open_f32_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
                      cudaStream_t st, bool timed)
 {
+  const UseMark mark {c, st};
   const int np = c->np, C = NCOMP (c->version), n = C * np;
   const int nchunk = open_nchunk (np);
   // layout of the scratch: ph, pl [np] float4; xf [n] float; partial float2
