@@ -938,12 +938,9 @@ matrix_fix_dev (Ctx *c, const double *d_pos, double *d_mat, cudaStream_t st)
   const int rc = dense_setup (c, c->sys);
   if (rc) return rc;
   DenseState *f = c->dfix;
-  if (*f->h_status)
-    {
-      *f->h_status = 0;
-      return set_error (STOKES_GPU_ETIMEOUT,
-                        "a tensor-core wait of the previous dense builder ran out");
-    }
+  const int failed = earlier_failure (c, f->h_status,
+                                      "a tensor-core wait of the previous dense builder ran out");
+  if (failed) return failed;
   FixPlan p = f->p;
   p.stall = g_test_gemm_stall;
   int *status = f->d_status;

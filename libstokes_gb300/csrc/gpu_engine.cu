@@ -832,6 +832,16 @@ check_status (Ctx *c)
   return STOKES_GPU_OK;
 }
 
+int
+earlier_failure (Ctx *c, int *word, const char *message)
+{
+  if (!word || !*(volatile int *) word) return STOKES_GPU_OK;
+  const cudaError_t e = wait_products (c);
+  if (e != cudaSuccess) return cuda_fail (e, message);
+  *word = 0;
+  return set_error (STOKES_GPU_ETIMEOUT, "%s", message);
+}
+
 cudaError_t
 status_word (int **host, int **dev)
 {

@@ -168,6 +168,9 @@ cudaEvent_t *phase_events (Ctx *c, bool timed);
 // memory that they write in place, so that a product needs no copy to report it
 // (a copy engine's turn at its end, 2-6 us)
 cudaError_t status_word (int **host, int **dev);
+// STOKES_GPU_ETIMEOUT when an earlier product or build raised the word; cleared
+// once those queued behind it, which may raise it again, are done
+int earlier_failure (Ctx *c, int *word, const char *message);
 // record a kernel-profiling mark on st when the window is open
 void kmark (Ctx *c, cudaStream_t st, const char *name);
 

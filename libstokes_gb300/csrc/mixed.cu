@@ -1627,13 +1627,8 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
       m->nchunk_k = std::max (1, std::min (64, (152 * 48 + np - 1) / np));
       if (m->nchunk_k * 32 > m->nkh) m->nchunk_k = std::max (1, m->nkh / 32);
     }
-  // a status word raised by a bounded device wait of the previous product
-  if (m->h_status && *m->h_status)
-    {
-      *m->h_status = 0;
-      return set_error (STOKES_GPU_ETIMEOUT,
-                        "a tensor-core wait of the previous mixed product ran out");
-    }
+  rc = earlier_failure (c, m->h_status, "a tensor-core wait of the previous mixed product ran out");
+  if (rc) return rc;
   cudaError_t e;
   if ((e = status_word (&m->h_status, &m->d_status)) != cudaSuccess) return cuda_fail (e, "status");
   if (!m->side)

@@ -367,13 +367,9 @@ atimes_fix_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y, cud
   FixPlan p = f->p;
   p.stall = g_test_gemm_stall;
   const int np = c->np, n = np * p.c;
-  // a status word raised by a bounded device wait of the previous product
-  if (*f->h_status)
-    {
-      *f->h_status = 0;
-      return set_error (STOKES_GPU_ETIMEOUT,
-                        "a tensor-core wait of the previous FP64 product ran out");
-    }
+  const int failed = earlier_failure (c, f->h_status,
+                                      "a tensor-core wait of the previous FP64 product ran out");
+  if (failed) return failed;
   const int nchunk = f->tabled ? 1 : real_chunks (np);
   cudaError_t e = f->partial.ensure (sizeof (double) * (size_t) nchunk * n);
   if (e != cudaSuccess) return cuda_fail (e, "real-space scratch");

@@ -1,12 +1,14 @@
 """A bounded wait of a product's tensor-core kernels that runs out is reported
 by the call that returns the product's result and leaves the context usable:
 calls that synchronise by themselves and whose last operation is a product
-(solves, Chebyshev, Brownian dynamics, batches).
+(solves, Chebyshev, Brownian dynamics, batches).  Of products queued on a
+caller's stream the next call reports it, once.
 
 The wait runs out on an mbarrier that nothing arrives at (stokes_gpu_test_
 stall_waits), after `polls` of about 20 us: long enough that a call has queued
 all of its products before the first one gives up."""
 import ctypes as C
+import time
 
 import numpy as np
 import pytest
@@ -117,3 +119,40 @@ def test_batch_creation_reports_its_wait(lib, stall):
     lib.stokes_gpu_batch_destroy(h)
     for s in systems:
         s.close()
+
+
+@pytest.mark.parametrize("precision,n", [(0, 100), (1, 600)])
+def test_queued_products_report_once(lib, stall, precision, n):
+    """Products on a caller's stream: the next call reports the wait that ran
+    out; those still queued behind it do not raise it a second time."""
+    import torch
+    from libstokes_gb300 import abi
+    s, pos = _system(0, n, precision)
+    x = torch.from_numpy(np.random.default_rng(4).standard_normal(s.n)).cuda()
+    p = torch.from_numpy(pos).cuda()
+    y, good = torch.zeros_like(x), torch.zeros_like(x)
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def product(out):
+        return lib.stokes_gpu_atimes_dev(s.sp, p.data_ptr(), x.data_ptr(), out.data_ptr(),
+                                         C.c_void_p(st.cuda_stream))
+
+    assert product(good) == abi.STOKES_GPU_OK
+    st.synchronize()
+    assert stall(4 * POLLS) == abi.STOKES_GPU_OK
+    t0 = time.perf_counter()
+    assert product(y) == abi.STOKES_GPU_OK
+    st.synchronize()
+    span = time.perf_counter() - t0                  # two waits that ran out
+    assert product(y) == abi.STOKES_GPU_ETIMEOUT
+    assert product(y) == abi.STOKES_GPU_OK
+    assert product(y) == abi.STOKES_GPU_OK           # queued behind the first
+    time.sleep(0.75 * span)                          # the first has raised the word
+    assert product(y) == abi.STOKES_GPU_ETIMEOUT
+    lib.stokes_gpu_test_stall_waits(0, 0)
+    torch.cuda.synchronize()
+    assert product(y) == abi.STOKES_GPU_OK
+    st.synchronize()
+    assert torch.equal(y, good)
+    s.close()
