@@ -823,7 +823,7 @@ dense_setup (Ctx *c, const struct stokes *sys)
   const size_t o_q = place (sizeof (uint4) * b.np), o_u = place (sizeof (unsigned long long) * 4 * b.np);
   cudaStream_t st = c->stream;
   // no build of this context may still be using the tables of the last set-up
-  cudaError_t e = f->arena.p ? cudaDeviceSynchronize () : cudaSuccess;
+  cudaError_t e = f->arena.p ? wait_products (c) : cudaSuccess;
   if (e == cudaSuccess) e = f->arena.ensure (bytes);
   char *base = (char *) f->arena.p;
   if (e == cudaSuccess)

@@ -1351,7 +1351,7 @@ upload_k (Ctx *c, MixedState *m)
 static int
 mix_setup (Ctx *c, MixedState *m)
 {
-  if (m->mix_fp == m->fp && m->mix.p) return STOKES_GPU_OK;
+  if (m->mix_fp == m->fp && m->mix_fp && m->mix.p) return STOKES_GPU_OK;
   MixPlan p {};
   p.np = c->np;
   p.c = NCOMP (c->version);
@@ -1443,7 +1443,8 @@ mix_setup (Ctx *c, MixedState *m)
   const size_t o_F = place (sizeof (float) * (size_t) p.nsplit * p.ncolf * p.Rp);
   const size_t o_yp = place (sizeof (float) * (size_t) p.nbitem * p.np * p.c);
   // no product of this context may still be using the tables of the last set-up
-  cudaError_t e = m->mix_id ? cudaDeviceSynchronize () : cudaSuccess;
+  cudaError_t e = m->mix_id ? wait_products (c) : cudaSuccess;
+  m->mix_fp = 0;                // until the set-up is whole
   if (e == cudaSuccess) e = m->mix.ensure (bytes);
   char *base = (char *) m->mix.p;
   if (e == cudaSuccess)

@@ -281,7 +281,7 @@ fix_setup (Ctx *c, const struct stokes *sys, const struct stokes *ts)
 
   cudaStream_t st = c->stream;
   // no product of this context may still be using the tables of the last set-up
-  cudaError_t e = f->id ? cudaDeviceSynchronize () : cudaSuccess;
+  cudaError_t e = f->id ? wait_products (c) : cudaSuccess;
   if (e == cudaSuccess) e = f->arena.ensure (bytes);
   char *base = (char *) f->arena.p;
   if (e == cudaSuccess)

@@ -1,5 +1,6 @@
 """Products queued on a caller's stream, with changes of the system between
-them and no synchronisation: each product uses the tables of its own call."""
+them and no synchronisation: each product uses the tables of its own call.  New
+tables wait for the products of their own system only."""
 import ctypes as C
 
 import numpy as np
@@ -68,4 +69,32 @@ def test_changes_between_queued_products(lib, precision, version, n, kind):
     for k, (a, b) in enumerate(zip(alone, queued)):
         assert torch.equal(a, b), (k, order[k])
     assert not torch.equal(alone[0], alone[1])
+    s.close()
+
+
+@pytest.mark.parametrize("call", ["fp64", "mixed", "matrix"])
+def test_new_tables_leave_other_streams_alone(lib, call):
+    """A change of box while a long kernel of somebody else's runs: the call
+    returns before that kernel ends."""
+    import torch
+    s, pos, side = _system(0, 600, int(call == "mixed"))
+    x = np.random.default_rng(9).standard_normal(s.n)
+
+    def change_and_call(k):
+        # (from the largest box down: the buffers have their size)
+        b = side * (1.0 - 1e-4 * k)
+        lib.stokes_set_l(s.sp, b, b, b)
+        lib.stokes_set_xi(s.sp, lib.xi_by_tratio(s.sp, 1.0), 1e-12)
+        return s.matrix() if call == "matrix" else s.atimes(x)
+
+    for k in range(4):
+        change_and_call(k)
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(other):
+        torch.cuda._sleep(1_000_000_000)         # half a second
+    change_and_call(4)
+    running = not other.query()
+    torch.cuda.synchronize()
+    assert running
     s.close()
