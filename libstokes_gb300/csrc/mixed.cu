@@ -81,7 +81,7 @@ struct MixedState {
   bool poly = false;
   double amax = 1.0;
   DevBuf prad, pqa, pself;
-  uint64_t poly_fp = 0;
+  uint64_t radii = 0, poly_fp = 0;      // hash of the radii; radii and split of the tables
 };
 
 constexpr int MX_WARPS = 8;      // warps per CTA in the mixed kernels
@@ -1111,15 +1111,22 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
   double amax = 1.0;
   if (poly)
     {
-      // the radii enter the split (xi a_max <= 0.5) and every table
+      // the split and its tables follow the largest radius alone (xi a_max <=
+      // 0.5); the radii themselves are in tables of their own (prad, pqa, pself)
       amax = 0.0;
+      m->radii = 1469598103934665603ull;
+      auto mix = [] (uint64_t &h, double v) {
+        uint64_t b;
+        memcpy (&b, &v, sizeof b);
+        h = (h ^ b) * 1099511628211ull;
+      };
       for (int q = 0; q < sys->np; q++)
         {
           amax = std::max (amax, sys->a[q]);
-          uint64_t b;
-          memcpy (&b, &sys->a[q], sizeof b);
-          fp = (fp ^ b) * 1099511628211ull;
+          mix (m->radii, sys->a[q]);
         }
+      mix (fp, amax);
+      fp = (fp ^ 0x706f6c79ull) * 1099511628211ull;     // not the key of equal spheres
     }
   if (fp == m->fp && m->made) return STOKES_GPU_OK;
   m->made = false;
@@ -1677,10 +1684,13 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
       if ((e = cudaStreamSynchronize (st)) != cudaSuccess) return cuda_fail (e, "mixed self matrix");
       m->self_fp = m->fp;
     }
-  if (m->poly && m->poly_fp != m->fp)
+  if (m->poly && m->poly_fp != (m->fp ^ m->radii))
     {
       // radii, squared radii and the self terms at the split
-      // (src/ewald.c:579-642 with this split's xi)
+      // (src/ewald.c:579-642 with this split's xi); remade alone when only the
+      // radii change (with the whole split remade a call took 650-700 us instead
+      // of 100 for 500-600 spheres)
+      if ((e = wait_products (c)) != cudaSuccess) return cuda_fail (e, "particle tables");
       std::vector<float> r ((size_t) np), q ((size_t) np);
       std::vector<double> sf ((size_t) 3 * np);
       const double xisp = m->xi / sqrt (M_PI), xi2 = m->xi * m->xi;
@@ -1705,7 +1715,7 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
                              cudaMemcpyHostToDevice, st);
       if (e == cudaSuccess) e = cudaStreamSynchronize (st);
       if (e != cudaSuccess) return cuda_fail (e, "particle tables");
-      m->poly_fp = m->fp;
+      m->poly_fp = m->fp ^ m->radii;
     }
   // 1024 rotations e^{2 pi i h / 1024} as FP32 pairs hi + lo, made once
   if (!m->rot.p)
