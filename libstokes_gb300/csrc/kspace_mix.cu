@@ -839,12 +839,18 @@ mix_plan_items (MixPlan &p, const std::vector<int> &nqm, std::vector<int4> &fwd,
         {
           const int l = (sets[0] + s - 1) / s;
           std::vector<int> len;
+          long long sum = 0;
           for (int k : sets)
             {
-              const int n = std::max (1, (k + l - 1) / l);
-              for (int z = 0; z < n; z++) len.push_back (DK * ((k + n - 1) / n));
+              const int n = std::max (1, (k + l - 1) / l), d = DK * ((k + n - 1) / n);
+              len.insert (len.end (), n, d);
+              sum += (long long) n * (d + START);
             }
           if (s > 1 && len.size () > 64) break;
+          // no schedule ends before the SMs' average
+          if (best >= 0
+              && (double) (sum * p.mt / SMS) * tile_time (tn) + len.size () / 24.0 >= best)
+            continue;
           const double t = (double) makespan (len, p.mt, START) * tile_time (tn) + len.size () / 24.0;
           if (best < 0 || t < best)
             {

@@ -51,6 +51,9 @@ struct MixedState {
   int nk_split = 0;      // rows of the re-tuned split; the rest: reference G term
   double selfc[3] = {0, 0, 0};
   std::vector<MixK> h_k;
+  std::vector<char> h_tables;   // of mix_setup
+  std::vector<float4> h_img;
+  bool img_made = false;        // h_img is on the device (img)
   DevBuf kt, qpos, tab, xf, pq, part_real, part_rec, selfbuf, rot;
   DevBuf img;                   // real-space lattice offsets (float4)
   int nimg = 1;
@@ -1130,12 +1133,6 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
     }
   if (fp == m->fp && m->made) return STOKES_GPU_OK;
   m->made = false;
-  // products queued on a caller's stream read the offsets, the k list and the
-  // buffers of the split before
-  {
-    const cudaError_t e = wait_products (c);
-    if (e != cudaSuccess) return cuda_fail (e, "mixed split");
-  }
   m->poly = poly;
   m->amax = amax;
 
@@ -1150,7 +1147,7 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
     {
       for (int it = 0; it < 200; it++)
         {
-          lsg_ewald_cutoffs (xi, eps, lmin, lmax, &rc, &kc);
+          lsg_ewald_cutoffs (xi, eps, lmin, lmax, &rc, nullptr);
           if (rc <= 0.4999 * lmin) break;
           xi *= 1.03;   // the cutoff must stay below half the box (minimum image)
         }
@@ -1163,11 +1160,11 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
           xi = std::min (eta / lv, XI_CAP);
         }
     }
-  if (images) lsg_ewald_cutoffs (xi, eps, lmin, lmax, &rc, &kc);
+  lsg_ewald_cutoffs (xi, eps, lmin, lmax, images ? &rc : nullptr, &kc);
   // lattice offsets within the cutoff of a minimum-image difference (just
   // the zero offset while the cutoff is below half the box)
   {
-    std::vector<float4> hi;
+    m->h_img.clear ();
     const int nx = (int) ceil (rc / sys->lx + 0.5), ny = (int) ceil (rc / sys->ly + 0.5),
               nz = (int) ceil (rc / sys->lz + 0.5);
     for (int a1 = -nx; a1 <= nx; a1++)
@@ -1183,17 +1180,10 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
             const double ey = std::max (0.0, fabs (ty) - 0.5 * sys->ly);
             const double ez = std::max (0.0, fabs (tz) - 0.5 * sys->lz);
             if (ex * ex + ey * ey + ez * ez > rc * rc) continue;
-            hi.push_back (make_float4 ((float) tx, (float) ty, (float) tz, 0.f));
+            m->h_img.push_back (make_float4 ((float) tx, (float) ty, (float) tz, 0.f));
           }
-    cudaError_t e = m->img.ensure (sizeof (float4) * hi.size ());
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync (m->img.p, hi.data (), sizeof (float4) * hi.size (),
-                           cudaMemcpyHostToDevice, c->stream);
-    // the product may run on another stream (nothing else need be uploaded: a
-    // return to the split of the reciprocal tables makes none)
-    if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
-    if (e != cudaSuccess) return cuda_fail (e, "mixed real-space images");
-    m->nimg = (int) hi.size ();
+    m->img_made = false;
+    m->nimg = (int) m->h_img.size ();
   }
   m->xi = xi;
   m->rc = rc;
@@ -1218,29 +1208,40 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
   // exp(-k^2 / 4 xi^2) is a product over the axes: (B1 + 1) (2 B2 + 2 B3 + 3)
   // exponentials instead of one per vector
   std::vector<double> e2 (2 * B2 + 1), e3 (2 * B3 + 1);
+  const double i4x = 1.0 / (4.0 * xi2);
   for (int m1 = 0; m1 <= B1; m1++)
     {
       const double k1 = k0x * m1;
       const double s2 = sys->shear_mode == 1 ? sl * m1 : 0.0, s3 = sys->shear_mode == 2 ? sl * m1 : 0.0;
-      auto gauss = [&] (double k) { return exp (-k * k / 4.0 / xi2); };
-      for (int m2 = -B2; m2 <= B2; m2++) e2[m2 + B2] = gauss (k1) * gauss (k0y * ((double) m2 - s2));
-      for (int m3 = -B3; m3 <= B3; m3++) e3[m3 + B3] = gauss (k0z * ((double) m3 - s3));
+      auto gauss = [&] (double k) { return exp (-k * k * i4x); };
+      if (m1 == 0 || s2 != 0.0)
+        for (int m2 = -B2; m2 <= B2; m2++) e2[m2 + B2] = gauss (k0y * ((double) m2 - s2));
+      if (m1 == 0 || s3 != 0.0)
+        for (int m3 = -B3; m3 <= B3; m3++) e3[m3 + B3] = gauss (k0z * ((double) m3 - s3));
+      const double e1 = pivol * gauss (k1);
       for (int m2 = -B2; m2 <= B2; m2++)
-        for (int m3 = -B3; m3 <= B3; m3++)
+        {
+          const double k2 = k0y * ((double) m2 - s2), k12 = k1 * k1 + k2 * k2;
+          if (k12 > kc2) continue;
+          // the line's part within the cutoff, a little wide
+          const double lim = sqrt (kc2 - k12) / k0z + 1e-6;
+          const int a3 = std::max (-B3, (int) ceil (s3 - lim)), b3 = std::min (B3, (int) floor (s3 + lim));
+          for (int m3 = a3; m3 <= b3; m3++)
           {
             // half space: m1 > 0, or m1 == 0 and (m2 > 0 or (m2 == 0 and m3 > 0))
             if (m1 == 0 && (m2 < 0 || (m2 == 0 && m3 <= 0))) continue;
-            const double k2 = k0y * ((double) m2 - s2), k3 = k0z * ((double) m3 - s3);
-            const double kk = k1 * k1 + k2 * k2 + k3 * k3;
+            const double k3 = k0z * ((double) m3 - s3);
+            const double kk = k12 + k3 * k3;
             if (kk > kc2) continue;
             const double k = sqrt (kk);
             if (k > kc) continue;
-            const double k4z = kk / 4.0 / xi2;
-            const double kexp = pivol * (1.0 + k4z * (1.0 + 2.0 * k4z)) / kk * (e2[m2 + B2] * e3[m3 + B3]);
+            // (one division a vector: they took most of the loop)
+            const double ik = 1.0 / k, k4z = kk * i4x;
+            const double kexp = e1 * (1.0 + k4z * (1.0 + 2.0 * k4z)) * (ik * ik) * (e2[m2 + B2] * e3[m3 + B3]);
             MixK r;
             memset (&r, 0, sizeof r);
             r.m1 = m1; r.m2 = m2; r.m3 = m3;
-            r.ex = (float) (k1 / k); r.ey = (float) (k2 / k); r.ez = (float) (k3 / k);
+            r.ex = (float) (k1 * ik); r.ey = (float) (k2 * ik); r.ez = (float) (k3 * ik);
             if (poly)
               {
                 // the per-k factors of the unequal-radius weights
@@ -1253,7 +1254,7 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
               }
             else
               {
-                r.ya = (float) (6.0 * (1.0 - kk / 3.0) * kexp);
+                r.ya = (float) ((6.0 - 2.0 * kk) * kexp);
                 r.yb = (float) (3.0 * k * kexp);
                 r.yc = (float) (1.5 * kk * kexp);
                 // G coupling with the sign that makes real + reciprocal
@@ -1261,13 +1262,14 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
                 // src/ewald.c:1060-1066)
                 r.yg = (float) (-3.0 * (1.0 - 4.0 / 15.0 * kk) * k * kexp);
                 r.yh = (float) (1.5 * kk * kexp);
-                r.ym = (float) (3.0 * (1.0 - kk / 5.0) * kk * kexp);
+                r.ym = (float) (3.0 * (1.0 - 0.2 * kk) * kk * kexp);
               }
             m->h_k.push_back (r);
             M[0] = std::max (M[0], abs (m1));
             M[1] = std::max (M[1], abs (m2));
             M[2] = std::max (M[2], abs (m3));
           }
+        }
     }
   m->nk_split = (int) m->h_k.size ();
   // libstokes' FTS result depends on its own xi through the sign of its
@@ -1338,12 +1340,36 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
   return STOKES_GPU_OK;
 }
 
-// the half-space list on the device, for the SIMT and unequal-radii kernels
-static int
-upload_k (Ctx *c, MixedState *m)
+// the lattice offsets to the device, after wait_products (see upload_split)
+static cudaError_t
+upload_images (Ctx *c, MixedState *m)
 {
-  if (m->kt_made) return STOKES_GPU_OK;
-  cudaError_t e = m->kt.ensure (sizeof (MixK) * std::max (m->nkh, 1));
+  if (m->img_made) return cudaSuccess;
+  const size_t n = sizeof (float4) * m->h_img.size ();
+  cudaError_t e = m->img.ensure (n);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync (m->img.p, m->h_img.data (), n, cudaMemcpyHostToDevice, c->stream);
+  m->img_made = e == cudaSuccess;
+  return e;
+}
+
+// lattice offsets and, for the SIMT and unequal-radii kernels, the half-space
+// list on the device.  Products queued on a caller's stream may still read those
+// of the split before, and the next one may run on another stream than the
+// uploads: a wait before and one after.  The host side of the split is made by
+// then, beside what is queued.
+static int
+upload_split (Ctx *c, MixedState *m, bool list)
+{
+  if (m->img_made && (m->kt_made || !list)) return STOKES_GPU_OK;
+  cudaError_t e = wait_products (c);
+  if (e == cudaSuccess) e = upload_images (c, m);
+  if (!list)
+    {
+      if (e == cudaSuccess) e = cudaStreamSynchronize (c->stream);
+      return e == cudaSuccess ? STOKES_GPU_OK : cuda_fail (e, "mixed real-space images");
+    }
+  if (e == cudaSuccess) e = m->kt.ensure (sizeof (MixK) * std::max (m->nkh, 1));
   if (e == cudaSuccess && m->nkh)
     e = cudaMemcpyAsync (m->kt.p, m->h_k.data (), sizeof (MixK) * m->nkh, cudaMemcpyHostToDevice,
                          c->stream);
@@ -1358,7 +1384,8 @@ upload_k (Ctx *c, MixedState *m)
 static int
 mix_setup (Ctx *c, MixedState *m)
 {
-  if (m->mix_fp == m->fp && m->mix_fp && m->mix.p) return STOKES_GPU_OK;
+  // (a return to the split of these tables)
+  if (m->mix_fp == m->fp && m->mix_fp && m->mix.p) return upload_split (c, m, false);
   MixPlan p {};
   p.np = c->np;
   p.c = NCOMP (c->version);
@@ -1371,13 +1398,17 @@ mix_setup (Ctx *c, MixedState *m)
   // quarters (|m2|, |m3|) in use, by length: the ones in use at |m1| are then
   // (nearly, on a sheared lattice) a prefix
   const int W = p.M[2] + 1;
-  std::vector<char> used ((size_t) (p.M[1] + 1) * W, 0);
-  for (const MixK &k : m->h_k) used[(size_t) abs (k.m2) * W + abs (k.m3)] = 1;
+  std::vector<int> top ((size_t) (p.M[1] + 1) * W, -1);         // largest |m1| of each
+  for (const MixK &k : m->h_k)
+    {
+      int &t = top[(size_t) abs (k.m2) * W + abs (k.m3)];
+      t = std::max (t, k.m1);
+    }
   const struct stokes *sys = c->sys;
   std::vector<std::pair<double, int>> order;
   for (int b = 0; b <= p.M[1]; b++)
     for (int d = 0; d <= p.M[2]; d++)
-      if (used[(size_t) b * W + d])
+      if (top[(size_t) b * W + d] >= 0)
         order.push_back ({(b / sys->ly) * (b / sys->ly) + (d / sys->lz) * (d / sys->lz), b * W + d});
   std::stable_sort (order.begin (), order.end ());
   p.nq = (int) order.size ();
@@ -1400,29 +1431,21 @@ mix_setup (Ctx *c, MixedState *m)
   // quarters of each |m1|, as prefixes that do not grow with |m1| (a column
   // tile covers the quarters of its smallest |m1|)
   std::vector<int> nqm ((size_t) p.M[0] + 1, 0), off ((size_t) p.M[0] + 2, 0);
-  for (const MixK &k : m->h_k)
-    nqm[k.m1] = std::max (nqm[k.m1], at[(size_t) abs (k.m2) * W + abs (k.m3)] + 1);
+  for (int k = 0; k < p.nq; k++) nqm[top[order[k].second]] = k + 1;
   for (int a = p.M[0] - 1; a >= 0; a--) nqm[a] = std::max (nqm[a], nqm[a + 1]);
   for (int a = 0; a <= p.M[0]; a++) off[a + 1] = off[a] + nqm[a];
-  // weights by sign pattern: each half-space vector (m1 >= 0) is one pattern
-  // of its octant point; patterns that name the same vector (m2 or m3 zero)
-  // get it once
-  std::vector<MixCoef> coef ((size_t) 4 * off[p.M[0] + 1]);
-  if (!coef.empty ()) memset (coef.data (), 0, sizeof (MixCoef) * coef.size ());
-  for (const MixK &k : m->h_k)
-    {
-      const int q = at[(size_t) abs (k.m2) * W + abs (k.m3)];
-      MixCoef &w = coef[(size_t) 4 * (off[k.m1] + q) + 2 * (k.m2 < 0) + (k.m3 < 0)];
-      w.ex = k.ex; w.ey = k.ey; w.ez = k.ez;
-      w.ya = k.ya; w.yb = k.yb; w.yc = k.yc; w.yg = k.yg; w.yh = k.yh; w.ym = k.ym;
-    }
   std::vector<int4> fitem, bitem;
   mix_plan_items (p, nqm, fitem, bitem);
   // one allocation: host tables (one copy), what stays zero where nothing
-  // writes it (table pads, rows and columns), the rest
-  std::vector<char> host;
+  // writes it (table pads, rows and columns), the rest.  The host side is kept
+  // with the state: a run with changing box or shear makes it for every product,
+  // and fresh memory of its size costs more than filling it (F N = 1000 540 us a
+  // product with a new shear, 685 with fresh memory and a division per weight).
+  std::vector<char> &host = m->h_tables;
+  host.clear ();
+  const size_t ncoef = (size_t) 4 * off[p.M[0] + 1];
   host.reserve (sizeof (int4) * (quart.size () + fitem.size () + bitem.size ())
-                + sizeof (MixCoef) * coef.size () + 8 * (nqm.size () + off.size ()) + 2048);
+                + sizeof (MixCoef) * ncoef + 8 * (nqm.size () + off.size ()) + 4096);
   size_t bytes = 0;
   auto place = [&] (size_t n) {
     const size_t o = bytes;
@@ -1432,15 +1455,26 @@ mix_setup (Ctx *c, MixedState *m)
   auto table = [&] (const void *src, size_t n) {
     const size_t o = place (n);
     host.resize (bytes);
-    if (n) memcpy (host.data () + o, src, n);
+    if (n && src) memcpy (host.data () + o, src, n);
     return o;
   };
   const size_t o_quart = table (quart.data (), sizeof (int4) * quart.size ());
   const size_t o_nqm = table (nqm.data (), sizeof (int) * nqm.size ());
   const size_t o_off = table (off.data (), sizeof (int) * off.size ());
-  const size_t o_coef = table (coef.data (), sizeof (MixCoef) * coef.size ());
+  const size_t o_coef = table (nullptr, sizeof (MixCoef) * ncoef);
   const size_t o_fit = table (fitem.data (), sizeof (int4) * fitem.size ());
   const size_t o_bit = table (bitem.data (), sizeof (int4) * bitem.size ());
+  // weights by sign pattern: each half-space vector (m1 >= 0) is one pattern
+  // of its octant point; patterns that name the same vector (m2 or m3 zero)
+  // get it once
+  MixCoef *coef = reinterpret_cast<MixCoef *> (host.data () + o_coef);
+  for (const MixK &k : m->h_k)
+    {
+      const int q = at[(size_t) abs (k.m2) * W + abs (k.m3)];
+      MixCoef &w = coef[(size_t) 4 * (off[k.m1] + q) + 2 * (k.m2 < 0) + (k.m3 < 0)];
+      w.ex = k.ex; w.ey = k.ey; w.ez = k.ez;
+      w.ya = k.ya; w.yb = k.yb; w.yc = k.yc; w.yg = k.yg; w.yh = k.yh; w.ym = k.ym;
+    }
   const size_t zero0 = bytes;
   const size_t o_T = place (sizeof (int) * (size_t) p.nT * p.ldT);
   const size_t o_ZF = place (mix_zf_bytes (p)), o_WB = place (mix_wb_bytes (p));
@@ -1450,8 +1484,9 @@ mix_setup (Ctx *c, MixedState *m)
   const size_t o_F = place (sizeof (float) * (size_t) p.nsplit * p.ncolf * p.Rp);
   const size_t o_yp = place (sizeof (float) * (size_t) p.nbitem * p.np * p.c);
   // no product of this context may still be using the tables of the last set-up
-  cudaError_t e = m->mix_id ? wait_products (c) : cudaSuccess;
+  cudaError_t e = wait_products (c);
   m->mix_fp = 0;                // until the set-up is whole
+  if (e == cudaSuccess) e = upload_images (c, m);
   if (e == cudaSuccess) e = m->mix.ensure (bytes);
   char *base = (char *) m->mix.p;
   if (e == cudaSuccess)
@@ -1624,7 +1659,7 @@ atimes_mixed_dev (Ctx *c, const double *d_pos, const double *d_x, double *d_y,
   const size_t off2 = off1 + (size_t) (m->M[1] + 1) * np;
   {
     m->tensor = use_gemms (sys) && m->nkh > 0;
-    rc = m->tensor ? mix_setup (c, m) : upload_k (c, m);
+    rc = m->tensor ? mix_setup (c, m) : upload_split (c, m, true);
     if (rc) return rc;
     m->mp.stall = g_test_gemm_stall;
   }
