@@ -184,10 +184,13 @@ bterm (const BSys &S, const float *xf, int j, float dx, float dy, float dz, GenU
 {
   constexpr int C = NComp<V>::value;
   const float rr = dx * dx + dy * dy + dz * dz, rm = 2.0f * S.rmin;
-  // 1 / r from the reciprocal square root with one Newton step (1 ulp)
+  // r and 1 / r from the reciprocal square root with one Newton step on the
+  // residual of both roundings (half an ulp; without it r was off by more than
+  // the square root and the division it replaces)
   float ri = rsqrtf (rr);
-  ri = ri * fmaf (-0.5f * rr, ri * ri, 1.5f);
-  float r = rr * ri;
+  const float h = rr * ri, res = fmaf (-h, ri, 1.0f) - fmaf (rr, ri, -h) * ri;
+  ri = fmaf (0.5f * ri, res, ri);
+  float r = fmaf (0.5f * h, res, h);
   if (r < rm)
     {
       r = rm;
@@ -198,7 +201,14 @@ bterm (const BSys &S, const float *xf, int j, float dx, float dy, float dz, GenU
 #pragma unroll
   for (int q = 0; q < C; q++) x[q] = xf[S.x_off + (size_t) C * j + q];
   radial_f32<V> (S.xi, S.xisp, r, ri, f);
-  apply_radial<V, float> (e, 1.0f, f, x, acc.v);
+  // the term by itself, then one rounding in the sum (three for FT when it is
+  // built up in the sum)
+  float t[C];
+#pragma unroll
+  for (int q = 0; q < C; q++) t[q] = 0.f;
+  apply_radial<V, float> (e, 1.0f, f, x, t);
+#pragma unroll
+  for (int q = 0; q < C; q++) acc.v[q] += t[q];
 }
 
 template <int V>
@@ -211,12 +221,24 @@ mb_real_warp (const BatchArgs &a, const BSys &S, int i, int chunk, float (*s_d)[
   const int j1 = (int) ((long long) S.np * (chunk + 1) / S.nchunk);
   const uint4 *qp = reinterpret_cast<const uint4 *> (a.qpos) + S.p_off;
   const uint4 qi = qp[i];
-  GenU<V, float> acc;
+  // acc: of the current 32 sources; sum: of those before.  In one running sum
+  // the error grows with its length, and the faster pair terms made longer sums
+  // (fewer chunks) the quicker choice.  64 systems, error against FP64: F 2.15e-7
+  // with the closed forms, 2.19 with the shared polynomials in one sum, 2.14 now;
+  // FT 2.02, 2.12, 1.98; 870, 595, 610 us a product.
+  GenU<V, float> acc, sum;
   acc.zero ();
+  sum.zero ();
   int qn = 0;
   const unsigned lt = (1u << lane) - 1u;
   for (int jb = j0; jb < j1; jb += 32)
     {
+#pragma unroll
+      for (int q = 0; q < C; q++)
+        {
+          sum.v[q] += acc.v[q];
+          acc.v[q] = 0.f;
+        }
       const int j = jb + lane;
       float d0x = 0.f, d0y = 0.f, d0z = 0.f;
       if (j < j1) bmin_image (S, qi, qp[j], d0x, d0y, d0z);
@@ -269,7 +291,7 @@ mb_real_warp (const BatchArgs &a, const BSys &S, int i, int chunk, float (*s_d)[
 #pragma unroll
   for (int q = 0; q < C; q++)
     {
-      const float v = warp_sum (acc.v[q]);
+      const float v = warp_sum (sum.v[q] + acc.v[q]);
       if (lane == 0) out[q] = v;
     }
 }
