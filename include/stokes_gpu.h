@@ -194,16 +194,15 @@ int stokes_gpu_count_mixed_real_terms (struct stokes *sys, long long *count);
  * xi, rc, kc, eta = xi V^(1/3), eps, half-space k count, max |m| per axis */
 int stokes_gpu_mixed_split (struct stokes *sys, double *info9);
 
-/* known-answer test of the tensor-core (tcgen05, 3xTF32) path on the
- * current GPU: largest error of a 128x16x32 product relative to the sum of
- * absolute products (expect ~1e-7) */
+/* known-answer test of the tensor-core path of the reciprocal-space GEMMs on
+ * the current GPU: f16 planes of 8-bit digits, one digit of a 128 x 128 operand
+ * against several of a 32 x 128 one in each tcgen05 instruction; largest error
+ * of the three digit sums relative to the sum of absolute products (the sums
+ * are integers below 2^24: expect 0) */
 int stokes_gpu_selftest_tensor (double *max_rel_err);
 
-/* known-answer test of the TMA path of the reciprocal-space GEMMs: operand
- * images (TF32 hi/lo planes) loaded by 3-d TMA boxes with 128-byte swizzle
- * (including zero-filled rows past the end), a 128 x 32 x 64 product in
- * 3xTF32 on the swizzled descriptors; largest error relative to the sum of
- * absolute products (expect ~1e-7) */
+/* the same with the second operand's planes loaded by 3-d TMA boxes of all
+ * planes (128-byte swizzle, zero-filled rows past the end) */
 int stokes_gpu_selftest_tma (double *max_rel_err);
 
 /* measured FMA throughput of the current GPU in GFLOP/s (2 flops per FMA),

@@ -1,13 +1,6 @@
 // tc_umma.cuh -- minimal tcgen05 (5th-generation tensor core) helpers for
-// sm_103a: TMEM allocation, shared-memory matrix descriptors, the TF32 MMA,
+// sm_103a: TMEM allocation, shared-memory matrix descriptors, the f16 MMA,
 // commit to an mbarrier, bounded mbarrier waits and TMEM loads.
-//
-// Operand layout used throughout (K-major, no swizzle): a tile of R rows by
-// 8 TF32 values (one MMA K step) is a grid of 8-row x 16-byte "core
-// matrices"; the two core matrices of a row group sit side by side
-// (LBO = 128 B apart along K) and consecutive 8-row groups are 256 B apart
-// (SBO).  umma_off() gives the byte offset of element (row, k) in a tile of
-// R rows and KT = 8 * nsteps columns.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -16,34 +9,11 @@
 namespace lsg {
 namespace umma {
 
-// byte offset of (row, k) inside a K-major no-swizzle tile of `rows` rows
-__host__ __device__ __forceinline__ uint32_t
-off (uint32_t row, uint32_t k, uint32_t rows)
-{
-  const uint32_t step = k >> 3, kk = (k >> 2) & 1u, e = k & 3u;
-  const uint32_t g = row >> 3, r = row & 7u;
-  return step * (rows * 32u) + g * 256u + kk * 128u + r * 16u + e * 4u;
-}
-
-// shared-memory matrix descriptor (tcgen05 format, version 1):
-// start >> 4 [0,14), LBO >> 4 [16,30), SBO >> 4 [32,46), version [46,48),
-// base offset [49,52) = 0, layout type [61,64) = 0 (no swizzle)
-__device__ __forceinline__ uint64_t
-smem_desc (uint32_t saddr, uint32_t lbo, uint32_t sbo)
-{
-  uint64_t d = 0;
-  d |= (uint64_t) ((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t) ((lbo >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t) ((sbo >> 4) & 0x3FFFu) << 32;
-  d |= (uint64_t) 1u << 46;
-  return d;
-}
-
 // descriptor of a K-major tile in the 128-byte swizzled layout that a TMA
-// load with CU_TENSOR_MAP_SWIZZLE_128B writes: rows of 128 bytes (32 TF32
+// load with CU_TENSOR_MAP_SWIZZLE_128B writes: rows of 128 bytes (64 f16
 // values), 8-row groups 1024 bytes apart (SBO), the 16-byte chunks of row r
 // permuted by r % 8; the tile must start on a 1024-byte boundary.  The k-th
-// K step of 8 values starts 32 k bytes in (the swizzle is applied to the
+// K step of 16 values starts 32 k bytes in (the swizzle is applied to the
 // address, so the start moves within the atom).  LBO is unused in this mode.
 __device__ __forceinline__ uint64_t
 smem_desc_sw128 (uint32_t saddr)
@@ -55,17 +25,6 @@ smem_desc_sw128 (uint32_t saddr)
   d |= (uint64_t) 1u << 46;                 // descriptor version
   d |= (uint64_t) 2u << 61;                 // layout: 128-byte swizzle
   return d;
-}
-
-// instruction descriptor, kind::tf32: D f32, A/B tf32, both K-major
-__host__ __device__ __forceinline__ uint32_t
-idesc_tf32 (uint32_t M, uint32_t N)
-{
-  return (1u << 4)            // D format: f32
-    | (2u << 7)               // A format: tf32
-    | (2u << 10)              // B format: tf32
-    | ((N >> 3) << 17)        // N / 8
-    | ((M >> 4) << 24);       // M / 16
 }
 
 // instruction descriptor, kind::f16: D f32, A/B f16, both K-major
@@ -81,25 +40,6 @@ __device__ __forceinline__ uint32_t
 smem_u32 (const void *p)
 {
   return (uint32_t) __cvta_generic_to_shared (p);
-}
-
-// TF32 rounding of an FP32 bit pattern, to nearest with ties away from zero
-// (the rounding of cvt.rna.tf32.f32): add half a TF32 unit to the magnitude
-// bits and clear the 13 bits below TF32's mantissa; a carry moves into the
-// exponent as it should.  Finite inputs.
-__device__ __forceinline__ uint32_t
-rna_tf32_bits (uint32_t u)
-{
-  return (u + 0x1000u) & 0xFFFFE000u;
-}
-
-// x = hi + lo with hi, lo representable in TF32 (the 3xTF32 split), in
-// integer and FP32 arithmetic
-__device__ __forceinline__ void
-split_tf32 (float x, uint32_t &hi, uint32_t &lo)
-{
-  hi = rna_tf32_bits (__float_as_uint (x));
-  lo = rna_tf32_bits (__float_as_uint (x - __uint_as_float (hi)));
 }
 
 // TMEM allocation by one full warp; the column address lands in *slot
@@ -118,22 +58,11 @@ tmem_dealloc (uint32_t taddr, uint32_t ncols)
                 :: "r"(taddr), "r"(ncols) : "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread
-__device__ __forceinline__ void
-mma_tf32 (uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
-{
-  asm volatile (
-    "{\n\t.reg .pred p;\n\t"
-    "setp.ne.b32 p, %4, 0;\n\t"
-    "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-    :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
-// the same with f16 operands (K = 16 per instruction), called by a whole
-// converged warp: one elected lane issues it.  The descriptors are then warp
-// uniform and live in uniform registers; issued from a branch on one lane each
-// MMA first moved them there (about 115 clocks an MMA instead of the 32 to 96
-// that the tensor pipe takes).
+// D[tmem] (+)= A[smem] * B[smem]^T, f16 operands (K = 16 per instruction),
+// called by a whole converged warp: one elected lane issues it.  The descriptors
+// are then warp uniform and live in uniform registers; issued from a branch on
+// one lane each MMA first moved them there (about 115 clocks an MMA instead of
+// the 32 to 96 that the tensor pipe takes).
 __device__ __forceinline__ void
 mma_f16 (uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
 {
@@ -145,15 +74,8 @@ mma_f16 (uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32
     :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-// arrive on an mbarrier once all previously issued MMAs of this thread are done
-__device__ __forceinline__ void
-mma_commit (uint64_t *mbar)
-{
-  asm volatile ("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                :: "r"(smem_u32 (mbar)) : "memory");
-}
-
-// the same from a whole converged warp (the lane that mma_f16 elects)
+// arrive on an mbarrier once all MMAs issued so far are done, from a whole
+// converged warp (the lane that mma_f16 elects)
 __device__ __forceinline__ void
 mma_commit_warp (uint64_t *mbar)
 {
@@ -174,25 +96,6 @@ __device__ __forceinline__ void
 fence_mbar_init ()
 {
   asm volatile ("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// wait for phase `parity` of the mbarrier with at most `limit` polls;
-// returns false when the limit ran out
-__device__ __forceinline__ bool
-mbar_wait (uint64_t *mbar, uint32_t parity, uint32_t limit)
-{
-  const uint32_t a = smem_u32 (mbar);
-  for (uint32_t it = 0; it < limit; it++)
-    {
-      uint32_t done;
-      asm volatile (
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(a), "r"(parity) : "memory");
-      if (done) return true;
-    }
-  return false;
 }
 
 // one arrival on an mbarrier (release at CTA scope)
@@ -277,25 +180,8 @@ fence_after_sync ()
   asm volatile ("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// 16 consecutive FP32 columns of this thread's TMEM lane (32x32b shape):
-// warp w of a warpgroup reads lanes 32 w .. 32 w + 31
-__device__ __forceinline__ void
-tmem_ld16 (uint32_t taddr, float v[16])
-{
-  uint32_t r[16];
-  asm volatile (
-    "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-    "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-      "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-      "=r"(r[14]), "=r"(r[15])
-    : "r"(taddr));
-  asm volatile ("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int q = 0; q < 16; q++) v[q] = __uint_as_float (r[q]);
-}
-
-// the same load without the wait: v holds the columns after tmem_ld_wait (v)
+// 16 consecutive FP32 columns of this thread's TMEM lane (32x32b shape): warp w
+// of a warpgroup reads lanes 32 w .. 32 w + 31; v holds them after tmem_ld_wait (v)
 __device__ __forceinline__ void
 tmem_ld16_issue (uint32_t taddr, float v[16])
 {
