@@ -388,9 +388,8 @@ mb_sfac (BatchArgs a)
   else mb_sfac_warp<1> (a, S, k);
 }
 
-// one warp per (system, particle): y_i = self x_i + sum real partials
-// + 2 sum_k cos(k.r_i) P + sin(k.r_i) Q
-// Back-projection: one warp per BP_N particles of a system, its lanes over the
+// Back-projection, y_i = self x_i + sum real partials + 2 sum_k cos(k.r_i) P +
+// sin(k.r_i) Q: one warp per BP_N particles of a system, its lanes over the
 // k vectors, so that their loads serve BP_N particles (one particle a warp with
 // its table read from global memory waited for L2 most of the time: 215 us of a
 // 64-system product, 140 with the table alone in shared memory)

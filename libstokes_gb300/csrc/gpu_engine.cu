@@ -792,12 +792,13 @@ mapped_host (const void *p)
   return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
 }
 
-// the positions as the mixed kernels read them from a host call: sys->pos in
-// place when it is pinned, else a copy in the context's pinned mirror. The
-// mixed kernels read each coordinate once (mk_prep, k_open_prep convert
-// them), so a read over the CPU-GPU link replaces the staging copy of
-// pageable memory. Called only between synchronised host calls, so no
-// kernel is reading the mirror while it is rewritten.
+// the positions as a host call's first kernel reads them: sys->pos in place
+// when it is pinned, else a copy in the context's pinned mirror. The mixed
+// kernels convert them over the CPU-GPU link (mk_prep_tc and mk_prep once per
+// group of table rows, 19 groups at FTS N = 1000; k_open_prep once), the FP64
+// product copies them first (k_gather), in place of a staging copy of pageable
+// memory. Called only between synchronised host calls, so no kernel is reading
+// the mirror while it is rewritten.
 static const double *
 mapped_positions (Ctx *c, const struct stokes *sys)
 {
@@ -856,9 +857,10 @@ status_word (int **host, int **dev)
   return cudaHostGetDevicePointer ((void **) dev, *host, 0);
 }
 
-// A pinned, mapped buffer of the context for a vector of a small host call: copying it on the host and letting the device read or write it there
-// is quicker than a copy of pageable memory, which waits twice (FT N = 333 65
-// -> 54 us a call).  Larger vectors are not staged.  FP64 kernels read x and the
+// A pinned, mapped buffer of the context for a vector of a small host call:
+// copying it on the host and letting the device read or write it there is
+// quicker than a copy of pageable memory, which waits twice (FT N = 333 65 -> 54
+// us a call).  Larger vectors are not staged.  FP64 kernels read x and the
 // positions several times: one kernel copies both from the pinned buffers
 // (k_gather; F N = 64 84 -> 78 us), where two copies took the copy engine's turn
 // each (89).
@@ -910,10 +912,10 @@ atimes_host (struct stokes *sys, const double *x, double *y, bool cube)
   // pinned host buffers (cudaHostAlloc, cudaHostRegister) are used in place
   // through their device mapping -- over the CPU-GPU link -- without a
   // staging copy and its latency: y always (each element is written once),
-  // x on the mixed paths, which read it twice (the FP64 kernels read x once
-  // per reciprocal vector or pair and take a device copy); small vectors in
-  // other host memory pass through the context's pinned buffers, larger ones
-  // through device copies
+  // x on the mixed paths, whose first kernel (once per group of table rows) and
+  // last one read it (the FP64 kernels read x once per reciprocal vector or
+  // pair and take a device copy); small vectors in other host memory pass
+  // through the context's pinned buffers, larger ones through device copies
   const bool mixed = c->precision == STOKES_GPU_MIXED;
   const size_t nb = sizeof (double) * n;
   const double *d_x = mixed ? (const double *) mapped_host (x) : nullptr;

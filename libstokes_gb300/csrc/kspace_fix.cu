@@ -41,7 +41,7 @@
 //
 // Shared memory rows are 128 bytes: 32 K values of an even digit and of the
 // next odd one side by side.  The rows of all even digits of B follow one
-// another, so one MMA takes a digit of A against all of them (see mma_role).
+// another, so one MMA takes a digit of A against all of them (issue_tile).
 // One MMA per digit pair (N = 64) took 78 clocks, 80 us of MMAs in the forward
 // GEMM of FTS N = 1000: it reads 6 KB of shared memory for 32 clocks of tensor
 // pipe.  Now a 16-wide K step is 13 MMAs that read 108 KB for 896 clocks.

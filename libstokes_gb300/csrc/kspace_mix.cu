@@ -111,7 +111,7 @@ unit_of (uint32_t mx, float &inverse)
   return E == 128 ? __int_as_float (0x7f800000) : __int_as_float ((E + 127) << 23);
 }
 
-// ---- operand builders (see worker_role) -----------------------------------
+// ---- operand builders (see run_tiles in digit_gemm.cuh) --------------------
 // Forward: rows r0 .. + 127, particles j0 .. + 63.  A warp makes two quarters
 // (eight rows), a lane two particles.
 struct BuildF {
@@ -948,6 +948,8 @@ launch_mix_backward (const MixPlan &p, const MixMaps &m, int *status, cudaStream
 {
   const cudaError_t e = launch_chained (p.rad ? k_bp_gemm<true> : k_bp_gemm<false>, dim3 (p.mt, p.nbitem),
                                         NT, SMEM_DYN, st, m.wb, p, status);
+  // the profile's name of the back-projection of unequal radii is the same on
+  // both paths: callers look for it
   kmark (prof, st, p.rad ? "mk_backproj_poly" : "k_bp_gemm");
   return e;
 }

@@ -316,9 +316,9 @@ constexpr int RG_QCAP = 64;      // queue entries per warp: 32 are added to at m
 // split's lattice offsets) and queues the accepted pairs (displacement and
 // source index, one float4 each) in shared memory; every 32 queued pairs the
 // lanes evaluate one term each, so the FP32 pipe only sees accepted terms.
-// With lattice offsets (cutoff beyond half the box) each lane tests all
-// offsets of its source into a bit mask and one warp prefix sum places the
-// accepted ones.  Each lane sums its terms per component (a few tens at
+// With lattice offsets (cutoff beyond half the box) each lane tests up to 32
+// offsets of its source into a bit mask, and each round queues one accepted
+// offset of every lane that has one.  Each lane sums its terms per component (a few tens at
 // most), the 32 lane sums meet in a shuffle tree (pairwise summation), the
 // G warps of the target meet with TwoSum (error-free, the rounding errors
 // carried along), and the result is written as the FP32 pair hi + lo,
@@ -1098,11 +1098,11 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
   // against FP64 is 2.92e-7 at 1e-8, 2.99e-7 at 3e-8, 3.03e-7 at 1e-7 --
   // FP32 rounding, not truncation, sets it -- and the cutoffs shrink)
   const double eps = env_double ("LIBSTOKES_GB300_MIXED_EPS", 3e-8);
-  // minimum image unless asked otherwise: with the real space overlapping
-  // the back-projection, lattice images were faster at no measured size
-  // (FTS N = 256-512 level at eta 8; N = 4096 283 against 273 us; N = 8192
-  // and 16384 level at eta 11, where the cutoff is below half the box)
-  // the exception are small systems on the SIMT path (small_system)
+  // minimum image unless asked otherwise: beside the GEMMs, a lower eta with
+  // lattice images is faster at no measured size (products in a row, us: FTS N =
+  // 512 37.0 at eta 8 and 9, 42.2 at 6 with images; N = 4096 211 at 12, 332 at 10
+  // with images; F N = 4096 110 at 10.4, 225 at 10 with images).  The exception
+  // are small systems on the SIMT path (small_system).
   const bool small = small_system (sys) && !use_gemms (sys);
   bool images = env_double ("LIBSTOKES_GB300_MIXED_IMAGES", small ? 1.0 : 0.0) != 0.0;
   double eta = env_double ("LIBSTOKES_GB300_MIXED_ETA",
