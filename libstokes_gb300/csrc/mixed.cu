@@ -1142,25 +1142,53 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
   // xi a <= 0.5 keeps the self, real and reciprocal parts of comparable size
   // (FP32 loses digits to their cancellation when xi a grows)
   const double XI_CAP = 0.5 / amax;
-  double xi = std::min (eta / lv, XI_CAP), rc = 0, kc = 0;
-  if (!images)
-    {
-      for (int it = 0; it < 200; it++)
-        {
-          lsg_ewald_cutoffs (xi, eps, lmin, lmax, &rc, nullptr);
-          if (rc <= 0.4999 * lmin) break;
-          xi *= 1.03;   // the cutoff must stay below half the box (minimum image)
-        }
-      // a small box would need xi above the cap for a minimum-image cutoff:
-      // take lattice images in real space instead (measured: F and FT at
-      // L = 6 reached 1e-5 against FP64 at the forced xi, 1e-7 with images)
-      if (rc > 0.4999 * lmin || xi > XI_CAP)
-        {
-          images = true;
-          xi = std::min (eta / lv, XI_CAP);
-        }
-    }
-  lsg_ewald_cutoffs (xi, eps, lmin, lmax, images ? &rc : nullptr, &kc);
+  double xi = 0, rc = 0, kc = 0;
+  bool with_images = images;
+  auto choose = [&] (double eta) {
+    xi = std::min (eta / lv, XI_CAP);
+    with_images = images;
+    if (!images)
+      {
+        for (int it = 0; it < 200; it++)
+          {
+            lsg_ewald_cutoffs (xi, eps, lmin, lmax, &rc, nullptr);
+            if (rc <= 0.4999 * lmin) break;
+            xi *= 1.03;   // the cutoff must stay below half the box (minimum image)
+          }
+        // a small box would need xi above the cap for a minimum-image cutoff:
+        // take lattice images in real space instead (measured: F and FT at
+        // L = 6 reached 1e-5 against FP64 at the forced xi, 1e-7 with images)
+        if (rc > 0.4999 * lmin || xi > XI_CAP)
+          {
+            with_images = true;
+            xi = std::min (eta / lv, XI_CAP);
+          }
+      }
+    lsg_ewald_cutoffs (xi, eps, lmin, lmax, with_images ? &rc : nullptr, &kc);
+  };
+  // largest |m| of the vectors within kc
+  auto largest_m = [&] {
+    const double s2 = sys->shear_mode == 1 ? fabs (sys->shear_shift / sys->lx) : 0.0;
+    const double s3 = sys->shear_mode == 2 ? fabs (sys->shear_shift / sys->lx) : 0.0;
+    const double k0x = 2.0 * M_PI / sys->lx;
+    int top = 0;
+    for (int m1 = 0; k0x * m1 <= kc; m1++)
+      {
+        const double k = sqrt (std::max (0.0, kc * kc - k0x * m1 * k0x * m1)) / (2.0 * M_PI);
+        top = std::max (top, std::max (m1, (int) std::max (k * sys->ly + s2 * m1, k * sys->lz + s3 * m1)));
+      }
+    return top;
+  };
+  choose (eta);
+  // the etas of large systems are those of a cube: in a long or flat box (3 : 1 :
+  // 1 at N = 20000, 8 : 8 : 1) they lead past the largest |m|; the largest eta that
+  // does not, down to that of small systems
+  if (getenv ("LIBSTOKES_GB300_MIXED_ETA") == nullptr)
+    for (double e = eta; e > 8.0 && largest_m () > MX_MTAB; )
+      {
+        e = std::max (8.0, 0.97 * e);
+        choose (e);
+      }
   // lattice offsets within the cutoff of a minimum-image difference (just
   // the zero offset while the cutoff is below half the box)
   {
