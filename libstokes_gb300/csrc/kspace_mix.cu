@@ -10,14 +10,17 @@
 //             |m3|), the Ewald weights, and back (k_kop)
 //   backward  y_q(i) = sum_mi f_x(i) sum_r A[r][i] G[n][r]     (k_bp_gemm)
 //
-// Operands are 24-bit fixed-point numbers in three 8-bit digits, exact in f16
-// (the top digit up to 256): |f| <= 1 for A; B in units of the largest entry
-// of its column within 128 K values, so that a column of very different
-// entries keeps its digits.  Six digit products (i + j < 3) in three
-// accumulators; 128 K values keep every sum below 2^24, so the FP32
-// accumulation of the tensor core is exact, and each 128-wide set is scaled
-// by its unit and added in FP32.  Rounding is 2^-25 of the largest entry per
-// operand, that of FP32.  The 3xTF32 split used before carried 22 bits, had to
+// Operands are fixed-point numbers in three 8-bit digits, exact in f16: A, |f|
+// <= 1, with 24 fractional bits (the top digit up to 256); B with 25 (up to 512)
+// in units of the largest entry of its column within 128 K values, so that a
+// column of very different entries keeps its digits.  Six digit products (i + j
+// < 3) in three accumulators; 128 K values keep every sum below 2^24, so the
+// FP32 accumulation of the tensor core is exact, and each 128-wide set is
+// scaled by its unit and added in FP32.  Rounding is 2^-25 for A and 2^-26 of
+// the largest entry for B: with 24 bits, forces of one size lost two of theirs
+// to the unit (the next power of two above the largest of 128), and products of
+// some hundred unequal spheres came out up to 27% further from FP64 than with
+// FP32 sums (F N = 600 1.96e-7, 2.39e-7 with 24 bits, 1.67e-7 now).  The 3xTF32 split used before carried 22 bits, had to
 // be drained every 32 K values (the tensor core truncates inexact sums) and
 // multiplied k and -k separately.  Kernel times between events, before and now
 // (at the same split, eta 11, for N = 12001):
@@ -59,7 +62,7 @@ constexpr int DK = 2;                   // tiles per set (K = 128)
 constexpr int KB = DK * KT;             // K values per unit
 constexpr int TN_MAX = 128;             // columns per tile at most
 constexpr uint32_t A_PLANE = TM * 128;
-constexpr float UNIT = 1.0f / 65536.0f; // of a product of two top digits
+constexpr float UNIT = 1.0f / 131072.0f;        // of a product of two top digits: 2^-8 of A, 2^-9 of B
 
 constexpr int NS = 2;                   // stages (three leave too little L1 for the builds' loads)
 constexpr uint32_t A_BYTES = ND * A_PLANE;
@@ -69,12 +72,15 @@ constexpr uint32_t SMEM_DYN = NS * stage_bytes (TN_MAX) + 1024;
 
 // ---- digits ---------------------------------------------------------------
 // a product of two 30-bit fractions (upper word: 28 fractional bits) as a
-// biased string of 24 fractional bits: bytes 0 and 1 are the lower digits plus
-// 128, the upper half the top digit plus 512
+// biased string of `bits` fractional bits: bytes 0 and 1 are the lower digits
+// plus 128, the upper half the top digit plus 512
+constexpr int A_BITS = 24, B_BITS = 25;
+template <int bits>
 __device__ __forceinline__ int
 biased (int hi)
 {
-  return (hi + ((0x02008080 << 4) + 8)) >> 4;
+  constexpr int sh = 28 - bits;
+  return (hi + ((0x02008080 << sh) + (1 << (sh - 1)))) >> sh;
 }
 
 __device__ __forceinline__ uint32_t
@@ -148,7 +154,7 @@ struct BuildF {
         {
           const int2 y = v[u][b >> 1], z = v[u][2 + (b & 1)];
           uint32_t d[ND];
-          digits (biased (__mulhi (y.x, z.x)), biased (__mulhi (y.y, z.y)), d);
+          digits (biased<A_BITS> (__mulhi (y.x, z.x)), biased<A_BITS> (__mulhi (y.y, z.y)), d);
           unsigned char *o = stage + chunk_off (8 * warp + 4 * u + b, lane >> 2) + (lane & 3) * 4;
 #pragma unroll
           for (int q = 0; q < ND; q++) *reinterpret_cast<uint32_t *> (o + q * A_PLANE) = d[q];
@@ -192,7 +198,7 @@ struct BuildB {
           {
             const int *f = v[2 * h + (u >> 1)];
             const int y = f[u & 1];
-            digits (biased (__mulhi (y, f[2])), biased (__mulhi (y, f[3])), w[u]);
+            digits (biased<A_BITS> (__mulhi (y, f[2])), biased<A_BITS> (__mulhi (y, f[3])), w[u]);
           }
 #pragma unroll
         for (int q = 0; q < ND; q++)
@@ -549,7 +555,7 @@ mk_prep_tc (MixPrep a)
             {
               const int jl = 8 * j8 + 2 * u + h;
               const int xs = __float2int_rn (s_x[q][jl] * inv * 0x1p30f);
-              v[h] = biased (__mulhi (s_f[rr][part][jl], xs));
+              v[h] = biased<B_BITS> (__mulhi (s_f[rr][part][jl], xs));
             }
           digits (v[0], v[1], d[u]);
         }
@@ -642,7 +648,7 @@ put_rows (const MixPlan &p, const KopLane &l, int first, float (&g)[C], uint32_t
         {
           float inv;
           unit_of (s_mx[q][l.sine], inv);
-          const int w = __float2int_rn (g[q] * inv * 0x1p24f) + 0x02008080;
+          const int w = __float2int_rn (g[q] * inv * 0x1p25f) + 0x02008080;     // B_BITS
           uint32_t d[ND];
           digits (w, w, d);
 #pragma unroll
