@@ -1066,7 +1066,12 @@ default_eta_images (int np)
 //   F    N = 64 24.6 / 38.6, 250 28.8 / 42.5, 400 37.0 / 42.4, 700 68 / 43
 //   FT   N = 64 22.7 / 40.4, 333 37.0 / 42.5, 500 45.2 / 44.6
 //   FTS  N = 64 24.7 / 41.5, 250 37.0 / 49.7, 400 52.6 / 50.8
-//   unequal radii: F 400 39 / 49, FT 333 43 / 51, FTS 250 45 / 67
+// Unequal radii: their pair terms carry more rounding, so F and FT take a higher
+// eta, at which the error against FP64 is that of the sums before (F N = 100, phi
+// 0.25, 1.59e-7 at eta 4, 1.43 at 6 and before; F 300, 0.05, 1.51, 1.24, 1.24; FT
+// 300, 0.05, 1.32 at 4, 1.10 at 4.5, 1.16 before), and turn earlier: F N = 150
+// 24.7 / 29 us in a row, 300 35 / 32; FT 150 27 / 36, 300 36 / 37, 400 45 / 41; FTS
+// (eta 4) 250 39 / 49.
 // Under the rmin clamp its kernel (mk_clamp) follows the real space, so F turns
 // earlier: a BD step of 33 products N = 250 1412 / 1493 us, 350 1718 / 1476; FT
 // 330 1545 / 1640, 400 1705 / 1700.
@@ -1077,8 +1082,16 @@ small_system (const struct stokes *sys)
 {
   const double lmin = fmin (sys->lx, fmin (sys->ly, sys->lz));
   const double lmax = fmax (sys->lx, fmax (sys->ly, sys->lz));
-  const int most = sys->version == 0 ? (sys->rmin > 0.0 ? 256 : 512) : (sys->version == 1 ? 400 : 256);
+  const bool early = sys->rmin > 0.0 || sys->a;
+  const int most = sys->version == 0 ? (early ? 256 : 512)
+                                     : (sys->version == 1 ? (sys->a ? 300 : 400) : 256);
   return sys->np <= most && lmax <= 2.0 * lmin;
+}
+
+static double
+small_eta (const struct stokes *sys)
+{
+  return !sys->a || sys->version == 2 ? 4.0 : (sys->version == 0 ? 6.0 : 4.5);
 }
 
 static bool
@@ -1106,7 +1119,7 @@ mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
   const bool small = small_system (sys) && !use_gemms (sys);
   bool images = env_double ("LIBSTOKES_GB300_MIXED_IMAGES", small ? 1.0 : 0.0) != 0.0;
   double eta = env_double ("LIBSTOKES_GB300_MIXED_ETA",
-                           small ? 4.0
+                           small ? small_eta (sys)
                                  : (images ? default_eta_images (sys->np)
                                            : default_eta (sys->version, sys->np)));
   uint64_t fp = mix_fingerprint (sys, eta + (images ? 1000.0 : 0.0), eps);

@@ -33,6 +33,7 @@ def _mean_error(version, n, phi):
 
 @pytest.mark.parametrize("version,n,phi,before", [
     (0, 600, 0.05, 1.529e-7), (0, 600, 0.25, 1.959e-7), (1, 600, 0.05, 1.429e-7),
+    (0, 100, 0.25, 1.428e-7), (0, 300, 0.05, 1.239e-7), (1, 300, 0.05, 1.155e-7),
     (1, 600, 0.25, 2.023e-7), (2, 300, 0.05, 1.164e-7), (2, 300, 0.25, 1.930e-7)])
 def test_error_of_unequal_spheres(lib, version, n, phi, before):
     assert _mean_error(version, n, phi) <= 1.05 * before
