@@ -1107,9 +1107,9 @@ use_gemms (const struct stokes *sys)
 static int
 mixed_setup (Ctx *c, const struct stokes *sys, MixedState *m)
 {
-  // truncation of the sums: 3e-8 (measured at FTS N = 1000: the error
-  // against FP64 is 2.92e-7 at 1e-8, 2.99e-7 at 3e-8, 3.03e-7 at 1e-7 --
-  // FP32 rounding, not truncation, sets it -- and the cutoffs shrink)
+  // truncation of the sums: 3e-8 (error against FP64 at 1e-8, 3e-8 and 1e-7:
+  // FTS N = 1000 2.05, 2.16, 2.08e-7, FTS N = 100 at phi 0.05 9.9, 10.0, 9.9e-8
+  // -- FP32 rounding, not truncation, sets it -- and the cutoffs shrink)
   const double eps = env_double ("LIBSTOKES_GB300_MIXED_EPS", 3e-8);
   // minimum image unless asked otherwise: beside the GEMMs, a lower eta with
   // lattice images is faster at no measured size (products in a row, us: FTS N =
